@@ -75,6 +75,7 @@ struct BwdParams {
   float* dq_acc;       // [T, H*D] fp32, zeroed by the launcher
   __nv_bfloat16* dqkv; // [T, (H+2Hkv)*D]
   int B, L, H, Hkv;
+  int window;          // > 0: the query at position i saw the keys j with i - window < j <= i; 0: all j <= i
   float scale;
 };
 
@@ -108,7 +109,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const int hkv = blockIdx.x % p.Hkv, b = blockIdx.x / p.Hkv;
   const int g = p.H / p.Hkv;
   const int kv0 = jb * BN;
-  const int nqb = (p.L + BM - 1) / BM;
+  // query blocks that see this key block: from the diagonal to the end, or to the last query whose window reaches back
+  const int q_end = p.window > 0 ? min(p.L, kv0 + BN - 1 + p.window) : p.L;
+  const int nqb = (q_end + BM - 1) / BM;
   const int i_start = kv0 / BM;
   const int nqi = nqb - i_start;
   const int n_it = g * nqi;
@@ -356,8 +359,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // a row past the end of the sequence gets lse = +inf: exp2(s - inf) = 0, so P and dS vanish without a mask
       const float lse2 = row_ok ? p.lse[(long long)hq * T + t] * 1.4426950408889634f : INFINITY;
       const float dlts = row_ok ? p.delta[(long long)hq * T + t] * p.scale : 0.f;
-      const bool diag = (kv0 + BN - 1) > q0;
-      const int lim = diag ? (qi - kv0) : 0x7fffffff;  // tile columns <= lim are visible to this row
+      // tile columns lo .. lim are visible to this row; `masked`: not all of them to every row of the block
+      const bool masked = (kv0 + BN - 1) > q0 || (p.window > 0 && q0 + BM - p.window > kv0);
+      const int lim = qi - kv0;
+      const int lo = p.window > 0 ? qi - p.window + 1 - kv0 : 0;
       int w = mbar_wait_bounded(sdp_full, it & 1u, abort_flag, err_word, ERR_WAIT_TMEM_FULL) ? 1 : 0;
       if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
       tc_fence_after_sync();
@@ -370,7 +375,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         tmem_ld_32x32b_x16(tmem_base + lane_addr + C::DP_COL + col0, dv);
         tmem_ld_wait();
         uint32_t pkP[8], pkS[8];
-        if (!diag) {
+        if (!masked) {
 #pragma unroll
           for (int e = 0; e < 16; e += 2) {
             const float p0 = fast_exp2(fmaf(__uint_as_float(sv[e]), c2, -lse2));
@@ -385,8 +390,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           for (int e = 0; e < 16; e += 2) {
             float p0 = fast_exp2(fmaf(__uint_as_float(sv[e]), c2, -lse2));
             float p1 = fast_exp2(fmaf(__uint_as_float(sv[e + 1]), c2, -lse2));
-            if ((col0 + e) > lim) p0 = 0.f;
-            if ((col0 + e + 1) > lim) p1 = 0.f;
+            if ((col0 + e) > lim || (col0 + e) < lo) p0 = 0.f;
+            if ((col0 + e + 1) > lim || (col0 + e + 1) < lo) p1 = 0.f;
             const float d0 = p0 * fmaf(__uint_as_float(dv[e]), p.scale, -dlts);
             const float d1 = p1 * fmaf(__uint_as_float(dv[e + 1]), p.scale, -dlts);
             pkP[e >> 1] = pack_bf16x2(p0, p1);
@@ -572,8 +577,8 @@ __global__ void dq_convert_rope_kernel(const float* __restrict__ acc, __nv_bfloa
 
 template <int D>
 static int launch_bwd(const void* dout, const void* qkv, const void* out, const float* lse, float* delta, void* dqkv,
-                      float* dq_acc, int B, int L, int H, int Hkv, const int* pos, const float* cos_tab,
-                      const float* sin_tab, cudaStream_t st) {
+                      float* dq_acc, int B, int L, int window, int H, int Hkv, const int* pos,
+                      const float* cos_tab, const float* sin_tab, cudaStream_t st) {
   using C = Cfg<D>;
   const long long width = (long long)(H + 2 * Hkv) * D;
   const long long T = (long long)B * L;
@@ -602,7 +607,7 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
     B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     attr = true;
   }
-  BwdParams p{lse, delta, dq_acc, (__nv_bfloat16*)dqkv, B, L, H, Hkv, 1.0f / sqrtf((float)D)};
+  BwdParams p{lse, delta, dq_acc, (__nv_bfloat16*)dqkv, B, L, H, Hkv, window, 1.0f / sqrtf((float)D)};
   dim3 grid(Hkv * B, (L + BN - 1) / BN);
   kern<<<grid, NTHREADS, C::SMEM_BYTES, st>>>(tmQKV, tmDO, tmDQ, p, device_err_word());
   B200_CUDA_CHECK(cudaGetLastError());
@@ -627,14 +632,15 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
 
 // dq_acc: fp32 scratch [T, H*D] (zeroed here); delta: fp32 scratch [H, T]. dqkv receives dQ | dK | dV.
 extern "C" int b200_flash_attn_bwd(const void* dout, const void* qkv, const void* out, const float* lse, float* delta,
-                                   void* dqkv, float* dq_acc, int B, int L, int H, int Hkv, int D, cudaStream_t st) {
+                                   void* dqkv, float* dq_acc, int B, int L, int window, int H, int Hkv, int D,
+                                   cudaStream_t st) {
   using namespace b200;
-  if (!dout || !qkv || !out || !lse || !delta || !dqkv || !dq_acc || B <= 0 || L <= 0 || H <= 0 || Hkv <= 0 ||
-      (H % Hkv) != 0)
+  if (!dout || !qkv || !out || !lse || !delta || !dqkv || !dq_acc || B <= 0 || L <= 0 || window < 0 || H <= 0 ||
+      Hkv <= 0 || (H % Hkv) != 0)
     return B200_ERR_ARG;
-  if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, H, Hkv, nullptr, nullptr, nullptr, st);
+  if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, nullptr, nullptr, nullptr, st);
   if (D == 128)
-    return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, H, Hkv, nullptr, nullptr, nullptr, st);
+    return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, nullptr, nullptr, nullptr, st);
   return B200_ERR_ARG;
 }
 
@@ -643,14 +649,15 @@ extern "C" int b200_flash_attn_bwd(const void* dout, const void* qkv, const void
 // and is rotated by the caller.
 extern "C" int b200_flash_attn_bwd_rope(const void* dout, const void* qkv, const void* out, const float* lse,
                                         float* delta, void* dqkv, float* dq_acc, const int* pos, const float* cos_tab,
-                                        const float* sin_tab, int B, int L, int H, int Hkv, int D, cudaStream_t st) {
+                                        const float* sin_tab, int B, int L, int window, int H, int Hkv, int D,
+                                        cudaStream_t st) {
   using namespace b200;
   if (!dout || !qkv || !out || !lse || !delta || !dqkv || !dq_acc || !pos || !cos_tab || !sin_tab || B <= 0 || L <= 0 ||
-      H <= 0 || Hkv <= 0 || (H % Hkv) != 0)
+      window < 0 || H <= 0 || Hkv <= 0 || (H % Hkv) != 0)
     return B200_ERR_ARG;
-  if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, H, Hkv, pos, cos_tab, sin_tab, st);
+  if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, pos, cos_tab, sin_tab, st);
   if (D == 128)
-    return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, H, Hkv, pos, cos_tab, sin_tab, st);
+    return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, pos, cos_tab, sin_tab, st);
   return B200_ERR_ARG;
 }
 

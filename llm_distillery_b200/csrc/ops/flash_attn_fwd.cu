@@ -15,6 +15,9 @@
 //                            moves the maximum, rescales O in TMEM and redoes the tile; final O / l and lse.
 // The score buffers alternate: S_{j+1} is computed while the softmax warps work on S_j, and S_{j+2} goes into S_j's
 // buffer as soon as P_j V_j has completed, so in the steady state the softmax warps never wait for the tensor core.
+// Sliding window: a block starts at the tile its first query's window reaches and masks the lower edge the way it masks
+// the diagonal; whole tiles in between take the unmasked path (7 B layer, 32 heads of 128, window 4096, 6001 positions:
+// about 0.5 ms; under a dense band mask in library attention 8.7 ms).
 // P never touches shared memory: an N = D MMA fed from shared memory on both sides is bound by shared-memory
 // bandwidth, and the softmax warps issue no st.shared and no proxy fence.
 // TMEM: 2 x 64 score columns + D output columns (<= 256); shared memory 56 KB (D = 64) / 112 KB (D = 128): two CTAs
@@ -67,6 +70,7 @@ struct FwdParams {
   // sit in a cache (row p of the K / V tensors = position p). q_off = 0 and K / V inside the same packed tensor as Q
   // is the ordinary whole-sequence call.
   int q_off;
+  int window;               // > 0: the query at position i sees the keys j with i - window < j <= i; 0: all j <= i
   int colQ0, colK0, colV0;  // first column of head 0 of Q / K / V in their tensors
 };
 
@@ -117,7 +121,9 @@ __global__ void __launch_bounds__(NTHREADS, 2)
   const int q0 = qb * BM;
   const int qpos0 = p.q_off + q0;                       // sequence position of the block's first query
   const int kv_end = p.q_off + min(p.L, q0 + BM);       // causal: keys < kv_end
-  const int n_kv = (kv_end + BN - 1) / BN;
+  // sliding window: the block's first query looks back furthest; tiles before that one are not walked
+  const int tile0 = p.window > 0 ? max(0, qpos0 - p.window + 1) / BN : 0;
+  const int n_kv = (kv_end + BN - 1) / BN - tile0;      // tiles tile0 .. tile0 + n_kv - 1, counted from 0 below
 
   if ((smem_u32(smem) & 1023u) != 0u) {  // swizzled tiles need a 1024-byte aligned base
     if (threadIdx.x == 0 && err_word) atomicCAS(err_word, 0u, (unsigned)ERR_BAD_ARG);
@@ -168,7 +174,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
         uint8_t* sK = smem + C::OFF_K + ks * C::T_BYTES;
         mbar_arrive_expect_tx(&k_full[ks], C::T_BYTES);
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) tma_load_3d(sK + c * (BN * 128), &tmK, &k_full[ks], colK + c * 64, j * BN, b);
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sK + c * (BN * 128), &tmK, &k_full[ks], colK + c * 64, (tile0 + j) * BN, b);
       }
     } else if (lane == 1) {
       for (int j = 0; j < n_kv; ++j) {
@@ -180,7 +186,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
         uint8_t* sV = smem + C::OFF_V + vs * C::T_BYTES;
         mbar_arrive_expect_tx(&v_full[vs], C::T_BYTES);
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) tma_load_3d(sV + c * (BN * 128), &tmV, &v_full[vs], colV + c * 64, j * BN, b);
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sV + c * (BN * 128), &tmV, &v_full[vs], colV + c * 64, (tile0 + j) * BN, b);
       }
     }
   } else if (warp == 1) {
@@ -255,11 +261,11 @@ __global__ void __launch_bounds__(NTHREADS, 2)
     bool ok = true;
 
     // One 32-column chunk of scores -> probabilities (bf16 pairs) with the running maximum and the row sum.
-    // `lim`: columns of this chunk with index <= lim are visible (>= 31: all of them). POLY8 of every 8 pairs of
+    // Columns lo .. lim of this chunk are visible (lo <= 0 and lim >= 31: all of them). POLY8 of every 8 pairs of
     // exponentials are evaluated on the FMA pipe.
-    auto chunk = [&](const uint32_t (&v)[32], const uint64_t nmb, const int lim, float& mx, uint64_t& sum2,
+    auto chunk = [&](const uint32_t (&v)[32], const uint64_t nmb, const int lo, const int lim, float& mx, uint64_t& sum2,
                      uint32_t (&pk)[16]) {
-      if (lim >= 31) {
+      if (lim >= 31 && lo <= 0) {
 #pragma unroll
         for (int t = 0; t < 32; t += 2) {
           const float s0 = __uint_as_float(v[t]), s1 = __uint_as_float(v[t + 1]);
@@ -275,8 +281,8 @@ __global__ void __launch_bounds__(NTHREADS, 2)
       } else {
 #pragma unroll
         for (int t = 0; t < 32; t += 2) {
-          const float s0 = t <= lim ? __uint_as_float(v[t]) : -INFINITY;
-          const float s1 = (t + 1) <= lim ? __uint_as_float(v[t + 1]) : -INFINITY;
+          const float s0 = (t <= lim && t >= lo) ? __uint_as_float(v[t]) : -INFINITY;
+          const float s1 = ((t + 1) <= lim && (t + 1) >= lo) ? __uint_as_float(v[t + 1]) : -INFINITY;
           mx = fmax3(mx, s0, s1);
           float x0, x1;
           unpack_f32x2(fma_f32x2(pack_f32x2(s0, s1), c2p, nmb), x0, x1);
@@ -293,32 +299,35 @@ __global__ void __launch_bounds__(NTHREADS, 2)
       int w = mbar_wait_bounded(&s_full[bsel], (j / NBUF) & 1u, abort_flag, err_word, ERR_WAIT_TMEM_FULL) ? 1 : 0;
       if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
       tc_fence_after_sync();
-      const int kv0 = j * BN;
+      const int kv0 = (tile0 + j) * BN;
       const bool diag = (kv0 + BN - 1) > qpos0;              // some keys of this tile are masked for some rows
-      const int lim = diag ? (qpos - kv0) : 0x3fffffff;      // tile columns <= lim are visible to this row
+      const int lim = diag ? (qpos - kv0) : 0x3fffffff;      // tile columns lo .. lim are visible to this row
+      const int lo = p.window > 0 ? qpos - p.window + 1 - kv0 : 0;
       uint32_t va[32], vb[32], pka[16], pkb[16];
       tmem_ld_32x32b_x32(tS, va);
       tmem_ld_32x32b_x32(tS + 32, vb);
       tmem_ld_wait();
       if (j == 0) {
-        // The first tile fixes the reference maximum (every row sees key 0, so it is finite). Later tiles are
-        // exponentiated against the maximum known so far and only redone when a score exceeds it by more than
-        // 2^kRescaleThreshold, which is rare once a row has seen a few hundred keys.
+        // The first tile fixes the reference maximum. Later tiles are exponentiated against the maximum known so far
+        // and only redone when a score exceeds it by more than 2^kRescaleThreshold, which is rare once a row has seen
+        // a few hundred keys. Without a window every row sees key 0; with one the later rows of the block may see
+        // nothing of the first tile: they start from a finite bound below any score, so that their first visible
+        // tile moves the maximum and nothing is ever inf - inf.
         float mx0 = -INFINITY;
 #pragma unroll
         for (int t = 0; t < 32; t += 2) {
-          mx0 = fmax3(mx0, t <= lim ? __uint_as_float(va[t]) : -INFINITY,
-                      (t + 1) <= lim ? __uint_as_float(va[t + 1]) : -INFINITY);
-          mx0 = fmax3(mx0, (t + 32) <= lim ? __uint_as_float(vb[t]) : -INFINITY,
-                      (t + 33) <= lim ? __uint_as_float(vb[t + 1]) : -INFINITY);
+          mx0 = fmax3(mx0, (t <= lim && t >= lo) ? __uint_as_float(va[t]) : -INFINITY,
+                      ((t + 1) <= lim && (t + 1) >= lo) ? __uint_as_float(va[t + 1]) : -INFINITY);
+          mx0 = fmax3(mx0, ((t + 32) <= lim && (t + 32) >= lo) ? __uint_as_float(vb[t]) : -INFINITY,
+                      ((t + 33) <= lim && (t + 33) >= lo) ? __uint_as_float(vb[t + 1]) : -INFINITY);
         }
-        m_used = mx0;
+        m_used = fmaxf(mx0, -1e30f);
       }
       float mx = m_used;
       uint64_t sum2 = 0ull;
       uint64_t nmb = pack_f32x2(-m_used * c2, -m_used * c2);
-      chunk(va, nmb, lim, mx, sum2, pka);
-      chunk(vb, nmb, lim - 32, mx, sum2, pkb);
+      chunk(va, nmb, lo, lim, mx, sum2, pka);
+      chunk(vb, nmb, lo - 32, lim - 32, mx, sum2, pkb);
       const bool need = (mx - m_used) * c2 > kRescaleThreshold;
       if (__any_sync(0xffffffffu, need)) {
         // a score outgrew the reference maximum: move the maximum, rescale what is accumulated, redo the tile
@@ -352,10 +361,10 @@ __global__ void __launch_bounds__(NTHREADS, 2)
         // S_j is still intact in TMEM (P_j is stored below): read it again rather than keep it in registers
         tmem_ld_32x32b_x32(tS, va);
         tmem_ld_wait();
-        chunk(va, nmb, lim, mx2, sum2, pka);
+        chunk(va, nmb, lo, lim, mx2, sum2, pka);
         tmem_ld_32x32b_x32(tS + 32, va);
         tmem_ld_wait();
-        chunk(va, nmb, lim - 32, mx2, sum2, pkb);
+        chunk(va, nmb, lo - 32, lim - 32, mx2, sum2, pkb);
       }
       // P_j over the first half of S_j (both halves of S_j are in registers by now)
       tmem_st_32x32b_x16(tS, pka);
@@ -416,8 +425,8 @@ __global__ void __launch_bounds__(NTHREADS, 2)
 
 template <int D>
 static int launch_fwd(const void* q, long long q_width, int colQ0, const void* k, const void* v, long long kv_width,
-                      int colK0, int colV0, long long kv_rows, void* out, float* lse, int B, int L, int q_off, int H,
-                      int Hkv, cudaStream_t st) {
+                      int colK0, int colV0, long long kv_rows, void* out, float* lse, int B, int L, int q_off, int window,
+                      int H, int Hkv, cudaStream_t st) {
   using C = Cfg<D>;
   CUtensorMap tmQ, tmK, tmV;
   int rc = make_tmap_3d(&tmQ, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)q_width, (uint64_t)L, (uint64_t)B,
@@ -444,7 +453,7 @@ static int launch_fwd(const void* q, long long q_width, int colQ0, const void* k
     B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     attr = true;
   }
-  FwdParams p{(__nv_bfloat16*)out, lse, B, L, H, Hkv, 1.0f / sqrtf((float)D), q_off, colQ0, colK0, colV0};
+  FwdParams p{(__nv_bfloat16*)out, lse, B, L, H, Hkv, 1.0f / sqrtf((float)D), q_off, window, colQ0, colK0, colV0};
   dim3 grid(H * B, (L + BM - 1) / BM);
   kern<<<grid, NTHREADS, C::SMEM_BYTES, st>>>(tmQ, tmK, tmV, p, device_err_word());
   B200_CUDA_CHECK(cudaGetLastError());
@@ -454,15 +463,16 @@ static int launch_fwd(const void* q, long long q_width, int colQ0, const void* k
 }  // namespace fa
 }  // namespace b200
 
-extern "C" int b200_flash_attn_fwd(const void* qkv, void* out, float* lse, int B, int L, int H, int Hkv, int D,
+// window > 0: sliding-window attention (the last `window` positions, the own one included); 0: plain causal.
+extern "C" int b200_flash_attn_fwd(const void* qkv, void* out, float* lse, int B, int L, int window, int H, int Hkv, int D,
                                    cudaStream_t st) {
   using namespace b200;
-  if (!qkv || !out || B <= 0 || L <= 0 || H <= 0 || Hkv <= 0 || (H % Hkv) != 0) return B200_ERR_ARG;
+  if (!qkv || !out || B <= 0 || L <= 0 || window < 0 || H <= 0 || Hkv <= 0 || (H % Hkv) != 0) return B200_ERR_ARG;
   const long long width = (long long)(H + 2 * Hkv) * D;
   if (D == 64)
-    return fa::launch_fwd<64>(qkv, width, 0, qkv, qkv, width, H * D, (H + Hkv) * D, L, out, lse, B, L, 0, H, Hkv, st);
+    return fa::launch_fwd<64>(qkv, width, 0, qkv, qkv, width, H * D, (H + Hkv) * D, L, out, lse, B, L, 0, window, H, Hkv, st);
   if (D == 128)
-    return fa::launch_fwd<128>(qkv, width, 0, qkv, qkv, width, H * D, (H + Hkv) * D, L, out, lse, B, L, 0, H, Hkv, st);
+    return fa::launch_fwd<128>(qkv, width, 0, qkv, qkv, width, H * D, (H + Hkv) * D, L, out, lse, B, L, 0, window, H, Hkv, st);
   return B200_ERR_ARG;
 }
 
@@ -471,16 +481,16 @@ extern "C" int b200_flash_attn_fwd(const void* qkv, void* out, float* lse, int B
 // row p = sequence position p, valid (and finite: allocate the caches zeroed) for p < q_off + L. The chunk's queries
 // are positions q_off .. q_off + L - 1 and see keys <= their own position. out [B*L, H*D], lse [H, B*L] (may be null).
 extern "C" int b200_flash_attn_fwd_cached(const void* qkv, const void* k_cache, const void* v_cache, long long cache_rows,
-                                          void* out, float* lse, int B, int L, int q_off, int H, int Hkv, int D,
-                                          cudaStream_t st) {
+                                          void* out, float* lse, int B, int L, int q_off, int window, int H, int Hkv,
+                                          int D, cudaStream_t st) {
   using namespace b200;
-  if (!qkv || !k_cache || !v_cache || !out || B <= 0 || L <= 0 || q_off < 0 || H <= 0 || Hkv <= 0 || (H % Hkv) != 0 ||
+  if (!qkv || !k_cache || !v_cache || !out || B <= 0 || L <= 0 || q_off < 0 || window < 0 || H <= 0 || Hkv <= 0 || (H % Hkv) != 0 ||
       cache_rows < (long long)q_off + L)
     return B200_ERR_ARG;
   const long long width = (long long)(H + 2 * Hkv) * D, kvw = (long long)Hkv * D;
   if (D == 64)
-    return fa::launch_fwd<64>(qkv, width, 0, k_cache, v_cache, kvw, 0, 0, cache_rows, out, lse, B, L, q_off, H, Hkv, st);
+    return fa::launch_fwd<64>(qkv, width, 0, k_cache, v_cache, kvw, 0, 0, cache_rows, out, lse, B, L, q_off, window, H, Hkv, st);
   if (D == 128)
-    return fa::launch_fwd<128>(qkv, width, 0, k_cache, v_cache, kvw, 0, 0, cache_rows, out, lse, B, L, q_off, H, Hkv, st);
+    return fa::launch_fwd<128>(qkv, width, 0, k_cache, v_cache, kvw, 0, 0, cache_rows, out, lse, B, L, q_off, window, H, Hkv, st);
   return B200_ERR_ARG;
 }

@@ -8,10 +8,11 @@ CUDA tensors run the sm_100a flash-attention kernels (csrc/ops/flash_attn.cu); C
 restatement below, which is also the oracle of the GPU tests.
 
 Sliding-window layers (Mistral v0.1, Phi-3, the windowed layers of hybrid models): a query at position i sees the
-keys j with i - window < j <= i. Up to ``window`` positions that IS causal attention and the paths above run. Longer
-sequences take ``windowed_fwd`` / ``windowed_bwd`` below: PyTorch's scaled-dot-product attention under a band mask, on
-either device - the flash kernels have no window, so this case is exact but runs at the library's speed. The same
-path, without a window, serves heads of other sizes than 64 and 128 on a GPU (Gemma's 256).
+keys j with i - window < j <= i. Up to ``window`` positions that IS causal attention. On longer sequences the flash
+kernels walk only the key tiles the window reaches and mask its edge: a layer of 32 heads of 128 at window 4096 and
+6001 positions takes about 0.5 ms against 8.7 ms for PyTorch's attention under a band mask, which visits every tile and
+wants the key / value heads repeated. ``windowed_fwd`` / ``windowed_bwd`` below are that masked path: they serve CPU
+tensors and, with or without a window, heads of other sizes than 64 and 128 on a GPU (Gemma's 256).
 """
 from __future__ import annotations
 
@@ -112,24 +113,24 @@ def attention_fwd(qkv: torch.Tensor, B: int, L: int, H: int, Hkv: int, d: int, w
     """Returns (out [T, H*d], lse [H, T] fp32). ``window``: the layer's sliding window, or None."""
     if window is not None and L <= window:
         window = None
-    if window is not None or _library_path(qkv, d):
+    if _library_path(qkv, d) or (window is not None and not qkv.is_cuda):
         return windowed_fwd(qkv, B, L, H, Hkv, d, window)
     if not qkv.is_cuda:
         return attention_reference_fwd(qkv, B, L, H, Hkv, d)
     from . import flash
-    return flash.flash_attn_fwd(qkv, B, L, H, Hkv, d)
+    return flash.flash_attn_fwd(qkv, B, L, H, Hkv, d, window)
 
 
 def attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window: int | None = None):
     """Returns dqkv with the layout of qkv."""
     if window is not None and L <= window:
         window = None
-    if window is not None or _library_path(qkv, d):
+    if _library_path(qkv, d) or (window is not None and not qkv.is_cuda):
         return windowed_bwd(dout, qkv, B, L, H, Hkv, d, window)
     if not qkv.is_cuda:
         return attention_reference_bwd(dout, qkv, out, lse, B, L, H, Hkv, d)
     from . import flash
-    return flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d)
+    return flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window=window)
 
 
 def attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin, window: int | None = None):
@@ -139,15 +140,15 @@ def attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin,
     from . import basic
     if window is not None and L <= window:
         window = None
-    if window is not None or _library_path(qkv, d):
+    if _library_path(qkv, d) or (window is not None and not qkv.is_cuda):
         return basic.rope_(windowed_bwd(dout, qkv, B, L, H, Hkv, d, window), pos, cos, sin, H + Hkv, d, inverse=True)
     if (qkv.is_cuda and qkv.dtype == torch.bfloat16 and pos.dtype == torch.int32 and cos.is_contiguous()
             and sin.is_contiguous() and 2 * cos.shape[1] == d):      # partial rotary: the separate kernel below
         from . import flash
-        dqkv = flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, rope=(pos, cos, sin))
+        dqkv = flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, rope=(pos, cos, sin), window=window)
         basic.rope_(dqkv[:, H * d:], pos, cos, sin, Hkv, d, inverse=True)      # the key heads
         return dqkv
-    dqkv = attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d)
+    dqkv = attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
     return basic.rope_(dqkv, pos, cos, sin, H + Hkv, d, inverse=True)
 
 
@@ -172,7 +173,7 @@ def attention_fwd_cached(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     values at rows q_off .. q_off+L-1). Inference only: no log-sum-exp is kept."""
     if window is not None and q_off + L <= window:
         window = None
-    if window is not None or _library_path(qkv, d):
+    if _library_path(qkv, d) or (window is not None and not qkv.is_cuda):
         n = q_off + L
         q = qkv[:, : H * d].reshape(B, L, H, d)
         k = k_cache[:, :n].reshape(B, n, Hkv, d)
@@ -181,4 +182,4 @@ def attention_fwd_cached(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     if not qkv.is_cuda:
         return attention_cached_reference_fwd(qkv, k_cache, v_cache, B, L, q_off, H, Hkv, d)
     from . import flash
-    return flash.flash_attn_fwd_cached(qkv, k_cache, v_cache, B, L, q_off, H, Hkv, d)
+    return flash.flash_attn_fwd_cached(qkv, k_cache, v_cache, B, L, q_off, H, Hkv, d, window)

@@ -99,3 +99,29 @@ def test_sequences_longer_than_a_sliding_window(B, L, H, Hkv, d, window):
     a, _ = attention.attention_fwd(qkv, B, L, H, Hkv, d, L)
     b, _ = attention.attention_fwd(qkv, B, L, H, Hkv, d)
     assert torch.equal(a, b) and _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("L,H,Hkv,d,window", [(65, 2, 1, 64, 1), (129, 2, 2, 128, 64), (500, 4, 1, 64, 63), (641, 2, 1, 128, 129),
+                                              (777, 2, 2, 64, 776), (1100, 4, 2, 128, 500)])
+def test_window_edges_against_the_band_mask(L, H, Hkv, d, window):
+    """Windows of one key, at and around the tile sizes, one short of the sequence: the flash kernels (whole sequence,
+    chunk behind a cache, backward) against the masked path in fp32. Bound: probabilities and outputs are rounded to
+    bf16 (2^-9 each), gradients are sums of up to ``window`` such terms - 2e-2 of the largest value."""
+    B = 2
+    torch.manual_seed(7 * L + window)
+    qkv = torch.randn(B * L, (H + 2 * Hkv) * d, device=DEV).bfloat16()
+    dout = torch.randn(B * L, H * d, device=DEV).bfloat16()
+    out, lse = attention.attention_fwd(qkv, B, L, H, Hkv, d, window)
+    dqkv = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
+    ro, _ = attention.windowed_fwd(qkv.float(), B, L, H, Hkv, d, window)
+    rd = attention.windowed_bwd(dout.float(), qkv.float(), B, L, H, Hkv, d, window)
+    for got, want in ((out, ro), (dqkv, rd)):
+        assert (got.float() - want).abs().max() <= 2e-2 * want.abs().max()
+    kv, n = Hkv * d, L // 3
+    c0 = L - n
+    kc, vc = (qkv[:, (H + i * Hkv) * d:(H + i * Hkv) * d + kv].reshape(B, L, kv).contiguous() for i in (0, 1))
+    rows = qkv.view(B, L, -1)[:, c0:].reshape(B * n, -1).contiguous()
+    got = attention.attention_fwd_cached(rows, kc, vc, B, n, c0, H, Hkv, d, window)
+    want = ro.view(B, L, -1)[:, c0:].reshape(B * n, -1)
+    assert (got.float() - want).abs().max() <= 2e-2 * want.abs().max()
+    assert _lib.take_device_error() == 0
