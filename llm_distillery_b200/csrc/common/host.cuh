@@ -42,6 +42,26 @@ int make_tmap_3d(CUtensorMap* out, const void* base, CUtensorMapDataType dtype, 
                  uint64_t d1, uint64_t d2, uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0, uint32_t b1,
                  uint32_t b2, CUtensorMapSwizzle swizzle);
 
+// Launch that may overlap the tail of the kernel before it on the stream (see pdl_wait / pdl_trigger in ptx.cuh: the
+// kernel must call them). Errors surface through cudaGetLastError like those of <<<>>>. About 1 us per launch in a chain
+// of short kernels (a 777-token training step, 1000 launches: 18.8 -> 17.7 ms). Not for kernels of less than one wave of
+// long CTAs: placed while the grid before them still runs, those pack onto few SMs (top-K over 128 rows of 128 256
+// logits: a collection batch with 64 such launches went from 144 to 152 ms), so loss/topk_logprob.cu launches plainly.
+template <class... P, class... A>
+static inline void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 static inline long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }
 

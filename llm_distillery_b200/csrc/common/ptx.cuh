@@ -149,6 +149,16 @@ __device__ __forceinline__ bool wait_equal_bounded(const unsigned int* addr, uns
   }
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// Kernels launched with launch_pdl (host.cuh) may start while the kernel before them on the stream drains: their set-up
+// (barriers, TMEM, descriptors) then costs nothing. pdl_wait returns when every earlier kernel has completed and its
+// writes are visible; a kernel calls it before its first access to global memory that another kernel may write or
+// read. pdl_trigger lets the next kernel's CTAs be scheduled where this grid leaves room. It comes AFTER the CTA's
+// TMEM allocation: the next kernel starts once every CTA of this grid has triggered, and could otherwise take the
+// columns a CTA of this one still needs.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -444,7 +444,7 @@ static int launch_rope_pair(const void* A, const void* W, int M, int N, int K, l
   const int tiles = ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  kern<<<2 * pairs, NUM_THREADS, smem_bytes, stream>>>(tmA, tmB, M, N, K, 1, rp, device_err_word(), 1, nullptr, 0);
+  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, rp, device_err_word(), 1, nullptr, 0);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -572,7 +572,7 @@ static int launch_swiglu_bwd_pair(const void* dY, const void* Wd, int M, int f, 
   const int tiles = ceil_div(M, PAIR_BM) * ceil_div(f, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  kern<<<2 * pairs, NUM_THREADS, smem_bytes, stream>>>(tmA, tmB, M, f, K, 1, sp, device_err_word(), 1, nullptr, 0);
+  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, f, K, 1, sp, device_err_word(), 1, nullptr, 0);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -600,7 +600,7 @@ static int launch_swiglu_pair(const void* A, const void* Wgu, int M, int f, int 
   const int tiles = ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  kern<<<2 * pairs, NUM_THREADS, smem_bytes, stream>>>(tmA, tmB, M, N, K, 1, sp, device_err_word(), 1, nullptr, f);
+  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, sp, device_err_word(), 1, nullptr, f);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -634,7 +634,7 @@ static int launch_store(const void* A, const void* B, int M, int N, int K, long 
   const int tiles = ceil_div(M, BM) * ceil_div(N, BN);
   const int grid = tiles < sm_count() ? tiles : sm_count();
   DescCfg dc = dc_override ? *dc_override : default_desc_cfg<BN, A_MN, B_MN>();
-  kern<<<grid, NUM_THREADS, smem_bytes, stream>>>(tmA, tmB, M, N, K, fmt, dc, sp, device_err_word());
+  launch_pdl(kern, grid, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, fmt, dc, sp, device_err_word());
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -729,7 +729,7 @@ static int launch_store_pair(const void* A, const void* B, int M, int N, int K, 
   }
   const long long units = (long long)tiles * k_splits;
   const int pairs = units < max_pairs ? (int)units : max_pairs;
-  kern<<<2 * pairs, NUM_THREADS, smem_bytes, stream>>>(tmA, tmB, M, N, K, fmt, sp, device_err_word(), k_splits, sync, 0);
+  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, fmt, sp, device_err_word(), k_splits, sync, 0);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

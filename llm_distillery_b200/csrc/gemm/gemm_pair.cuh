@@ -81,6 +81,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   cluster_sync_all();  // both CTAs' barriers exist before any remote arrive / pair TMA
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   const int m_tiles = (M + PAIR_BM - 1) / PAIR_BM;
   const int n_tiles = (N + PAIR_BN - 1) / PAIR_BN;

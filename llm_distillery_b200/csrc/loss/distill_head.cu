@@ -235,7 +235,7 @@ static int launch_head(const void* Hc, const void* W, int M, int N, int Kdim, lo
     }
     const int tiles = ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
     const int pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
-    kern<<<2 * pairs, NUM_THREADS, smem_bytes, stream>>>(tmA, tmB, M, N, Kdim, 1, ep, device_err_word(), 1, nullptr, 0);
+    launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, Kdim, 1, ep, device_err_word(), 1, nullptr, 0);
     B200_CUDA_CHECK(cudaGetLastError());
     return B200_OK;
   }
@@ -249,7 +249,7 @@ static int launch_head(const void* Hc, const void* W, int M, int N, int Kdim, lo
   }
   const int tiles = ceil_div(M, BM) * ceil_div(N, BN);
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  kern<<<grid, NUM_THREADS, smem_bytes, stream>>>(tmA, tmB, M, N, Kdim, 1, default_desc_cfg<BN, false, false>(), ep,
+  launch_pdl(kern, grid, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, Kdim, 1, default_desc_cfg<BN, false, false>(), ep,
                                                   device_err_word());
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -272,6 +272,8 @@ struct RowParams {
 };
 
 __global__ void __launch_bounds__(128) distill_rows_kernel(RowParams p) {
+  pdl_wait();
+  pdl_trigger();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= p.M) return;
@@ -389,6 +391,8 @@ struct VpPeers { const void* p[16]; };
 __global__ void __launch_bounds__(128) vp_combine_kernel(VpPeers pmax, VpPeers psum, VpPeers zk, int world,
                                                         int n_tiles, int M, int K, float* __restrict__ out_pmax,
                                                         float* __restrict__ out_psum, float* __restrict__ out_zk) {
+  pdl_wait();
+  pdl_trigger();
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= M) return;
@@ -460,7 +464,7 @@ int b200_vp_combine(const void* const* pmax_ptrs, const void* const* psum_ptrs, 
     b.p[i] = psum_ptrs[i];
     c.p[i] = zk_ptrs[i];
   }
-  vp_combine_kernel<<<ceil_div(M, 4), 128, 0, st>>>(a, b, c, world, n_tiles, M, K, out_pmax, out_psum, out_zk);
+  launch_pdl(vp_combine_kernel, ceil_div(M, 4), 128, 0, st, a, b, c, world, n_tiles, M, K, out_pmax, out_psum, out_zk);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -472,7 +476,7 @@ int b200_distill_rows(const float* pmax, const float* psum, const float* zk, con
   if (kind != 4 && (!zk || !u || !ids || !loss || !a || !A || K <= 0)) return B200_ERR_ARG;
   RowParams p{pmax, psum, zk, u, ids, lse, loss, a, A, M, K, n_tiles, vocab, kind, inv_T};
   const int warps_per_block = 4;
-  distill_rows_kernel<<<ceil_div(M, warps_per_block), warps_per_block * 32, 0, st>>>(p);
+  launch_pdl(distill_rows_kernel, ceil_div(M, warps_per_block), warps_per_block * 32, 0, st, p);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

@@ -25,6 +25,8 @@ __device__ __forceinline__ long long lower_bound(const long long* __restrict__ s
 __global__ void __launch_bounds__(256) segment_reduce_kernel(const float* __restrict__ x,
                                                              const long long* __restrict__ seg,
                                                              float* __restrict__ out, long long M, int n_seg, int op) {
+  pdl_wait();
+  pdl_trigger();
   const int warp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (warp >= n_seg) return;
@@ -54,7 +56,7 @@ extern "C" int b200_segment_reduce(const float* x, const long long* seg, float* 
   using namespace b200;
   if (!seg || !out || M < 0 || n_seg <= 0 || op < 0 || op > 2 || (op != 2 && !x)) return B200_ERR_ARG;
   const int blocks = ceil_div(n_seg * 32, 256);
-  seg::segment_reduce_kernel<<<blocks, 256, 0, st>>>(x, seg, out, M, n_seg, op);
+  launch_pdl(seg::segment_reduce_kernel, blocks, 256, 0, st, x, seg, out, M, n_seg, op);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

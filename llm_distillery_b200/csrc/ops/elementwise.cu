@@ -51,6 +51,8 @@ __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __
                                                         const __nv_bfloat16* __restrict__ w,
                                                         __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ hout,
                                                         float* __restrict__ rstd, int rows, int h, float eps) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[NT / 32];
   const int nvec = h >> 3;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -112,6 +114,8 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(const __nv_bfloat
                                                               __nv_bfloat16* __restrict__ y,
                                                               __nv_bfloat16* __restrict__ hout,
                                                               float* __restrict__ rstd, int rows, float eps) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int h = VPL * 256;
   const int lane = threadIdx.x & 31;
   const int nwarps = gridDim.x * 4;
@@ -168,6 +172,8 @@ __global__ void __launch_bounds__(NT) rmsnorm_bwd_kernel(const __nv_bfloat16* __
                                                         const __nv_bfloat16* __restrict__ dres,
                                                         __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial,
                                                         int rows, int h) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[NT / 32];
   const int nvec = h >> 3;
   float dwacc[MAX_VEC][8];
@@ -248,6 +254,8 @@ __global__ void __launch_bounds__(128, 5) rmsnorm_bwd_warp_kernel(const __nv_bfl
                                                               const __nv_bfloat16* __restrict__ dres,
                                                               __nv_bfloat16* __restrict__ dx,
                                                               float* __restrict__ dw_partial, int rows, int nwarps) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int h = VPL * 256;
   extern __shared__ float4 sdw_all[];
   const int lane = threadIdx.x & 31;
@@ -323,6 +331,8 @@ __global__ void __launch_bounds__(128, 5) rmsnorm_bwd_warp_kernel(const __nv_bfl
 // out[j] (+)= sum_b partial[b][j]; block = 32 columns x 8 row groups, reduced through shared memory
 __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                                      int nblk, int h, int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + tx;
@@ -351,6 +361,8 @@ __global__ void __launch_bounds__(256) headnorm_fwd_kernel(const __nv_bfloat16* 
                                                           const __nv_bfloat16* __restrict__ wk,
                                                           float* __restrict__ rstd, long long T, int H, int Hkv,
                                                           long long ld, float eps) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int d = EPL * 32;
   const int lane = threadIdx.x & 31;
   const int nh = H + 2 * Hkv, nn = H + Hkv;
@@ -396,6 +408,8 @@ __global__ void __launch_bounds__(256) headnorm_bwd_kernel(__nv_bfloat16* __rest
                                                           const float* __restrict__ rstd,
                                                           float* __restrict__ partial, long long T, int H, int Hkv,
                                                           long long ld) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int d = EPL * 32;
   __shared__ float sdw[8][2 * d];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -459,6 +473,8 @@ __global__ void __launch_bounds__(256) headnorm_bwd_kernel(__nv_bfloat16* __rest
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict__ pos, const float* __restrict__ cs,
                             const float* __restrict__ sn, long long T, int nh, int d, int rot, long long row_stride,
                             float sign) {
+  pdl_wait();
+  pdl_trigger();
   // one thread rotates 8 pairs: a 16-byte vector from each half of the rotated part
   const int half = rot >> 1;
   const int vecs_per_head = half >> 3;
@@ -496,6 +512,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict
 // x[t, j] += bias[j] in place (bf16, 16-byte vectors): the q/k/v projection bias of Qwen2-style attention
 __global__ void bias_add_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ bias, long long T,
                                 int N, long long ld) {
+  pdl_wait();
+  pdl_trigger();
   const int nv = N >> 3;
   const long long total = T * nv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -516,6 +534,8 @@ __global__ void bias_add_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloat
 // Block = 32 column vectors (256 columns) x 8 row lanes; grid.y row groups stride over the rows.
 __global__ void __launch_bounds__(256) bias_grad_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ out,
                                                         long long T, int N, long long ld) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[8][32][9];
   const int cv = threadIdx.x & 31, rl = threadIdx.x >> 5;
   const int v = blockIdx.x * 32 + cv;  // column vector index
@@ -545,6 +565,8 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const __nv_bfloat16* __r
 // act[t, j] = silu(gu[t, j]) * gu[t, f + j]      gu is [T, 2f]
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act, long long T,
                                   int f) {
+  pdl_wait();
+  pdl_trigger();
   const int fv = f >> 3;
   const long long total = T * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -564,6 +586,8 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 // dgu[t, j] = dact * u * dsilu(g) ; dgu[t, f + j] = dact * silu(g)
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dact,
                                   __nv_bfloat16* __restrict__ dgu, long long T, int f) {
+  pdl_wait();
+  pdl_trigger();
   const int fv = f >> 3;
   const long long total = T * fv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -590,6 +614,8 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 
 __global__ void embed_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ W,
                                  __nv_bfloat16* __restrict__ out, long long T, int h, int vocab) {
+  pdl_wait();
+  pdl_trigger();
   const int hv = h >> 3;
   const long long total = T * hv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -605,6 +631,8 @@ __global__ void embed_fwd_kernel(const long long* __restrict__ ids, const __nv_b
 // dW[ids[t], :] += dout[t, :]   (fp32 gradient buffer, atomics: rows repeat)
 __global__ void embed_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dout,
                                  float* __restrict__ dW, long long T, int h, int vocab) {
+  pdl_wait();
+  pdl_trigger();
   const int hv = h >> 3;
   const long long total = T * hv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -624,6 +652,8 @@ __global__ void embed_bwd_kernel(const long long* __restrict__ ids, const __nv_b
 // dst[rows[i], :] = src[i, :]   (rows unique; dst pre-zeroed by the launcher). Backward of a row gather.
 __global__ void scatter_rows_kernel(const long long* __restrict__ rows, const __nv_bfloat16* __restrict__ src,
                                     __nv_bfloat16* __restrict__ dst, long long n, int h, long long dst_rows) {
+  pdl_wait();
+  pdl_trigger();
   const int hv = h >> 3;
   const long long total = n * hv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -639,6 +669,8 @@ __global__ void scatter_rows_kernel(const long long* __restrict__ rows, const __
 // bf16 <-> fp32 conversions over flat buffers (n elements), with optional scale / accumulate.
 __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n,
                                         float scale) {
+  pdl_wait();
+  pdl_trigger();
   const long long nv = n >> 3;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv;
        i += (long long)gridDim.x * blockDim.x) {
@@ -652,6 +684,8 @@ __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ in, __nv_bfloa
 }
 __global__ void cast_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ in, float* __restrict__ out, long long n,
                                         float scale, int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   const long long nv = n >> 3;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv;
        i += (long long)gridDim.x * blockDim.x) {
@@ -701,7 +735,7 @@ int b200_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, voi
   const int grid = rows < sm_count() * 8 ? rows : sm_count() * 8;
   const int wblocks = ceil_div(rows, 4) < sm_count() * 5 ? ceil_div(rows, 4) : sm_count() * 5;  // 4 rows per 128-thread CTA
 #define B200_RMS_FWD_WARP(VPL)                                                                                        \
-  rmsnorm_fwd_warp_kernel<VPL><<<wblocks, 128, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res,            \
+  launch_pdl(rmsnorm_fwd_warp_kernel<VPL>, wblocks, 128, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,            \
                                                         (const __nv_bfloat16*)w, (__nv_bfloat16*)y,                   \
                                                         (__nv_bfloat16*)hout, rstd, rows, eps)
   if (h == 2048) B200_RMS_FWD_WARP(8);
@@ -709,7 +743,7 @@ int b200_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, voi
   else if (h == 512) B200_RMS_FWD_WARP(2);
   else if (h == 256) B200_RMS_FWD_WARP(1);
   else
-    rmsnorm_fwd_kernel<<<grid, NT, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
+    launch_pdl(rmsnorm_fwd_kernel, grid, NT, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
                                             (__nv_bfloat16*)y, (__nv_bfloat16*)hout, rstd, rows, h, eps);
 #undef B200_RMS_FWD_WARP
   B200_CUDA_CHECK(cudaGetLastError());
@@ -723,7 +757,7 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
     return B200_ERR_ARG;
   const int grid = b200_rmsnorm_bwd_blocks(rows);  // partial rows: one per block, or one per warp in the warp kernels
 #define B200_RMS_BWD_WARP(VPL)                                                                                       \
-  rmsnorm_bwd_warp_kernel<VPL><<<ceil_div(grid, 4), 128, 4 * (VPL) * 256 * 4, st>>>(                                                   \
+  launch_pdl(rmsnorm_bwd_warp_kernel<VPL>, ceil_div(grid, 4), 128, 4 * (VPL) * 256 * 4, st,                                                    \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,   \
       (__nv_bfloat16*)dx, dw_partial, rows, grid)
   if (h == 2048) B200_RMS_BWD_WARP(8);
@@ -731,12 +765,12 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
   else if (h == 512) B200_RMS_BWD_WARP(2);
   else if (h == 256) B200_RMS_BWD_WARP(1);
   else
-    rmsnorm_bwd_kernel<<<grid, NT, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+    launch_pdl(rmsnorm_bwd_kernel, grid, NT, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
                                             rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, rows, h);
 #undef B200_RMS_BWD_WARP
   B200_CUDA_CHECK(cudaGetLastError());
   const bool warp_kernel = h == 2048 || h == 1024 || h == 512 || h == 256;    // one partial row per 4-warp CTA there
-  colsum_kernel<<<ceil_div(h, 32), 256, 0, st>>>(dw_partial, dw_out, warp_kernel ? ceil_div(grid, 4) : grid, h,
+  launch_pdl(colsum_kernel, ceil_div(h, 32), 256, 0, st, dw_partial, dw_out, warp_kernel ? ceil_div(grid, 4) : grid, h,
                                                  dw_accumulate);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -751,10 +785,10 @@ int b200_headnorm_fwd(const void* x, void* y, const void* wq, const void* wk, fl
   const long long items = T * (H + 2 * Hkv);
   const int grid = grid_for(items * 32, 256);
   if (d == 128)
-    headnorm_fwd_kernel<4><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, (const __nv_bfloat16*)wq,
+    launch_pdl(headnorm_fwd_kernel<4>, grid, 256, 0, st, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, (const __nv_bfloat16*)wq,
                                                  (const __nv_bfloat16*)wk, rstd, T, H, Hkv, ld, eps);
   else
-    headnorm_fwd_kernel<2><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, (const __nv_bfloat16*)wq,
+    launch_pdl(headnorm_fwd_kernel<2>, grid, 256, 0, st, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, (const __nv_bfloat16*)wq,
                                                  (const __nv_bfloat16*)wk, rstd, T, H, Hkv, ld, eps);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -777,13 +811,13 @@ int b200_headnorm_bwd(void* g, const void* x, const void* wq, const void* wk, co
     return B200_ERR_ARG;
   const int grid = b200_headnorm_bwd_blocks(T, H, Hkv);
   if (d == 128)
-    headnorm_bwd_kernel<4><<<grid, 256, 0, st>>>((__nv_bfloat16*)g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq,
+    launch_pdl(headnorm_bwd_kernel<4>, grid, 256, 0, st, (__nv_bfloat16*)g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq,
                                                  (const __nv_bfloat16*)wk, rstd, dw_partial, T, H, Hkv, ld);
   else
-    headnorm_bwd_kernel<2><<<grid, 256, 0, st>>>((__nv_bfloat16*)g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq,
+    launch_pdl(headnorm_bwd_kernel<2>, grid, 256, 0, st, (__nv_bfloat16*)g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq,
                                                  (const __nv_bfloat16*)wk, rstd, dw_partial, T, H, Hkv, ld);
   B200_CUDA_CHECK(cudaGetLastError());
-  colsum_kernel<<<ceil_div(2 * d, 32), 256, 0, st>>>(dw_partial, dw_out, grid, 2 * d, dw_accumulate);
+  launch_pdl(colsum_kernel, ceil_div(2 * d, 32), 256, 0, st, dw_partial, dw_out, grid, 2 * d, dw_accumulate);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -795,7 +829,7 @@ int b200_rope_partial(void* x, const int* pos, const float* cos_tab, const float
       (row_stride & 7))
     return B200_ERR_ARG;
   const long long total = T * nh * (rot >> 4);
-  rope_kernel<<<grid_for(total, 256), 256, 0, st>>>((__nv_bfloat16*)x, pos, cos_tab, sin_tab, T, nh, d, rot,
+  launch_pdl(rope_kernel, grid_for(total, 256), 256, 0, st, (__nv_bfloat16*)x, pos, cos_tab, sin_tab, T, nh, d, rot,
                                                    row_stride, inverse ? -1.f : 1.f);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -808,7 +842,7 @@ int b200_rope(void* x, const int* pos, const float* cos_tab, const float* sin_ta
 
 int b200_bias_add(void* x, const void* bias, long long T, int N, long long ld, cudaStream_t st) {
   if (!x || !bias || T <= 0 || N <= 0 || (N & 7) || (ld & 7)) return B200_ERR_ARG;
-  bias_add_kernel<<<grid_for(T * (N >> 3), 256), 256, 0, st>>>((__nv_bfloat16*)x, (const __nv_bfloat16*)bias, T, N, ld);
+  launch_pdl(bias_add_kernel, grid_for(T * (N >> 3), 256), 256, 0, st, (__nv_bfloat16*)x, (const __nv_bfloat16*)bias, T, N, ld);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -821,21 +855,21 @@ int b200_bias_grad(const void* dy, float* out, long long T, int N, long long ld,
   if (gy > 64) gy = 64;
   if (gy < 1) gy = 1;
   dim3 grid((unsigned)ceil_div(N, 256), (unsigned)gy);
-  bias_grad_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)dy, out, T, N, ld);
+  launch_pdl(bias_grad_kernel, grid, 256, 0, st, (const __nv_bfloat16*)dy, out, T, N, ld);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
 
 int b200_swiglu_fwd(const void* gu, void* act, long long T, int f, cudaStream_t st) {
   if (!gu || !act || T <= 0 || (f & 7)) return B200_ERR_ARG;
-  swiglu_fwd_kernel<<<grid_for(T * (f >> 3), 256), 256, 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)act, T, f);
+  launch_pdl(swiglu_fwd_kernel, grid_for(T * (f >> 3), 256), 256, 0, st, (const __nv_bfloat16*)gu, (__nv_bfloat16*)act, T, f);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
 
 int b200_swiglu_bwd(const void* gu, const void* dact, void* dgu, long long T, int f, cudaStream_t st) {
   if (!gu || !dact || !dgu || T <= 0 || (f & 7)) return B200_ERR_ARG;
-  swiglu_bwd_kernel<<<grid_for(T * (f >> 3), 256), 256, 0, st>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dact,
+  launch_pdl(swiglu_bwd_kernel, grid_for(T * (f >> 3), 256), 256, 0, st, (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dact,
                                                                 (__nv_bfloat16*)dgu, T, f);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -843,7 +877,7 @@ int b200_swiglu_bwd(const void* gu, const void* dact, void* dgu, long long T, in
 
 int b200_embed_fwd(const long long* ids, const void* W, void* out, long long T, int h, int vocab, cudaStream_t st) {
   if (!ids || !W || !out || T <= 0 || (h & 7)) return B200_ERR_ARG;
-  embed_fwd_kernel<<<grid_for(T * (h >> 3), 256), 256, 0, st>>>(ids, (const __nv_bfloat16*)W, (__nv_bfloat16*)out, T, h,
+  launch_pdl(embed_fwd_kernel, grid_for(T * (h >> 3), 256), 256, 0, st, ids, (const __nv_bfloat16*)W, (__nv_bfloat16*)out, T, h,
                                                                vocab);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -851,7 +885,7 @@ int b200_embed_fwd(const long long* ids, const void* W, void* out, long long T, 
 
 int b200_embed_bwd(const long long* ids, const void* dout, float* dW, long long T, int h, int vocab, cudaStream_t st) {
   if (!ids || !dout || !dW || T <= 0 || (h & 7)) return B200_ERR_ARG;
-  embed_bwd_kernel<<<grid_for(T * (h >> 3), 256), 256, 0, st>>>(ids, (const __nv_bfloat16*)dout, dW, T, h, vocab);
+  launch_pdl(embed_bwd_kernel, grid_for(T * (h >> 3), 256), 256, 0, st, ids, (const __nv_bfloat16*)dout, dW, T, h, vocab);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -860,7 +894,7 @@ int b200_scatter_rows(const long long* rows, const void* src, void* dst, long lo
                       cudaStream_t st) {
   if (!rows || !src || !dst || n <= 0 || (h & 7) || dst_rows <= 0) return B200_ERR_ARG;
   B200_CUDA_CHECK(cudaMemsetAsync(dst, 0, (size_t)dst_rows * h * 2, st));
-  scatter_rows_kernel<<<grid_for(n * (h >> 3), 256), 256, 0, st>>>(rows, (const __nv_bfloat16*)src, (__nv_bfloat16*)dst,
+  launch_pdl(scatter_rows_kernel, grid_for(n * (h >> 3), 256), 256, 0, st, rows, (const __nv_bfloat16*)src, (__nv_bfloat16*)dst,
                                                                   n, h, dst_rows);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -869,7 +903,7 @@ int b200_scatter_rows(const long long* rows, const void* src, void* dst, long lo
 int b200_cast_f32_to_bf16(const float* in, void* out, long long n, float scale, cudaStream_t st) {
   if (!in || !out || n <= 0) return B200_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return B200_ERR_ARG;
-  cast_f32_to_bf16_kernel<<<grid_for(n >> 3, 256), 256, 0, st>>>(in, (__nv_bfloat16*)out, n, scale);
+  launch_pdl(cast_f32_to_bf16_kernel, grid_for(n >> 3, 256), 256, 0, st, in, (__nv_bfloat16*)out, n, scale);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -877,7 +911,7 @@ int b200_cast_f32_to_bf16(const float* in, void* out, long long n, float scale, 
 int b200_cast_bf16_to_f32(const void* in, float* out, long long n, float scale, int accumulate, cudaStream_t st) {
   if (!in || !out || n <= 0) return B200_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return B200_ERR_ARG;
-  cast_bf16_to_f32_kernel<<<grid_for(n >> 3, 256), 256, 0, st>>>((const __nv_bfloat16*)in, out, n, scale, accumulate);
+  launch_pdl(cast_bf16_to_f32_kernel, grid_for(n >> 3, 256), 256, 0, st, (const __nv_bfloat16*)in, out, n, scale, accumulate);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -940,10 +974,10 @@ extern "C" int b200_rmsnorm_bwd_noalloc(const void* dy, const void* x, const voi
   const int grid = rows < B200_RMSNORM_NOALLOC_MAX_BLOCKS ? rows : B200_RMSNORM_NOALLOC_MAX_BLOCKS;
   // every block writes its own partial row (all h columns) before the column sum reads rows [0, grid):
   // nothing left over from an earlier call is ever read
-  rmsnorm_bwd_kernel<<<grid, NT, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+  launch_pdl(rmsnorm_bwd_kernel, grid, NT, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
                                           rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, h);
   B200_CUDA_CHECK(cudaGetLastError());
-  colsum_kernel<<<ceil_div(h, 32), 256, 0, st>>>(scratch, dw_out, grid, h, dw_accumulate);
+  launch_pdl(colsum_kernel, ceil_div(h, 32), 256, 0, st, scratch, dw_out, grid, h, dw_accumulate);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

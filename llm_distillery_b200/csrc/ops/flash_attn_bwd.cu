@@ -150,6 +150,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   const int colK = p.H * D + hkv * D;
   const int colV = (p.H + p.Hkv) * D + hkv * D;
@@ -479,6 +481,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 template <int D>
 __global__ void delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
                              float* __restrict__ delta, long long T, int H) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int LPG = D / 8;  // lanes per (t,h)
   const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x);
   const long long grp = gid / LPG;
@@ -509,6 +513,8 @@ __global__ void delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_
 // dqkv[t, 0:H*D] = bf16(dq_acc[t, :])
 __global__ void dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dqkv, long long T, int HD,
                                   long long width) {
+  pdl_wait();
+  pdl_trigger();
   const int hv = HD >> 3;
   const long long total = T * hv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -532,6 +538,8 @@ __global__ void dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* 
 __global__ void dq_convert_rope_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dqkv,
                                        const int* __restrict__ pos, const float* __restrict__ cs,
                                        const float* __restrict__ sn, long long T, int H, int D, long long width) {
+  pdl_wait();
+  pdl_trigger();
   const int half = D >> 1;
   const int vph = half >> 3;                 // vector pairs per head
   const int vpt = H * vph;
@@ -596,7 +604,7 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
   if (rc != B200_OK) return rc;
   {
     const long long threads = T * H * (D / 8);
-    delta_kernel<D><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)dout,
+    launch_pdl(delta_kernel<D>, (unsigned)((threads + 255) / 256), 256, 0, st, (const __nv_bfloat16*)dout,
                                                                       (const __nv_bfloat16*)out, delta, T, H);
     B200_CUDA_CHECK(cudaGetLastError());
   }
@@ -609,7 +617,7 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
   }
   BwdParams p{lse, delta, dq_acc, (__nv_bfloat16*)dqkv, B, L, H, Hkv, window, 1.0f / sqrtf((float)D)};
   dim3 grid(Hkv * B, (L + BN - 1) / BN);
-  kern<<<grid, NTHREADS, C::SMEM_BYTES, st>>>(tmQKV, tmDO, tmDQ, p, device_err_word());
+  launch_pdl(kern, grid, NTHREADS, C::SMEM_BYTES, st, tmQKV, tmDO, tmDQ, p, device_err_word());
   B200_CUDA_CHECK(cudaGetLastError());
   {
     const bool rot = pos != nullptr;
@@ -618,10 +626,10 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
     const long long cap = (long long)sm_count() * 8;
     if (blocks > cap) blocks = cap;
     if (rot)
-      dq_convert_rope_kernel<<<(unsigned)blocks, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, pos, cos_tab, sin_tab, T, H,
+      launch_pdl(dq_convert_rope_kernel, (unsigned)blocks, 256, 0, st, dq_acc, (__nv_bfloat16*)dqkv, pos, cos_tab, sin_tab, T, H,
                                                               D, width);
     else
-      dq_convert_kernel<<<(unsigned)blocks, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, T, (int)HD, width);
+      launch_pdl(dq_convert_kernel, (unsigned)blocks, 256, 0, st, dq_acc, (__nv_bfloat16*)dqkv, T, (int)HD, width);
     B200_CUDA_CHECK(cudaGetLastError());
   }
   return B200_OK;
@@ -671,7 +679,7 @@ extern "C" int b200_dq_convert_rope(const float* acc, void* dqkv, const int* pos
   long long blocks = (work + 255) / 256;
   const long long cap = (long long)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  fab::dq_convert_rope_kernel<<<(unsigned)blocks, 256, 0, st>>>(acc, (__nv_bfloat16*)dqkv, pos, cos_tab, sin_tab, T, H, D,
+  launch_pdl(fab::dq_convert_rope_kernel, (unsigned)blocks, 256, 0, st, acc, (__nv_bfloat16*)dqkv, pos, cos_tab, sin_tab, T, H, D,
                                                               width);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;

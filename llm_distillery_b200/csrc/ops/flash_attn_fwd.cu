@@ -156,6 +156,8 @@ __global__ void __launch_bounds__(NTHREADS, 2)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   const int colQ = p.colQ0 + hq * D;
   const int colK = p.colK0 + hkv * D;
@@ -455,7 +457,7 @@ static int launch_fwd(const void* q, long long q_width, int colQ0, const void* k
   }
   FwdParams p{(__nv_bfloat16*)out, lse, B, L, H, Hkv, 1.0f / sqrtf((float)D), q_off, window, colQ0, colK0, colV0};
   dim3 grid(H * B, (L + BM - 1) / BM);
-  kern<<<grid, NTHREADS, C::SMEM_BYTES, st>>>(tmQ, tmK, tmV, p, device_err_word());
+  launch_pdl(kern, grid, NTHREADS, C::SMEM_BYTES, st, tmQ, tmK, tmV, p, device_err_word());
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

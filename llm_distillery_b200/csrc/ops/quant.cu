@@ -26,6 +26,8 @@ __global__ void __launch_bounds__(256) dequant_nf4_kernel(const uint8_t* __restr
                                                           const int8_t* __restrict__ absmax_code,
                                                           const float* __restrict__ absmax_scale, float offset,
                                                           __nv_bfloat16* __restrict__ out, long long n) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float lut[16];
   if (threadIdx.x < 16) lut[threadIdx.x] = kNF4[threadIdx.x];
   __syncthreads();
@@ -51,6 +53,8 @@ __global__ void __launch_bounds__(256) dequant_nf4_kernel(const uint8_t* __restr
 __global__ void __launch_bounds__(256) dequant_int8_kernel(const int8_t* __restrict__ code,
                                                            const float* __restrict__ row_scale,
                                                            __nv_bfloat16* __restrict__ out, long long rows, int cols) {
+  pdl_wait();
+  pdl_trigger();
   const int gpr = cols >> 4;
   const long long groups = rows * gpr;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < groups;
@@ -87,7 +91,7 @@ int b200_dequant_nf4(const void* packed, const void* absmax_code, const float* a
                      long long n, cudaStream_t st) {
   if (!packed || !absmax_code || !absmax_scale || !out || n <= 0 || (n & 63)) return B200_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(packed) & 7) || (reinterpret_cast<uintptr_t>(out) & 15)) return B200_ERR_ARG;
-  quant::dequant_nf4_kernel<<<quant::grid_for(n >> 4), 256, 0, st>>>((const uint8_t*)packed, (const int8_t*)absmax_code,
+  launch_pdl(quant::dequant_nf4_kernel, quant::grid_for(n >> 4), 256, 0, st, (const uint8_t*)packed, (const int8_t*)absmax_code,
                                                                     absmax_scale, offset, (__nv_bfloat16*)out, n);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -96,7 +100,7 @@ int b200_dequant_nf4(const void* packed, const void* absmax_code, const float* a
 int b200_dequant_int8(const void* code, const float* row_scale, void* out, long long rows, int cols, cudaStream_t st) {
   if (!code || !row_scale || !out || rows <= 0 || cols <= 0 || (cols & 15)) return B200_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(code) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return B200_ERR_ARG;
-  quant::dequant_int8_kernel<<<quant::grid_for(rows * (cols >> 4)), 256, 0, st>>>((const int8_t*)code, row_scale,
+  launch_pdl(quant::dequant_int8_kernel, quant::grid_for(rows * (cols >> 4)), 256, 0, st, (const int8_t*)code, row_scale,
                                                                                  (__nv_bfloat16*)out, rows, cols);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;

@@ -16,6 +16,8 @@ struct AdamArgs {
 __global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ master, __nv_bfloat16* __restrict__ model,
                                                   const float* __restrict__ grad, float* __restrict__ m,
                                                   float* __restrict__ v, long long n, AdamArgs a) {
+  pdl_wait();
+  pdl_trigger();
   const long long nv = n >> 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv;
        i += (long long)gridDim.x * blockDim.x) {
@@ -67,6 +69,8 @@ struct SimpleArgs {
 __global__ void __launch_bounds__(256) simple_kernel(float* __restrict__ master, __nv_bfloat16* __restrict__ model,
                                                     const float* __restrict__ grad, float* __restrict__ s0,
                                                     float* __restrict__ s1, long long n, SimpleArgs a) {
+  pdl_wait();
+  pdl_trigger();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     float p = master[i];
@@ -99,6 +103,8 @@ __global__ void __launch_bounds__(QB) adam8_kernel(float* __restrict__ master, _
                                                   const float* __restrict__ grad, int8_t* __restrict__ mq,
                                                   uint8_t* __restrict__ vq, float* __restrict__ mabs,
                                                   float* __restrict__ vabs, long long n, AdamArgs a) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[QB / 32];
   __shared__ float bcast[2];
   for (long long blk = blockIdx.x; blk * QB < n; blk += gridDim.x) {
@@ -152,6 +158,8 @@ __global__ void __launch_bounds__(QB) adam8_kernel(float* __restrict__ master, _
 
 // sum of squares of a flat fp32 buffer (for gradient-norm logging), atomically added into out[0].
 __global__ void sumsq_kernel(const float* __restrict__ x, long long n, float scale, float* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
   float s = 0.f;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const float v = x[i] * scale;
@@ -183,7 +191,7 @@ int b200_adam_step(float* master, void* model, const float* grad, float* m, floa
   if (!master || !grad || !m || !v || n <= 0 || step < 1) return B200_ERR_ARG;
   AdamArgs a{lr, beta1, beta2, eps, weight_decay, 1.f - powf(beta1, (float)step), 1.f - powf(beta2, (float)step),
              grad_scale, decoupled};
-  adam_kernel<<<opt_grid(n, 4), 256, 0, st>>>(master, (__nv_bfloat16*)model, grad, m, v, n, a);
+  launch_pdl(adam_kernel, opt_grid(n, 4), 256, 0, st, master, (__nv_bfloat16*)model, grad, m, v, n, a);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -196,7 +204,7 @@ int b200_adam8_step(float* master, void* model, const float* grad, void* mq, voi
              grad_scale, decoupled};
   long long blocks = (n + QB - 1) / QB;
   const long long cap = (long long)sm_count() * 8;
-  adam8_kernel<<<(int)(blocks < cap ? blocks : cap), QB, 0, st>>>(master, (__nv_bfloat16*)model, grad, (int8_t*)mq,
+  launch_pdl(adam8_kernel, (int)(blocks < cap ? blocks : cap), QB, 0, st, master, (__nv_bfloat16*)model, grad, (int8_t*)mq,
                                                                   (uint8_t*)vq, mabs, vabs, n, a);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -207,14 +215,14 @@ int b200_simple_opt_step(float* master, void* model, const float* grad, float* s
                          int first_step, float grad_scale, cudaStream_t st) {
   if (!master || !grad || !s0 || n <= 0 || kind < 0 || kind > 2 || (kind == 1 && !s1)) return B200_ERR_ARG;
   SimpleArgs a{lr, weight_decay, momentum, alpha, eps, grad_scale, kind, nesterov, first_step};
-  simple_kernel<<<opt_grid(n, 1), 256, 0, st>>>(master, (__nv_bfloat16*)model, grad, s0, s1, n, a);
+  launch_pdl(simple_kernel, opt_grid(n, 1), 256, 0, st, master, (__nv_bfloat16*)model, grad, s0, s1, n, a);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
 
 int b200_sumsq(const float* x, long long n, float scale, float* out, cudaStream_t st) {
   if (!x || !out || n <= 0) return B200_ERR_ARG;
-  sumsq_kernel<<<opt_grid(n, 4), 256, 0, st>>>(x, n, scale, out);
+  launch_pdl(sumsq_kernel, opt_grid(n, 4), 256, 0, st, x, n, scale, out);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
