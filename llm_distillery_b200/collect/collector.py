@@ -69,7 +69,7 @@ class TeacherCollector:
             r1 = min(M, r0 + self.chunk_rows)
             lg = logits[: r1 - r0]
             if Hc.is_cuda and Hc.dtype in (torch.bfloat16, torch.float16):
-                basic.gemm(Hc[r0:r1], W, out=lg)
+                basic.gemm(Hc[r0:r1], W, out=lg, split_k=True)
             else:
                 lg.copy_(Hc[r0:r1].float() @ W.float().t())
             if self.enable_topk:

@@ -3,6 +3,7 @@
 // with A and B each either K-major or MN-major, so forward (NT), dgrad (NN) and wgrad (TN)
 // GEMMs of a linear layer all run without a transpose pass.
 #include "gemm_pair.cuh"
+#include "gemm_cluster.cuh"
 #include <stdlib.h>
 #include <atomic>
 #include "../common/host.cuh"
@@ -664,6 +665,22 @@ static bool split_k_enabled() {
   return on != 0;
 }
 
+// K slices of a split launch on `max_pairs` SM pairs: rounds of the pair grid in units of one whole tile, ceil(tiles * s /
+// pairs) / s, plus 1.5 % per extra slice for its read-modify-write epilogue; split only when that buys at least 7 %.
+// `rounds` (may be null) receives the cost.
+static int pair_k_splits(int tiles, int num_kb, int max_pairs, double* rounds) {
+  const double unsplit = (double)((tiles + max_pairs - 1) / max_pairs);
+  double best = unsplit;
+  int k_splits = 1;
+  for (int s = 2; s <= SPLIT_MAX_SLICES && num_kb / s >= 16; ++s) {
+    const double c = (double)((tiles * s + max_pairs - 1) / max_pairs) / s * (1.0 + 0.015 * (s - 1));
+    if (c < best - 1e-9) { best = c; k_splits = s; }
+  }
+  if (best > 0.93 * unsplit) { best = unsplit; k_splits = 1; }
+  if (rounds) *rounds = best;
+  return k_splits;
+}
+
 // Two-SM (cta_group::2) launch: 256 x 256 tiles, one CTA pair per tile.
 template <bool A_MN, bool B_MN>
 static int launch_store_pair(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int fmt,
@@ -703,15 +720,7 @@ static int launch_store_pair(const void* A, const void* B, int M, int N, int K, 
     if (forced > 0) {
       k_splits = forced;
     } else {
-      // rounds of the pair grid in units of one whole tile: ceil(tiles * s / pairs) / s, plus 1.5 % per extra slice for
-      // its read-modify-write epilogue; split only when that buys at least 7 %
-      const double unsplit = (double)((tiles + max_pairs - 1) / max_pairs);
-      double best = unsplit;
-      for (int s2 = 2; s2 <= SPLIT_MAX_SLICES && num_kb / s2 >= 16; ++s2) {
-        const double c = (double)((tiles * s2 + max_pairs - 1) / max_pairs) / s2 * (1.0 + 0.015 * (s2 - 1));
-        if (c < best - 1e-9) { best = c; k_splits = s2; }
-      }
-      if (best > 0.93 * unsplit) k_splits = 1;
+      k_splits = pair_k_splits(tiles, num_kb, max_pairs, nullptr);
     }
     if (k_splits > num_kb) k_splits = num_kb;
     if (k_splits > SPLIT_MAX_SLICES) k_splits = SPLIT_MAX_SLICES;
@@ -734,6 +743,202 @@ static int launch_store_pair(const void* A, const void* B, int M, int N, int K, 
   return B200_OK;
 }
 
+// ------------------------------------------------------------------------------------------- cluster split-K launches
+// Epilogues of the cluster kernel (gemm_cluster.cuh): the same arithmetic as the TMEM epilogues above, on four columns
+// of a row per call.
+__device__ __forceinline__ uint2 pack_bf16x4(const float (&v)[4]) {
+  return make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+}
+__device__ __forceinline__ void unpack_bf16x4(const uint2& q, float (&f)[4]) {
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+}
+
+struct ClusterStore {
+  using Params = StoreParams;
+  static constexpr bool SPLIT_B = false;
+  template <int BN>
+  static constexpr int items() { return BN / 4; }
+  template <int BN, class Get>
+  static __device__ __forceinline__ void item(const Params& p, int row, int n0, int N, int it, Get get) {
+    const int col = n0 + it * 4;
+    if (col >= N) return;
+    const int nv = min(4, N - col);
+    const float4 a = get(it);
+    float v[4] = {a.x * p.alpha, a.y * p.alpha, a.z * p.alpha, a.w * p.alpha};
+    if (p.resid) {
+      const __nv_bfloat16* rp = p.resid + (long long)row * p.ldr + col;
+      if (nv == 4 && !(reinterpret_cast<uintptr_t>(rp) & 7)) {
+        float r[4];
+        unpack_bf16x4(*reinterpret_cast<const uint2*>(rp), r);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] += r[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < nv) v[j] += __bfloat162float(rp[j]);
+      }
+    }
+    if (p.out_f32) {
+      float* cp = reinterpret_cast<float*>(p.C) + (long long)row * p.ldc + col;
+      if (nv == 4 && !(reinterpret_cast<uintptr_t>(cp) & 15)) {
+        float4 o = make_float4(v[0], v[1], v[2], v[3]);
+        if (p.accumulate) {
+          const float4 c = *reinterpret_cast<const float4*>(cp);
+          o.x += c.x; o.y += c.y; o.z += c.z; o.w += c.w;
+        }
+        *reinterpret_cast<float4*>(cp) = o;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < nv) cp[j] = p.accumulate ? cp[j] + v[j] : v[j];
+      }
+    } else if (p.fmt == 1) {
+      __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)row * p.ldc + col;
+      if (nv == 4 && !(reinterpret_cast<uintptr_t>(cp) & 7)) {
+        if (p.accumulate) {
+          float c[4];
+          unpack_bf16x4(*reinterpret_cast<const uint2*>(cp), c);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] += c[j];
+        }
+        *reinterpret_cast<uint2*>(cp) = pack_bf16x4(v);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < nv) cp[j] = __float2bfloat16(v[j] + (p.accumulate ? __bfloat162float(cp[j]) : 0.f));
+      }
+    } else {
+      __half* cp = reinterpret_cast<__half*>(p.C) + (long long)row * p.ldc + col;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < nv) cp[j] = __float2half(v[j] + (p.accumulate ? __half2float(cp[j]) : 0.f));
+    }
+  }
+};
+
+struct ClusterSwiglu {
+  using Params = SwigluParams;
+  static constexpr bool SPLIT_B = true;
+  template <int BN>
+  static constexpr int items() { return BN / 8; }
+  template <int BN, class Get>
+  static __device__ __forceinline__ void item(const Params& p, int row, int f0, int N, int it, Get get) {
+    const int col = f0 + it * 4;
+    if (col >= p.f) return;
+    const float4 g4 = get(it), u4 = get(it + BN / 8);
+    const float g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
+    const uint2 qg = pack_bf16x4(g), qu = pack_bf16x4(u);
+    float gr[4], ur[4], a[4];
+    unpack_bf16x4(qg, gr);
+    unpack_bf16x4(qu, ur);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[j] = __fdividef(gr[j], 1.f + __expf(-gr[j])) * ur[j];
+    __nv_bfloat16* gp = p.gu + (long long)row * p.ld_gu + col;
+    *reinterpret_cast<uint2*>(gp) = qg;
+    *reinterpret_cast<uint2*>(gp + p.f) = qu;
+    *reinterpret_cast<uint2*>(p.act + (long long)row * p.ld_act + col) = pack_bf16x4(a);
+  }
+};
+
+struct ClusterRope {      // a tile holds whole heads: BN is a multiple of d
+  using Params = RopeParams;
+  static constexpr bool SPLIT_B = false;
+  template <int BN>
+  static constexpr int items() { return BN / 8; }
+  template <int BN, class Get>
+  static __device__ __forceinline__ void item(const Params& p, int row, int n0, int N, int it, Get get) {
+    const int per_head = p.d >> 3;                         // pairs of 4-column chunks in a head
+    const int head = it / per_head, w = it - head * per_head;
+    const int ca = head * (p.d >> 2) + w, cb = ca + per_head;
+    const int col = n0 + ca * 4;
+    if (col >= N) return;
+    const float4 a4 = get(ca), b4 = get(cb);
+    const float af[4] = {a4.x, a4.y, a4.z, a4.w}, bf[4] = {b4.x, b4.y, b4.z, b4.w};
+    float a[4], b[4];
+    unpack_bf16x4(pack_bf16x4(af), a);
+    unpack_bf16x4(pack_bf16x4(bf), b);
+    if (col < p.n_rot) {
+      const long long e = (long long)p.pos[row] * (p.d >> 1) + w * 4;
+      const float4 c4 = *reinterpret_cast<const float4*>(p.cs + e);
+      const float4 s4 = *reinterpret_cast<const float4*>(p.sn + e);
+      const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float fa = a[j], fb = b[j];
+        a[j] = __fmaf_rn(fa, cc[j], -__fmul_rn(fb, ss[j]));
+        b[j] = __fmaf_rn(fb, cc[j], __fmul_rn(fa, ss[j]));
+      }
+    }
+    __nv_bfloat16* cp = p.C + (long long)row * p.ldc + col;
+    *reinterpret_cast<uint2*>(cp) = pack_bf16x4(a);
+    *reinterpret_cast<uint2*>(cp + (p.d >> 1)) = pack_bf16x4(b);
+  }
+};
+
+struct ClusterSwigluBwd {
+  using Params = SwigluBwdParams;
+  static constexpr bool SPLIT_B = false;
+  template <int BN>
+  static constexpr int items() { return BN / 4; }
+  template <int BN, class Get>
+  static __device__ __forceinline__ void item(const Params& p, int row, int n0, int N, int it, Get get) {
+    const int col = n0 + it * 4;
+    if (col >= p.f) return;
+    const __nv_bfloat16* gp = p.gu + (long long)row * p.ld_gu + col;
+    float g[4], u[4], d[4], dg[4], du[4];
+    unpack_bf16x4(__ldg(reinterpret_cast<const uint2*>(gp)), g);
+    unpack_bf16x4(__ldg(reinterpret_cast<const uint2*>(gp + p.f)), u);
+    const float4 a = get(it);
+    const float af[4] = {a.x, a.y, a.z, a.w};
+    unpack_bf16x4(pack_bf16x4(af), d);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float sgm = __fdividef(1.f, 1.f + __expf(-g[j]));
+      const float silu = g[j] * sgm;
+      dg[j] = d[j] * u[j] * (sgm + silu * (1.f - sgm));
+      du[j] = d[j] * silu;
+    }
+    __nv_bfloat16* op = p.dgu + (long long)row * p.ld_dgu + col;
+    *reinterpret_cast<uint2*>(op) = pack_bf16x4(dg);
+    *reinterpret_cast<uint2*>(op + p.f) = pack_bf16x4(du);
+  }
+};
+
+// N: columns of B's output space covered by tiles of BN (2 f for the gate / up projection, whose tiles take BN/2 gate and
+// BN/2 up rows: f = b_half > 0).
+template <int BN, bool A_MN, bool B_MN, class Epi>
+static int launch_cluster(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int fmt,
+                          const typename Epi::Params& ep, int slices, int b_half, cudaStream_t stream) {
+  using S = SmemCluster<BN>;
+  CUtensorMap tmA, tmB;
+  const CUtensorMapDataType dt = fmt == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  int rc;
+  if (!A_MN)
+    rc = make_tmap_2d(&tmA, A, dt, 2, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, BK, BM, CU_TENSOR_MAP_SWIZZLE_128B);
+  else
+    rc = make_tmap_2d(&tmA, A, dt, 2, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc != B200_OK) return rc;
+  if (!B_MN)
+    rc = make_tmap_2d(&tmB, B, dt, 2, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, BK, Epi::SPLIT_B ? BN / 2 : BN,
+                      CU_TENSOR_MAP_SWIZZLE_128B);
+  else
+    rc = make_tmap_2d(&tmB, B, dt, 2, (uint64_t)N, (uint64_t)K, (uint64_t)ldb * 2, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc != B200_OK) return rc;
+  auto kern = gemm_cluster_kernel<BN, A_MN, B_MN, Epi>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES));
+    attr_set = true;
+  }
+  const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, BN);
+  launch_pdl_cluster(kern, dim3((unsigned)(tiles * slices)), dim3(NUM_THREADS), S::BYTES, stream, slices, tmA, tmB, M, N, K,
+                     fmt, ep, device_err_word(), b_half);
+  B200_CUDA_CHECK(cudaGetLastError());
+  return B200_OK;
+}
+
 // 0 = never, 1 = whenever the shape allows, unset = heuristic (enough 256 x 256 tiles to fill the SM pairs)
 static int pair_mode() {
   static int mode = -2;
@@ -750,6 +955,56 @@ static bool use_pair(int M, int N, int K) {
   if (mode == 1) return true;
   const long long tiles = (long long)ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
   return (tiles >= sm_count() / 2 && K >= 256) || (tiles >= sm_count() / 8 && K >= 4096);
+}
+
+// Which kernel takes a GEMM: the cluster kernel with tiles of 128 x bn and `slices` CTAs per tile, or (bn = 0) the
+// kernels of 128 x 256 and 256 x 256 tiles. The K slices decide the order of the additions, so the choice of `slices` is a
+// function of the sizes alone and is the same for the plain GEMM and for the ones with a fused epilogue. split = false
+// keeps the order of additions that the large tiles have. The forward pass of training asks for that, and under the
+// reference loss the backward pass too: that loss divides by the largest row and clips a difference of two
+// cross-entropies, and turned a last bit of an activation into 0.1 to 0.7 % of its value (38 runs of five students, 200
+// to 1100 tokens; the KL losses: 0.001 %), so that the loss of a conversation would depend on the batch that it is in.
+//
+// Times in microseconds, least squares over 137 sizes from 32 to 3000 tokens on layers of 256 to 28672 (B200, weights
+// from HBM; within 6 - 9 %): a cluster CTA costs a fixed part (launch, first loads, exchange, epilogue) and a part per K
+// block, more of both when two share an SM; the 256 x 256 kernel pays per round of its SM pairs. Clusters do not pack
+// onto the last SMs of the chip (294 CTAs in clusters of 3 or 6 ran as two rounds), so split tiles stop at 7/8 of the
+// resident CTAs. Examples, one CTA per tile before / cluster now: 93 x 2048 x 5632 37.8 / 11.0, 93 x 2560 x 2048 17.2 /
+// 7.4, 777 x 896 x 9728 59.3 / 21.4, 896 x 896 x 776 (weight gradient) 11.3 / 9.4; 2048 x 2048 x 2048 stays where it is
+// (17.7, cluster 20.2: tiles of 128 x 128 read twice the operand bytes per product and are bound by the L2).
+struct TilePlan { int bn, slices; };
+static TilePlan plan_tiles(int M, int N, int K, bool f32, bool split) {
+  static const double kCost[2][2][4] = {   // [bn = 64, 128][one CTA per SM, two]: fixed, per K block, split, per slice
+      {{4.15, 0.301, 0.73, -0.045}, {4.67, 0.337, 0.92, 0.055}},
+      {{4.91, 0.377, 1.44, -0.124}, {6.19, 0.455, 1.14, 0.156}}};
+  const int sms = sm_count(), num_kb = ceil_div(K, BK);
+  const long long pair_tiles = (long long)ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
+  TilePlan plan{0, 1};
+  double rounds = (double)((pair_tiles + sms / 2 - 1) / (sms / 2));
+  if (f32 && pair_tiles <= SPLIT_MAX_TILES && split_k_enabled()) {
+    const int s = pair_k_splits((int)pair_tiles, num_kb, sms / 2, &rounds);
+    if (!split && s > 1 && use_pair(M, N, K)) return plan;      // that order of additions stays
+  }
+  double least = 0.95 * (4.8 + rounds * (0.328 * num_kb + (f32 ? 3.2 : 1.3)));
+  for (int w = 0; w < 2; ++w) {
+    const int bn = w ? 128 : 64;
+    const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, bn);
+    for (int s = 1; s <= (split ? CLUSTER_MAX_SLICES : 1) && s <= num_kb; ++s) {
+      const long long ctas = tiles * s;
+      if (ctas > (s > 1 ? 2LL * sms * 7 / 8 : 2LL * sms)) break;
+      const double* c = kCost[w][ctas > sms];
+      const double us = c[0] + c[1] * ceil_div(num_kb, s) + (s > 1 ? c[2] : 0.0) + c[3] * s;
+      if (us < least) { least = us; plan = TilePlan{bn, s}; }
+    }
+  }
+  return plan;
+}
+
+template <bool A_MN, bool B_MN, class Epi>
+static int launch_cluster_bn(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int fmt,
+                             const typename Epi::Params& ep, TilePlan plan, int b_half, cudaStream_t stream) {
+  return plan.bn == 64 ? launch_cluster<64, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, plan.slices, b_half, stream)
+                       : launch_cluster<128, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, plan.slices, b_half, stream);
 }
 
 }  // namespace gemm
@@ -772,13 +1027,15 @@ int b200_gemm_reset_split_sync(cudaStream_t stream) {
 // launch. f must be a multiple of 128; row strides (elements) multiples of 8. Returns B200_ERR_ARG for shapes the fused
 // kernel does not take (the caller then runs the GEMM and the SwiGLU kernel).
 int b200_gemm_swiglu(const void* x, const void* Wgu, void* gu, void* act, int M, int f, int K, long long ldx,
-                     long long ldw, long long ld_gu, long long ld_act, cudaStream_t stream) {
+                     long long ldw, long long ld_gu, long long ld_act, int split_k, cudaStream_t stream) {
   using namespace b200;
   using namespace b200::gemm;
   if (!x || !Wgu || !gu || !act || M <= 0 || f <= 0 || K <= 0 || (f % PAIR_HALF_N) || (ldx & 7) || (ldw & 7) ||
       (ld_gu & 7) || (ld_act & 7) || (reinterpret_cast<uintptr_t>(gu) & 15) || (reinterpret_cast<uintptr_t>(act) & 15))
     return B200_ERR_ARG;
   SwigluParams sp{reinterpret_cast<__nv_bfloat16*>(gu), ld_gu, reinterpret_cast<__nv_bfloat16*>(act), ld_act, f};
+  const TilePlan plan = plan_tiles(M, 2 * f, K, false, split_k != 0);
+  if (plan.bn) return launch_cluster_bn<false, false, ClusterSwiglu>(x, Wgu, M, 2 * f, K, ldx, ldw, 1, sp, plan, f, stream);
   return launch_swiglu_pair(x, Wgu, M, f, K, ldx, ldw, sp, stream);
 }
 
@@ -786,7 +1043,7 @@ int b200_gemm_swiglu(const void* x, const void* Wgu, void* gu, void* act, int M,
 // epilogue (pos int32 [M]; cos / sin fp32 [max_pos, d/2]). d = 64 or 128, N a multiple of 128.
 int b200_gemm_rope(const void* x, const void* W, void* out, const int* pos, const float* cos_tab, const float* sin_tab,
                    int M, int N, int K, int n_rot_heads, int d, long long ldx, long long ldw, long long ldo,
-                   cudaStream_t stream) {
+                   int split_k, cudaStream_t stream) {
   using namespace b200;
   using namespace b200::gemm;
   if (!x || !W || !out || !pos || !cos_tab || !sin_tab || M <= 0 || N <= 0 || K <= 0 || (d != 64 && d != 128) ||
@@ -794,19 +1051,26 @@ int b200_gemm_rope(const void* x, const void* W, void* out, const int* pos, cons
       (reinterpret_cast<uintptr_t>(out) & 15))
     return B200_ERR_ARG;
   RopeParams rp{reinterpret_cast<__nv_bfloat16*>(out), ldo, pos, cos_tab, sin_tab, d, n_rot_heads * d};
+  TilePlan plan = plan_tiles(M, N, K, false, split_k != 0);
+  if (plan.bn) {
+    if (plan.bn < d) plan.bn = d;            // a tile holds whole heads
+    return launch_cluster_bn<false, false, ClusterRope>(x, W, M, N, K, ldx, ldw, 1, rp, plan, 0, stream);
+  }
   return launch_rope_pair(x, W, M, N, K, ldx, ldw, rp, stream);
 }
 
 // dgu[M, 2f] = SwiGLU backward of (gu, d(act)) with d(act) = dy[M, K] Wd[K, f] taken straight from the accumulator
 // (never written). f a multiple of 128; strides multiples of 8. B200_ERR_ARG for shapes the fused kernel does not take.
 int b200_gemm_swiglu_bwd(const void* dy, const void* Wd, const void* gu, void* dgu, int M, int f, int K, long long ld_dy,
-                         long long ldw, long long ld_gu, long long ld_dgu, cudaStream_t stream) {
+                         long long ldw, long long ld_gu, long long ld_dgu, int split_k, cudaStream_t stream) {
   using namespace b200;
   using namespace b200::gemm;
   if (!dy || !Wd || !gu || !dgu || M <= 0 || f <= 0 || K <= 0 || (f % PAIR_HALF_N) || (ld_dy & 7) || (ldw & 7) ||
       (ld_gu & 7) || (ld_dgu & 7) || (reinterpret_cast<uintptr_t>(gu) & 15) || (reinterpret_cast<uintptr_t>(dgu) & 15))
     return B200_ERR_ARG;
   SwigluBwdParams sp{reinterpret_cast<const __nv_bfloat16*>(gu), ld_gu, reinterpret_cast<__nv_bfloat16*>(dgu), ld_dgu, f};
+  const TilePlan plan = plan_tiles(M, f, K, false, split_k != 0);
+  if (plan.bn) return launch_cluster_bn<false, true, ClusterSwigluBwd>(dy, Wd, M, f, K, ld_dy, ldw, 1, sp, plan, 0, stream);
   return launch_swiglu_bwd_pair(dy, Wd, M, f, K, ld_dy, ldw, sp, stream);
 }
 
@@ -815,10 +1079,11 @@ int b200_gemm_swiglu_bwd(const void* dy, const void* Wd, const void* gu, void* d
 //   b_mn = 0: B is [N,K] with row stride ldb;   b_mn = 1: B is stored [K,N] with row stride ldb
 //   fmt: 1 = bf16 operands, 0 = fp16.  out_f32: C is fp32, else the operand type.
 // Strides are in elements and must be multiples of 8 (16 bytes); base pointers 16-byte aligned.
+// split_k: K may be cut over the CTAs of a cluster (plan_tiles).
 // desc_cfg: optional 6 x uint32 override of the matrix-descriptor byte offsets (testing hook), else null.
 int b200_gemm(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
               long long ldc, int a_mn, int b_mn, int fmt, int out_f32, int accumulate, float alpha,
-              const void* residual, long long ldr, const unsigned int* desc_cfg, cudaStream_t stream) {
+              const void* residual, long long ldr, const unsigned int* desc_cfg, int split_k, cudaStream_t stream) {
   using namespace b200;
   using namespace b200::gemm;
   if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return B200_ERR_ARG;
@@ -838,6 +1103,18 @@ int b200_gemm(const void* A, const void* B, void* C, int M, int N, int K, long l
     dco.a_lbo = desc_cfg[0]; dco.a_sbo = desc_cfg[1]; dco.a_kadv = desc_cfg[2];
     dco.b_lbo = desc_cfg[3]; dco.b_sbo = desc_cfg[4]; dco.b_kadv = desc_cfg[5];
     dcp = &dco;
+  }
+  if (!dcp && pair_mode() < 0) {
+    const TilePlan plan = plan_tiles(M, N, K, out_f32 != 0, split_k != 0);
+    if (plan.bn) {
+      if (!a_mn && !b_mn)
+        return launch_cluster_bn<false, false, ClusterStore>(A, B, M, N, K, lda, ldb, fmt, sp, plan, 0, stream);
+      if (!a_mn && b_mn)
+        return launch_cluster_bn<false, true, ClusterStore>(A, B, M, N, K, lda, ldb, fmt, sp, plan, 0, stream);
+      if (a_mn && b_mn)
+        return launch_cluster_bn<true, true, ClusterStore>(A, B, M, N, K, lda, ldb, fmt, sp, plan, 0, stream);
+      return launch_cluster_bn<true, false, ClusterStore>(A, B, M, N, K, lda, ldb, fmt, sp, plan, 0, stream);
+    }
   }
   if (!dcp && use_pair(M, N, K)) {
     if (!a_mn && !b_mn) return launch_store_pair<false, false>(A, B, M, N, K, lda, ldb, fmt, sp, stream);

@@ -62,6 +62,7 @@ class DistillEngine:
                  jsd_renorm: bool = False, vocab_parallel: bool = False, max_rows_per_rank: int = 0):
         self.model = model
         self.loss_kind = loss
+        model.ordered_sums = loss == "reference"      # the one loss that turns a last bit into per mille of its value
         self.temperature = float(temperature)
         self.alpha = float(alpha)
         self.vocab = min(crop_to_size or model.cfg.vocab_size, model.cfg.vocab_size)

@@ -67,7 +67,7 @@ def _rows(pmax, psum, zk, u, ids, M, K, nt, vocab, kind, inv_T):
     return lse, loss, a, A
 
 
-def _backward_chunks(Hc, W, ids, a, A, lse, g, inv_T, vocab, w_slot, need_dh: bool):
+def _backward_chunks(Hc, W, ids, a, A, lse, g, inv_T, vocab, w_slot, need_dh: bool, split_k: bool):
     """dH [M,h] (or None) and the LM-head weight gradient (into the slot, or returned) from the dlogits pass."""
     M, h = Hc.shape
     K = ids.shape[1]
@@ -90,15 +90,16 @@ def _backward_chunks(Hc, W, ids, a, A, lse, g, inv_T, vocab, w_slot, need_dh: bo
                                            _lib.stream()), "b200_lmhead_dlogits")
         dzv = dz[:n, :vocab]
         if need_dh:
-            basic.gemm(dzv, Wc, b_mn=True, out=dH[r0:r1])
+            basic.gemm(dzv, Wc, b_mn=True, out=dH[r0:r1], split_k=split_k)
         if want_w:
             if w_slot is not None:
-                basic.gemm(dzv, Hc[r0:r1], a_mn=True, b_mn=True, out=w_slot.buf[:vocab], accumulate=not w_slot.fresh)
+                basic.gemm(dzv, Hc[r0:r1], a_mn=True, b_mn=True, out=w_slot.buf[:vocab], accumulate=not w_slot.fresh,
+                           split_k=split_k)
                 if w_slot.fresh and vocab < W.shape[0]:
                     w_slot.buf[vocab:].zero_()
                 w_slot.fresh = False
             else:
-                basic.gemm(dzv, Hc[r0:r1], a_mn=True, b_mn=True, out=dW[:vocab], accumulate=True)
+                basic.gemm(dzv, Hc[r0:r1], a_mn=True, b_mn=True, out=dW[:vocab], accumulate=True, split_k=split_k)
     return dH, (dW.to(W.dtype) if dW is not None else None)
 
 
@@ -119,7 +120,8 @@ class _LmHeadStatsFn(torch.autograd.Function):
         a = (dzk if dzk is not None else torch.zeros(ids.shape, device=Hc.device)).float().contiguous()
         A = (-(dlse.float()) if dlse is not None else torch.zeros(M, device=Hc.device)).contiguous()
         g = torch.ones(M, dtype=torch.float32, device=Hc.device)
-        dH, dW = _backward_chunks(Hc, ctx.W, ids, a, A, lse, g, ctx.inv_T, ctx.vocab, ctx.slot, ctx.needs_input_grad[0])
+        dH, dW = _backward_chunks(Hc, ctx.W, ids, a, A, lse, g, ctx.inv_T, ctx.vocab, ctx.slot, ctx.needs_input_grad[0],
+                                  split_k=False)      # the reference loss is ill-conditioned: one order of additions
         return dH, dW, None, None, None
 
 
@@ -137,7 +139,8 @@ class _FusedDistillFn(torch.autograd.Function):
     def backward(ctx, dloss):
         Hc, ids, lse, a, A = ctx.saved_tensors
         g = dloss.float().contiguous()
-        dH, dW = _backward_chunks(Hc, ctx.W, ids, a, A, lse, g, ctx.inv_T, ctx.vocab, ctx.slot, ctx.needs_input_grad[0])
+        dH, dW = _backward_chunks(Hc, ctx.W, ids, a, A, lse, g, ctx.inv_T, ctx.vocab, ctx.slot, ctx.needs_input_grad[0],
+                                  split_k=True)
         return dH, dW, None, None, None, None, None
 
 

@@ -38,15 +38,15 @@ def _slot(p: torch.Tensor):
     return getattr(p, "grad_slot", None) if p.requires_grad else None
 
 
-def _wgrad(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor, slot):
+def _wgrad(dy: torch.Tensor, x: torch.Tensor, w: torch.Tensor, slot, split_k: bool = False):
     """Weight gradient of y = x w^T. With a slot: accumulated in place (fp32), returns None. Else returns dW."""
     if not w.requires_grad:
         return None
     if slot is not None:
-        basic.linear_wgrad(dy, x, out=slot.buf, accumulate=not slot.fresh)
+        basic.linear_wgrad(dy, x, out=slot.buf, accumulate=not slot.fresh, split_k=split_k)
         slot.fresh = False
         return None
-    return basic.linear_wgrad(dy, x, out_dtype=w.dtype)
+    return basic.linear_wgrad(dy, x, out_dtype=w.dtype, split_k=split_k)
 
 
 def _bias_grad(dy: torch.Tensor, b: torch.Tensor | None, slot):
@@ -118,14 +118,17 @@ class DecoderLayerFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, h, pos, cos, sin, w_ln1, w_qkv, w_o, w_ln2, w_gu, w_d, meta, b_qkv=None, w_qn=None, w_kn=None,
-                b_o=None, b_gu=None, b_d=None, rmul=1.0):
+                b_o=None, b_gu=None, b_d=None, rmul=1.0, split=(False, False)):
+        # split: whether GEMMs of few tiles may cut K, in the forward and in the backward pass (gemm.cu: plan_tiles)
+        ctx.split_bwd = split[1]
+        split = split[0]
         B, L, H, Hkv, d, eps, recompute, window = meta
         n1, _, rstd1 = basic.rmsnorm_fwd(h, w_ln1, eps)
         qk_saved = ()
         if b_qkv is None and w_qn is None:                    # rotation in the epilogue of the q/k/v GEMM
-            qkv = basic.linear_rope_fwd(n1, w_qkv, pos, cos, sin, H + Hkv, d)
+            qkv = basic.linear_rope_fwd(n1, w_qkv, pos, cos, sin, H + Hkv, d, split_k=split)
         else:
-            qkv = basic.linear_fwd(n1, w_qkv)
+            qkv = basic.linear_fwd(n1, w_qkv, split_k=split)
             if b_qkv is not None:
                 basic.bias_add_(qkv, b_qkv)
             if w_qn is not None:                              # per-head norm of q and k (Qwen3), before the rotation
@@ -136,16 +139,16 @@ class DecoderLayerFn(torch.autograd.Function):
         att, lse = attention.attention_fwd(qkv, B, L, H, Hkv, d, window)
         # rmul (Granite's residual_multiplier) scales a branch, bias included, before it joins the residual stream: it is
         # the alpha of the GEMM whose epilogue adds the residual
-        h1 = basic.gemm(att, w_o, residual=h, alpha=rmul)
+        h1 = basic.gemm(att, w_o, residual=h, alpha=rmul, split_k=split)
         if b_o is not None:
             basic.bias_add_(h1, b_o if rmul == 1.0 else b_o * rmul)
         n2, _, rstd2 = basic.rmsnorm_fwd(h1, w_ln2, eps)
         if b_gu is None:
-            gu, act = basic.linear_swiglu_fwd(n2, w_gu)
+            gu, act = basic.linear_swiglu_fwd(n2, w_gu, split_k=split)
         else:
-            gu = basic.bias_add_(basic.linear_fwd(n2, w_gu), b_gu)
+            gu = basic.bias_add_(basic.linear_fwd(n2, w_gu, split_k=split), b_gu)
             act = basic.swiglu_fwd(gu)
-        h2 = basic.gemm(act, w_d, residual=h1, alpha=rmul)
+        h2 = basic.gemm(act, w_d, residual=h1, alpha=rmul, split_k=split)
         if b_d is not None:
             basic.bias_add_(h2, b_d if rmul == 1.0 else b_d * rmul)
         ctx.rmul = rmul
@@ -167,6 +170,7 @@ class DecoderLayerFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dh2):
         B, L, H, Hkv, d, eps, recompute, window = ctx.meta
+        sp = ctx.split_bwd
         w_ln1, w_qkv, w_o, w_ln2, w_gu, w_d = ctx.weights
         s_ln1, s_qkv, s_o, s_ln2, s_gu, s_d = ctx.slots
         if UNIT_PRE[0] is not None:
@@ -209,21 +213,21 @@ class DecoderLayerFn(torch.autograd.Function):
         rmul = ctx.rmul
         db2 = dh2 if rmul == 1.0 else dh2 * rmul
         g_bd = _bias_grad(db2, b_d, sb_d)
-        g_d = _wgrad(db2, act, w_d, s_d)
+        g_d = _wgrad(db2, act, w_d, s_d, sp)
         del act
-        dgu = basic.linear_dgrad_swiglu_bwd(db2, w_d, gu)     # dgrad of the down projection + SwiGLU backward
+        dgu = basic.linear_dgrad_swiglu_bwd(db2, w_d, gu, split_k=sp)     # dgrad of the down projection + SwiGLU backward
         del db2
         g_bgu = _bias_grad(dgu, b_gu, sb_gu)
-        g_gu = _wgrad(dgu, n2, w_gu, s_gu)
-        dn2 = basic.linear_dgrad(dgu, w_gu)
+        g_gu = _wgrad(dgu, n2, w_gu, s_gu, sp)
+        dn2 = basic.linear_dgrad(dgu, w_gu, sp)
         del dgu
         dh1, dw2 = basic.rmsnorm_bwd(dn2, h1, w_ln2, rstd2, dres=dh2)
         g_ln2 = _vec_grad(dw2, w_ln2, s_ln2)
         # attention branch
         db1 = dh1 if rmul == 1.0 else dh1 * rmul
         g_bo = _bias_grad(db1, b_o, sb_o)
-        g_o = _wgrad(db1, att, w_o, s_o)
-        datt = basic.linear_dgrad(db1, w_o)
+        g_o = _wgrad(db1, att, w_o, s_o, sp)
+        datt = basic.linear_dgrad(db1, w_o, sp)
         del db1
         dqkv = attention.attention_bwd_unrotated(datt, qkv, att, lse, B, L, H, Hkv, d, pos, cos, sin, window)
         del datt
@@ -239,15 +243,15 @@ class DecoderLayerFn(torch.autograd.Function):
                 ctx.b_slot.fresh = False
             else:
                 g_b = basic.bias_grad(dqkv).to(ctx.b_qkv.dtype)
-        g_qkv = _wgrad(dqkv, n1, w_qkv, s_qkv)
-        dn1 = basic.linear_dgrad(dqkv, w_qkv)
+        g_qkv = _wgrad(dqkv, n1, w_qkv, s_qkv, sp)
+        dn1 = basic.linear_dgrad(dqkv, w_qkv, sp)
         del dqkv
         dh, dw1 = basic.rmsnorm_bwd(dn1, h, w_ln1, rstd1, dres=dh1)
         g_ln1 = _vec_grad(dw1, w_ln1, s_ln1)
         if LAYER_BACKWARD_DONE[0] is not None:
             LAYER_BACKWARD_DONE[0](w_ln1)
         return (dh, None, None, None, g_ln1, g_qkv, g_o, g_ln2, g_gu, g_d, None, g_b, g_qn, g_kn, g_bo, g_bgu, g_bd,
-                None)
+                None, None)
 
 
 class FinalNormFn(torch.autograd.Function):
@@ -355,6 +359,7 @@ class LlamaModel(nn.Module):
         else:
             self.lm_head = nn.Parameter(torch.empty(cfg.vocab_size, cfg.hidden_size, **kw))
         self.grad_checkpointing = False
+        self.ordered_sums = False  # backward GEMMs keep one order of additions whatever their size (see gemm.cu: plan_tiles)
         self._rope = None
         self.quant = None          # FrozenQuantLinears when the decoder layers' matrices are frozen NF4 / int8
 
@@ -448,6 +453,7 @@ class LlamaModel(nn.Module):
         meta = (B, L, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, cfg.rms_norm_eps,
                 bool(self.grad_checkpointing and torch.is_grad_enabled()))
         rmul = float(cfg.residual_multiplier)
+        split = (not torch.is_grad_enabled(), not self.ordered_sums)
         tables = self.layer_rope(cos, sin)
         meta7 = meta
         for li, (layer, (cos, sin)) in enumerate(zip(self.layers, tables)):
@@ -482,7 +488,7 @@ class LlamaModel(nn.Module):
                                      layer.post_attention_layernorm, layer.gate_up_proj, layer.down_proj, meta,
                                      getattr(layer, "qkv_bias", None), getattr(layer, "q_norm", None),
                                      getattr(layer, "k_norm", None), getattr(layer, "o_bias", None),
-                                     getattr(layer, "gate_up_bias", None), getattr(layer, "down_bias", None), rmul)
+                                     getattr(layer, "gate_up_bias", None), getattr(layer, "down_bias", None), rmul, split)
         if pre is not None:
             pre(self.norm, False)
         y = FinalNormFn.apply(h, self.norm, cfg.rms_norm_eps)
@@ -533,9 +539,9 @@ class LlamaModel(nn.Module):
                     continue
                 n1, _, _ = basic.rmsnorm_fwd(h, layer.input_layernorm, cfg.rms_norm_eps)
                 if not hasattr(layer, "qkv_bias") and not cfg.qk_norm and not cfg.qk_norm_full:
-                    qkv = basic.linear_rope_fwd(n1, layer.qkv_proj, pos, cos, sin, H + Hkv, d)
+                    qkv = basic.linear_rope_fwd(n1, layer.qkv_proj, pos, cos, sin, H + Hkv, d, split_k=True)
                 else:
-                    qkv = basic.linear_fwd(n1, layer.qkv_proj)
+                    qkv = basic.linear_fwd(n1, layer.qkv_proj, split_k=True)
                     if hasattr(layer, "qkv_bias"):
                         basic.bias_add_(qkv, layer.qkv_bias)
                     if cfg.qk_norm_full:
@@ -548,7 +554,7 @@ class LlamaModel(nn.Module):
                 vc[:, c0:c0 + n] = qkv[:, (H + Hkv) * d:].reshape(B, n, kv)
                 att = attention.attention_fwd_cached(qkv, kc, vc, B, n, c0, H, Hkv, d, window)
                 rm = float(cfg.residual_multiplier)
-                h1 = basic.gemm(att, layer.o_proj, residual=h, alpha=rm)
+                h1 = basic.gemm(att, layer.o_proj, residual=h, alpha=rm, split_k=True)
                 if cfg.o_bias:
                     basic.bias_add_(h1, layer.o_bias if rm == 1.0 else layer.o_bias * rm)
                 n2, _, _ = basic.rmsnorm_fwd(h1, layer.post_attention_layernorm, cfg.rms_norm_eps)
@@ -565,8 +571,8 @@ class LlamaModel(nn.Module):
                     h = basic.bias_add_(basic.gemm(act, layer.down_proj, residual=h1, alpha=rm),
                                         layer.down_bias if rm == 1.0 else layer.down_bias * rm)
                     continue
-                _, act = basic.linear_swiglu_fwd(n2, layer.gate_up_proj)
-                h = basic.gemm(act, layer.down_proj, residual=h1, alpha=rm)
+                _, act = basic.linear_swiglu_fwd(n2, layer.gate_up_proj, split_k=True)
+                h = basic.gemm(act, layer.down_proj, residual=h1, alpha=rm, split_k=True)
             y, _, _ = basic.rmsnorm_fwd(h, self.norm, cfg.rms_norm_eps)
             if cfg.logits_scaling != 1.0:
                 y = y * (1.0 / cfg.logits_scaling)

@@ -37,7 +37,7 @@ _VP, _I, _LL, _F = c_void_p, c_int, c_longlong, c_float
 
 _SIGS = {
     # name: argtypes
-    "b200_gemm": [_VP, _VP, _VP, _I, _I, _I, _LL, _LL, _LL, _I, _I, _I, _I, _I, _F, _VP, _LL, _VP, _VP],
+    "b200_gemm": [_VP, _VP, _VP, _I, _I, _I, _LL, _LL, _LL, _I, _I, _I, _I, _I, _F, _VP, _LL, _VP, _I, _VP],
     "b200_rmsnorm_fwd": [_VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _F, _VP],
     "b200_rmsnorm_bwd": [_VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _VP],
     "b200_rmsnorm_bwd_blocks": [_I],
@@ -57,9 +57,9 @@ _SIGS = {
     "b200_sm_count": [],
     "b200_segment_reduce": [_VP, _VP, _VP, _LL, _I, _I, _VP],
     "b200_gemm_reset_split_sync": [_VP],
-    "b200_gemm_swiglu": [_VP, _VP, _VP, _VP, _I, _I, _I, _LL, _LL, _LL, _LL, _VP],
-    "b200_gemm_rope": [_VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _LL, _LL, _LL, _VP],
-    "b200_gemm_swiglu_bwd": [_VP, _VP, _VP, _VP, _I, _I, _I, _LL, _LL, _LL, _LL, _VP],
+    "b200_gemm_swiglu": [_VP, _VP, _VP, _VP, _I, _I, _I, _LL, _LL, _LL, _LL, _I, _VP],
+    "b200_gemm_rope": [_VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _LL, _LL, _LL, _I, _VP],
+    "b200_gemm_swiglu_bwd": [_VP, _VP, _VP, _VP, _I, _I, _I, _LL, _LL, _LL, _LL, _I, _VP],
     "b200_headnorm_fwd": [_VP, _VP, _VP, _VP, _VP, _LL, _I, _I, _I, _LL, _F, _VP],
     "b200_headnorm_bwd_blocks": [_LL, _I, _I],
     "b200_headnorm_bwd": [_VP, _VP, _VP, _VP, _VP, _VP, _VP, _I, _LL, _I, _I, _I, _LL, _VP],

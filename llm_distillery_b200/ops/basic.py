@@ -32,8 +32,9 @@ def _fmt(dtype: torch.dtype) -> int:
 # ------------------------------------------------------------------------------------------------ GEMM
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,
          out_dtype: torch.dtype | None = None, accumulate: bool = False, alpha: float = 1.0,
-         residual: torch.Tensor | None = None, desc_cfg: list[int] | None = None) -> torch.Tensor:
-    """C[M,N] = alpha * A @ B^T (+ C) (+ residual).
+         residual: torch.Tensor | None = None, desc_cfg: list[int] | None = None, split_k: bool = False) -> torch.Tensor:
+    """C[M,N] = alpha * A @ B^T (+ C) (+ residual). ``split_k``: the reduction may be cut into slices that are added in
+    order (faster for outputs of few tiles; the last bits then depend on the sizes).
 
     ``a`` is [M,K] (``a_mn=False``) or stored transposed as [K,M] (``a_mn=True``); ``b`` is [N,K] or stored as [K,N].
     Rows must be contiguous (stride(1) == 1); row strides must be multiples of 8 elements.
@@ -79,25 +80,25 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     rc = _lib.kernels().b200_gemm(
         _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0), int(a_mn), int(b_mn),
         fmt, out_f32, int(accumulate), float(alpha), _lib.ptr(residual), residual.stride(0) if residual is not None else 0,
-        ctypes.cast(cfg, c_void_p) if cfg is not None else c_void_p(0), _lib.stream())
+        ctypes.cast(cfg, c_void_p) if cfg is not None else c_void_p(0), int(split_k), _lib.stream())
     _lib.check(rc, "b200_gemm")
     return out
 
 
-def linear_fwd(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
+def linear_fwd(x: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None = None, split_k: bool = False) -> torch.Tensor:
     """y[T,N] = x[T,K] @ w[N,K]^T (+ residual)."""
-    return gemm(x, w, residual=residual)
+    return gemm(x, w, residual=residual, split_k=split_k)
 
 
-def linear_dgrad(dy: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def linear_dgrad(dy: torch.Tensor, w: torch.Tensor, split_k: bool = False) -> torch.Tensor:
     """dx[T,K] = dy[T,N] @ w[N,K]  (w is read as an MN-major B operand: no transpose copy)."""
-    return gemm(dy, w, b_mn=True)
+    return gemm(dy, w, b_mn=True, split_k=split_k)
 
 
 def linear_wgrad(dy: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = None, accumulate: bool = False,
-                 out_dtype: torch.dtype | None = None) -> torch.Tensor:
+                 out_dtype: torch.dtype | None = None, split_k: bool = False) -> torch.Tensor:
     """dW[N,K] (+)= dy[T,N]^T @ x[T,K]  (both operands MN-major)."""
-    return gemm(dy, x, a_mn=True, b_mn=True, out=out, accumulate=accumulate, out_dtype=out_dtype)
+    return gemm(dy, x, a_mn=True, b_mn=True, out=out, accumulate=accumulate, out_dtype=out_dtype, split_k=split_k)
 
 
 # ------------------------------------------------------------------------------------------------ RMSNorm
@@ -158,21 +159,21 @@ def rmsnorm_bwd(dy: torch.Tensor, h: torch.Tensor, w: torch.Tensor, rstd: torch.
 
 
 def linear_rope_fwd(x: torch.Tensor, w: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
-                    n_heads: int, head_dim: int) -> torch.Tensor:
+                    n_heads: int, head_dim: int, split_k: bool = False) -> torch.Tensor:
     """qkv[T, N] = x w^T with the rotary embedding applied to the first ``n_heads`` heads of every row. On the GPU one
-    launch when the shape allows (bf16, head_dim 64 or 128, N a multiple of 128, a few hundred rows): the rotation sits
-    in the GEMM's epilogue. Same values as ``linear_fwd`` followed by ``rope_``."""
+    launch when the shape allows (bf16, head_dim 64 or 128, N a multiple of 128): the rotation sits in the
+    GEMM's epilogue. Same values as ``linear_fwd`` followed by ``rope_``."""
     T, N = x.shape[0], w.shape[0]
-    if (_native(x, w) and x.dtype == _BF16 and w.dtype == _BF16 and head_dim in (64, 128) and N % 128 == 0 and T >= 512
+    if (_native(x, w) and x.dtype == _BF16 and w.dtype == _BF16 and head_dim in (64, 128) and N % 128 == 0
             and x.stride(-1) == 1 and w.stride(-1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
             and pos.dtype == torch.int32 and cos.dtype == torch.float32 and cos.shape[1] == head_dim // 2
             and cos.is_contiguous() and sin.is_contiguous()):
         out = torch.empty((T, N), dtype=x.dtype, device=x.device)
         _lib.check(_lib.kernels().b200_gemm_rope(_lib.ptr(x), _lib.ptr(w), _lib.ptr(out), _lib.ptr(pos), _lib.ptr(cos),
                                                  _lib.ptr(sin), T, N, x.shape[1], n_heads, head_dim, x.stride(0),
-                                                 w.stride(0), out.stride(0), _lib.stream()), "b200_gemm_rope")
+                                                 w.stride(0), out.stride(0), int(split_k), _lib.stream()), "b200_gemm_rope")
         return out
-    return rope_(linear_fwd(x, w), pos, cos, sin, n_heads, head_dim)
+    return rope_(linear_fwd(x, w, split_k=split_k), pos, cos, sin, n_heads, head_dim)
 
 
 # ------------------------------------------------------------------------------------------------ per-head q/k norm
@@ -394,15 +395,15 @@ def swiglu_fwd(gu: torch.Tensor) -> torch.Tensor:
 def swiglu_fusable(x: torch.Tensor, w_gu: torch.Tensor) -> bool:
     """Whether ``linear_swiglu_fwd`` runs as one launch for these operands."""
     f = w_gu.shape[0] // 2
-    return bool(_native(x, w_gu) and x.dtype == _BF16 and w_gu.dtype == _BF16 and f % 128 == 0 and x.shape[0] >= 512
+    return bool(_native(x, w_gu) and x.dtype == _BF16 and w_gu.dtype == _BF16 and f % 128 == 0
                 and x.stride(-1) == 1 and w_gu.stride(-1) == 1 and x.stride(0) % 8 == 0 and w_gu.stride(0) % 8 == 0)
 
 
 def linear_swiglu_fwd(x: torch.Tensor, w_gu: torch.Tensor, out_gu: torch.Tensor | None = None,
-                      out_act: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
+                      out_act: torch.Tensor | None = None, split_k: bool = False) -> tuple[torch.Tensor, torch.Tensor]:
     """(gu, act) with gu[T, 2f] = x w_gu^T (gate rows first, then up rows) and act[T, f] = silu(gate) * up. On the GPU
-    one launch does both when the shape allows (bf16, f a multiple of 128, at least a few hundred rows): the SwiGLU
-    sits in the epilogue of the gate / up GEMM. Same values as ``linear_fwd`` followed by ``swiglu_fwd``.
+    one launch does both when the shape allows (bf16, f a multiple of 128): the SwiGLU sits in the
+    epilogue of the gate / up GEMM. Same values as ``linear_fwd`` followed by ``swiglu_fwd``.
     ``out_gu`` / ``out_act`` (row slices of larger buffers are fine) receive the results when given."""
     T = x.shape[0]
     f = w_gu.shape[0] // 2
@@ -411,9 +412,9 @@ def linear_swiglu_fwd(x: torch.Tensor, w_gu: torch.Tensor, out_gu: torch.Tensor 
         act = out_act if out_act is not None else torch.empty((T, f), dtype=x.dtype, device=x.device)
         _lib.check(_lib.kernels().b200_gemm_swiglu(_lib.ptr(x), _lib.ptr(w_gu), _lib.ptr(gu), _lib.ptr(act), T, f,
                                                    x.shape[1], x.stride(0), w_gu.stride(0), gu.stride(0), act.stride(0),
-                                                   _lib.stream()), "b200_gemm_swiglu")
+                                                   int(split_k), _lib.stream()), "b200_gemm_swiglu")
         return gu, act
-    gu = gemm(x, w_gu, out=out_gu) if out_gu is not None else linear_fwd(x, w_gu)
+    gu = gemm(x, w_gu, out=out_gu, split_k=split_k)
     act = swiglu_fwd(gu)
     if out_act is not None:
         out_act.copy_(act)
@@ -425,12 +426,12 @@ def swiglu_bwd_fusable(dy: torch.Tensor, w_d: torch.Tensor, gu: torch.Tensor) ->
     """Whether ``linear_dgrad_swiglu_bwd`` runs as one launch for these operands."""
     f = w_d.shape[1]
     return bool(_native(dy, w_d, gu) and dy.dtype == _BF16 and w_d.dtype == _BF16 and gu.dtype == _BF16 and f % 128 == 0
-                and dy.shape[0] >= 512 and dy.stride(-1) == 1 and w_d.stride(-1) == 1 and gu.stride(-1) == 1
+                and dy.stride(-1) == 1 and w_d.stride(-1) == 1 and gu.stride(-1) == 1
                 and dy.stride(0) % 8 == 0 and w_d.stride(0) % 8 == 0 and gu.stride(0) % 8 == 0)
 
 
 def linear_dgrad_swiglu_bwd(dy: torch.Tensor, w_d: torch.Tensor, gu: torch.Tensor,
-                            out: torch.Tensor | None = None) -> torch.Tensor:
+                            out: torch.Tensor | None = None, split_k: bool = False) -> torch.Tensor:
     """dgu[T, 2f] = SwiGLU backward of (gu, dact) with dact = dy[T, h] w_d[h, f] - the gradient through the down
     projection and the activation. On the GPU one launch when the shape allows: the dgrad GEMM's epilogue reads gate /
     up, rounds its accumulator to bf16 and writes d(gate), d(up); dact is never stored. Same values as
@@ -441,9 +442,9 @@ def linear_dgrad_swiglu_bwd(dy: torch.Tensor, w_d: torch.Tensor, gu: torch.Tenso
         dgu = out if out is not None else torch.empty((T, 2 * f), dtype=gu.dtype, device=gu.device)
         _lib.check(_lib.kernels().b200_gemm_swiglu_bwd(_lib.ptr(dy), _lib.ptr(w_d), _lib.ptr(gu), _lib.ptr(dgu), T, f,
                                                        dy.shape[1], dy.stride(0), w_d.stride(0), gu.stride(0),
-                                                       dgu.stride(0), _lib.stream()), "b200_gemm_swiglu_bwd")
+                                                       dgu.stride(0), int(split_k), _lib.stream()), "b200_gemm_swiglu_bwd")
         return dgu
-    dgu = swiglu_bwd(gu, linear_dgrad(dy, w_d))
+    dgu = swiglu_bwd(gu, linear_dgrad(dy, w_d, split_k))
     if out is not None:
         out.copy_(dgu)
         return out

@@ -150,3 +150,69 @@ def test_qkv_gemm_with_rotary_embedding_in_the_epilogue(T, H, Hkv, d, K):
     assert torch.equal(got, ref)
     assert torch.equal(got[:, (H + Hkv) * d:], plain[:, (H + Hkv) * d:])
     assert not torch.equal(got[:, : H * d], plain[:, : H * d])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (93, 2048, 5632), (128, 128, 512), (129, 72, 200), (300, 1152, 896),
+                                   (257, 896, 1024), (896, 256, 776)])
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+def test_few_tiles_split_over_a_cluster(M, N, K, layout):
+    """Outputs of few tiles: K is cut over the CTAs of a cluster and the partial tiles are added in slice order. Every
+    store form against fp64, nothing outside the output, and the same bits twice. Bound: operands are exact bf16, the
+    fp32 sums err by about sqrt(K) 2^-24 of the sum of |products| / sqrt(K), far below the 2^-9 of the bf16 store."""
+    a_mn, b_mn = layout == "tn", layout != "nt"
+    if a_mn and M % 8:
+        pytest.skip("row strides are multiples of 8 elements")
+    torch.manual_seed(M + N + K)
+    a = torch.randn((K, M) if a_mn else (M, K), device=DEV).bfloat16()
+    b = (torch.randn((K, N) if b_mn else (N, K), device=DEV) * 0.1).bfloat16()
+    kw = dict(a_mn=a_mn, b_mn=b_mn, split_k=True)
+    ref = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double()
+    scale = ref.abs().max().item()
+    guard = torch.full((M + 2, N + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    out = guard[1:-1, :N]
+    basic.gemm(a, b, out=out, **kw)
+    assert _lib.take_device_error() == 0
+    assert (guard[0] == 7).all() and (guard[-1] == 7).all() and (guard[1:-1, N:] == 7).all()
+    assert (out.double() - ref).abs().max().item() <= 2 ** -8 * scale
+    assert torch.equal(out, basic.gemm(a, b, **kw))
+    res = torch.randn(M, N, device=DEV).bfloat16()
+    got = basic.gemm(a, b, residual=res, alpha=0.5, **kw)
+    want = 0.5 * ref + res.double()
+    assert (got.double() - want).abs().max().item() <= 2 ** -8 * want.abs().max().item()
+    acc = torch.randn(M, N, device=DEV)
+    want = acc.double() + ref
+    basic.gemm(a, b, out=acc, accumulate=True, **kw)
+    assert (acc.double() - want).abs().max().item() <= 1e-5 * (want.abs().max().item() + K ** 0.5)
+
+
+@pytest.mark.parametrize("T", [1, 31, 130, 511, 777])
+def test_one_slice_keeps_the_order_of_the_large_tiles(T):
+    """Without ``split_k`` a row's result has the same bits whichever kernel its batch size picks."""
+    torch.manual_seed(T)
+    a = torch.randn(4096, 1400, device=DEV).bfloat16()
+    b = (torch.randn(896, 1400, device=DEV) * 0.1).bfloat16()
+    assert torch.equal(basic.gemm(a[:T], b), basic.gemm(a, b)[:T])
+    assert torch.equal(basic.gemm(a[:T], b, out_dtype=torch.float32), basic.gemm(a, b, out_dtype=torch.float32)[:T])
+
+
+@pytest.mark.parametrize("T", [1, 31, 130, 511, 777])
+@pytest.mark.parametrize("split", [False, True])
+def test_fused_epilogues_on_few_rows(T, split):
+    """The projections with rotary embedding and SwiGLU (forward and backward) in the cluster kernel's epilogue: the
+    bits of GEMM + separate kernel, for heads of 64 and 128 and for row counts off the tile."""
+    torch.manual_seed(T)
+    K, f = 896, 1408
+    x = torch.randn(T, K, device=DEV).bfloat16()
+    w = (torch.randn(2 * f, K, device=DEV) * 0.05).bfloat16()
+    gu, act = basic.linear_swiglu_fwd(x, w, split_k=split)
+    assert torch.equal(gu, basic.linear_fwd(x, w, split_k=split)) and torch.equal(act, basic.swiglu_fwd(gu))
+    wd = (torch.randn(K, f, device=DEV) * 0.05).bfloat16()
+    dact = basic.linear_dgrad(x, wd, split)
+    assert torch.equal(basic.linear_dgrad_swiglu_bwd(x, wd, gu, split_k=split), basic.swiglu_bwd(gu, dact))
+    for H, Hkv, d in ((14, 2, 64), (6, 1, 128)):
+        wq = (torch.randn((H + 2 * Hkv) * d, K, device=DEV) * 0.05).bfloat16()
+        pos = (torch.arange(T, device=DEV, dtype=torch.int32) * 5) % 300
+        cos, sin = basic.rope_tables(300, d, 10000.0, DEV)
+        got = basic.linear_rope_fwd(x, wq, pos, cos, sin, H + Hkv, d, split_k=split)
+        assert torch.equal(got, basic.rope_(basic.linear_fwd(x, wq, split_k=split), pos, cos, sin, H + Hkv, d))
+    assert _lib.take_device_error() == 0
