@@ -453,9 +453,12 @@ class LlamaModel(nn.Module):
         meta = (B, L, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, cfg.rms_norm_eps,
                 bool(self.grad_checkpointing and torch.is_grad_enabled()))
         rmul = float(cfg.residual_multiplier)
-        split = (not torch.is_grad_enabled(), not self.ordered_sums)
+        training = torch.is_grad_enabled()
+        split = (not training, not self.ordered_sums)
+        plain = not (cfg.qk_norm or cfg.o_bias or cfg.mlp_bias) and rmul == 1.0
         tables = self.layer_rope(cos, sin)
         meta7 = meta
+        from . import layer_native
         for li, (layer, (cos, sin)) in enumerate(zip(self.layers, tables)):
             meta = meta7 + (cfg.layer_window(li, L),)       # the layer's sliding window when the sequence is longer
             if pre is not None:
@@ -484,6 +487,13 @@ class LlamaModel(nn.Module):
                                      getattr(layer, "shared_down_proj", None),
                                      getattr(layer, "shared_expert_gate", None))
                 continue
+            if plain:
+                b_qkv = getattr(layer, "qkv_bias", None)
+                w = (layer.input_layernorm, layer.qkv_proj, layer.o_proj, layer.post_attention_layernorm, layer.gate_up_proj,
+                     layer.down_proj)
+                if layer_native.fits(h, pos, cos, w, b_qkv, cfg.head_dim, training):
+                    h = layer_native.NativeLayerFn.apply(h, pos, cos, sin, *w, b_qkv, meta, split)
+                    continue
             h = DecoderLayerFn.apply(h, pos, cos, sin, layer.input_layernorm, layer.qkv_proj, layer.o_proj,
                                      layer.post_attention_layernorm, layer.gate_up_proj, layer.down_proj, meta,
                                      getattr(layer, "qkv_bias", None), getattr(layer, "q_norm", None),

@@ -71,6 +71,8 @@ KERNELS_PER_CALL = {"b200_rmsnorm_bwd": 2, "b200_flash_attn_bwd": 3, "b200_flash
                     "b200_rmsnorm_bwd_blocks": 0, "b200_last_cuda_error": 0, "b200_take_device_error": 0,
                     "b200_gemm_reset_split_sync": 0, "b200_headnorm_bwd_blocks": 0, "b200_headnorm_bwd": 2}
 LAUNCH_COUNT = [0]
+# launchers that return something else than an int status
+RESTYPES: dict = {}
 
 
 class _CountingLib:
@@ -110,7 +112,7 @@ def kernels():
             except AttributeError:
                 continue
             fn.argtypes = args
-            fn.restype = c_int
+            fn.restype = RESTYPES.get(name, c_int)
         _KERNELS = _CountingLib(lib)
     return _KERNELS
 
@@ -124,7 +126,7 @@ def register(name: str, argtypes: list) -> None:
         except AttributeError:  # declared by Python but not built into the library yet: calling it will raise
             return
         fn.argtypes = argtypes
-        fn.restype = c_int
+        fn.restype = RESTYPES.get(name, c_int)
 
 
 def host() -> ctypes.CDLL:
