@@ -16,8 +16,12 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
-from ..ops import attention, basic
+from ..ops import _lib, attention, basic
+from ..ops._lib import _F, _I, _LL, _VP
 from . import llama as _ll
+
+_lib.register("b200_expert_sort", [_VP, _LL, _I, _I, _VP, _VP, _VP, _VP, _VP])
+_lib.register("b200_moe_combine", [_VP, _VP, _VP, _VP, _VP, _LL, _I, _I, _F, _VP])
 
 
 # ------------------------------------------------------------------------------------------------ routing
@@ -32,14 +36,36 @@ def route(n2: torch.Tensor, w_router: torch.Tensor, k: int, renorm: bool = True)
 
 
 def permutation(top_e: torch.Tensor, n_experts: int):
-    """(order, inverse, counts): ``order`` lists the T*k (token, choice) pairs sorted by expert (stable, so tokens keep
-    their order inside an expert's slab), ``inverse`` undoes it, ``counts`` are the slab lengths as Python ints."""
+    """(order, inverse, token, counts): ``order`` lists the T*k (token, choice) pairs sorted by expert (stable, so tokens
+    keep their order inside an expert's slab), ``inverse`` undoes it, ``token`` is the token of each sorted pair,
+    ``counts`` are the slab lengths as Python ints. One kernel on a GPU for up to 32 experts (csrc/ops/moe.cu)."""
     flat = top_e.reshape(-1)
+    k = top_e.shape[1]
+    if flat.is_cuda and flat.is_contiguous() and n_experts <= 32 and flat.numel():
+        order, inverse, token = (torch.empty_like(flat) for _ in range(3))
+        counts = torch.empty(n_experts, dtype=torch.int64, device=flat.device)
+        _lib.check(_lib.kernels().b200_expert_sort(_lib.ptr(flat), flat.numel(), n_experts, k, _lib.ptr(order),
+                                                   _lib.ptr(inverse), _lib.ptr(token), _lib.ptr(counts), _lib.stream()),
+                   "b200_expert_sort")
+        return order, inverse, token, counts.tolist()
     order = torch.argsort(flat, stable=True)
     inverse = torch.empty_like(order)
     inverse[order] = torch.arange(order.numel(), device=order.device)
     counts = torch.bincount(flat, minlength=n_experts).tolist()
-    return order, inverse, counts
+    return order, inverse, torch.div(order, k, rounding_mode="floor"), counts
+
+
+def combine(y: torch.Tensor, inverse: torch.Tensor, top_w: torch.Tensor, h1: torch.Tensor | None, rmul: float = 1.0):
+    """(h1 +) rmul * sum_k weight * y of each token in y's dtype, or None where the kernel does not apply."""
+    T, k = top_w.shape
+    h = y.shape[1]
+    if not (y.is_cuda and y.dtype == torch.bfloat16 and h % 8 == 0 and y.is_contiguous() and T
+            and top_w.dtype == torch.float32 and (h1 is None or (h1.dtype == y.dtype and h1.is_contiguous()))):
+        return None
+    out = torch.empty((T, h), dtype=y.dtype, device=y.device)
+    _lib.check(_lib.kernels().b200_moe_combine(_lib.ptr(y), _lib.ptr(inverse), _lib.ptr(top_w.contiguous()), _lib.ptr(h1),
+                                               _lib.ptr(out), T, k, h, float(rmul), _lib.stream()), "b200_moe_combine")
+    return out
 
 
 def experts_forward(x_perm: torch.Tensor, counts: list[int], w_gu: torch.Tensor, w_d: torch.Tensor):
@@ -90,9 +116,12 @@ def moe_mlp(n2: torch.Tensor, w_router: torch.Tensor, w_gu: torch.Tensor, w_d: t
     down matrix, gate vector) of a shared expert, or None."""
     T, h = n2.shape
     _, top_e, top_w = route(n2, w_router, k, renorm)
-    order, inverse, counts = permutation(top_e, w_gu.shape[0])
-    x_perm = n2.index_select(0, torch.div(order, k, rounding_mode="floor"))
-    _, _, y = experts_forward(x_perm, counts, w_gu, w_d)
+    _, inverse, tok, counts = permutation(top_e, w_gu.shape[0])
+    _, _, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d)
+    if shared is None:
+        out = combine(y, inverse, top_w, None)
+        if out is not None:
+            return out
     y_tok = y.index_select(0, inverse).view(T, k, h)
     out = (y_tok.float() * top_w.unsqueeze(-1)).sum(1)
     if shared is not None:
@@ -110,7 +139,8 @@ class AttnBlockFn(torch.autograd.Function):
         B, L, H, Hkv, d, eps, recompute, window = meta
         ctx.rmul = rmul          # Granite's residual multiplier: the branch is scaled before it joins the stream
         n1, _, rstd1 = basic.rmsnorm_fwd(h, w_ln1, eps)
-        qkv = basic.linear_fwd(n1, w_qkv)
+        plain = b_qkv is None and w_qn is None               # rotation in the epilogue of the q/k/v GEMM
+        qkv = basic.linear_rope_fwd(n1, w_qkv, pos, cos, sin, H + Hkv, d) if plain else basic.linear_fwd(n1, w_qkv)
         if b_qkv is not None:
             basic.bias_add_(qkv, b_qkv)
         qk_saved = ()
@@ -121,7 +151,8 @@ class AttnBlockFn(torch.autograd.Function):
             qkv_raw = qkv
             qkv, rstd_qk = basic.headnorm_fwd(qkv_raw, w_qn, w_kn, H, Hkv, d, eps)
             qk_saved = (qkv_raw, rstd_qk)
-        basic.rope_(qkv, pos, cos, sin, H + Hkv, d)
+        if not plain:
+            basic.rope_(qkv, pos, cos, sin, H + Hkv, d)
         att, lse = attention.attention_fwd(qkv, B, L, H, Hkv, d, window)
         h1 = basic.gemm(att, w_o, residual=h, alpha=rmul)
         ctx.meta = meta
@@ -224,18 +255,18 @@ class MoEBlockFn(torch.autograd.Function):
         T, hdim = h1.shape
         n2, _, rstd2 = basic.rmsnorm_fwd(h1, w_ln2, eps)
         probs, top_e, top_w = route(n2, w_router, k, renorm)
-        order, inverse, counts = permutation(top_e, w_gu.shape[0])
-        tok = torch.div(order, k, rounding_mode="floor")
-        x_perm = n2.index_select(0, tok)
-        gu, act, y = experts_forward(x_perm, counts, w_gu, w_d)
-        y_tok = y.index_select(0, inverse).view(T, k, hdim)
-        branch = (y_tok.float() * top_w.unsqueeze(-1)).sum(1)
+        order, inverse, tok, counts = permutation(top_e, w_gu.shape[0])
+        gu, act, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d)
         shared_saved = ()
-        if w_sgu is not None:
-            gu_s, act_s, y_s, gate = shared_expert_forward(n2, w_sgu, w_sd, w_sg)
-            branch = branch + gate * y_s.float()
-            shared_saved = (gu_s, act_s, y_s, gate)
-        h2 = (h1.float() + (branch if rmul == 1.0 else branch * rmul)).to(h1.dtype)
+        h2 = combine(y, inverse, top_w, h1, rmul) if w_sgu is None else None
+        if h2 is None:
+            y_tok = y.index_select(0, inverse).view(T, k, hdim)
+            branch = (y_tok.float() * top_w.unsqueeze(-1)).sum(1)
+            if w_sgu is not None:
+                gu_s, act_s, y_s, gate = shared_expert_forward(n2, w_sgu, w_sd, w_sg)
+                branch = branch + gate * y_s.float()
+                shared_saved = (gu_s, act_s, y_s, gate)
+            h2 = (h1.float() + (branch if rmul == 1.0 else branch * rmul)).to(h1.dtype)
         ctx.meta = meta
         ctx.counts = counts
         ctx.weights = (w_ln2, w_router, w_gu, w_d)

@@ -1,0 +1,37 @@
+"""Expert sort and weighted combination against their PyTorch restatements."""
+import pytest
+import torch
+
+from llm_distillery_b200.models import moe
+from llm_distillery_b200.ops import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,k,E", [(1, 1, 1), (1, 2, 8), (511, 2, 8), (6124, 2, 8), (1025, 8, 32), (3000, 4, 33)])
+def test_expert_sort_is_the_stable_sort(T, k, E):
+    g = torch.Generator("cuda").manual_seed(T)
+    top_e = (torch.rand(T, k, device="cuda", generator=g) ** 2 * E).long().clamp_(max=E - 1)     # uneven, some empty
+    order, inverse, token, counts = moe.permutation(top_e, E)
+    flat = top_e.reshape(-1)
+    want = torch.argsort(flat, stable=True)
+    assert torch.equal(order, want) and torch.equal(token, want // k)
+    assert torch.equal(order[inverse], torch.arange(T * k, device="cuda"))
+    assert counts == torch.bincount(flat, minlength=E).tolist()
+
+
+@pytest.mark.parametrize("T,k,h,resid,rmul", [(1, 1, 8, True, 1.0), (257, 2, 2048, True, 1.0), (33, 8, 264, False, 1.0),
+                                              (100, 4, 512, True, 0.25)])
+def test_combine_matches_the_gathered_sum(T, k, h, resid, rmul):
+    g = torch.Generator("cuda").manual_seed(T + h)
+    y = torch.randn(T * k, h, device="cuda", generator=g).bfloat16()
+    inverse = torch.randperm(T * k, device="cuda", generator=g)
+    w = torch.rand(T, k, device="cuda", generator=g)
+    h1 = torch.randn(T, h, device="cuda", generator=g).bfloat16() if resid else None
+    got = moe.combine(y, inverse, w, h1, rmul)
+    want = (y[inverse].view(T, k, h).double() * w.double().unsqueeze(-1)).sum(1) * rmul
+    if resid:
+        want = want + h1.double()
+    # fp32 sums of at most 9 terms, then one rounding to bf16 (2^-9 of the value)
+    assert ((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5).all()
+    assert _lib.take_device_error() == 0
