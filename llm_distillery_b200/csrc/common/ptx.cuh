@@ -210,6 +210,22 @@ __device__ __forceinline__ void tma_store_wait_read0() {
 }
 __device__ __forceinline__ void tma_store_wait_all0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// ---------------------------------------------------------------- one thread of a converged warp
+// The warps that issue tcgen05 instructions run their loops - waits, counters, descriptors - with all 32 lanes and let one
+// elected lane issue: the operands are then warp-uniform values. In a loop that only lane 0 runs they are not, and each
+// instruction paid for moving them (a K block of 64 in the few-tile GEMM: 0.30 us, elected 0.25 us).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
 // ---------------------------------------------------------------- tcgen05 / TMEM
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),

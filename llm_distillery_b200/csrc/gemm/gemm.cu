@@ -908,10 +908,10 @@ struct ClusterSwigluBwd {
 
 // N: columns of B's output space covered by tiles of BN (2 f for the gate / up projection, whose tiles take BN/2 gate and
 // BN/2 up rows: f = b_half > 0).
-template <int BN, bool A_MN, bool B_MN, class Epi>
+template <int BN, bool DEEP, bool A_MN, bool B_MN, class Epi>
 static int launch_cluster(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int fmt,
                           const typename Epi::Params& ep, int slices, int b_half, cudaStream_t stream) {
-  using S = SmemCluster<BN>;
+  using S = SmemCluster<BN, DEEP>;
   CUtensorMap tmA, tmB;
   const CUtensorMapDataType dt = fmt == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   int rc;
@@ -926,7 +926,7 @@ static int launch_cluster(const void* A, const void* B, int M, int N, int K, lon
   else
     rc = make_tmap_2d(&tmB, B, dt, 2, (uint64_t)N, (uint64_t)K, (uint64_t)ldb * 2, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != B200_OK) return rc;
-  auto kern = gemm_cluster_kernel<BN, A_MN, B_MN, Epi>;
+  auto kern = gemm_cluster_kernel<BN, DEEP, A_MN, B_MN, Epi>;
   static bool attr_set = false;
   if (!attr_set) {
     B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES));
@@ -965,18 +965,24 @@ static bool use_pair(int M, int N, int K) {
 // cross-entropies, and turned a last bit of an activation into 0.1 to 0.7 % of its value (38 runs of five students, 200
 // to 1100 tokens; the KL losses: 0.001 %), so that the loss of a conversation would depend on the batch that it is in.
 //
-// Times in microseconds, least squares over 137 sizes from 32 to 3000 tokens on layers of 256 to 28672 (B200, weights
-// from HBM; within 6 - 9 %): a cluster CTA costs a fixed part (launch, first loads, exchange, epilogue) and a part per K
+// Times in microseconds, least squares over sizes from 93 to 3000 tokens on layers of 256 to 14336 (B200, weights from
+// HBM; within 4 - 8 %): a cluster CTA costs a fixed part (launch, first loads, exchange, epilogue) and a part per K
 // block, more of both when two share an SM; the 256 x 256 kernel pays per round of its SM pairs. Clusters do not pack
 // onto the last SMs of the chip (294 CTAs in clusters of 3 or 6 ran as two rounds), so split tiles stop at 7/8 of the
 // resident CTAs. Examples, one CTA per tile before / cluster now: 93 x 2048 x 5632 37.8 / 11.0, 93 x 2560 x 2048 17.2 /
-// 7.4, 777 x 896 x 9728 59.3 / 21.4, 896 x 896 x 776 (weight gradient) 11.3 / 9.4; 2048 x 2048 x 2048 stays where it is
-// (17.7, cluster 20.2: tiles of 128 x 128 read twice the operand bytes per product and are bound by the L2).
+// 7.4, 777 x 896 x 9728 59.3 / 21.4 (43.4 in one slice), 896 x 896 x 776 (weight gradient) 11.3 / 7.7; 2048 x 2048 x 2048
+// stays where it is (17.7, cluster 20.2: tiles of 128 x 128 read twice the operand bytes per product and are bound by the L2).
 struct TilePlan { int bn, slices; };
+// A CTA may take the shared memory of two where the grid fits the SMs at one each; clusters only up to 3/4 of them (147
+// CTAs in clusters of 3 with an SM each ran as two rounds: 37.5 us, in shared SMs 30).
+static bool deep_ring(long long ctas, int slices) {
+  return ctas <= (slices > 1 ? sm_count() * 3 / 4 : sm_count());
+}
 static TilePlan plan_tiles(int M, int N, int K, bool f32, bool split) {
-  static const double kCost[2][2][4] = {   // [bn = 64, 128][one CTA per SM, two]: fixed, per K block, split, per slice
-      {{4.15, 0.301, 0.73, -0.045}, {4.67, 0.337, 0.92, 0.055}},
-      {{4.91, 0.377, 1.44, -0.124}, {6.19, 0.455, 1.14, 0.156}}};
+  // [bn = 64, 128][deep ring, one CTA per SM, two]: fixed, per K block, split, per slice
+  static const double kCost[2][3][4] = {
+      {{4.33, 0.256, 0.78, -0.081}, {4.73, 0.295, 0.0, 0.064}, {4.05, 0.331, 1.34, 0.134}},
+      {{6.04, 0.275, 1.20, -0.249}, {6.56, 0.396, 0.0, 0.055}, {6.05, 0.457, 0.89, 0.219}}};
   const int sms = sm_count(), num_kb = ceil_div(K, BK);
   const long long pair_tiles = (long long)ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
   TilePlan plan{0, 1};
@@ -992,7 +998,7 @@ static TilePlan plan_tiles(int M, int N, int K, bool f32, bool split) {
     for (int s = 1; s <= (split ? CLUSTER_MAX_SLICES : 1) && s <= num_kb; ++s) {
       const long long ctas = tiles * s;
       if (ctas > (s > 1 ? 2LL * sms * 7 / 8 : 2LL * sms)) break;
-      const double* c = kCost[w][ctas > sms];
+      const double* c = kCost[w][deep_ring(ctas, s) ? 0 : ctas > sms ? 2 : 1];
       const double us = c[0] + c[1] * ceil_div(num_kb, s) + (s > 1 ? c[2] : 0.0) + c[3] * s;
       if (us < least) { least = us; plan = TilePlan{bn, s}; }
     }
@@ -1003,8 +1009,13 @@ static TilePlan plan_tiles(int M, int N, int K, bool f32, bool split) {
 template <bool A_MN, bool B_MN, class Epi>
 static int launch_cluster_bn(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int fmt,
                              const typename Epi::Params& ep, TilePlan plan, int b_half, cudaStream_t stream) {
-  return plan.bn == 64 ? launch_cluster<64, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, plan.slices, b_half, stream)
-                       : launch_cluster<128, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, plan.slices, b_half, stream);
+  const bool deep = deep_ring((long long)ceil_div(M, BM) * ceil_div(N, plan.bn) * plan.slices, plan.slices);
+  const int s = plan.slices;
+  if (plan.bn == 64)
+    return deep ? launch_cluster<64, true, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, stream)
+                : launch_cluster<64, false, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, stream);
+  return deep ? launch_cluster<128, true, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, stream)
+              : launch_cluster<128, false, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, stream);
 }
 
 }  // namespace gemm

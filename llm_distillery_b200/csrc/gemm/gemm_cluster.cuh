@@ -19,9 +19,11 @@
 namespace b200 {
 namespace gemm {
 
-template <int BN>
+// A CTA's ring: 96 KB where two CTAs share an SM; twice that (DEEP) where the grid leaves each CTA an SM of its own, since
+// a single chain of K blocks runs at the latency of its loads over the blocks in flight.
+template <int BN, bool DEEP>
 struct SmemCluster {
-  static constexpr int STAGES = BN == 64 ? 4 : 3;       // 96 KB either way: two CTAs per SM
+  static constexpr int STAGES = (BN == 64 ? 4 : 3) * (DEEP ? 2 : 1);
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -47,11 +49,11 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
 // Epi concept: Params; SPLIT_B (the tile's B rows are BN/2 rows at n and BN/2 rows b_half_stride below them);
 // items<BN>() work items per row; item<BN>(p, row, n0, N, it, get) with get(chunk) = the four accumulator columns
 // 4 * chunk .. 4 * chunk + 3 of the row.
-template <int BN, bool A_MN, bool B_MN, class Epi>
-__global__ void __launch_bounds__(NUM_THREADS, 2)
+template <int BN, bool DEEP, bool A_MN, bool B_MN, class Epi>
+__global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
     gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
                         int K, int fmt, typename Epi::Params ep, unsigned int* err_word, int b_half_stride) {
-  using S = SmemCluster<BN>;
+  using S = SmemCluster<BN, DEEP>;
   constexpr int STAGES = S::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -123,19 +125,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc_f16(fmt, BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      constexpr DescCfg dc = default_desc_cfg<BN, A_MN, B_MN>();
-      bool ok = true;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const uint32_t it = kb - kb0, s = it % STAGES, ph = (it / STAGES) & 1u;
-        if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag, err_word, ERR_WAIT_FULL)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after_sync();
-        const uint32_t a_base = smem_u32(smem + s * S::STAGE_BYTES);
-        const uint32_t b_base = a_base + S::A_BYTES;
+    const uint32_t idesc = make_idesc_f16(fmt, BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    constexpr DescCfg dc = default_desc_cfg<BN, A_MN, B_MN>();
+    for (int kb = kb0; kb < kb1; ++kb) {
+      const uint32_t it = kb - kb0, s = it % STAGES, ph = (it / STAGES) & 1u;
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[s], ph, abort_flag, err_word, ERR_WAIT_FULL)))
+        break;
+      tc_fence_after_sync();
+      const uint32_t a_base = smem_u32(smem + s * S::STAGE_BYTES);
+      const uint32_t b_base = a_base + S::A_BYTES;
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k) {
           const uint64_t da = make_smem_desc_sw128(a_base + k * dc.a_kadv, dc.a_lbo, dc.a_sbo);
@@ -143,8 +142,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
           umma_f16_ss(tmem_base, da, db, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
         }
         umma_commit(&empty_bar[s]);
+        if (kb + 1 == kb1) umma_commit(done_bar);
       }
-      if (ok) umma_commit(done_bar);
+      __syncwarp();
     }
   } else {
     // accumulator -> shared memory. done_bar means every MMA has read its stage, so the ring is free.

@@ -158,7 +158,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
-    if (lane == 0 && cta == 0) {
+    if (cta == 0) {
       const uint32_t idesc = make_idesc_f16(fmt, PAIR_BM, PAIR_BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       constexpr uint32_t a_lbo = A_MN ? BK * 128 : 16, a_kadv = A_MN ? UMMA_K * 128 : UMMA_K * 2;
       constexpr uint32_t b_lbo = B_MN ? BK * 128 : 16, b_kadv = B_MN ? UMMA_K * 128 : UMMA_K * 2;
@@ -169,28 +169,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         unit_range(unit, tile, kb0, kb1);
         const uint32_t acc = tl & 1u;
         const uint32_t aph = (tl >> 1) & 1u;
-        if (!mbar_wait_bounded(&tempty_bar[acc], aph ^ 1u, abort_flag, err_word, ERR_WAIT_TMEM_EMPTY)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&tempty_bar[acc], aph ^ 1u, abort_flag, err_word, ERR_WAIT_TMEM_EMPTY)))
+          break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * PAIR_BN;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1u;
-          if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag, err_word, ERR_WAIT_FULL)) {
+          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[s], ph, abort_flag, err_word, ERR_WAIT_FULL))) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
           const uint32_t a_base = smem_u32(smem + s * S::STAGE_BYTES);
           const uint32_t b_base = a_base + S::A_BYTES;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t da = make_smem_desc_sw128(a_base + k * a_kadv, a_lbo, 1024);
-            const uint64_t db = make_smem_desc_sw128(b_base + k * b_kadv, b_lbo, 1024);
-            umma_f16_ss_pair(d_tmem, da, db, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              const uint64_t da = make_smem_desc_sw128(a_base + k * a_kadv, a_lbo, 1024);
+              const uint64_t db = make_smem_desc_sw128(b_base + k * b_kadv, b_lbo, 1024);
+              umma_f16_ss_pair(d_tmem, da, db, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+            }
+            umma_commit_pair(&empty_bar[s], 0x3);
+            if (kb + 1 == kb1) umma_commit_pair(&tfull_bar[acc], 0x3);
           }
-          umma_commit_pair(&empty_bar[s], 0x3);
+          __syncwarp();
         }
-        if (ok) umma_commit_pair(&tfull_bar[acc], 0x3);
       }
     }
   } else {

@@ -190,7 +190,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
   } else if (warp < FIRST_WORK_WARP) {
     // ------------------------------------------------------------------ MMA issuers (one elected thread per warp)
-    if (lane == 0) {
+    {
+      auto spin = [&](uint64_t* bar, uint32_t parity, unsigned int code) {
+        return __all_sync(0xffffffffu, mbar_spin_bounded(bar, parity, abort_flag, err_word, code)) != 0;
+      };
       const uint32_t sK = smem_u32(smem + C::OFF_K);
       const uint32_t sV = smem_u32(smem + C::OFF_V);
       const uint32_t sP = smem_u32(smem + C::OFF_P);
@@ -210,25 +213,28 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         const uint32_t idesc_kk = make_idesc_f16(1, BM, BN, 0, 0);
         const uint64_t kQ = make_smem_desc_sw128(sQ0, 16, 1024), kDO = make_smem_desc_sw128(sDO0, 16, 1024);
         const uint64_t kK = make_smem_desc_sw128(sK, 16, 1024), kV = make_smem_desc_sw128(sV, 16, 1024);
-        bool ok = mbar_spin_bounded(kv_full, 0, abort_flag, err_word, ERR_WAIT_FULL);
+        bool ok = spin(kv_full, 0, ERR_WAIT_FULL);
         for (int it = 0; ok && it < n_it; ++it) {
-          if (!mbar_spin_bounded(&qdo_full[it % ST], (it / ST) & 1u, abort_flag, err_word, ERR_WAIT_FULL)) break;
+          if (!spin(&qdo_full[it % ST], (it / ST) & 1u, ERR_WAIT_FULL)) break;
           if (it > 0) {
             if constexpr (C::PIPE) {
-              if (!mbar_spin_bounded(pds_ready, (it - 1) & 1u, abort_flag, err_word, ERR_WAIT_AUX)) break;
+              if (!spin(pds_ready, (it - 1) & 1u, ERR_WAIT_AUX)) break;
             } else {  // dQ shares its TMEM columns with S: they are free when the drain of pair it - 1 is through
-              if (!mbar_spin_bounded(dq_empty, (it - 1) & 1u, abort_flag, err_word, ERR_WAIT_AUX)) break;
+              if (!spin(dq_empty, (it - 1) & 1u, ERR_WAIT_AUX)) break;
             }
           }
           tc_fence_after_sync();
           const uint64_t stage = stage_off(it);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < D / 16; ++k)
-            umma_f16_ss(tmem_base + C::S_COL, kQ + stage + koff(k), kK + koff(k), idesc_kk, k != 0 ? 1u : 0u);
+            for (int k = 0; k < D / 16; ++k)
+              umma_f16_ss(tmem_base + C::S_COL, kQ + stage + koff(k), kK + koff(k), idesc_kk, k != 0 ? 1u : 0u);
 #pragma unroll
-          for (int k = 0; k < D / 16; ++k)
-            umma_f16_ss(tmem_base + C::DP_COL, kDO + stage + koff(k), kV + koff(k), idesc_kk, k != 0 ? 1u : 0u);
-          umma_commit(sdp_full);
+            for (int k = 0; k < D / 16; ++k)
+              umma_f16_ss(tmem_base + C::DP_COL, kDO + stage + koff(k), kV + koff(k), idesc_kk, k != 0 ? 1u : 0u);
+            umma_commit(sdp_full);
+          }
+          __syncwarp();
         }
       } else if (warp == 2 || warp == 3) {
         // dV += P^T dO (warp 2) ; dK += dS^T Q (warp 3): reduction over the 128 queries, 16 per step = 2048 B per step
@@ -238,42 +244,43 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         const uint64_t tB = make_smem_desc_sw128(warp == 2 ? sDO0 : sQ0, BM * 128, 1024);
         const uint32_t dcol = tmem_base + (warp == 2 ? C::DV_COL : C::DK_COL);
         for (int it = 0; it < n_it; ++it) {
-          if (!mbar_spin_bounded(pds_ready, it & 1u, abort_flag, err_word, ERR_WAIT_AUX)) break;
+          if (!spin(pds_ready, it & 1u, ERR_WAIT_AUX)) break;
           tc_fence_after_sync();
           const uint64_t stage = stage_off(it);
-          if (it == 0) {
+          if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < BM / 16; ++k)
-              umma_f16_ss(dcol, tA + (uint64_t)(k * 128), tB + stage + (uint64_t)(k * 128), idesc_tt, k != 0 ? 1u : 0u);
-          } else {
-#pragma unroll
-            for (int k = 0; k < BM / 16; ++k)
-              umma_f16_ss(dcol, tA + (uint64_t)(k * 128), tB + stage + (uint64_t)(k * 128), idesc_tt, 1u);
+              umma_f16_ss(dcol, tA + (uint64_t)(k * 128), tB + stage + (uint64_t)(k * 128), idesc_tt,
+                          (it != 0 || k != 0) ? 1u : 0u);
+            umma_commit(pair_bar(it));
           }
-          umma_commit(pair_bar(it));
+          __syncwarp();
         }
       } else {
         // dQ = dS K (reduction over the 128 keys; dS K-major, K MN-major) into the pair's accumulator
         const uint32_t idesc_kt = make_idesc_f16(1, BM, D, 0, 1);
         const uint64_t kDS = make_smem_desc_sw128(sDS, 16, 1024);
         const uint64_t tK = make_smem_desc_sw128(sK, BN * 128, 1024);
-        bool ok = mbar_spin_bounded(kv_full, 0, abort_flag, err_word, ERR_WAIT_FULL);
+        bool ok = spin(kv_full, 0, ERR_WAIT_FULL);
         for (int it = 0; ok && it < n_it; ++it) {
-          if (!mbar_spin_bounded(pds_ready, it & 1u, abort_flag, err_word, ERR_WAIT_AUX)) break;
+          if (!spin(pds_ready, it & 1u, ERR_WAIT_AUX)) break;
           uint32_t dq_col = C::DQ_COL;
           if constexpr (C::PIPE) {
             dq_col = (it & 1) ? C::DQ_COL1 : C::DQ_COL;
             if (it >= 2) {  // the drain of pair it-2 has emptied this accumulator
-              if (!mbar_spin_bounded((it & 1) ? dq_empty1 : dq_empty, ((it >> 1) - 1) & 1u, abort_flag, err_word,
+              if (!spin((it & 1) ? dq_empty1 : dq_empty, ((it >> 1) - 1) & 1u,
                                      ERR_WAIT_AUX))
                 break;
             }
           }
           tc_fence_after_sync();
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BN / 16; ++k)
-            umma_f16_ss(tmem_base + dq_col, kDS + koff(k), tK + (uint64_t)(k * 128), idesc_kt, k != 0 ? 1u : 0u);
-          umma_commit(pair_bar(it));
+            for (int k = 0; k < BN / 16; ++k)
+              umma_f16_ss(tmem_base + dq_col, kDS + koff(k), tK + (uint64_t)(k * 128), idesc_kt, k != 0 ? 1u : 0u);
+            umma_commit(pair_bar(it));
+          }
+          __syncwarp();
         }
       }
     }

@@ -193,38 +193,36 @@ __global__ void __launch_bounds__(NTHREADS, 2)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ O += P_j V_j
-    if (lane == 0) {
+    {
       const uint32_t idesc_o = make_idesc_f16(1, BM, D, 0, 1);
       // descriptors are constants plus a stage offset (the address field counts 16-byte units): built once
       uint64_t dV[BN / 16];
 #pragma unroll
       for (int k = 0; k < BN / 16; ++k)   // V is MN-major (D contiguous), 64-wide D chunks BN*128 bytes apart
         dV[k] = make_smem_desc_sw128(smem_u32(smem + C::OFF_V) + k * (16 * 128), BN * 128, 1024);
-      bool ok = true;
       for (int j = 0; j < n_kv; ++j) {
         const int bsel = j % NBUF, vs = j % VS;
         // P_j is in TMEM (over the first half of S_j) once the softmax warps have arrived
-        if (!mbar_spin_bounded(&p_ready[bsel], (j / NBUF) & 1u, abort_flag, err_word, ERR_WAIT_AUX)) { ok = false; break; }
-        if (!mbar_spin_bounded(&v_full[vs], (j / VS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_spin_bounded(&p_ready[bsel], (j / NBUF) & 1u, abort_flag, err_word, ERR_WAIT_AUX) &&
+                                         mbar_spin_bounded(&v_full[vs], (j / VS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)))
+          break;
         tc_fence_after_sync();
         const uint64_t stage = static_cast<uint64_t>((vs * C::T_BYTES) >> 4);
         const uint32_t pcol = tmem_base + C::S_COL + bsel * BN;   // bsel = j % NBUF
         // BN/16 k-steps over keys. A = P from TMEM (16 bf16 of a row = 8 columns per step)
-        if (j == 0) {
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < BN / 16; ++k)
-            umma_f16_ts(tmem_base + C::O_COL, pcol + k * 8, dV[k] + stage, idesc_o, k != 0 ? 1u : 0u);
-        } else {
-#pragma unroll
-          for (int k = 0; k < BN / 16; ++k) umma_f16_ts(tmem_base + C::O_COL, pcol + k * 8, dV[k] + stage, idesc_o, 1u);
+            umma_f16_ts(tmem_base + C::O_COL, pcol + k * 8, dV[k] + stage, idesc_o, (j != 0 || k != 0) ? 1u : 0u);
+          umma_commit(&pv_done[bsel]);
+          if (j + 1 == n_kv) umma_commit(o_final);   // a barrier of its own for the last tile: the epilogue waits on nothing else
         }
-        umma_commit(&pv_done[bsel]);
+        __syncwarp();
       }
-      if (ok) umma_commit(o_final);   // a barrier of its own for the last tile: the epilogue waits on nothing else
     }
   } else if (warp == 2) {
     // ------------------------------------------------------------------ S_t = Q K_t^T
-    if (lane == 0) {
+    {
       const uint32_t idesc_s = make_idesc_f16(1, BM, BN, 0, 0);
       uint64_t dQ[D / 16], dK[D / 16];
 #pragma unroll
@@ -233,20 +231,25 @@ __global__ void __launch_bounds__(NTHREADS, 2)
         dQ[k] = make_smem_desc_sw128(smem_u32(smem) + sub * (BM * 128) + kk * 32, 16, 1024);
         dK[k] = make_smem_desc_sw128(smem_u32(smem + C::OFF_K) + sub * (BN * 128) + kk * 32, 16, 1024);
       }
-      bool ok = mbar_spin_bounded(q_full, 0, abort_flag, err_word, ERR_WAIT_FULL);
+      const bool ok = __all_sync(0xffffffffu, mbar_spin_bounded(q_full, 0, abort_flag, err_word, ERR_WAIT_FULL));
       for (int t = 0; ok && t < n_kv; ++t) {
         const int ks = t % KS;
         // buffer t % NBUF held S_{t-NBUF} and then P_{t-NBUF}: it is free when that tile's P V has completed
-        if (t >= NBUF && !mbar_spin_bounded(&pv_done[t % NBUF], ((t - NBUF) / NBUF) & 1u, abort_flag, err_word, ERR_WAIT_AUX))
+        if (!__all_sync(0xffffffffu,
+                        (t < NBUF || mbar_spin_bounded(&pv_done[t % NBUF], ((t - NBUF) / NBUF) & 1u, abort_flag, err_word,
+                                                       ERR_WAIT_AUX)) &&
+                            mbar_spin_bounded(&k_full[ks], (t / KS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)))
           break;
-        if (!mbar_spin_bounded(&k_full[ks], (t / KS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)) break;
         tc_fence_after_sync();
         const uint64_t stage = static_cast<uint64_t>((ks * C::T_BYTES) >> 4);
         const uint32_t dcol = tmem_base + C::S_COL + (t % NBUF) * BN;
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) umma_f16_ss(dcol, dQ[k], dK[k] + stage, idesc_s, k != 0 ? 1u : 0u);
-        umma_commit(&s_full[t % NBUF]);
-        umma_commit(&k_empty[ks]);
+          for (int k = 0; k < D / 16; ++k) umma_f16_ss(dcol, dQ[k], dK[k] + stage, idesc_s, k != 0 ? 1u : 0u);
+          umma_commit(&s_full[t % NBUF]);
+          umma_commit(&k_empty[ks]);
+        }
+        __syncwarp();
       }
     }
   } else {
