@@ -12,13 +12,14 @@ namespace ew {
 constexpr int NT = 256;
 constexpr int MAX_VEC = 4;  // 16-byte vectors cached per thread: rows up to NT*MAX_VEC*8 = 8192 elements
 
+template <int NTB = NT>
 __device__ __forceinline__ float block_sum(float v, float* red) {
   v = warp_sum(v);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   __syncthreads();
   if (l == 0) red[w] = v;
   __syncthreads();
-  float t = (threadIdx.x < (NT / 32)) ? red[threadIdx.x] : 0.f;
+  float t = (threadIdx.x < (NTB / 32)) ? red[threadIdx.x] : 0.f;
   if (w == 0) {
     t = warp_sum(t);
     if (l == 0) red[0] = t;
@@ -46,23 +47,25 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 }
 
 // y = rmsnorm(x (+ res)) * w ; if res != null also writes h = x + res to `hout`. rstd[row] saved for backward.
-__global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
+// One block of NTB threads per row, NV vectors of 8 per thread (rows up to NV * NTB * 8 elements).
+template <int NV, int NTB>
+__global__ void __launch_bounds__(NTB) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                         const __nv_bfloat16* __restrict__ res,
                                                         const __nv_bfloat16* __restrict__ w,
                                                         __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ hout,
                                                         float* __restrict__ rstd, int rows, int h, float eps) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float red[NT / 32];
+  __shared__ float red[NTB / 32];
   const int nvec = h >> 3;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * h);
     const uint4* rr = res ? reinterpret_cast<const uint4*>(res + (size_t)row * h) : nullptr;
-    float vals[MAX_VEC][8];
+    float vals[NV][8];
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < MAX_VEC; ++i) {
-      const int v = threadIdx.x + i * NT;
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * NTB;
       if (v < nvec) {
         unpack8(xr[v], vals[i]);
         if (rr) {
@@ -81,12 +84,12 @@ __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __
         for (int j = 0; j < 8; ++j) ss += vals[i][j] * vals[i][j];
       }
     }
-    const float tot = block_sum(ss, red);
+    const float tot = block_sum<NTB>(ss, red);
     const float rs = rsqrtf(tot / (float)h + eps);
     if (threadIdx.x == 0 && rstd) rstd[row] = rs;
 #pragma unroll
-    for (int i = 0; i < MAX_VEC; ++i) {
-      const int v = threadIdx.x + i * NT;
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * NTB;
       if (v < nvec) {
         float w8[8], o[8];
         unpack8(reinterpret_cast<const uint4*>(w)[v], w8);
@@ -165,7 +168,10 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(const __nv_bfloat
 }
 
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres) ; dw partial sums per block in fp32.
-__global__ void __launch_bounds__(NT) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
+// NV and NTB as in the forward kernel: with arrays for the longest row (NV = 4) a thread held 170 registers and an SM one
+// block, 8000 rows of 4096 took 210 us; sized for the row (NV = 2) several blocks share it.
+template <int NV, int NTB>
+__global__ void __launch_bounds__(NTB) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                         const __nv_bfloat16* __restrict__ x,
                                                         const __nv_bfloat16* __restrict__ w,
                                                         const float* __restrict__ rstd,
@@ -174,24 +180,24 @@ __global__ void __launch_bounds__(NT) rmsnorm_bwd_kernel(const __nv_bfloat16* __
                                                         int rows, int h) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float red[NT / 32];
+  __shared__ float red[NTB / 32];
   const int nvec = h >> 3;
-  float dwacc[MAX_VEC][8];
-  float w8[MAX_VEC][8];
+  float dwacc[NV][8];
+  float w8[NV][8];
 #pragma unroll
-  for (int i = 0; i < MAX_VEC; ++i) {
-    const int v = threadIdx.x + i * NT;
+  for (int i = 0; i < NV; ++i) {
+    const int v = threadIdx.x + i * NTB;
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
     if (v < nvec) unpack8(reinterpret_cast<const uint4*>(w)[v], w8[i]);
   }
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const float rs = rstd[row];
-    float xh[MAX_VEC][8], g[MAX_VEC][8];
+    float xh[NV][8], g[NV][8];
     float dot = 0.f;
 #pragma unroll
-    for (int i = 0; i < MAX_VEC; ++i) {
-      const int v = threadIdx.x + i * NT;
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * NTB;
       if (v < nvec) {
         float d8[8];
         unpack8(reinterpret_cast<const uint4*>(x + (size_t)row * h)[v], xh[i]);
@@ -205,27 +211,30 @@ __global__ void __launch_bounds__(NT) rmsnorm_bwd_kernel(const __nv_bfloat16* __
         }
       }
     }
-    const float c = block_sum(dot, red) / (float)h;
+    const float c = block_sum<NTB>(dot, red) / (float)h;
 #pragma unroll
-    for (int i = 0; i < MAX_VEC; ++i) {
-      const int v = threadIdx.x + i * NT;
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * NTB;
       if (v < nvec) {
         float o[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rs * (g[i][j] - xh[i][j] * c);
-        if (dres) {
+        for (int j = 0; j < 8; ++j) o[j] = __fmaf_rn(-xh[i][j], c, g[i][j]);
+        if (dres) {         // fused multiply-adds by name: every instantiation rounds alike
           float r8[8];
           unpack8(reinterpret_cast<const uint4*>(dres + (size_t)row * h)[v], r8);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += r8[j];
+          for (int j = 0; j < 8; ++j) o[j] = __fmaf_rn(rs, o[j], r8[j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] *= rs;
         }
         reinterpret_cast<uint4*>(dx + (size_t)row * h)[v] = pack8(o);
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < MAX_VEC; ++i) {
-    const int v = threadIdx.x + i * NT;
+  for (int i = 0; i < NV; ++i) {
+    const int v = threadIdx.x + i * NTB;
     if (v < nvec) {
       float* p = dw_partial + (size_t)blockIdx.x * h + (size_t)v * 8;
       *reinterpret_cast<float4*>(p) = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
@@ -338,6 +347,9 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ p
   const int j = blockIdx.x * 32 + tx;
   float s = 0.f;
   if (j < h)
+    // loads of 16 rows in flight (the additions keep their order): one at a time the chain of a few hundred rows was
+    // all this kernel did
+#pragma unroll 16
     for (int b = ty; b < nblk; b += 8) s += partial[(size_t)b * h + j];
   red[ty][tx] = s;
   __syncthreads();
@@ -719,6 +731,17 @@ static inline int grid_for(long long work_items, int threads, int per_sm = 8) {
 }  // namespace ew
 }  // namespace b200
 
+// The block-per-row kernels in the size that holds a row of h elements (h <= NT * MAX_VEC * 8): half a block for rows
+// that half a block covers, else as many vectors per thread as the row needs. The sums do not depend on it.
+#define B200_RMS_BY_WIDTH(KERNEL, h, grid, st, ...)                                        \
+  do {                                                                                     \
+    if ((h) <= NT / 2 * 8) launch_pdl(KERNEL<1, NT / 2>, grid, NT / 2, 0, st, __VA_ARGS__); \
+    else if ((h) <= NT * 8) launch_pdl(KERNEL<1, NT>, grid, NT, 0, st, __VA_ARGS__);       \
+    else if ((h) <= NT * 16) launch_pdl(KERNEL<2, NT>, grid, NT, 0, st, __VA_ARGS__);      \
+    else if ((h) <= NT * 24) launch_pdl(KERNEL<3, NT>, grid, NT, 0, st, __VA_ARGS__);      \
+    else launch_pdl(KERNEL<MAX_VEC, NT>, grid, NT, 0, st, __VA_ARGS__);                    \
+  } while (0)
+
 extern "C" {
 using namespace b200;
 using namespace b200::ew;
@@ -743,8 +766,8 @@ int b200_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, voi
   else if (h == 512) B200_RMS_FWD_WARP(2);
   else if (h == 256) B200_RMS_FWD_WARP(1);
   else
-    launch_pdl(rmsnorm_fwd_kernel, grid, NT, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
-                                            (__nv_bfloat16*)y, (__nv_bfloat16*)hout, rstd, rows, h, eps);
+    B200_RMS_BY_WIDTH(rmsnorm_fwd_kernel, h, grid, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,
+                      (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)hout, rstd, rows, h, eps);
 #undef B200_RMS_FWD_WARP
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -765,8 +788,8 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
   else if (h == 512) B200_RMS_BWD_WARP(2);
   else if (h == 256) B200_RMS_BWD_WARP(1);
   else
-    launch_pdl(rmsnorm_bwd_kernel, grid, NT, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
-                                            rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, rows, h);
+    B200_RMS_BY_WIDTH(rmsnorm_bwd_kernel, h, grid, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
+                      (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, rows, h);
 #undef B200_RMS_BWD_WARP
   B200_CUDA_CHECK(cudaGetLastError());
   const bool warp_kernel = h == 2048 || h == 1024 || h == 512 || h == 256;    // one partial row per 4-warp CTA there
@@ -974,8 +997,8 @@ extern "C" int b200_rmsnorm_bwd_noalloc(const void* dy, const void* x, const voi
   const int grid = rows < B200_RMSNORM_NOALLOC_MAX_BLOCKS ? rows : B200_RMSNORM_NOALLOC_MAX_BLOCKS;
   // every block writes its own partial row (all h columns) before the column sum reads rows [0, grid):
   // nothing left over from an earlier call is ever read
-  launch_pdl(rmsnorm_bwd_kernel, grid, NT, 0, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
-                                          rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, h);
+  B200_RMS_BY_WIDTH(rmsnorm_bwd_kernel, h, grid, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
+                    (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, h);
   B200_CUDA_CHECK(cudaGetLastError());
   launch_pdl(colsum_kernel, ceil_div(h, 32), 256, 0, st, scratch, dw_out, grid, h, dw_accumulate);
   B200_CUDA_CHECK(cudaGetLastError());

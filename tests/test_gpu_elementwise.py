@@ -157,3 +157,21 @@ def test_per_head_qk_norm_fwd_bwd(T, H, Hkv, d):
     assert torch.allclose(dwq.cpu(), dwq_ref, atol=2e-2 * scale, rtol=2e-2)
     assert torch.allclose(dwk.cpu(), dwk_ref, atol=2e-2 * scale, rtol=2e-2)
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("h", [8, 1016, 1032, 2056, 4096, 4104, 6144, 6152, 8192])
+def test_rmsnorm_row_widths_of_the_block_kernels(h):
+    """Rows at the edges of the block-per-row sizes, forward and backward with a residual gradient, against fp32."""
+    torch.manual_seed(h)
+    rows = 37
+    x, dy, dres = (torch.randn(rows, h, device=DEV).bfloat16() for _ in range(3))
+    w = (1 + 0.1 * torch.randn(h, device=DEV)).bfloat16()
+    y, _, rstd = basic.rmsnorm_fwd(x, w, 1e-5)
+    dx, dw = basic.rmsnorm_bwd(dy, x, w, rstd, dres=dres)
+    xf, wf = x.float().requires_grad_(), w.float().requires_grad_()
+    ref = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-5) * wf
+    ref.backward(dy.float())
+    # one rounding to bf16 of values of a few units: 2^-9 relative
+    assert torch.allclose(y.float(), ref, atol=1e-4, rtol=2 ** -8)
+    assert torch.allclose(dx.float(), xf.grad + dres.float(), atol=1e-3, rtol=2 ** -7)
+    assert torch.allclose(dw, wf.grad, atol=1e-3 * rows ** 0.5, rtol=1e-4)
