@@ -16,13 +16,15 @@ does the same with this package's own storage and kernels:
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
 from ._lib import _VP, _LL, _I, _F
 
-_lib.register("b200_dequant_nf4", [_VP, _VP, _VP, _F, _VP, _LL, _VP])
-_lib.register("b200_dequant_int8", [_VP, _VP, _VP, _LL, _I, _VP])
+_lib.register("b200_dequant_nf4", [_VP, _VP, _VP, _VP, _VP, _VP, _I, _VP])
+_lib.register("b200_dequant_int8", [_VP, _VP, _VP, _VP, _VP, _I, _VP])
 
 NF4 = torch.tensor([-1.0, -0.6961928009986877, -0.5250730514526367, -0.39491748809814453, -0.28444138169288635,
                     -0.18477343022823334, -0.09105003625154495, 0.0, 0.07958029955625534, 0.16093020141124725,
@@ -76,18 +78,35 @@ def dequantize_reference(q: dict, dtype=torch.float32) -> torch.Tensor:
     return vals.to(dtype).reshape(q["shape"])
 
 
+def dequantize_all(qs: list[dict], outs: list[torch.Tensor]) -> None:
+    """Every out (compute dtype, its q's shape, contiguous) = dequantised weights; on CUDA one launch for up to four
+    matrices of one kind and bf16 outputs."""
+    if not all(o.is_cuda and o.dtype == torch.bfloat16 and q["kind"] == qs[0]["kind"] for q, o in zip(qs, outs)) or len(qs) > 4:
+        for q, o in zip(qs, outs):
+            dequantize_into(q, o)
+        return
+    n = len(qs)
+    ptrs = ctypes.c_void_p * n
+    out = ptrs(*[o.data_ptr() for o in outs])
+    lib = _lib.kernels()
+    if qs[0]["kind"] == "nf4":
+        arr = [ptrs(*[q[key].data_ptr() for q in qs]) for key in ("packed", "absmax_code", "absmax_scale")]
+        off = (ctypes.c_float * n)(*[float(q["offset"]) for q in qs])
+        counts = (ctypes.c_longlong * n)(*[o.numel() for o in outs])
+        _lib.check(lib.b200_dequant_nf4(*arr, off, out, counts, n, _lib.stream()), "b200_dequant_nf4")
+    else:
+        arr = [ptrs(*[q[key].data_ptr() for q in qs]) for key in ("code", "row_scale")]
+        rows = (ctypes.c_longlong * n)(*[o.shape[0] for o in outs])
+        cols = (ctypes.c_int * n)(*[o.shape[1] for o in outs])
+        _lib.check(lib.b200_dequant_int8(*arr, out, rows, cols, n, _lib.stream()), "b200_dequant_int8")
+
+
 def dequantize_into(q: dict, out: torch.Tensor) -> None:
     """out (compute dtype, q's shape, contiguous) = dequantised weights; a kernel on CUDA for bf16 outputs."""
     if out.is_cuda and out.dtype == torch.bfloat16:
-        lib = _lib.kernels()
-        if q["kind"] == "nf4":
-            _lib.check(lib.b200_dequant_nf4(_lib.ptr(q["packed"]), _lib.ptr(q["absmax_code"]), _lib.ptr(q["absmax_scale"]),
-                                            float(q["offset"]), _lib.ptr(out), out.numel(), _lib.stream()), "b200_dequant_nf4")
-        else:
-            _lib.check(lib.b200_dequant_int8(_lib.ptr(q["code"]), _lib.ptr(q["row_scale"]), _lib.ptr(out), out.shape[0],
-                                             out.shape[1], _lib.stream()), "b200_dequant_int8")
-        return
-    out.copy_(dequantize_reference(q, out.dtype))
+        dequantize_all([q], [out])
+    else:
+        out.copy_(dequantize_reference(q, out.dtype))
 
 
 def packed_bytes(q: dict) -> int:
@@ -126,9 +145,9 @@ class FrozenQuantLinears:
 
     def materialize(self, layer_index: int) -> None:
         layer = self.model.layers[layer_index]
+        packed = self.layers[layer_index]
         with torch.no_grad():
-            for n in LINEARS:
-                dequantize_into(self.layers[layer_index][n], getattr(layer, n).data)
+            dequantize_all([packed[n] for n in LINEARS], [getattr(layer, n).data for n in LINEARS])
 
     def before_layer(self, first_param) -> None:
         """Hook form of ``materialize``: called with the layer's first parameter before its forward / backward."""

@@ -90,3 +90,20 @@ def test_dequant_kernels_match_the_restatement_and_training_runs(kind):
     assert losses[2] < losses[0]
     from llm_distillery_b200.ops import _lib
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["nf4", "int8"])
+def test_matrices_of_a_layer_in_one_launch(kind):
+    """Up to four matrices of different sizes expand in one launch: each equals the restatement bit for bit, nothing is
+    written behind it."""
+    shapes = [(64, 64), (192, 320), (1, 64), (257, 128)]
+    quantize = quant.quantize_nf4 if kind == "nf4" else quant.quantize_int8
+    for n in (1, 3, 4):
+        g = torch.Generator("cuda").manual_seed(n)
+        qs = [quantize(torch.randn(*s, device="cuda", generator=g)) for s in shapes[:n]]
+        buf = [torch.full((s[0] * s[1] + 64,), 7.0, dtype=torch.bfloat16, device="cuda") for s in shapes[:n]]
+        outs = [b[:-64].view(s) for b, s in zip(buf, shapes)]
+        quant.dequantize_all(qs, outs)
+        for q, o, b in zip(qs, outs, buf):
+            assert torch.equal(o, quant.dequantize_reference(q, torch.float32).bfloat16()) and (b[-64:] == 7).all()
