@@ -4,7 +4,7 @@ What the reference does per batch (classes/teacher/inference_worker.py:66-85, re
 full forward, ``[:, :, :crop].float()``, log_softmax over the cropped vocabulary, ``torch.topk``, copy EVERYTHING to
 the host, then keep the content positions on the CPU. Here the content rows are gathered on the device before
 the LM head, so the vocabulary-sized work is done only for rows that are kept; logits exist only for one row
-chunk at a time (fp32, sized to stay L2-resident) between the tcgen05 GEMM and the exact top-K kernel; fp16
+chunk at a time (fp32; 96 MB, or 512 rows where that is more) between the tcgen05 GEMM and the exact top-K kernel; fp16
 log-probs + int32 ids go to pinned host memory on a copy stream, and the caller queues the next batch before it takes
 delivery of this one (``submit`` / ``fetch``).
 """
