@@ -20,6 +20,7 @@ from dataclasses import dataclass, field
 import torch
 
 from ..loss.head import distill_head_loss
+from ..models.llama import LlamaModel
 from ..ops import basic
 from .optim import FlatOptimizer, FlatParams
 from .schedule import LRSchedule
@@ -62,7 +63,6 @@ class DistillEngine:
                  jsd_renorm: bool = False, vocab_parallel: bool = False, max_rows_per_rank: int = 0):
         self.model = model
         self.loss_kind = loss
-        model.ordered_sums = loss == "reference"      # the one loss that turns a last bit into per mille of its value
         self.temperature = float(temperature)
         self.alpha = float(alpha)
         self.vocab = min(crop_to_size or model.cfg.vocab_size, model.cfg.vocab_size)
@@ -96,7 +96,12 @@ class DistillEngine:
 
     # ---- forward of one micro-batch: (sum over conversations of per-conversation loss, logs)
     def loss_on_batch(self, mb: HostBatch):
-        hs = self.model.hidden_states(mb.input_ids)
+        if isinstance(self.model, LlamaModel):
+            # one order of additions in the forward, so that training and validation see the same loss, and under the
+            # reference loss in the backward too: it is the one that turns a last bit into per mille of its value
+            hs = self.model.hidden_states(mb.input_ids, split_k=(False, self.loss_kind != "reference"))
+        else:
+            hs = self.model.hidden_states(mb.input_ids)
         Hc = hs if mb.rows is None else basic.GatherRowsFn.apply(hs, mb.rows)
         logp = mb.logp if mb.logp.dtype == torch.float32 else mb.logp.float()
         if self.vp_loss is not None:

@@ -359,7 +359,10 @@ class LlamaModel(nn.Module):
         else:
             self.lm_head = nn.Parameter(torch.empty(cfg.vocab_size, cfg.hidden_size, **kw))
         self.grad_checkpointing = False
-        self.ordered_sums = False  # backward GEMMs keep one order of additions whatever their size (see gemm.cu: plan_tiles)
+        # True: GEMMs add in one order whatever their size (gemm.cu: plan_tiles), so that the last bits of a conversation do
+        # not depend on the batch that it is in. False: GEMMs of few tiles may cut K. None, a new model: not chosen, as True;
+        # a TeacherCollector then chooses False, since it takes no loss of its forward
+        self.ordered_sums = None
         self._rope = None
         self.quant = None          # FrozenQuantLinears when the decoder layers' matrices are frozen NF4 / int8
 
@@ -436,8 +439,9 @@ class LlamaModel(nn.Module):
         return [(cos, sin) if flags[i] else ident for i in range(n)]
 
     # ---- forward
-    def hidden_states(self, input_ids: torch.Tensor) -> torch.Tensor:
-        """input_ids [B, L] int64 -> final-norm hidden states [B*L, h]."""
+    def hidden_states(self, input_ids: torch.Tensor, split_k: tuple[bool, bool] | None = None) -> torch.Tensor:
+        """input_ids [B, L] int64 -> final-norm hidden states [B*L, h]. ``split_k``: whether GEMMs of few tiles may cut K, in
+        the forward (without gradients only) and in the backward pass; None: as ``ordered_sums`` says."""
         cfg = self.cfg
         B, L = input_ids.shape
         dev = self.embed_tokens.device
@@ -454,7 +458,8 @@ class LlamaModel(nn.Module):
                 bool(self.grad_checkpointing and torch.is_grad_enabled()))
         rmul = float(cfg.residual_multiplier)
         training = torch.is_grad_enabled()
-        split = (not training, not self.ordered_sums)
+        fwd, bwd = split_k if split_k is not None else (self.ordered_sums is False,) * 2
+        split = (fwd and not training, bwd)
         plain = not (cfg.qk_norm or cfg.o_bias or cfg.mlp_bias) and rmul == 1.0
         tables = self.layer_rope(cos, sin)
         meta7 = meta
@@ -514,6 +519,7 @@ class LlamaModel(nn.Module):
         rotated keys and its values for all positions seen so far ([B, L, Hkv*d] each, zero-filled beyond), and the
         chunk's queries attend to positions <= their own. Same result as ``hidden_states`` up to rounding."""
         cfg = self.cfg
+        split = self.ordered_sums is False
         B, L = input_ids.shape
         if chunk_len <= 0 or chunk_len >= L:
             return self.hidden_states(input_ids)
@@ -549,9 +555,9 @@ class LlamaModel(nn.Module):
                     continue
                 n1, _, _ = basic.rmsnorm_fwd(h, layer.input_layernorm, cfg.rms_norm_eps)
                 if not hasattr(layer, "qkv_bias") and not cfg.qk_norm and not cfg.qk_norm_full:
-                    qkv = basic.linear_rope_fwd(n1, layer.qkv_proj, pos, cos, sin, H + Hkv, d, split_k=True)
+                    qkv = basic.linear_rope_fwd(n1, layer.qkv_proj, pos, cos, sin, H + Hkv, d, split_k=split)
                 else:
-                    qkv = basic.linear_fwd(n1, layer.qkv_proj, split_k=True)
+                    qkv = basic.linear_fwd(n1, layer.qkv_proj, split_k=split)
                     if hasattr(layer, "qkv_bias"):
                         basic.bias_add_(qkv, layer.qkv_bias)
                     if cfg.qk_norm_full:
@@ -564,7 +570,7 @@ class LlamaModel(nn.Module):
                 vc[:, c0:c0 + n] = qkv[:, (H + Hkv) * d:].reshape(B, n, kv)
                 att = attention.attention_fwd_cached(qkv, kc, vc, B, n, c0, H, Hkv, d, window)
                 rm = float(cfg.residual_multiplier)
-                h1 = basic.gemm(att, layer.o_proj, residual=h, alpha=rm, split_k=True)
+                h1 = basic.gemm(att, layer.o_proj, residual=h, alpha=rm, split_k=split)
                 if cfg.o_bias:
                     basic.bias_add_(h1, layer.o_bias if rm == 1.0 else layer.o_bias * rm)
                 n2, _, _ = basic.rmsnorm_fwd(h1, layer.post_attention_layernorm, cfg.rms_norm_eps)
@@ -581,8 +587,8 @@ class LlamaModel(nn.Module):
                     h = basic.bias_add_(basic.gemm(act, layer.down_proj, residual=h1, alpha=rm),
                                         layer.down_bias if rm == 1.0 else layer.down_bias * rm)
                     continue
-                _, act = basic.linear_swiglu_fwd(n2, layer.gate_up_proj, split_k=True)
-                h = basic.gemm(act, layer.down_proj, residual=h1, alpha=rm, split_k=True)
+                _, act = basic.linear_swiglu_fwd(n2, layer.gate_up_proj, split_k=split)
+                h = basic.gemm(act, layer.down_proj, residual=h1, alpha=rm, split_k=split)
             y, _, _ = basic.rmsnorm_fwd(h, self.norm, cfg.rms_norm_eps)
             if cfg.logits_scaling != 1.0:
                 y = y * (1.0 / cfg.logits_scaling)
