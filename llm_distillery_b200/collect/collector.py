@@ -4,7 +4,7 @@ What the reference does per batch (classes/teacher/inference_worker.py:66-85, re
 full forward, ``[:, :, :crop].float()``, log_softmax over the cropped vocabulary, ``torch.topk``, copy EVERYTHING to
 the host, then keep the content positions on the CPU. Here the content rows are gathered on the device before
 the LM head, so the vocabulary-sized work is done only for rows that are kept; logits exist only for one row
-chunk at a time (fp32; 96 MB, or 512 rows where that is more) between the tcgen05 GEMM and the exact top-K kernel; fp16
+chunk at a time (fp32; up to 128 MB, or 512 rows where that is more) between the tcgen05 GEMM and the exact top-K kernel; fp16
 log-probs + int32 ids go to pinned host memory on a copy stream, and the caller queues the next batch before it takes
 delivery of this one (``submit`` / ``fetch``).
 """
@@ -16,10 +16,13 @@ import torch
 from ..data.convo import ConvoTokenized, TeacherRows
 from ..ops import _lib, basic, topk as topk_ops
 
+DEFAULT_CHUNK_BYTES = (96 << 20, 128 << 20)
+
 
 class TeacherCollector:
-    def __init__(self, model, *, topk: int, crop_to_size: int, enable_topk: bool = True, logits_chunk_bytes: int = 96 << 20,
-                 prefill_chunk_len: int = 0):
+    def __init__(self, model, *, topk: int, crop_to_size: int, enable_topk: bool = True,
+                 logits_chunk_bytes: int | None = None, prefill_chunk_len: int = 0):
+        # logits_chunk_bytes: a bound on the logits of a chunk (128 rows are the least); None: ``rows_per_chunk`` decides
         self.model = model
         # > 0: sequences longer than this are run through the model in chunks of this many positions against a
         # key / value cache (LlamaModel.hidden_states_chunked); 0: one pass over the whole sequence
@@ -32,21 +35,22 @@ class TeacherCollector:
         # way (93 tokens of a 1.1 B model: 0.060 rms), the last bits of a row then depend on the rows of its batch
         if getattr(model, "ordered_sums", True) is None:
             model.ordered_sums = False
-        self.chunk_rows = self._rows_per_chunk(logits_chunk_bytes)
+        pairs = _lib.kernels().b200_sm_count() // 2 if self.device.type == "cuda" else 0
+        self.chunk_rows = self.rows_per_chunk(self.vocab, logits_chunk_bytes, pairs)
 
-    def _rows_per_chunk(self, chunk_bytes: int) -> int:
-        """Rows of logits that exist at a time. At least 512 unless the caller asks for less memory than the default: with
-        the 128 rows that 96 MB hold of a 128 k vocabulary, every chunk read the whole head for half a row of tiles and
+    @staticmethod
+    def rows_per_chunk(vocab: int, chunk_bytes: int | None, sm_pairs: int) -> int:
+        """Rows of fp32 logits that exist at a time. With ``chunk_bytes`` as many multiples of 128 as it holds, at least
+        128. Without: 96 - 128 MB of them, and at least 512 rows (263 MB of a 128 k vocabulary, 311 MB of 152 k): with the
+        128 rows that 96 MB hold of a 128 k vocabulary, every chunk read the whole head for half a row of tiles and
         the top-K kernel had fewer rows than SMs (0.39 ms per chunk, 64 of them in 8192 rows; a chunk of 512 takes about
-        0.6 ms). Between that and twice as many rows, the count whose 256 x 256 tiles waste least of their last round
-        over the SM pairs (32 k vocabulary: 1024 rows are 6.8 rounds run as 7, 768 rows 5.1 run as 6)."""
-        fit = chunk_bytes // (4 * self.vocab)
-        if self.device.type != "cuda" or chunk_bytes < (96 << 20):
-            return max(128, fit // 128 * 128)
-        pairs = max(1, _lib.kernels().b200_sm_count() // 2)
-        low = max(512, fit // 256 * 256)
-        return min(range(low, min(2 * low, low + 2048) + 1, 256),
-                   key=lambda r: (-(-(r // 256) * -(-self.vocab // 256) // pairs) / r, r))
+        0.6 ms). Inside these bounds the count whose 256 x 256 tiles waste least of their last round over the SM pairs (32 k
+        vocabulary: 1024 rows are 6.8 rounds run as 7, 768 rows 5.1 run as 6)."""
+        if chunk_bytes is not None or sm_pairs <= 0:
+            return max(128, (DEFAULT_CHUNK_BYTES[0] if chunk_bytes is None else chunk_bytes) // (4 * vocab) // 128 * 128)
+        low, high = (max(512, b // (4 * vocab) // 256 * 256) for b in DEFAULT_CHUNK_BYTES)
+        return min(range(low, min(high, low + 2048) + 1, 256),
+                   key=lambda r: (-(-(r // 256) * -(-vocab // 256) // sm_pairs) / r, r))
 
     @torch.no_grad()
     def submit(self, tokens: np.ndarray, convos: list[ConvoTokenized], positions=None) -> dict:
