@@ -12,7 +12,8 @@ keys j with i - window < j <= i. Up to ``window`` positions that IS causal atten
 kernels walk only the key tiles the window reaches and mask its edge: a layer of 32 heads of 128 at window 4096 and
 6001 positions takes about 0.5 ms against 8.7 ms for PyTorch's attention under a band mask, which visits every tile and
 wants the key / value heads repeated. ``windowed_fwd`` / ``windowed_bwd`` below are that masked path: they serve CPU
-tensors and, with or without a window, heads of other sizes than 64 and 128 on a GPU (Gemma's 256).
+tensors and, with or without a window, heads of other sizes than 64 and 128 on a GPU (Gemma's 256), and windowed calls
+of other types than bf16.
 """
 from __future__ import annotations
 
@@ -68,9 +69,21 @@ def attention_reference_bwd(dout, qkv, out, lse, B, L, H, Hkv, d):
     return dqkv.to(qkv.dtype)
 
 
-def _library_path(qkv: torch.Tensor, d: int) -> bool:
-    """Heads the flash kernels do not take (they take 64 and 128) go to the library path on a GPU, e.g. Gemma's 256."""
-    return qkv.is_cuda and d not in (64, 128)
+def _library_path(d: int, window: int | None, qkv: torch.Tensor, *others: torch.Tensor | None) -> bool:
+    """Whether a call takes the masked path: on a GPU heads that the flash kernels do not take (they take 64 and 128, not
+    e.g. Gemma's 256), and windowed calls where ``qkv`` or one of the ``others`` is not bf16; on the CPU every windowed
+    call. (Without a window the kernels' wrappers refuse other types.)"""
+    if not qkv.is_cuda:
+        return window is not None
+    return d not in (64, 128) or (window is not None and not all(t is not None and t.dtype == torch.bfloat16
+                                                                 for t in (qkv, *others)))
+
+
+def _dense(window: int | None, t: torch.Tensor | None) -> torch.Tensor | None:
+    """The operand of a windowed call on a GPU as both paths read it: contiguous rows from a 16-byte boundary on."""
+    if window is None or t is None or not t.is_cuda or (t.is_contiguous() and t.data_ptr() % 16 == 0):
+        return t
+    return t.clone(memory_format=torch.contiguous_format)
 
 
 def _band_mask(n_q: int, n_k: int, q_off: int, window: int, device) -> torch.Tensor:
@@ -113,7 +126,8 @@ def attention_fwd(qkv: torch.Tensor, B: int, L: int, H: int, Hkv: int, d: int, w
     """Returns (out [T, H*d], lse [H, T] fp32). ``window``: the layer's sliding window, or None."""
     if window is not None and L <= window:
         window = None
-    if _library_path(qkv, d) or (window is not None and not qkv.is_cuda):
+    qkv = _dense(window, qkv)
+    if _library_path(d, window, qkv):
         return windowed_fwd(qkv, B, L, H, Hkv, d, window)
     if not qkv.is_cuda:
         return attention_reference_fwd(qkv, B, L, H, Hkv, d)
@@ -125,12 +139,13 @@ def attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window: int | None = Non
     """Returns dqkv with the layout of qkv."""
     if window is not None and L <= window:
         window = None
-    if _library_path(qkv, d) or (window is not None and not qkv.is_cuda):
+    qkv, out = _dense(window, qkv), _dense(window, out)
+    if _library_path(d, window, qkv, out):
         return windowed_bwd(dout, qkv, B, L, H, Hkv, d, window)
     if not qkv.is_cuda:
         return attention_reference_bwd(dout, qkv, out, lse, B, L, H, Hkv, d)
     from . import flash
-    return flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window=window)
+    return flash.flash_attn_bwd(dout.to(qkv.dtype), qkv, out, lse, B, L, H, Hkv, d, window=window)
 
 
 def attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin, window: int | None = None):
@@ -140,12 +155,13 @@ def attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin,
     from . import basic
     if window is not None and L <= window:
         window = None
-    if _library_path(qkv, d) or (window is not None and not qkv.is_cuda):
+    qkv, out = _dense(window, qkv), _dense(window, out)
+    if _library_path(d, window, qkv, out):
         return basic.rope_(windowed_bwd(dout, qkv, B, L, H, Hkv, d, window), pos, cos, sin, H + Hkv, d, inverse=True)
     if (qkv.is_cuda and qkv.dtype == torch.bfloat16 and pos.dtype == torch.int32 and cos.is_contiguous()
             and sin.is_contiguous() and 2 * cos.shape[1] == d):      # partial rotary: the separate kernel below
         from . import flash
-        dqkv = flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, rope=(pos, cos, sin), window=window)
+        dqkv = flash.flash_attn_bwd(dout.to(qkv.dtype), qkv, out, lse, B, L, H, Hkv, d, rope=(pos, cos, sin), window=window)
         basic.rope_(dqkv[:, H * d:], pos, cos, sin, Hkv, d, inverse=True)      # the key heads
         return dqkv
     dqkv = attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
@@ -173,7 +189,8 @@ def attention_fwd_cached(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     values at rows q_off .. q_off+L-1). Inference only: no log-sum-exp is kept."""
     if window is not None and q_off + L <= window:
         window = None
-    if _library_path(qkv, d) or (window is not None and not qkv.is_cuda):
+    qkv, k_cache, v_cache = (_dense(window, t) for t in (qkv, k_cache, v_cache))
+    if _library_path(d, window, qkv, k_cache, v_cache):
         n = q_off + L
         q = qkv[:, : H * d].reshape(B, L, H, d)
         k = k_cache[:, :n].reshape(B, n, Hkv, d)

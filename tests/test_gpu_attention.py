@@ -125,3 +125,50 @@ def test_window_edges_against_the_band_mask(L, H, Hkv, d, window):
     want = ro.view(B, L, -1)[:, c0:].reshape(B * n, -1)
     assert (got.float() - want).abs().max() <= 2e-2 * want.abs().max()
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("form", ["fp32", "fp16", "strided", "offset"])
+@pytest.mark.parametrize("d", [64, 128])
+def test_windowed_calls_take_tensors_that_the_flash_kernels_do_not(form, d):
+    """Types other than bf16 (in the masked path), column slices of wider rows and bases off 16 bytes (copied), forward,
+    backward and behind a cache: against the same calls in fp32 on the CPU. Bound: 2^-9 per rounding to bf16 (2^-11 for fp16, and
+    TF32 is off), gradients are sums of such terms - 2e-2 of the largest value."""
+    B, L, H, Hkv, window = 2, 150, 4, 2, 40
+    torch.manual_seed(d)
+    width = (H + 2 * Hkv) * d
+    dtype = {"fp32": torch.float32, "fp16": torch.float16}.get(form, torch.bfloat16)
+    qkv = torch.randn(B * L, width + 8, device=DEV).to(dtype)
+    dout = torch.randn(B * L, H * d, device=DEV).to(dtype)
+    if form == "strided":
+        qkv = qkv[:, 8:]
+    elif form == "offset":
+        qkv = torch.cat([qkv.new_zeros(1), qkv[:, 8:].reshape(-1)])[1:].view(B * L, width)
+        assert qkv.is_contiguous() and qkv.data_ptr() % 16
+    else:
+        qkv = qkv[:, 8:].contiguous()
+    out, lse = attention.attention_fwd(qkv, B, L, H, Hkv, d, window)
+    dqkv = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
+    kv = Hkv * d
+    kc, vc = (qkv[:, (H + i * Hkv) * d:(H + i * Hkv) * d + kv].reshape(B, L, kv) for i in (0, 1))
+    n = 30
+    rows = qkv.reshape(B, L, -1)[:, L - n:].reshape(B * n, -1)
+    got_c = attention.attention_fwd_cached(rows, kc, vc, B, n, L - n, H, Hkv, d, window)
+    ro, rl = attention.attention_fwd(qkv.float().cpu(), B, L, H, Hkv, d, window)
+    rd = attention.attention_bwd(dout.float().cpu(), qkv.float().cpu(), ro, rl, B, L, H, Hkv, d, window)
+    rc = ro.view(B, L, -1)[:, L - n:].reshape(B * n, -1)
+    for got, want in ((out, ro), (dqkv, rd), (got_c, rc)):
+        assert got.dtype == dtype and (got.float().cpu() - want).abs().max() <= 2e-2 * want.abs().max()
+    with pytest.raises((TypeError, _lib.NativeError)):           # without a window such tensors stay refused
+        attention.attention_fwd(qkv, B, L, H, Hkv, d)
+
+
+def test_windowed_backward_takes_a_gradient_of_another_type():
+    B, L, H, Hkv, d, window = 1, 150, 2, 1, 64, 40
+    torch.manual_seed(0)
+    qkv = torch.randn(B * L, (H + 2 * Hkv) * d, device=DEV).bfloat16()
+    dout = torch.randn(B * L, H * d, device=DEV).bfloat16()
+    out, lse = attention.attention_fwd(qkv, B, L, H, Hkv, d, window)
+    a = attention.attention_bwd(dout.float(), qkv, out, lse, B, L, H, Hkv, d, window)
+    b = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
+    # query gradients of two key blocks meet by atomic adds of two terms onto zero: any order gives the same bits
+    assert torch.equal(a, b) and _lib.take_device_error() == 0
