@@ -656,6 +656,7 @@ extern "C" int b200_flash_attn_bwd(const void* dout, const void* qkv, const void
   if (!dout || !qkv || !out || !lse || !delta || !dqkv || !dq_acc || B <= 0 || L <= 0 || window < 0 || H <= 0 ||
       Hkv <= 0 || (H % Hkv) != 0)
     return B200_ERR_ARG;
+  if (window >= L) window = 0;      // causal; also keeps the sum of position and window inside 32 bits
   if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, nullptr, nullptr, nullptr, st);
   if (D == 128)
     return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, nullptr, nullptr, nullptr, st);
@@ -673,6 +674,7 @@ extern "C" int b200_flash_attn_bwd_rope(const void* dout, const void* qkv, const
   if (!dout || !qkv || !out || !lse || !delta || !dqkv || !dq_acc || !pos || !cos_tab || !sin_tab || B <= 0 || L <= 0 ||
       window < 0 || H <= 0 || Hkv <= 0 || (H % Hkv) != 0)
     return B200_ERR_ARG;
+  if (window >= L) window = 0;      // causal; also keeps the sum of position and window inside 32 bits
   if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, pos, cos_tab, sin_tab, st);
   if (D == 128)
     return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, pos, cos_tab, sin_tab, st);

@@ -473,6 +473,7 @@ extern "C" int b200_flash_attn_fwd(const void* qkv, void* out, float* lse, int B
                                    cudaStream_t st) {
   using namespace b200;
   if (!qkv || !out || B <= 0 || L <= 0 || window < 0 || H <= 0 || Hkv <= 0 || (H % Hkv) != 0) return B200_ERR_ARG;
+  if (window >= L) window = 0;      // causal; also keeps the sums of position and window inside 32 bits
   const long long width = (long long)(H + 2 * Hkv) * D;
   if (D == 64)
     return fa::launch_fwd<64>(qkv, width, 0, qkv, qkv, width, H * D, (H + Hkv) * D, L, out, lse, B, L, 0, window, H, Hkv, st);
@@ -492,6 +493,7 @@ extern "C" int b200_flash_attn_fwd_cached(const void* qkv, const void* k_cache, 
   if (!qkv || !k_cache || !v_cache || !out || B <= 0 || L <= 0 || q_off < 0 || window < 0 || H <= 0 || Hkv <= 0 || (H % Hkv) != 0 ||
       cache_rows < (long long)q_off + L)
     return B200_ERR_ARG;
+  if (window >= (long long)q_off + L) window = 0;
   const long long width = (long long)(H + 2 * Hkv) * D, kvw = (long long)Hkv * D;
   if (D == 64)
     return fa::launch_fwd<64>(qkv, width, 0, k_cache, v_cache, kvw, 0, 0, cache_rows, out, lse, B, L, q_off, window, H, Hkv, st);

@@ -13,13 +13,18 @@ _lib.register("b200_dq_convert_rope", [_VP, _VP, _VP, _VP, _VP, _LL, _I, _I, _LL
 _lib.register("b200_flash_attn_bwd_rope", [_VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP])
 
 
+def _window(window: int | None, positions: int) -> int:
+    """The C argument: 0 where every position is inside the window (a Python int of any size would be cut to 32 bits)."""
+    return 0 if window is None or window >= positions else window
+
+
 def flash_attn_fwd(qkv: torch.Tensor, B: int, L: int, H: int, Hkv: int, d: int, window: int | None = None):
     if qkv.dtype != torch.bfloat16 or not qkv.is_contiguous():
         raise TypeError("flash_attn_fwd: qkv must be contiguous bf16")
     T = B * L
     out = torch.empty((T, H * d), dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty((H, T), dtype=torch.float32, device=qkv.device)
-    rc = _lib.kernels().b200_flash_attn_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), B, L, window or 0, H, Hkv, d,
+    rc = _lib.kernels().b200_flash_attn_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), B, L, _window(window, L), H, Hkv, d,
                                             _lib.stream())
     _lib.check(rc, "b200_flash_attn_fwd")
     return out, lse
@@ -38,11 +43,12 @@ def flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, rope=None, window: int 
         pos, cos, sin = rope
         rc = _lib.kernels().b200_flash_attn_bwd_rope(_lib.ptr(dout), _lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse),
                                                      _lib.ptr(delta), _lib.ptr(dqkv), _lib.ptr(dq_acc), _lib.ptr(pos),
-                                                     _lib.ptr(cos), _lib.ptr(sin), B, L, window or 0, H, Hkv, d, _lib.stream())
+                                                     _lib.ptr(cos), _lib.ptr(sin), B, L, _window(window, L), H, Hkv, d,
+                                                     _lib.stream())
         _lib.check(rc, "b200_flash_attn_bwd_rope")
         return dqkv
     rc = _lib.kernels().b200_flash_attn_bwd(_lib.ptr(dout), _lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(delta),
-                                            _lib.ptr(dqkv), _lib.ptr(dq_acc), B, L, window or 0, H, Hkv, d, _lib.stream())
+                                            _lib.ptr(dqkv), _lib.ptr(dq_acc), B, L, _window(window, L), H, Hkv, d, _lib.stream())
     _lib.check(rc, "b200_flash_attn_bwd")
     return dqkv
 
@@ -54,6 +60,6 @@ def flash_attn_fwd_cached(qkv, k_cache, v_cache, B, L, q_off, H, Hkv, d, window:
         raise ValueError("key / value caches must be [B, rows, Hkv*d]")
     out = torch.empty((B * L, H * d), dtype=qkv.dtype, device=qkv.device)
     rc = _lib.kernels().b200_flash_attn_fwd_cached(_lib.ptr(qkv), _lib.ptr(k_cache), _lib.ptr(v_cache), k_cache.shape[1],
-                                                   _lib.ptr(out), None, B, L, q_off, window or 0, H, Hkv, d, _lib.stream())
+                                                   _lib.ptr(out), None, B, L, q_off, _window(window, q_off + L), H, Hkv, d, _lib.stream())
     _lib.check(rc, "b200_flash_attn_fwd_cached")
     return out

@@ -172,3 +172,36 @@ def test_windowed_backward_takes_a_gradient_of_another_type():
     b = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
     # query gradients of two key blocks meet by atomic adds of two terms onto zero: any order gives the same bits
     assert torch.equal(a, b) and _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("window", [300, 2 ** 31 - 1, 2 ** 31, 2 ** 32 + 7])
+def test_windows_at_and_beyond_the_sequence_are_causal(window):
+    """Through the kernels' own wrappers and, where it fits 32 bits, the C entries: the bits of the call without a window."""
+    from llm_distillery_b200.ops import flash
+    B, L, H, Hkv, d = 1, 300, 2, 1, 64
+    torch.manual_seed(3)
+    qkv = torch.randn(B * L, (H + 2 * Hkv) * d, device=DEV).bfloat16()
+    dout = torch.randn(B * L, H * d, device=DEV).bfloat16()
+    out, lse = flash.flash_attn_fwd(qkv, B, L, H, Hkv, d)
+    a, al = flash.flash_attn_fwd(qkv, B, L, H, Hkv, d, window)
+    assert torch.equal(a, out) and torch.equal(al, lse)
+    want = flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d)
+
+    def near(got):      # query gradients of three key blocks meet by atomic adds in no fixed order: a last bit of bf16
+        assert torch.equal(got[:, H * d:], want[:, H * d:])
+        assert (got.float() - want.float()).abs().max() <= 2 ** -7 * want.float().abs().max()
+    near(flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window=window))
+    kc, vc = (qkv[:, (H + i) * d:(H + 1 + i) * d].reshape(B, L, d).contiguous() for i in (0, 1))
+    rows = qkv[200:].contiguous()
+    assert torch.equal(flash.flash_attn_fwd_cached(rows, kc, vc, B, 100, 200, H, Hkv, d, window),
+                       flash.flash_attn_fwd_cached(rows, kc, vc, B, 100, 200, H, Hkv, d))
+    if window < 2 ** 31:
+        lib, p = _lib.kernels(), _lib.ptr
+        o2, l2, dq = torch.empty_like(out), torch.empty_like(lse), torch.empty_like(qkv)
+        _lib.check(lib.b200_flash_attn_fwd(p(qkv), p(o2), p(l2), B, L, window, H, Hkv, d, _lib.stream()), "fwd")
+        delta, acc = torch.empty_like(lse), torch.empty((B * L, H * d), dtype=torch.float32, device=DEV)
+        _lib.check(lib.b200_flash_attn_bwd(p(dout), p(qkv), p(o2), p(l2), p(delta), p(dq), p(acc), B, L, window, H, Hkv, d,
+                                           _lib.stream()), "bwd")
+        assert torch.equal(o2, out)
+        near(dq)
+    assert _lib.take_device_error() == 0
