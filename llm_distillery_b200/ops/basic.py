@@ -164,6 +164,7 @@ def linear_rope_fwd(x: torch.Tensor, w: torch.Tensor, pos: torch.Tensor, cos: to
     launch when the shape allows (bf16, head_dim 64 or 128, N a multiple of 128): the rotation sits in the
     GEMM's epilogue. Same values as ``linear_fwd`` followed by ``rope_``."""
     T, N = x.shape[0], w.shape[0]
+    _same_reduction("linear_rope_fwd", x.shape[1], w.shape[1])
     if (_native(x, w) and x.dtype == _BF16 and w.dtype == _BF16 and head_dim in (64, 128) and N % 128 == 0
             and x.stride(-1) == 1 and w.stride(-1) == 1 and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
             and pos.dtype == torch.int32 and cos.dtype == torch.float32 and cos.shape[1] == head_dim // 2
@@ -392,6 +393,24 @@ def swiglu_fwd(gu: torch.Tensor) -> torch.Tensor:
     return act
 
 
+def _same_reduction(what: str, k: int, kw: int) -> None:
+    """The fused launches read both operands by one K, as ``gemm`` does: refused alike."""
+    if k != kw:
+        raise ValueError(f"{what}: reduction dims differ ({k} vs {kw})")
+
+
+def _target(out: torch.Tensor | None, rows: int, cols: int, device) -> torch.Tensor:
+    """What an epilogue of 16-byte bf16 stores writes to: the caller's ``out`` where it can, else a tensor to copy from."""
+    if out is not None and out.dtype == _BF16 and tuple(out.shape) == (rows, cols) and out.stride(1) == 1 \
+            and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0:
+        return out
+    return torch.empty((rows, cols), dtype=_BF16, device=device)
+
+
+def _deliver(t: torch.Tensor, out: torch.Tensor | None) -> torch.Tensor:
+    return t if out is None or out is t else out.copy_(t)
+
+
 def swiglu_fusable(x: torch.Tensor, w_gu: torch.Tensor) -> bool:
     """Whether ``linear_swiglu_fwd`` runs as one launch for these operands."""
     f = w_gu.shape[0] // 2
@@ -407,19 +426,15 @@ def linear_swiglu_fwd(x: torch.Tensor, w_gu: torch.Tensor, out_gu: torch.Tensor 
     ``out_gu`` / ``out_act`` (row slices of larger buffers are fine) receive the results when given."""
     T = x.shape[0]
     f = w_gu.shape[0] // 2
+    _same_reduction("linear_swiglu_fwd", x.shape[1], w_gu.shape[1])
     if swiglu_fusable(x, w_gu):
-        gu = out_gu if out_gu is not None else torch.empty((T, 2 * f), dtype=x.dtype, device=x.device)
-        act = out_act if out_act is not None else torch.empty((T, f), dtype=x.dtype, device=x.device)
+        gu, act = _target(out_gu, T, 2 * f, x.device), _target(out_act, T, f, x.device)
         _lib.check(_lib.kernels().b200_gemm_swiglu(_lib.ptr(x), _lib.ptr(w_gu), _lib.ptr(gu), _lib.ptr(act), T, f,
                                                    x.shape[1], x.stride(0), w_gu.stride(0), gu.stride(0), act.stride(0),
                                                    int(split_k), _lib.stream()), "b200_gemm_swiglu")
-        return gu, act
+        return _deliver(gu, out_gu), _deliver(act, out_act)
     gu = gemm(x, w_gu, out=out_gu, split_k=split_k)
-    act = swiglu_fwd(gu)
-    if out_act is not None:
-        out_act.copy_(act)
-        act = out_act
-    return gu, act
+    return gu, _deliver(swiglu_fwd(gu), out_act)
 
 
 def swiglu_bwd_fusable(dy: torch.Tensor, w_d: torch.Tensor, gu: torch.Tensor) -> bool:
@@ -438,17 +453,14 @@ def linear_dgrad_swiglu_bwd(dy: torch.Tensor, w_d: torch.Tensor, gu: torch.Tenso
     ``linear_dgrad`` followed by ``swiglu_bwd``. ``out`` (a row slice of a larger buffer is fine) receives the result."""
     T = dy.shape[0]
     f = w_d.shape[1]
+    _same_reduction("linear_dgrad_swiglu_bwd", dy.shape[1], w_d.shape[0])
     if swiglu_bwd_fusable(dy, w_d, gu):
-        dgu = out if out is not None else torch.empty((T, 2 * f), dtype=gu.dtype, device=gu.device)
+        dgu = _target(out, T, 2 * f, gu.device)
         _lib.check(_lib.kernels().b200_gemm_swiglu_bwd(_lib.ptr(dy), _lib.ptr(w_d), _lib.ptr(gu), _lib.ptr(dgu), T, f,
                                                        dy.shape[1], dy.stride(0), w_d.stride(0), gu.stride(0),
                                                        dgu.stride(0), int(split_k), _lib.stream()), "b200_gemm_swiglu_bwd")
-        return dgu
-    dgu = swiglu_bwd(gu, linear_dgrad(dy, w_d, split_k))
-    if out is not None:
-        out.copy_(dgu)
-        return out
-    return dgu
+        return _deliver(dgu, out)
+    return _deliver(swiglu_bwd(gu, linear_dgrad(dy, w_d, split_k)), out)
 
 
 def swiglu_bwd(gu: torch.Tensor, dact: torch.Tensor) -> torch.Tensor:

@@ -216,3 +216,28 @@ def test_fused_epilogues_on_few_rows(T, split):
         got = basic.linear_rope_fwd(x, wq, pos, cos, sin, H + Hkv, d, split_k=split)
         assert torch.equal(got, basic.rope_(basic.linear_fwd(x, wq, split_k=split), pos, cos, sin, H + Hkv, d))
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("T", [1, 33, 600])
+@pytest.mark.parametrize("form", ["fp32", "odd stride", "offset"])
+def test_fused_epilogues_copy_to_outputs_they_cannot_store_to(T, form):
+    """Outputs of another type, with rows off 16 bytes or from an odd base receive the values of the call without them."""
+    torch.manual_seed(T)
+    K, f = 320, 256
+    x = torch.randn(T, K, device=DEV).bfloat16()
+    w = (torch.randn(2 * f, K, device=DEV) * 0.1).bfloat16()
+    wd = (torch.randn(K, f, device=DEV) * 0.1).bfloat16()
+
+    def output(cols):
+        if form == "fp32":
+            return torch.zeros(T, cols, device=DEV)
+        if form == "odd stride":
+            return torch.zeros(T, cols + 3, device=DEV, dtype=torch.bfloat16)[:, :cols]
+        return torch.zeros(T * cols + 1, device=DEV, dtype=torch.bfloat16)[1:].view(T, cols)
+    gu, act = basic.linear_swiglu_fwd(x, w)
+    og, oa, od = output(2 * f), output(f), output(2 * f)
+    rg, ra = basic.linear_swiglu_fwd(x, w, og, oa)
+    assert rg is og and ra is oa and torch.equal(og, gu.to(og.dtype)) and torch.equal(oa, act.to(oa.dtype))
+    dgu = basic.linear_dgrad_swiglu_bwd(x, wd, gu)
+    assert basic.linear_dgrad_swiglu_bwd(x, wd, gu, out=od) is od and torch.equal(od, dgu.to(od.dtype))
+    assert _lib.take_device_error() == 0
