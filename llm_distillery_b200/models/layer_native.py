@@ -24,17 +24,26 @@ for _n in ("b200_layer_fwd", "b200_layer_bwd", "b200_layer_saved_bytes", "b200_l
     _lib.KERNELS_PER_CALL[_n] = 0          # the calls return how many kernels they launched
 
 
-def fits(h, pos, cos, weights, b_qkv, d: int, training: bool) -> bool:
-    if not h.is_cuda or h.dtype != torch.bfloat16 or d not in (64, 128) or 2 * cos.shape[1] != d:
+def fits(h, pos, cos, sin, weights, b_qkv, heads, training: bool) -> bool:
+    """``heads`` = (query heads, key heads, head size). The C calls take sizes from the activations and trust the rest, so
+    what the separate calls would refuse is left to them."""
+    H, Hkv, d = heads
+    T, w = h.shape
+    if not h.is_cuda or h.dtype != torch.bfloat16 or d not in (64, 128) or w % 8 or w > 8192:
         return False
-    if pos.dtype != torch.int32 or cos.dtype != torch.float32 or not cos.is_contiguous() or h.shape[1] % 8 or h.shape[1] > 8192:
+    if pos.dtype != torch.int32 or not pos.is_contiguous() or pos.shape != (T,):
         return False
-    for w in weights if b_qkv is None else weights + (b_qkv,):
-        if w.dtype != torch.bfloat16 or not w.is_cuda or not w.is_contiguous():
+    for t in (cos, sin):
+        if t.dtype != torch.float32 or not t.is_contiguous() or 2 * t.shape[1] != d or t.shape != cos.shape:
             return False
-        if training and w.requires_grad and getattr(w, "grad_slot", None) is None:
+    n, f = (H + 2 * Hkv) * d, weights[4].shape[0] // 2
+    shapes = ((w,), (n, w), (w, H * d), (w,), (2 * f, w), (w, f), (n,))
+    for t, shape in zip(weights if b_qkv is None else weights + (b_qkv,), shapes):
+        if t.dtype != torch.bfloat16 or not t.is_cuda or not t.is_contiguous() or t.shape != shape:
             return False
-    return weights[4].shape[0] % 16 == 0
+        if training and t.requires_grad and getattr(t, "grad_slot", None) is None:
+            return False
+    return f % 8 == 0
 
 
 def _launched(rc: int, what: str) -> None:

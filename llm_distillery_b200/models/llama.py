@@ -460,6 +460,7 @@ class LlamaModel(nn.Module):
         training = torch.is_grad_enabled()
         fwd, bwd = split_k if split_k is not None else (self.ordered_sums is False,) * 2
         split = (fwd and not training, bwd)
+        heads = meta[2:5]
         plain = not (cfg.qk_norm or cfg.o_bias or cfg.mlp_bias) and rmul == 1.0
         tables = self.layer_rope(cos, sin)
         meta7 = meta
@@ -496,7 +497,7 @@ class LlamaModel(nn.Module):
                 b_qkv = getattr(layer, "qkv_bias", None)
                 w = (layer.input_layernorm, layer.qkv_proj, layer.o_proj, layer.post_attention_layernorm, layer.gate_up_proj,
                      layer.down_proj)
-                if layer_native.fits(h, pos, cos, w, b_qkv, cfg.head_dim, training):
+                if layer_native.fits(h, pos, cos, sin, w, b_qkv, heads, training):
                     h = layer_native.NativeLayerFn.apply(h, pos, cos, sin, *w, b_qkv, meta, split)
                     continue
             h = DecoderLayerFn.apply(h, pos, cos, sin, layer.input_layernorm, layer.qkv_proj, layer.o_proj,
