@@ -99,13 +99,9 @@ class NativeLayerFn(torch.autograd.Function):
             x, pos, cos, sin, saved = ctx.saved_tensors
         dout = dout.contiguous()
         h, f = x.shape[1], weights[4].shape[0] // 2
-        grads, acc = [], 0
-        for i, w in enumerate(weights + (b_qkv,)):
-            slot = llama._slot(w) if w is not None else None
-            grads.append(0 if slot is None else slot.buf.data_ptr())
-            if slot is not None:
-                acc |= 0 if slot.fresh else 1 << i
-                slot.fresh = False
+        slots = [llama._slot(w) if w is not None else None for w in weights + (b_qkv,)]
+        grads = [0 if s is None else s.buf.data_ptr() for s in slots]
+        acc = sum(1 << i for i, s in enumerate(slots) if s is not None and not s.fresh)
         lib = _lib.kernels()
         scratch = torch.empty(lib.b200_layer_scratch_bytes(B, L, H, Hkv, d, h, f), dtype=torch.uint8, device=x.device)
         dx = torch.empty_like(x)
@@ -115,6 +111,9 @@ class NativeLayerFn(torch.autograd.Function):
                                      w1.data_ptr(), wq.data_ptr(), wo.data_ptr(), w2.data_ptr(), wg.data_ptr(), wd.data_ptr(),
                                      saved.data_ptr(), scratch.data_ptr(), dx.data_ptr(), *grads, acc, B, L, window, H, Hkv,
                                      d, h, f, int(ctx.split[1]), _lib.stream()), "b200_layer_bwd")
+        for s in slots:
+            if s is not None:
+                s.fresh = False
         if llama.LAYER_BACKWARD_DONE[0] is not None:
             llama.LAYER_BACKWARD_DONE[0](weights[0])
         return (dx,) + (None,) * 12

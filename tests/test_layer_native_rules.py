@@ -41,3 +41,32 @@ N = (H + 2 * HKV) * D
     ("h", _t(T, W, dtype=torch.float32)), ("qkv", _t(W, N).t())])
 def test_other_layers_are_left_to_the_separate_calls(name, tensor):
     assert not _case(**{name: tensor})
+
+
+@pytest.mark.parametrize("rc", [-2, 20])
+def test_gradient_slots_are_taken_as_written_only_by_a_call_that_ran(monkeypatch, rc):
+    """A backward call that fails leaves the slots fresh, as they are: the next pass must not add to what is in them."""
+    class Lib:
+        def __getattr__(self, name):
+            if name == "b200_last_cuda_error":
+                return lambda: b""
+            return lambda *a: {"b200_layer_fwd": 8, "b200_layer_bwd": rc}.get(name, 64)
+
+    class Slot:
+        def __init__(self, w):
+            self.buf, self.fresh = torch.zeros(w.shape), True
+    monkeypatch.setattr(layer_native._lib, "kernels", Lib)
+    monkeypatch.setattr(layer_native._lib, "stream", lambda: None)
+    n = (H + 2 * HKV) * D
+    w = [torch.zeros(s, dtype=torch.bfloat16).requires_grad_() for s in ((W,), (n, W), (W, H * D), (W,), (2 * F, W), (W, F))]
+    for t in w:
+        t.grad_slot = Slot(t)
+    x = torch.zeros(T, W, dtype=torch.bfloat16).requires_grad_()
+    tables = torch.zeros(T, dtype=torch.int32), torch.zeros(16, D // 2), torch.zeros(16, D // 2)
+    y = layer_native.NativeLayerFn.apply(x, *tables, *w, None, (1, T, H, HKV, D, 1e-5, False, None), (False, False))
+    if rc < 0:
+        with pytest.raises(layer_native._lib.NativeError):
+            y.backward(torch.zeros_like(y))
+    else:
+        y.backward(torch.zeros_like(y))
+    assert all(t.grad_slot.fresh == (rc < 0) for t in w)
