@@ -520,7 +520,7 @@ class LlamaModel(nn.Module):
         rotated keys and its values for all positions seen so far ([B, L, Hkv*d] each, zero-filled beyond), and the
         chunk's queries attend to positions <= their own. Same result as ``hidden_states`` up to rounding."""
         cfg = self.cfg
-        split = self.ordered_sums is False
+        split = self.ordered_sums is False and not cfg.num_local_experts      # expert layers: see models/moe.py
         B, L = input_ids.shape
         if chunk_len <= 0 or chunk_len >= L:
             return self.hidden_states(input_ids)

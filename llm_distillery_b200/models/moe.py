@@ -10,6 +10,8 @@ expert's two GEMMs on its contiguous slab of rows with the same tcgen05 GEMM ker
 gate/up projection of all experts fills one buffer, so SwiGLU is one launch), and combines by GATHERING each token's k
 results - a fixed order of additions, no atomic scatter. Routing arithmetic ([T, E] tensors) is PyTorch in fp32.
 The number of rows per expert comes back to the host once per layer (the GEMM shapes depend on it).
+No GEMM here cuts K (``basic.gemm``'s split_k), in inference either: behind a router a last bit can be another expert, and
+an expert's row count, which the cut would depend on, changes with every batch.
 """
 from __future__ import annotations
 
@@ -78,7 +80,7 @@ def experts_forward(x_perm: torch.Tensor, counts: list[int], w_gu: torch.Tensor,
         offs.append(o)
         o += c
     if all(c == 0 or basic.swiglu_fusable(x_perm[o:o + c], w_gu[e]) for e, (o, c) in enumerate(zip(offs, counts))):
-        # every expert has enough rows for the GEMM that applies SwiGLU in its epilogue
+        # sizes that the GEMM with SwiGLU in its epilogue takes, whatever the experts' row counts
         act = torch.empty((n, two_f // 2), dtype=x_perm.dtype, device=x_perm.device)
         for e, (o, c) in enumerate(zip(offs, counts)):
             if c:
