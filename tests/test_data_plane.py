@@ -20,7 +20,8 @@ from tests.ref_import import import_reference, reference_root
 
 # ------------------------------------------------------------------ config
 def test_config_merge_and_bool_parsing(tmp_path):
-    ref_cfg = os.path.join(reference_root() or "", "config.json")
+    root = reference_root()          # without one a relative path would name this repository's own config.json
+    ref_cfg = os.path.join(root, "config.json") if root else ""
     if not os.path.exists(ref_cfg):
         pytest.skip("reference config.json not available")
     base = json.load(open(ref_cfg))
