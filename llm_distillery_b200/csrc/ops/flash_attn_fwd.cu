@@ -24,6 +24,7 @@
 // share an SM.
 //
 // Layout: qkv [T, (H + 2*Hkv) * D] bf16 with T = B*L; out [T, H*D] bf16; lse [H, T] fp32 (natural log).
+#include <float.h>
 #include "../common/ptx.cuh"
 #include "../common/host.cuh"
 
@@ -316,8 +317,8 @@ __global__ void __launch_bounds__(NTHREADS, 2)
         // The first tile fixes the reference maximum. Later tiles are exponentiated against the maximum known so far
         // and only redone when a score exceeds it by more than 2^kRescaleThreshold, which is rare once a row has seen
         // a few hundred keys. Without a window every row sees key 0; with one the later rows of the block may see
-        // nothing of the first tile: they start from a finite bound below any score, so that their first visible
-        // tile moves the maximum and nothing is ever inf - inf.
+        // nothing of the first tile: they start from the lowest finite value, which no finite score is below, so that
+        // their first visible tile moves the maximum and nothing is ever inf - inf.
         float mx0 = -INFINITY;
 #pragma unroll
         for (int t = 0; t < 32; t += 2) {
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
           mx0 = fmax3(mx0, ((t + 32) <= lim && (t + 32) >= lo) ? __uint_as_float(vb[t]) : -INFINITY,
                       ((t + 33) <= lim && (t + 33) >= lo) ? __uint_as_float(vb[t + 1]) : -INFINITY);
         }
-        m_used = fmaxf(mx0, -1e30f);
+        m_used = fmaxf(mx0, -FLT_MAX);
       }
       float mx = m_used;
       uint64_t sum2 = 0ull;
@@ -388,7 +389,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
       int w3 = mbar_wait_bounded(o_final, 0, abort_flag, err_word, ERR_WAIT_AUX) ? 1 : 0;
       if (__all_sync(0xffffffffu, w3)) {
         tc_fence_after_sync();
-        const float inv = l > 0.f ? 1.f / l : 0.f;
+        const float inv = 1.f / l;   // l = 0: every visible score was -inf, 0 * inf = NaN as in a softmax over them
         const bool row_ok = qi < p.L;
         const long long t = (long long)b * p.L + qi;
         __nv_bfloat16* orow = p.out + t * (long long)(p.H * D) + hq * D;

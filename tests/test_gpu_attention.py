@@ -205,3 +205,35 @@ def test_windows_at_and_beyond_the_sequence_are_causal(window):
         assert torch.equal(o2, out)
         near(dq)
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("window", [None, 1, 40, 130])
+def test_scores_of_any_size(d, window):
+    """Scores far below zero, a head whose scores all overflow to -inf, and NaN in one key. The values of position p are
+    p, so the output of a row is the mean position over its largest scores: the others are 2^13 / sqrt(d) lower, their
+    probability is exactly 0. Bound: two roundings to bf16, 2^-8."""
+    B, L, H = 1, 333, 2
+    ks = -(2.0 ** 8) * (1 + (torch.arange(L) * 5 % 7) / 8)              # exact in bf16
+    qkv = torch.empty(B * L, 3, H, d)
+    qkv[:, 0, 0], qkv[:, 0, 1] = 4.0, 2.0 ** 100                          # scores of -2^10 d and less, and -inf
+    qkv[:, 1, 0], qkv[:, 1, 1] = ks.view(L, 1), ks.view(L, 1) * 2.0 ** 40
+    qkv[:, 2] = torch.arange(L).float().view(L, 1, 1)
+    qkv = qkv.reshape(B * L, -1).bfloat16().to(DEV)
+    out, _ = attention.attention_fwd(qkv, B, L, H, H, d, window)
+    out = out.float().cpu().view(L, H, d)
+    see = torch.tril(torch.ones(L, L, dtype=torch.bool))
+    if window is not None:
+        see &= ~torch.tril(see, -window)
+    s = ks.double().view(1, L).expand(L, L).masked_fill(~see, -float("inf"))
+    top = (s == s.amax(1, keepdim=True)).double()
+    want = (top @ torch.arange(L).bfloat16().double()) / top.sum(1)
+    assert ((out[:, 0].double() - want.view(L, 1)).abs() <= 2 ** -8 * want.view(L, 1)).all()
+    assert out[:, 1].isnan().all()                                       # the softmax over nothing but -inf
+    nan_at = 100
+    qkv = torch.randn(B * L, 3 * H * d, device=DEV).bfloat16()
+    qkv[nan_at, H * d:2 * H * d] = float("nan")
+    out, _ = attention.attention_fwd(qkv, B, L, H, H, d, window)
+    bad = out.isnan().any(1).cpu()
+    assert torch.equal(bad, see[:, nan_at])                              # the rows that see the key, and no other
+    assert _lib.take_device_error() == 0
