@@ -14,7 +14,8 @@ constexpr int SORT_MAX_EXPERTS = 32;
 // hundred thousand small numbers that sit in L2, and the point is latency (the host waits for the counts): each thread
 // counts its contiguous run of keys per expert in shared memory, one scan over (expert, thread) turns the counts into
 // positions, and the same run is walked again in order. 12248 pairs of 8 experts: the ten launches of a library radix
-// sort, histogram, scatter and division that this replaces took about 90 us.
+// sort, histogram, scatter and division that this replaces took about 90 us. The runs grow with the pairs and one block
+// does not: the caller goes to the library beyond 32768 of them (models/moe.py: SORT_MAX_PAIRS, with both sides' times).
 __global__ void __launch_bounds__(SORT_THREADS, 1)
     expert_sort_kernel(const long long* __restrict__ experts, long long n, int E, int k, long long* __restrict__ order,
                        long long* __restrict__ inverse, long long* __restrict__ token, long long* __restrict__ counts) {

@@ -20,6 +20,27 @@ def test_expert_sort_is_the_stable_sort(T, k, E):
     assert counts == torch.bincount(flat, minlength=E).tolist()
 
 
+@pytest.mark.parametrize("T,k,dtype,native", [(16384, 2, torch.int64, True), (16385, 2, torch.int64, False),
+                                              (4096, 8, torch.int64, True), (16384, 8, torch.int64, False),
+                                              (100, 2, torch.int32, False), (100, 2, torch.uint8, False)])
+def test_which_sort_takes_the_pairs(monkeypatch, T, k, dtype, native):
+    """Many pairs are left to the library, whose sort is ahead there, and so are indices that the kernel would misread."""
+    top_e = torch.randint(0, 32, (T, k), device="cuda", generator=torch.Generator("cuda").manual_seed(T + k)).to(dtype)
+    calls, real = [], _lib.kernels()
+
+    class Recorder:
+        def __getattr__(self, name):
+            calls.append(name)
+            return getattr(real, name)
+    monkeypatch.setattr(_lib, "kernels", Recorder)
+    order, inverse, token, counts = moe.permutation(top_e, 32)
+    assert ("b200_expert_sort" in calls) == native
+    flat = top_e.reshape(-1)
+    want = torch.argsort(flat, stable=True)
+    assert torch.equal(order, want) and torch.equal(token, want // k) and counts == torch.bincount(flat.long(), minlength=32).tolist()
+    assert torch.equal(order[inverse], torch.arange(T * k, device="cuda"))
+
+
 @pytest.mark.parametrize("T,k,h,resid,rmul", [(1, 1, 8, True, 1.0), (257, 2, 2048, True, 1.0), (33, 8, 264, False, 1.0),
                                               (100, 4, 512, True, 0.25)])
 def test_combine_matches_the_gathered_sum(T, k, h, resid, rmul):
