@@ -187,12 +187,50 @@ def test_few_tiles_split_over_a_cluster(M, N, K, layout):
 
 @pytest.mark.parametrize("T", [1, 31, 130, 511, 777])
 def test_one_slice_keeps_the_order_of_the_large_tiles(T):
-    """Without ``split_k`` a row's result has the same bits whichever kernel its batch size picks."""
+    """Without ``split_k`` a row's result has the same bits in the few-tile kernel and in the one of 128 x 256 tiles
+    (4096 x 896 are 64 tiles of 256 x 256, too few for the pair kernel; the next test has that one)."""
     torch.manual_seed(T)
     a = torch.randn(4096, 1400, device=DEV).bfloat16()
     b = (torch.randn(896, 1400, device=DEV) * 0.1).bfloat16()
     assert torch.equal(basic.gemm(a[:T], b), basic.gemm(a, b)[:T])
     assert torch.equal(basic.gemm(a[:T], b, out_dtype=torch.float32), basic.gemm(a, b, out_dtype=torch.float32)[:T])
+
+
+@pytest.mark.parametrize("T", [1, 130, 777, 2048])
+def test_one_slice_keeps_the_order_of_the_pair_kernel(T):
+    """The same against the 256 x 256 kernel (8192 x 2304: 288 tiles), for the plain, rotary and SwiGLU forms. bf16 outputs
+    only: that kernel cuts the K of fp32 outputs by their tile count, with or without ``split_k``."""
+    torch.manual_seed(T)
+    K, N, d = 1400, 2304, 128
+    a = torch.randn(8192, K, device=DEV).bfloat16()
+    w = (torch.randn(N, K, device=DEV) * 0.1).bfloat16()
+    pos = torch.arange(8192, device=DEV, dtype=torch.int32) % 300
+    cos, sin = basic.rope_tables(300, d, 10000.0, DEV)
+    assert torch.equal(basic.gemm(a[:T], w), basic.gemm(a, w)[:T])
+    assert torch.equal(basic.linear_rope_fwd(a[:T], w, pos[:T], cos, sin, 14, d), basic.linear_rope_fwd(a, w, pos, cos, sin, 14, d)[:T])
+    for few, many in zip(basic.linear_swiglu_fwd(a[:T], w), basic.linear_swiglu_fwd(a, w)):
+        assert torch.equal(few, many[:T])
+    assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 64, 64), (128, 128, 512), (136, 72, 200), (304, 1152, 896)])
+@pytest.mark.parametrize("layout,dtype", [("nt", torch.float16), ("nn", torch.float16), ("tn", torch.float16),
+                                          ("tt", torch.float16), ("tt", torch.bfloat16)])
+def test_few_tiles_split_in_fp16_and_with_a_alone_transposed(M, N, K, layout, dtype):
+    """Forms that the models do not use: fp16 operands, and A stored [K, M] beside B stored [N, K]. Bound: one rounding of
+    the result, 2^-11 (fp16) or 2^-8, and the 32-bit sums, which are far below."""
+    a_mn, b_mn = layout[0] == "t", layout[1] == "n"
+    torch.manual_seed(M + N + K)
+    a = torch.randn((K, M) if a_mn else (M, K), device=DEV).to(dtype)
+    b = (torch.randn((K, N) if b_mn else (N, K), device=DEV) * 0.1).to(dtype)
+    ref = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double()
+    got = basic.gemm(a, b, a_mn=a_mn, b_mn=b_mn, split_k=True)
+    eps = 2 ** -11 if dtype == torch.float16 else 2 ** -8
+    assert got.dtype == dtype and ((got.double() - ref).abs() <= eps * ref.abs() + 1e-5 * K ** 0.5).all()
+    acc = basic.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=got.clone(), accumulate=True, split_k=True)
+    want = got.double() + ref
+    assert ((acc.double() - want).abs() <= eps * want.abs() + 1e-5 * K ** 0.5).all()
+    assert _lib.take_device_error() == 0
 
 
 @pytest.mark.parametrize("T", [1, 31, 130, 511, 777])

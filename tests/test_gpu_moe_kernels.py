@@ -56,3 +56,22 @@ def test_combine_matches_the_gathered_sum(T, k, h, resid, rmul):
     # fp32 sums of at most 9 terms, then one rounding to bf16 (2^-9 of the value)
     assert ((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5).all()
     assert _lib.take_device_error() == 0
+
+
+def test_combine_passes_on_what_is_not_finite():
+    """NaN, infinities and the product of zero and infinity as the gathered sum has them."""
+    T, k, h = 64, 2, 40
+    torch.manual_seed(0)
+    y = torch.randn(T * k, h, device="cuda").bfloat16()
+    y[3, 0], y[8, 1], y[8, 2], y[20, 3], y[21, 3] = (float(v) for v in ("nan", "inf", "-inf", "inf", "-inf"))
+    w = torch.rand(T, k, device="cuda")
+    w[4, 0] = 0.0                                      # times the infinities of row 8
+    w[30, 1] = float("nan")
+    inverse = torch.arange(T * k, device="cuda")
+    for h1 in (None, torch.randn(T, h, device="cuda").bfloat16()):
+        got = moe.combine(y, inverse, w, h1)
+        want = (y.view(T, k, h).float() * w.unsqueeze(-1)).sum(1) + (0 if h1 is None else h1.float())
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        ok = want.isfinite()
+        assert ((got.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-5)[ok].all() and not ok.all()
+    assert _lib.take_device_error() == 0
