@@ -211,9 +211,11 @@ __device__ __forceinline__ void tma_store_wait_read0() {
 __device__ __forceinline__ void tma_store_wait_all0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---------------------------------------------------------------- one thread of a converged warp
-// The warps that issue tcgen05 instructions run their loops - waits, counters, descriptors - with all 32 lanes and let one
-// elected lane issue: the operands are then warp-uniform values. In a loop that only lane 0 runs they are not, and each
-// instruction paid for moving them (a K block of 64 in the few-tile GEMM: 0.30 us, elected 0.25 us).
+// The warps that issue tcgen05 instructions in the few-tile and the CTA-pair GEMM and in flash attention run their loops -
+// waits, counters, descriptors - with all 32 lanes and let one elected lane issue: the operands are then warp-uniform
+// values. In a loop that only lane 0 runs they are not, and each instruction paid for moving them (a K block of 64 in the
+// few-tile GEMM: 0.30 us, elected 0.25 us). The one-SM GEMM of 128 x 256 tiles (gemm_core.cuh, comm/tp_gemm.cu) still
+// issues from lane 0.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile(

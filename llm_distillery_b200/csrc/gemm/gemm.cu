@@ -960,8 +960,9 @@ static bool use_pair(int M, int N, int K) {
 // Which kernel takes a GEMM: the cluster kernel with tiles of 128 x bn and `slices` CTAs per tile, or (bn = 0) the
 // kernels of 128 x 256 and 256 x 256 tiles. The K slices decide the order of the additions, so the choice of `slices` is a
 // function of the sizes alone and is the same for the plain GEMM and for the ones with a fused epilogue. split = false
-// keeps the order of additions that the large tiles have. Every forward pass that a loss is taken of asks for that,
-// training or validation, and under the reference loss the backward pass too: that loss divides by the largest row and clips a difference of two
+// keeps the order of additions that the large tiles have (fp32 outputs of the 256 x 256 kernel are still cut by
+// pair_k_splits). Every forward pass that a loss is taken of asks for that, training or validation, and under the
+// reference loss the backward pass too: that loss divides by the largest row and clips a difference of two
 // cross-entropies, and turned a last bit of an activation into 0.1 to 0.7 % of its value (38 runs of five students, 200
 // to 1100 tokens; the KL losses: 0.001 %), so that the loss of a conversation would depend on the batch that it is in.
 //

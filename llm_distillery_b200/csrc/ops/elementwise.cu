@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(const __nv_bfloat
 }
 
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres) ; dw partial sums per block in fp32.
-// NV and NTB as in the forward kernel: with arrays for the longest row (NV = 4) a thread held 170 registers and an SM one
+// NV and NTB as in the forward kernel: with arrays for the longest row (NV = 4) a thread held 157 registers and an SM one
 // block, 8000 rows of 4096 took 210 us; sized for the row (NV = 2) several blocks share it.
 template <int NV, int NTB>
 __global__ void __launch_bounds__(NTB) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,

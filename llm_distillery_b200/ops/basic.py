@@ -34,7 +34,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          out_dtype: torch.dtype | None = None, accumulate: bool = False, alpha: float = 1.0,
          residual: torch.Tensor | None = None, desc_cfg: list[int] | None = None, split_k: bool = False) -> torch.Tensor:
     """C[M,N] = alpha * A @ B^T (+ C) (+ residual). ``split_k``: the reduction may be cut into slices that are added in
-    order (faster for outputs of few tiles; the last bits then depend on the sizes).
+    order (faster for outputs of few tiles; the last bits then depend on the sizes). Without it a row of a bf16 or fp16
+    result has the same bits whatever the other rows; fp32 outputs of many tiles are cut by their tile count either way.
 
     ``a`` is [M,K] (``a_mn=False``) or stored transposed as [K,M] (``a_mn=True``); ``b`` is [N,K] or stored as [K,N].
     Rows must be contiguous (stride(1) == 1); row strides must be multiples of 8 elements.
