@@ -24,22 +24,27 @@ for _n in ("b200_layer_fwd", "b200_layer_bwd", "b200_layer_saved_bytes", "b200_l
     _lib.KERNELS_PER_CALL[_n] = 0          # the calls return how many kernels they launched
 
 
-def fits(h, pos, cos, sin, weights, b_qkv, heads, training: bool) -> bool:
+def tables_fit(pos, cos, sin, tokens: int, d: int) -> bool:
+    if pos.dtype != torch.int32 or not pos.is_contiguous() or pos.shape != (tokens,):
+        return False
+    return all(t.dtype == torch.float32 and t.is_contiguous() and 2 * t.shape[1] == d and t.shape == cos.shape for t in (cos, sin))
+
+
+def fits(h, pos, cos, sin, weights, b_qkv, heads, training: bool, tables: bool | None = None) -> bool:
     """``heads`` = (query heads, key heads, head size). The C calls take sizes from the activations and trust the rest, so
-    what the separate calls would refuse is left to them."""
+    what the separate calls would refuse is left to them. ``tables``: what ``tables_fit`` said of the positions and tables,
+    for a caller that runs several layers on them (this check of a layer is 3 us of the host's time, with theirs 5)."""
     H, Hkv, d = heads
     T, w = h.shape
-    if not h.is_cuda or h.dtype != torch.bfloat16 or d not in (64, 128) or w % 8 or w > 8192:
+    bf16 = torch.bfloat16
+    if not h.is_cuda or h.dtype != bf16 or d not in (64, 128) or w % 8 or w > 8192:
         return False
-    if pos.dtype != torch.int32 or not pos.is_contiguous() or pos.shape != (T,):
+    if not (tables_fit(pos, cos, sin, T, d) if tables is None else tables):
         return False
-    for t in (cos, sin):
-        if t.dtype != torch.float32 or not t.is_contiguous() or 2 * t.shape[1] != d or t.shape != cos.shape:
-            return False
     n, f = (H + 2 * Hkv) * d, weights[4].shape[0] // 2
     shapes = ((w,), (n, w), (w, H * d), (w,), (2 * f, w), (w, f), (n,))
     for t, shape in zip(weights if b_qkv is None else weights + (b_qkv,), shapes):
-        if t.dtype != torch.bfloat16 or not t.is_cuda or not t.is_contiguous() or t.shape != shape:
+        if t.shape != shape or t.dtype != bf16 or not t.is_cuda or not t.is_contiguous():
             return False
         if training and t.requires_grad and getattr(t, "grad_slot", None) is None:
             return False

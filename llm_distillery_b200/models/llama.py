@@ -465,7 +465,9 @@ class LlamaModel(nn.Module):
         tables = self.layer_rope(cos, sin)
         meta7 = meta
         from . import layer_native
-        for li, (layer, (cos, sin)) in enumerate(zip(self.layers, tables)):
+        checked, tables_ok = None, False
+        for li, (layer, table) in enumerate(zip(self.layers, tables)):
+            cos, sin = table
             meta = meta7 + (cfg.layer_window(li, L),)       # the layer's sliding window when the sequence is longer
             if pre is not None:
                 pre(layer.first_param, False)
@@ -497,7 +499,9 @@ class LlamaModel(nn.Module):
                 b_qkv = getattr(layer, "qkv_bias", None)
                 w = (layer.input_layernorm, layer.qkv_proj, layer.o_proj, layer.post_attention_layernorm, layer.gate_up_proj,
                      layer.down_proj)
-                if layer_native.fits(h, pos, cos, sin, w, b_qkv, heads, training):
+                if table is not checked:
+                    checked, tables_ok = table, layer_native.tables_fit(pos, cos, sin, B * L, cfg.head_dim)
+                if layer_native.fits(h, pos, cos, sin, w, b_qkv, heads, training, tables_ok):
                     h = layer_native.NativeLayerFn.apply(h, pos, cos, sin, *w, b_qkv, meta, split)
                     continue
             h = DecoderLayerFn.apply(h, pos, cos, sin, layer.input_layernorm, layer.qkv_proj, layer.o_proj,
