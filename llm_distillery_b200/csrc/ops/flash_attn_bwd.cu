@@ -1,32 +1,36 @@
 // Causal GQA flash-attention backward for sm_100a on tcgen05 tensor cores.
 //
-// One CTA owns one (batch, kv-head, 128-key block): K_j and V_j stay resident in shared memory, dK_j and dV_j
-// accumulate in TMEM over every query head of the group and every query block at or after the diagonal, and
-// are written once. dQ is produced per (query block, key block) pair, staged in shared memory and added into an fp32
-// buffer by TMA reduce-add (whole 32-byte sectors per request instead of scattered per-thread atomics, which bound
-// an earlier version of this kernel), then converted to bf16 by a small kernel.
+// One CTA owns one (batch, kv-head, 128-key block) and a share of the query heads of its group: K_j and V_j stay resident
+// in shared memory, dK_j and dV_j accumulate in TMEM over those query heads and every query block at or after the diagonal.
+// dQ is produced per (query block, key block) pair, staged in shared memory and added into an fp32 buffer by TMA
+// reduce-add (whole 32-byte sectors per request), then converted to bf16 by a small kernel.
 //
-// Per iteration (query head hq, query block i), five tcgen05.mma groups:
-//   S  = Q_i K_j^T                 (A K-major, B K-major)        -> TMEM
-//   dP = dO_i V_j^T                (A K-major, B K-major)        -> TMEM
-//   softmax warps: P = exp2(S*c - lse), dS = P * (dP - delta) * scale, both written to smem in bf16
-//   dV += P^T  dO_i                (A = P  read MN-major, B = dO MN-major)
-//   dK += dS^T Q_i                 (A = dS read MN-major, B = Q  MN-major)
-//   dQ  = dS   K_j                 (A = dS K-major,       B = K  MN-major)
-// A [q x k] tile written row-per-thread in the 128B-swizzled K-major layout is, byte for byte, also the
-// MN-major layout of its transpose, so P and dS are stored once and read both ways.
+// Everything is computed TRANSPOSED (thread = key row, tile columns = queries), five tcgen05.mma groups per pair:
+//   S^T  = K_j Q_i^T               (A K-major, B K-major)               -> TMEM
+//   dP^T = V_j dO_i^T              (A K-major, B K-major)               -> TMEM
+//   compute warps: P = exp2(S*c - lse), dS = P * (dP - delta) * scale; P^T goes back into TMEM over S^T, dS^T into TMEM over
+//   dP^T (head dim 64) and into shared memory, both bf16
+//   dV += P^T  dO_i                (A = P^T from TMEM, B = dO MN-major)
+//   dK += dS^T Q_i                 (A = dS^T from TMEM (64) or shared memory K-major (128), B = Q MN-major)
+//   dQ  = dS   K_j                 (A = dS^T read MN-major, B = K MN-major)
+// so that P never touches shared memory and dS is read from it once (64): per pair the MMAs read 144 KB of operands there
+// where the form with queries as rows read 224 KB, at 128 B per clock the busiest path of that form.
 //
-// Roles: warp 0 TMA producer (Q_i / dO_i ring); warps 1-4 issue the MMA groups, one group each (S and dP; dV; dK; dQ):
-// every tcgen05 instruction - an MMA, a commit, a completed mbarrier wait - costs its issuing thread on the order of a
-// hundred cycles here, so one thread issuing the 32 MMAs of a pair needed ~3.8 K cycles per pair and was what bound
-// the kernel (the tensor core needs ~1.3 K); warps 5-20 softmax + dQ drain + epilogue: each TMEM lane quadrant is
-// served by four warps that split the tile's columns.
-// What bounds the kernel now is shared-memory bandwidth: a pair's MMAs read ~224 KB of operands from shared memory
-// (every operand of the five groups lives there) next to ~100 KB of P / dS / dQ-staging traffic from the warps, at
-// ~128 B per clock. Two variants measured no faster and were dropped: the next pair's S / dP MMAs issued ahead of
-// this pair's dV / dK / dQ (0.654 against 0.648 ms at head dim 64), and dedicated dQ drain warps with packed f32x2
-// softmax arithmetic (0.673 ms). Less operand traffic needs P^T / dS^T (and K, V) as TMEM operands, i.e. the
-// transposed S^T = K Q^T formulation.
+// Roles (512 threads): warp 0 loads (TMA: Q_i and dO_i rings; -lse and -delta of a query block, scaled, through registers);
+// warp 1 issues S and dP, warp 2 dV, warp 3 dK and dQ; warps 4-7 drain dQ (each its own 32 rows: TMEM -> staging -> TMA
+// reduce, no barrier between them); warps 8-15 compute, two per TMEM lane quadrant, 64 query columns each.
+// Order: S of the next pair is issued while the compute warps work on this one, so they go from dS_i straight to the
+// exponentials of pair i + 1 while dK_i, dP_{i+1} and dQ_i run. Head dim 64: two S buffers; P_i in the lower half of its
+// buffer, dQ_i in the upper half. Head dim 128 (S, dP, dV, dK take all 512 columns): one S buffer, dQ_i over dP_i.
+// The compute warps' fixed work is 16 K exponentials a pair (1024 clocks of the MUFU unit). Neither they (all of them taken
+// out: 7 % faster at head dim 64) nor the reduce-adds (2.5 %) bound the kernel, but the chain dS_i -> dK_i -> dP_{i+1} -> dS_{i+1}
+// with its barriers, about 3500 clocks a pair at head dim 64 and 4600 at 128.
+// All three kernels of a backward pass, B200, queries as rows and one S / dP buffer before / now: 8 x 2048, 32/4 heads of 64
+// 638 / 570 us; 4 x 4096, 32/8 of 64 1136 / 994; 2 x 4096, 32/8 of 128 1199 / 808; 1 x 777, 14/2 of 64 122 / 34.
+//
+// Few key blocks (short sequences, few kv heads) leave SMs idle while each CTA walks all query heads of its group: then a
+// cluster of up to 8 CTAs shares the heads, and the partial dK / dV meet through distributed shared memory, added in the
+// order of the CTAs' ranks (`head_split` below; results repeat bit for bit).
 #include "../common/ptx.cuh"
 #include "../common/host.cuh"
 
@@ -35,47 +39,56 @@ namespace fab {
 
 constexpr int BM = 128;  // queries per block
 constexpr int BN = 128;  // keys per block
-constexpr int NSPLIT = 4;        // softmax/drain warps per TMEM lane quadrant: each takes 1/4 of a tile's columns
-constexpr int NISSUE = 4;                        // MMA-issuing warps: S/dP, dV, dK, dQ
-constexpr int FIRST_WORK_WARP = 1 + NISSUE;      // warp 0 is the TMA producer
-constexpr int NTHREADS = 32 * FIRST_WORK_WARP + 4 * NSPLIT * 32;  // + 16 softmax/drain warps
-constexpr int NWORK = 4 * NSPLIT * 32;          // threads that arrive on the softmax/drain barriers
+constexpr int NTHREADS = 512;
+constexpr int FIRST_DRAIN_WARP = 4;
+constexpr int FIRST_COMPUTE_WARP = 8;
+constexpr int NCOMPUTE_WARPS = 8;
+constexpr int SUB = 128 * 128;   // bytes of a [128 rows x 64] bf16 sub-tile with 128-byte rows
 
 template <int D>
 struct Cfg {
-  static constexpr int STAGES = (D == 64) ? 2 : 1;
+  static constexpr int QS = (D == 64) ? 3 : 2;     // Q ring: Q_i is read by S_i first and by dK_i last
+  static constexpr int OS = (D == 64) ? 2 : 1;     // dO ring: dP_i first, dV_i last
+  static constexpr int NSB = (D == 64) ? 2 : 1;    // S buffers in TMEM
+  static constexpr int NDS = (D == 64) ? 2 : 1;    // dS buffers in shared memory
+  static constexpr bool DS_TMEM = (D == 64);       // dK reads dS^T from TMEM (else from shared memory)
   static constexpr int KV_BYTES = BN * D * 2;   // one of K or V
-  static constexpr int QDO_BYTES = BM * D * 2;  // one of Q or dO
-  static constexpr int STAGE_BYTES = 2 * QDO_BYTES;
+  static constexpr int Q_BYTES = BM * D * 2;    // one of Q or dO
   static constexpr int P_BYTES = BM * BN * 2;
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = KV_BYTES;
-  static constexpr int OFF_QDO = 2 * KV_BYTES;
-  static constexpr int OFF_P = OFF_QDO + STAGES * STAGE_BYTES;
-  static constexpr int OFF_DS = OFF_P + P_BYTES;
-  static constexpr int OFF_DQS = OFF_DS + P_BYTES;  // dQ staging: two [128 x 32] fp32 sub-tiles, 128B-swizzled
-  static constexpr int DQS_BYTES = 2 * BM * 128;
-  static constexpr int OFF_BAR = OFF_DQS + DQS_BYTES;
-  static constexpr int SMEM_BYTES = OFF_BAR + 256;
-  static constexpr bool ALIAS = (D == 128);  // dQ shares TMEM columns with S
+  static constexpr int OFF_Q = 2 * KV_BYTES;
+  static constexpr int OFF_DO = OFF_Q + QS * Q_BYTES;
+  static constexpr int OFF_DS = OFF_DO + OS * Q_BYTES;
+  static constexpr int OFF_DQS = OFF_DS + NDS * P_BYTES;   // dQ staging: per drain warp two [32 x 32] fp32 tiles, 128B-swizzled
+  static constexpr int DQS_BYTES = 4 * 2 * 4096;
+  static constexpr int OFF_STAT = OFF_DQS + DQS_BYTES;     // per Q stage: -lse (log2 units) and -delta * scale of 128 queries
+  static constexpr int STAT_BYTES = 2 * BM * 4;
+  static constexpr int OFF_BAR = OFF_STAT + QS * STAT_BYTES;
+  static constexpr int SMEM_BYTES = OFF_BAR + 512;
+  static constexpr int RED_PITCH = 2 * D + 4;              // floats per key row of the cluster's dK | dV exchange (over K, V, Q ...)
+  static_assert(BN * RED_PITCH * 4 <= OFF_DQS, "the exchange may not reach the staging tiles, which the TMA may still read");
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
   static constexpr uint32_t S_COL = 0;
-  static constexpr uint32_t DP_COL = 128;
-  static constexpr uint32_t DV_COL = 256;
-  static constexpr uint32_t DK_COL = 256 + D;
-  static constexpr uint32_t DQ_COL = ALIAS ? 0 : 256 + 2 * D;
-  // head dim 64 leaves 64 TMEM columns free: a second dQ accumulator lets the pair loop run two pairs deep
-  static constexpr bool PIPE = !ALIAS;
-  static constexpr uint32_t DQ_COL1 = PIPE ? 256 + 3 * D : DQ_COL;
+  static constexpr uint32_t DP_COL = NSB * 128;
+  static constexpr uint32_t DV_COL = DP_COL + 128;
+  static constexpr uint32_t DK_COL = DV_COL + D;
   static constexpr uint32_t TMEM_COLS = 512;
+  static_assert(DK_COL + D == TMEM_COLS, "TMEM budget");
+  // P^T, 16 queries per 8 columns: at the start of the S buffer (64: dQ needs 64 whole columns behind it, so the second
+  // warp of a quadrant stores over scores of the first), or each warp's at the start of its own half (128)
+  static constexpr uint32_t P_HALF = (D == 64) ? 32 : 64;
+  // dQ of a pair: the upper half of its S buffer (64), or over dP (128)
+  static __device__ __forceinline__ uint32_t dq_col(int buf) { return D == 64 ? S_COL + buf * 128 + 64 : DP_COL; }
 };
 
 struct BwdParams {
   const float* lse;    // [H, T]
   const float* delta;  // [H, T]
-  float* dq_acc;       // [T, H*D] fp32, zeroed by the launcher
   __nv_bfloat16* dqkv; // [T, (H+2Hkv)*D]
   int B, L, H, Hkv;
   int window;          // > 0: the query at position i saw the keys j with i - window < j <= i; 0: all j <= i
+  int hsplit;          // CTAs (one cluster) that share the query heads of a group
   float scale;
 };
 
@@ -84,39 +97,45 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmDO,
                      const __grid_constant__ CUtensorMap tmDQ, BwdParams p, unsigned int* err_word) {
   using C = Cfg<D>;
-  constexpr int ST = C::STAGES;
+  constexpr int QS = C::QS, OS = C::OS, NSB = C::NSB;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
+  // Barriers that more than one pair can complete before their waiter looks are kept per buffer: a parity wait must never
+  // be overtaken by two phases. Beside each: who arrives.
   uint64_t* kv_full = bars + 0;
-  uint64_t* qdo_full = bars + 1;   // [2]
-  uint64_t* qdo_empty = bars + 3;  // [2]
-  uint64_t* sdp_full = bars + 5;
-  uint64_t* pds_ready = bars + 6;
-  uint64_t* dq_full = bars + 7;
-  uint64_t* dq_empty = bars + 8;
-  uint64_t* stage_full = bars + 9;   // dQ staging tile written by the drain threads (all of them arrive)
-  uint64_t* stage_free = bars + 10;  // ... and read out by the TMA reduce
-  uint64_t* dq_full1 = bars + 11;    // second dQ accumulator (pipelined variant)
-  uint64_t* dq_empty1 = bars + 12;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+  uint64_t* q_full = bars + 1;      // [QS] TMA bytes + the loader's statistics
+  uint64_t* q_empty = bars + 4;     // [QS] dK
+  uint64_t* do_full = bars + 7;     // [OS]
+  uint64_t* do_empty = bars + 9;    // [OS] dP, dV
+  uint64_t* s_full = bars + 11;     // [NSB]
+  uint64_t* p_ready = bars + 13;    // [NSB] compute warps
+  uint64_t* dv_done = bars + 15;    // [NSB]
+  uint64_t* dq_full = bars + 17;    // [NSB]
+  uint64_t* dq_empty = bars + 19;   // [NSB] drain warps
+  uint64_t* dp_full = bars + 21;
+  uint64_t* ds_ready = bars + 22;   // compute warps
+  uint64_t* dk_done = bars + 23;
+  uint64_t* s_read = bars + 24;     // [2][4] the first warp of a quadrant has read its half of S: the other may store P there
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 32);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nkb = (p.L + BN - 1) / BN;
-  // blockIdx.y = key block (block 0 has the most work), blockIdx.x = (kv head, batch): blocks are handed out x-fastest,
-  // so all the heavy key blocks of every head start first and the light ones fill the tail
+  // blockIdx.y = key block (block 0 has the most work), blockIdx.x = (batch, kv head, share of the heads): blocks are handed
+  // out x-fastest, so all the heavy key blocks of every head start first and the light ones fill the tail
   const int jb = blockIdx.y;
-  const int hkv = blockIdx.x % p.Hkv, b = blockIdx.x / p.Hkv;
+  const int part = blockIdx.x % p.hsplit;
+  const int bh = blockIdx.x / p.hsplit;
+  const int hkv = bh % p.Hkv, b = bh / p.Hkv;
   const int g = p.H / p.Hkv;
+  const int h_first = hkv * g + g * part / p.hsplit, h_last = hkv * g + g * (part + 1) / p.hsplit;
   const int kv0 = jb * BN;
   // query blocks that see this key block: from the diagonal to the end, or to the last query whose window reaches back
   const int q_end = p.window > 0 ? min(p.L, kv0 + BN - 1 + p.window) : p.L;
   const int nqb = (q_end + BM - 1) / BM;
   const int i_start = kv0 / BM;
   const int nqi = nqb - i_start;
-  const int n_it = g * nqi;
+  const int n_it = (h_last - h_first) * nqi;
   const long long T = (long long)p.B * p.L;
-  (void)nkb;
 
   if ((smem_u32(smem) & 1023u) != 0u) {
     if (threadIdx.x == 0 && err_word) atomicCAS(err_word, 0u, (unsigned)ERR_BAD_ARG);
@@ -127,18 +146,25 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     tma_prefetch_desc(&tmDO);
     tma_prefetch_desc(&tmDQ);
     mbar_init(kv_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&qdo_full[s], 1);
-      mbar_init(&qdo_empty[s], 1);
+    for (int s = 0; s < QS; ++s) {
+      mbar_init(&q_full[s], 2);
+      mbar_init(&q_empty[s], 1);
     }
-    mbar_init(sdp_full, 1);
-    mbar_init(pds_ready, NWORK);
-    mbar_init(dq_full, 3);     // "pair done": the dV, dK and dQ issuers each commit to it
-    mbar_init(dq_empty, NWORK);
-    mbar_init(stage_full, NWORK);
-    mbar_init(stage_free, 1);
-    mbar_init(dq_full1, 3);
-    mbar_init(dq_empty1, NWORK);
+    for (int s = 0; s < OS; ++s) {
+      mbar_init(&do_full[s], 1);
+      mbar_init(&do_empty[s], 2);
+    }
+    for (int s = 0; s < NSB; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&p_ready[s], NCOMPUTE_WARPS);
+      mbar_init(&dv_done[s], 1);
+      mbar_init(&dq_full[s], 1);
+      mbar_init(&dq_empty[s], 4);
+    }
+    mbar_init(dp_full, 1);
+    mbar_init(ds_ready, NCOMPUTE_WARPS);
+    mbar_init(dk_done, 1);
+    for (int s = 0; s < 8; ++s) mbar_init(&s_read[s], 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -155,316 +181,395 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
   const int colK = p.H * D + hkv * D;
   const int colV = (p.H + p.Hkv) * D + hkv * D;
+  auto spin = [&](uint64_t* bar, uint32_t parity, unsigned int code) {
+    return __all_sync(0xffffffffu, mbar_spin_bounded(bar, parity, abort_flag, err_word, code)) != 0;
+  };
 
-  if (warp == 0) {
-    if (lane == 0) {
-      mbar_arrive_expect_tx(kv_full, 2 * C::KV_BYTES);
-#pragma unroll
-      for (int c = 0; c < D / 64; ++c) {
-        tma_load_3d(smem + C::OFF_K + c * (BN * 128), &tmQKV, kv_full, colK + c * 64, kv0, b);
-        tma_load_3d(smem + C::OFF_V + c * (BN * 128), &tmQKV, kv_full, colV + c * 64, kv0, b);
-      }
-      for (int it = 0; it < n_it; ++it) {
-        const int s = it % ST;
-        const uint32_t ph = (it / ST) & 1u;
-        const int hq = hkv * g + it / nqi;
-        const int q0 = (i_start + it % nqi) * BM;
-        (void)ph;
-        if (it >= ST) {
-          // the stage was read by pair it - ST: free once that pair's dV, dK and dQ MMAs are done (the S / dP MMAs of a
-          // pair complete before its softmax and so before these are even issued)
-          const int pd = it - ST;
-          uint64_t* done = (C::PIPE && (pd & 1)) ? dq_full1 : dq_full;
-          const uint32_t par = C::PIPE ? ((pd >> 1) & 1u) : (pd & 1u);
-          if (!mbar_spin_bounded(done, par, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
-        }
-        uint8_t* sQ = smem + C::OFF_QDO + s * C::STAGE_BYTES;
-        uint8_t* sDO = sQ + C::QDO_BYTES;
-        mbar_arrive_expect_tx(&qdo_full[s], C::STAGE_BYTES);
+  // Registers: 128 a thread at launch; the compute warps hold 64 probabilities and 64 scores. 4 x (64 + 104 + 2 x 168) x 32 =
+  // 64512 of the 65536 that the block was launched with.
+  if (warp < FIRST_DRAIN_WARP) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    if (warp == 0) {
+      // ---------------------------------------------------------------- loads
+      if (elect_one()) {
+        mbar_arrive_expect_tx(kv_full, 2 * C::KV_BYTES);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
-          tma_load_3d(sQ + c * (BM * 128), &tmQKV, &qdo_full[s], hq * D + c * 64, q0, b);
-          tma_load_3d(sDO + c * (BM * 128), &tmDO, &qdo_full[s], hq * D + c * 64, q0, b);
+          tma_load_3d(smem + C::OFF_K + c * SUB, &tmQKV, kv_full, colK + c * 64, kv0, b);
+          tma_load_3d(smem + C::OFF_V + c * SUB, &tmQKV, kv_full, colV + c * 64, kv0, b);
         }
       }
-    }
-  } else if (warp < FIRST_WORK_WARP) {
-    // ------------------------------------------------------------------ MMA issuers (one elected thread per warp)
-    {
-      auto spin = [&](uint64_t* bar, uint32_t parity, unsigned int code) {
-        return __all_sync(0xffffffffu, mbar_spin_bounded(bar, parity, abort_flag, err_word, code)) != 0;
+      __syncwarp();
+      float st_l[4], st_d[4];      // statistics of the next query block: loaded one pair ahead
+      auto load_stats = [&](int hq, int qb) {
+        const long long row = (long long)hq * T + (long long)b * p.L;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int qi = qb * BM + j * 32 + lane;
+          const bool ok = qi < p.L;
+          st_l[j] = ok ? p.lse[row + qi] : INFINITY;   // rows past the end: exp2(s - inf) = 0, P and dS vanish
+          st_d[j] = ok ? p.delta[row + qi] : 0.f;
+        }
       };
-      const uint32_t sK = smem_u32(smem + C::OFF_K);
-      const uint32_t sV = smem_u32(smem + C::OFF_V);
-      const uint32_t sP = smem_u32(smem + C::OFF_P);
-      const uint32_t sDS = smem_u32(smem + C::OFF_DS);
+      int hq = h_first, qb = i_start;
+      load_stats(hq, qb);
+      for (int it = 0; it < n_it; ++it) {
+        const int qs = it % QS, os = it % OS;
+        const int hq_now = hq, q0 = qb * BM;
+        if (it >= QS && !spin(&q_empty[qs], (it / QS - 1) & 1u, ERR_WAIT_EMPTY)) break;
+        if (elect_one()) {
+          uint8_t* sQ = smem + C::OFF_Q + qs * C::Q_BYTES;
+          mbar_arrive_expect_tx(&q_full[qs], C::Q_BYTES);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sQ + c * SUB, &tmQKV, &q_full[qs], hq_now * D + c * 64, q0, b);
+        }
+        __syncwarp();
+        float* stat = reinterpret_cast<float*>(smem + C::OFF_STAT + qs * C::STAT_BYTES);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          stat[j * 32 + lane] = -(st_l[j] * 1.4426950408889634f);
+          stat[BM + j * 32 + lane] = -(st_d[j] * p.scale);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&q_full[qs]);
+        if (++qb == nqb) {
+          qb = i_start;
+          ++hq;
+        }
+        if (it + 1 < n_it) load_stats(hq, qb);
+        if (it >= OS && !spin(&do_empty[os], (it / OS - 1) & 1u, ERR_WAIT_EMPTY)) break;
+        if (elect_one()) {
+          uint8_t* sDO = smem + C::OFF_DO + os * C::Q_BYTES;
+          mbar_arrive_expect_tx(&do_full[os], C::Q_BYTES);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sDO + c * SUB, &tmDO, &do_full[os], hq_now * D + c * 64, q0, b);
+        }
+        __syncwarp();
+      }
+    } else {
+      // ---------------------------------------------------------------- MMA issuers (warp-uniform loops, one elected lane issues)
       // Base descriptors, built once: inside the loops an MMA's operands are a base plus a constant (k-step) and a
       // stage offset. The address field counts 16-byte units and never carries out of its 14 bits below 256 KB.
-      const uint32_t sQ0 = smem_u32(smem + C::OFF_QDO), sDO0 = sQ0 + C::QDO_BYTES;
+      const uint32_t sK = smem_u32(smem + C::OFF_K), sV = smem_u32(smem + C::OFF_V), sQ = smem_u32(smem + C::OFF_Q),
+                     sDO = smem_u32(smem + C::OFF_DO), sDS = smem_u32(smem + C::OFF_DS);
       auto koff = [](int k) -> uint64_t {   // k-step inside a K-major tile: 64-column sub-tiles 16 KB apart, 32 B per step
-        return static_cast<uint64_t>(((k >> 2) * (128 * 128) + (k & 3) * 32) >> 4);
+        return static_cast<uint64_t>(((k >> 2) * SUB + (k & 3) * 32) >> 4);
       };
-      auto stage_off = [](int it) -> uint64_t { return static_cast<uint64_t>(((it % ST) * C::STAGE_BYTES) >> 4); };
-      // "pair done" barrier of pair `it` (count 3) and the parity of its phase
-      auto pair_bar = [&](int it) -> uint64_t* { return (C::PIPE && (it & 1)) ? dq_full1 : dq_full; };
+      auto units = [](int n, int bytes) -> uint64_t { return static_cast<uint64_t>((n * bytes) >> 4); };
       if (warp == 1) {
-        // S = Q K^T and dP = dO V^T (both operands K-major) -> TMEM. Pair it + 1 is issued as soon as the softmax warps
-        // have read S / dP of pair it, i.e. AHEAD of pair it's dV / dK / dQ, which the other issuers handle.
-        const uint32_t idesc_kk = make_idesc_f16(1, BM, BN, 0, 0);
-        const uint64_t kQ = make_smem_desc_sw128(sQ0, 16, 1024), kDO = make_smem_desc_sw128(sDO0, 16, 1024);
+        const uint32_t idesc_kk = make_idesc_f16(1, BN, BM, 0, 0);
+        const uint64_t kQ = make_smem_desc_sw128(sQ, 16, 1024), kDO = make_smem_desc_sw128(sDO, 16, 1024);
         const uint64_t kK = make_smem_desc_sw128(sK, 16, 1024), kV = make_smem_desc_sw128(sV, 16, 1024);
-        bool ok = spin(kv_full, 0, ERR_WAIT_FULL);
-        for (int it = 0; ok && it < n_it; ++it) {
-          if (!spin(&qdo_full[it % ST], (it / ST) & 1u, ERR_WAIT_FULL)) break;
-          if (it > 0) {
-            if constexpr (C::PIPE) {
-              if (!spin(pds_ready, (it - 1) & 1u, ERR_WAIT_AUX)) break;
-            } else {  // dQ shares its TMEM columns with S: they are free when the drain of pair it - 1 is through
-              if (!spin(dq_empty, (it - 1) & 1u, ERR_WAIT_AUX)) break;
-            }
+        auto issue_s = [&](int it) -> bool {
+          if (!spin(&q_full[it % QS], (it / QS) & 1u, ERR_WAIT_FULL)) return false;
+          if (it >= NSB) {      // the buffer held P (read by dV) and, head dim 64, dQ of pair it - NSB
+            const int o = it - NSB;
+            if (!spin(&dv_done[o % NSB], (o / NSB) & 1u, ERR_WAIT_AUX)) return false;
+            if (D == 64 && !spin(&dq_empty[o % NSB], (o / NSB) & 1u, ERR_WAIT_AUX)) return false;
           }
           tc_fence_after_sync();
-          const uint64_t stage = stage_off(it);
+          const uint64_t q = kQ + units(it % QS, C::Q_BYTES);
+          const uint32_t dst = tmem_base + C::S_COL + (it % NSB) * 128;
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < D / 16; ++k) umma_f16_ss(dst, kK + koff(k), q + koff(k), idesc_kk, k != 0 ? 1u : 0u);
+            umma_commit(&s_full[it % NSB]);
+          }
+          __syncwarp();
+          return true;
+        };
+        bool ok = spin(kv_full, 0, ERR_WAIT_FULL) && issue_s(0);
+        for (int it = 0; ok && it < n_it; ++it) {
+          if (!spin(&do_full[it % OS], (it / OS) & 1u, ERR_WAIT_FULL)) break;
+          if (it > 0) {   // dP of pair it - 1 has been read, and what took its columns since: dS^T by dK (64), dQ by the drain (128)
+            if (D == 64 ? !spin(dk_done, (it - 1) & 1u, ERR_WAIT_AUX) : !spin(&dq_empty[0], (it - 1) & 1u, ERR_WAIT_AUX)) break;
+          }
+          tc_fence_after_sync();
+          const uint64_t o = kDO + units(it % OS, C::Q_BYTES);
           if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < D / 16; ++k)
-              umma_f16_ss(tmem_base + C::S_COL, kQ + stage + koff(k), kK + koff(k), idesc_kk, k != 0 ? 1u : 0u);
-#pragma unroll
-            for (int k = 0; k < D / 16; ++k)
-              umma_f16_ss(tmem_base + C::DP_COL, kDO + stage + koff(k), kV + koff(k), idesc_kk, k != 0 ? 1u : 0u);
-            umma_commit(sdp_full);
+              umma_f16_ss(tmem_base + C::DP_COL, kV + koff(k), o + koff(k), idesc_kk, k != 0 ? 1u : 0u);
+            umma_commit(dp_full);
+            umma_commit(&do_empty[it % OS]);
           }
           __syncwarp();
+          if (it + 1 < n_it && !issue_s(it + 1)) break;
         }
-      } else if (warp == 2 || warp == 3) {
-        // dV += P^T dO (warp 2) ; dK += dS^T Q (warp 3): reduction over the 128 queries, 16 per step = 2048 B per step
-        // in both tiles, both operands MN-major
-        const uint32_t idesc_tt = make_idesc_f16(1, BN, D, 1, 1);
-        const uint64_t tA = make_smem_desc_sw128(warp == 2 ? sP : sDS, BM * 128, 1024);
-        const uint64_t tB = make_smem_desc_sw128(warp == 2 ? sDO0 : sQ0, BM * 128, 1024);
-        const uint32_t dcol = tmem_base + (warp == 2 ? C::DV_COL : C::DK_COL);
+      } else if (warp == 2) {
+        const uint32_t idesc = make_idesc_f16(1, BN, D, 0, 1);
+        const uint64_t tDO = make_smem_desc_sw128(sDO, SUB, 1024);
         for (int it = 0; it < n_it; ++it) {
-          if (!spin(pds_ready, it & 1u, ERR_WAIT_AUX)) break;
+          const int bf = it % NSB;
+          if (!spin(&p_ready[bf], (it / NSB) & 1u, ERR_WAIT_AUX)) break;
+          if (!spin(&do_full[it % OS], (it / OS) & 1u, ERR_WAIT_FULL)) break;
           tc_fence_after_sync();
-          const uint64_t stage = stage_off(it);
+          const uint64_t o = tDO + units(it % OS, C::Q_BYTES);
+          const uint32_t pcol = tmem_base + C::S_COL + bf * 128;
           if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < BM / 16; ++k)
-              umma_f16_ss(dcol, tA + (uint64_t)(k * 128), tB + stage + (uint64_t)(k * 128), idesc_tt,
+              umma_f16_ts(tmem_base + C::DV_COL, pcol + (k >> 2) * C::P_HALF + (k & 3) * 8, o + (uint64_t)(k * 128), idesc,
                           (it != 0 || k != 0) ? 1u : 0u);
-            umma_commit(pair_bar(it));
+            umma_commit(&dv_done[bf]);
+            umma_commit(&do_empty[it % OS]);
           }
           __syncwarp();
         }
       } else {
-        // dQ = dS K (reduction over the 128 keys; dS K-major, K MN-major) into the pair's accumulator
-        const uint32_t idesc_kt = make_idesc_f16(1, BM, D, 0, 1);
-        const uint64_t kDS = make_smem_desc_sw128(sDS, 16, 1024);
-        const uint64_t tK = make_smem_desc_sw128(sK, BN * 128, 1024);
+        const uint32_t idesc_dk = make_idesc_f16(1, BN, D, 0, 1);      // A = dS^T with queries as its K dimension
+        const uint32_t idesc_dq = make_idesc_f16(1, BM, D, 1, 1);
+        const uint64_t tQ = make_smem_desc_sw128(sQ, SUB, 1024), tK = make_smem_desc_sw128(sK, SUB, 1024);
+        const uint64_t kDS = make_smem_desc_sw128(sDS, 16, 1024), tDS = make_smem_desc_sw128(sDS, SUB, 1024);
         bool ok = spin(kv_full, 0, ERR_WAIT_FULL);
         for (int it = 0; ok && it < n_it; ++it) {
-          if (!spin(pds_ready, it & 1u, ERR_WAIT_AUX)) break;
-          uint32_t dq_col = C::DQ_COL;
-          if constexpr (C::PIPE) {
-            dq_col = (it & 1) ? C::DQ_COL1 : C::DQ_COL;
-            if (it >= 2) {  // the drain of pair it-2 has emptied this accumulator
-              if (!spin((it & 1) ? dq_empty1 : dq_empty, ((it >> 1) - 1) & 1u,
-                                     ERR_WAIT_AUX))
-                break;
-            }
-          }
+          if (!spin(ds_ready, it & 1u, ERR_WAIT_AUX)) break;
           tc_fence_after_sync();
+          const uint64_t q = tQ + units(it % QS, C::Q_BYTES);
+          const uint64_t ds = units(it % C::NDS, C::P_BYTES);
+          const uint32_t dq = tmem_base + C::dq_col(it % NSB);
           if (elect_one()) {
+            auto dk = [&]() {
 #pragma unroll
-            for (int k = 0; k < BN / 16; ++k)
-              umma_f16_ss(tmem_base + dq_col, kDS + koff(k), tK + (uint64_t)(k * 128), idesc_kt, k != 0 ? 1u : 0u);
-            umma_commit(pair_bar(it));
+              for (int k = 0; k < BM / 16; ++k) {
+                const uint32_t acc = (it != 0 || k != 0) ? 1u : 0u;
+                if constexpr (C::DS_TMEM)   // a compute warp's 64 queries lie at the start of its own half of dP's columns
+                  umma_f16_ts(tmem_base + C::DK_COL, tmem_base + C::DP_COL + (k >> 2) * 64 + (k & 3) * 8,
+                              q + (uint64_t)(k * 128), idesc_dk, acc);
+                else
+                  umma_f16_ss(tmem_base + C::DK_COL, kDS + ds + koff(k), q + (uint64_t)(k * 128), idesc_dk, acc);
+              }
+              umma_commit(dk_done);
+              umma_commit(&q_empty[it % QS]);
+            };
+            auto dqm = [&]() {
+#pragma unroll
+              for (int k = 0; k < BN / 16; ++k)
+                umma_f16_ss(dq, tDS + ds + (uint64_t)(k * 128), tK + (uint64_t)(k * 128), idesc_dq, k != 0 ? 1u : 0u);
+              umma_commit(&dq_full[it % NSB]);
+            };
+            // first what the next dP waits for: dK frees dP's columns (64), dQ has to be drained from them (128)
+            if constexpr (D == 64) {
+              dk();
+              dqm();
+            } else {
+              dqm();
+              dk();
+            }
           }
           __syncwarp();
         }
       }
     }
-  } else {
+  } else if (warp < FIRST_COMPUTE_WARP) {
+    // ------------------------------------------------------------------ dQ: TMEM -> staging -> TMA reduce-add
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
     const int quad = warp & 3;
-    const int part = (warp - FIRST_WORK_WARP) >> 2;  // which quarter of the columns this warp handles
-    const int r = quad * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const float c2 = p.scale * 1.4426950408889634f;
-    uint8_t* sP = smem + C::OFF_P;
-    uint8_t* sDS = smem + C::OFF_DS;
-    constexpr int DW = D / NSPLIT;     // columns of dQ / dK / dV per warp: 16 (D = 64) or 32 (D = 128)
-    constexpr int ROUNDS = D / 64;     // the dQ staging area holds two 32-column sub-tiles per round
-    const int dc0 = part * DW;         // first dQ / dK / dV column of this warp
-    bool ok = true;
-    uint32_t rd = 0;  // staging rounds so far
-    uint8_t* sDQ = smem + C::OFF_DQS;
-    const int st = dc0 >> 5;               // 32-column sub-tile of dQ this warp contributes to
-    const int chunkbase = (dc0 & 31) >> 2;  // first 16-byte chunk (4 floats) inside the 128-byte row
-    // Drain the dQ accumulator of pair `itd` into the fp32 gradient: TMEM -> registers -> swizzled staging tile in
-    // shared memory (row r, 128-byte rows of 32 floats) -> TMA reduce-add issued by one thread. The staging area holds
-    // two 32-column sub-tiles: D = 128 takes two rounds, and in each round only the warps whose columns belong to
-    // that round write (everybody arrives on the barriers). The caller has waited for the pair's dq_full barrier.
-    auto drain = [&](int itd) {
-      const int hq = hkv * g + itd / nqi;
-      const int q0 = (i_start + itd % nqi) * BM;
-      const uint32_t dq_col = (C::PIPE && (itd & 1)) ? C::DQ_COL1 : C::DQ_COL;
-      uint32_t v[DW];
-      if constexpr (DW == 32) tmem_ld_32x32b_x32(tmem_base + lane_addr + dq_col + dc0, v);
-      else tmem_ld_32x32b_x16(tmem_base + lane_addr + dq_col + dc0, v);
-      tmem_ld_wait();
+    uint8_t* stage = smem + C::OFF_DQS + quad * 8192;
+    int hq = h_first, qb = i_start;
+    for (int it = 0; it < n_it; ++it) {
+      const int bf = it % NSB;
+      if (!spin(&dq_full[bf], (it / NSB) & 1u, ERR_WAIT_AUX)) break;
+      tc_fence_after_sync();
+      const uint32_t src = tmem_base + lane_addr + C::dq_col(bf);
 #pragma unroll
-      for (int rr = 0; rr < ROUNDS; ++rr) {
-        // the previous round's reduce must have finished READING the staging tile. The thread that issued it checks
-        // that only now, a whole softmax phase later, so that the TMA engine's latency is off the critical path.
-        if (warp == FIRST_WORK_WARP && lane == 0 && rd > 0) {
-          tma_store_wait_read0();
-          mbar_arrive(stage_free);
+      for (int rr = 0; rr < D / 64; ++rr) {
+        uint32_t v0[32], v1[32];
+        tmem_ld_32x32b_x32(src + rr * 64, v0);
+        tmem_ld_32x32b_x32(src + rr * 64 + 32, v1);
+        tmem_ld_wait();
+        if (rr + 1 == D / 64) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&dq_empty[bf]);
         }
+        if (lane == 0) tma_store_wait_read0();   // the reduce before this one has read the staging tiles
         __syncwarp();
-        if (rd > 0) {
-          int w3 = mbar_wait_bounded(stage_free, (rd - 1) & 1u, abort_flag, err_word, ERR_WAIT_AUX) ? 1 : 0;
-          if (!__all_sync(0xffffffffu, w3)) { ok = false; break; }
-        }
-        if ((st >> 1) == rr) {
-          uint8_t* rowp = sDQ + (st & 1) * (BM * 128) + r * 128;
+        uint8_t* rowp = stage + lane * 128;
 #pragma unroll
-          for (int q4 = 0; q4 < DW / 4; ++q4)
-            *reinterpret_cast<uint4*>(rowp + (((chunkbase + q4) ^ (r & 7)) * 16)) =
-                make_uint4(v[q4 * 4], v[q4 * 4 + 1], v[q4 * 4 + 2], v[q4 * 4 + 3]);
+        for (int c = 0; c < 8; ++c) {
+          const int off = (c ^ (lane & 7)) * 16;
+          *reinterpret_cast<uint4*>(rowp + off) = make_uint4(v0[c * 4], v0[c * 4 + 1], v0[c * 4 + 2], v0[c * 4 + 3]);
+          *reinterpret_cast<uint4*>(rowp + 4096 + off) = make_uint4(v1[c * 4], v1[c * 4 + 1], v1[c * 4 + 2], v1[c * 4 + 3]);
         }
         fence_proxy_async_smem();
-        mbar_arrive(stage_full);
-        if (warp == FIRST_WORK_WARP && lane == 0) {
-          if (mbar_wait_bounded(stage_full, rd & 1u, abort_flag, err_word, ERR_WAIT_AUX)) {
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh)
-              tma_reduce_add_3d(&tmDQ, sDQ + hh * (BM * 128), hq * D + (rr * 2 + hh) * 32, q0, b);
-            tma_store_commit();
+        __syncwarp();
+        if (lane == 0) {
+          const int q0 = qb * BM + quad * 32;
+          if (q0 < p.L) {
+            tma_reduce_add_3d(&tmDQ, stage, hq * D + rr * 64, q0, b);
+            tma_reduce_add_3d(&tmDQ, stage + 4096, hq * D + rr * 64 + 32, q0, b);
           }
+          tma_store_commit();
         }
         __syncwarp();
-        ++rd;
       }
-      if (ok) {
-        tc_fence_before_sync();
-        mbar_arrive((C::PIPE && (itd & 1)) ? dq_empty1 : dq_empty);
+      if (++qb == nqb) {
+        qb = i_start;
+        ++hq;
       }
-    };
-    // dq_full of pair itd: one barrier per accumulator, each used by every second pair in the pipelined variant
-    auto wait_dq_full = [&](int itd) -> bool {
-      uint64_t* bar = (C::PIPE && (itd & 1)) ? dq_full1 : dq_full;
-      const uint32_t parity = C::PIPE ? ((itd >> 1) & 1u) : (itd & 1u);
-      int w2 = mbar_wait_bounded(bar, parity, abort_flag, err_word, ERR_WAIT_AUX) ? 1 : 0;
-      if (!__all_sync(0xffffffffu, w2)) return false;
-      tc_fence_after_sync();
-      return true;
-    };
-    for (int it = 0; ok && it < n_it; ++it) {
-      const int hq = hkv * g + it / nqi;
-      const int q0 = (i_start + it % nqi) * BM;
-      const int qi = q0 + r;
-      const bool row_ok = qi < p.L;
-      const long long t = (long long)b * p.L + qi;
-      // a row past the end of the sequence gets lse = +inf: exp2(s - inf) = 0, so P and dS vanish without a mask
-      const float lse2 = row_ok ? p.lse[(long long)hq * T + t] * 1.4426950408889634f : INFINITY;
-      const float dlts = row_ok ? p.delta[(long long)hq * T + t] * p.scale : 0.f;
-      // tile columns lo .. lim are visible to this row; `masked`: not all of them to every row of the block
+    }
+    if (lane == 0) tma_store_wait_all0();
+  } else {
+    // ------------------------------------------------------------------ softmax, dS and the epilogue
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    const int quad = warp & 3;
+    const int half = (warp - FIRST_COMPUTE_WARP) >> 2;   // which 64 query columns of the tile
+    const int r = quad * 32 + lane;                      // key row
+    const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
+    const float c2 = p.scale * 1.4426950408889634f;
+    const uint64_t c2p = pack_f32x2(c2, c2), scp = pack_f32x2(p.scale, p.scale);
+    const uint32_t tS0 = tmem_base + lane_addr + C::S_COL + half * 64;
+    const uint32_t tDP = tmem_base + lane_addr + C::DP_COL + half * 64;
+    bool ok = true;
+    int qb = i_start;
+    for (int it = 0; it < n_it; ++it) {
+      const int bf = it % NSB, qs = it % QS;
+      const int q0 = qb * BM;
+      if (++qb == nqb) qb = i_start;
+      // tile columns lo .. hi (counted from this warp's first) are visible to this key; `masked`: not all of them to every key
       const bool masked = (kv0 + BN - 1) > q0 || (p.window > 0 && q0 + BM - p.window > kv0);
-      const int lim = qi - kv0;
-      const int lo = p.window > 0 ? qi - p.window + 1 - kv0 : 0;
-      int w = mbar_wait_bounded(sdp_full, it & 1u, abort_flag, err_word, ERR_WAIT_TMEM_FULL) ? 1 : 0;
-      if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
+      const int lo = kv0 + r - q0 - half * 64;
+      const int hi = p.window > 0 ? lo + p.window - 1 : 0x3fffffff;
+      const float* stat = reinterpret_cast<const float*>(smem + C::OFF_STAT + qs * C::STAT_BYTES) + half * 64;
+
+      // P = exp2(S * c - lse): S_it complete implies that the statistics of its queries are there
+      if (!spin(&s_full[bf], (it / NSB) & 1u, ERR_WAIT_TMEM_FULL) || !spin(&q_full[qs], (it / QS) & 1u, ERR_WAIT_FULL)) {
+        ok = false;
+        break;
+      }
       tc_fence_after_sync();
-      // this warp's 32 columns of S and dP, 16 at a time (keeps the register count under the 18-warp budget)
+      uint32_t s[2][32];
+      tmem_ld_32x32b_x32(tS0 + bf * 128, s[0]);
+      tmem_ld_32x32b_x32(tS0 + bf * 128 + 32, s[1]);
+      tmem_ld_wait_for(s[0]);
+      tmem_ld_wait_for(s[1]);
+      if (D == 64 && half == 0) {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_read[bf * 4 + quad]);
+      }
+      uint32_t pk[32];
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const int col0 = part * 32 + hf * 16;
-        uint32_t sv[16], dv[16];
-        tmem_ld_32x32b_x16(tmem_base + lane_addr + C::S_COL + col0, sv);
-        tmem_ld_32x32b_x16(tmem_base + lane_addr + C::DP_COL + col0, dv);
-        tmem_ld_wait();
-        uint32_t pkP[8], pkS[8];
-        if (!masked) {
+      for (int c = 0; c < 2; ++c) {
 #pragma unroll
-          for (int e = 0; e < 16; e += 2) {
-            const float p0 = fast_exp2(fmaf(__uint_as_float(sv[e]), c2, -lse2));
-            const float p1 = fast_exp2(fmaf(__uint_as_float(sv[e + 1]), c2, -lse2));
-            const float d0 = p0 * fmaf(__uint_as_float(dv[e]), p.scale, -dlts);
-            const float d1 = p1 * fmaf(__uint_as_float(dv[e + 1]), p.scale, -dlts);
-            pkP[e >> 1] = pack_bf16x2(p0, p1);
-            pkS[e >> 1] = pack_bf16x2(d0, d1);
+        for (int e = 0; e < 32; e += 4) {
+          const ulonglong2 nl = *reinterpret_cast<const ulonglong2*>(stat + c * 32 + e);
+          float x0, x1, x2, x3;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[c][e]), __uint_as_float(s[c][e + 1])), c2p, nl.x), x0, x1);
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[c][e + 2]), __uint_as_float(s[c][e + 3])), c2p, nl.y), x2, x3);
+          float y0 = fast_exp2(x0), y1 = fast_exp2(x1), y2 = fast_exp2(x2), y3 = fast_exp2(x3);
+          if (masked) {
+            const int q = c * 32 + e;
+            if (q < lo || q > hi) y0 = 0.f;
+            if (q + 1 < lo || q + 1 > hi) y1 = 0.f;
+            if (q + 2 < lo || q + 2 > hi) y2 = 0.f;
+            if (q + 3 < lo || q + 3 > hi) y3 = 0.f;
           }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 16; e += 2) {
-            float p0 = fast_exp2(fmaf(__uint_as_float(sv[e]), c2, -lse2));
-            float p1 = fast_exp2(fmaf(__uint_as_float(sv[e + 1]), c2, -lse2));
-            if ((col0 + e) > lim || (col0 + e) < lo) p0 = 0.f;
-            if ((col0 + e + 1) > lim || (col0 + e + 1) < lo) p1 = 0.f;
-            const float d0 = p0 * fmaf(__uint_as_float(dv[e]), p.scale, -dlts);
-            const float d1 = p1 * fmaf(__uint_as_float(dv[e + 1]), p.scale, -dlts);
-            pkP[e >> 1] = pack_bf16x2(p0, p1);
-            pkS[e >> 1] = pack_bf16x2(d0, d1);
-          }
-        }
-        if (C::PIPE && hf == 0 && it > 0) {
-          // P / dS in shared memory still belong to pair it-1 until its dV / dK / dQ MMAs are done (they were issued
-          // behind this pair's S / dP MMAs); the first 16 columns above were computed while waiting for that
-          if (!wait_dq_full(it - 1)) { ok = false; break; }
-        }
-        // columns col0 .. col0+15 of row r: 64-column sub-tile col0/64, 16-byte chunks (col0 % 64)/8 + {0, 1}
-        const int sub = col0 >> 6;
-        const int chunk0 = (col0 & 63) >> 3;
-        const int off = sub * (BM * 128) + r * 128;
-#pragma unroll
-        for (int q4 = 0; q4 < 2; ++q4) {
-          const int ch = (chunk0 + q4) ^ (r & 7);
-          *reinterpret_cast<uint4*>(sP + off + ch * 16) =
-              make_uint4(pkP[q4 * 4], pkP[q4 * 4 + 1], pkP[q4 * 4 + 2], pkP[q4 * 4 + 3]);
-          *reinterpret_cast<uint4*>(sDS + off + ch * 16) =
-              make_uint4(pkS[q4 * 4], pkS[q4 * 4 + 1], pkS[q4 * 4 + 2], pkS[q4 * 4 + 3]);
+          s[c][e] = __float_as_uint(y0);
+          s[c][e + 1] = __float_as_uint(y1);
+          s[c][e + 2] = __float_as_uint(y2);
+          s[c][e + 3] = __float_as_uint(y3);
+          pk[c * 16 + (e >> 1)] = pack_bf16x2(y0, y1);
+          pk[c * 16 + (e >> 1) + 1] = pack_bf16x2(y2, y3);
         }
       }
-      if (!ok) break;
+      if (D == 64 && half == 1) {    // these columns are the first warp's scores: long read by now
+        if (!spin(&s_read[bf * 4 + quad], (it / NSB) & 1u, ERR_WAIT_AUX)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+      }
+      {
+        const uint32_t dst = tmem_base + lane_addr + C::S_COL + bf * 128 + half * C::P_HALF;
+        tmem_st_32x32b_x16(dst, *reinterpret_cast<const uint32_t(*)[16]>(&pk[0]));
+        tmem_st_32x32b_x16(dst + 16, *reinterpret_cast<const uint32_t(*)[16]>(&pk[16]));
+        tmem_st_wait();
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_ready[bf]);
+
+      // dS = P * (dP - delta) * scale
+      if (!spin(dp_full, it & 1u, ERR_WAIT_TMEM_FULL)) {
+        ok = false;
+        break;
+      }
+      // the one dS tile of head dim 128 is read by dK of the pair before until that is done; with two tiles the drain of
+      // dQ_{it-2}, which S_it waited for, has shown that theirs is free
+      if (C::NDS == 1 && it > 0 && !spin(dk_done, (it - 1) & 1u, ERR_WAIT_AUX)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after_sync();
+      uint8_t* srow = smem + C::OFF_DS + (it % C::NDS) * C::P_BYTES + half * SUB + r * 128;
+      uint32_t dv[2][32];
+      tmem_ld_32x32b_x32(tDP, dv[0]);
+      tmem_ld_wait_for(dv[0]);
+      tmem_ld_32x32b_x32(tDP + 32, dv[1]);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (c == 1) tmem_ld_wait_for(dv[1]);
+        uint32_t pd[16];
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          const ulonglong2 nd = *reinterpret_cast<const ulonglong2*>(stat + BM + c * 32 + e);
+          const uint64_t t0 = fma_f32x2(pack_f32x2(__uint_as_float(dv[c][e]), __uint_as_float(dv[c][e + 1])), scp, nd.x);
+          const uint64_t t1 = fma_f32x2(pack_f32x2(__uint_as_float(dv[c][e + 2]), __uint_as_float(dv[c][e + 3])), scp, nd.y);
+          float y0, y1, y2, y3;
+          unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(s[c][e]), __uint_as_float(s[c][e + 1])), t0), y0, y1);
+          unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(s[c][e + 2]), __uint_as_float(s[c][e + 3])), t1), y2, y3);
+          pd[e >> 1] = pack_bf16x2(y0, y1);
+          pd[(e >> 1) + 1] = pack_bf16x2(y2, y3);
+        }
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4)
+          *reinterpret_cast<uint4*>(srow + ((c * 4 + q4) ^ (r & 7)) * 16) =
+              make_uint4(pd[q4 * 4], pd[q4 * 4 + 1], pd[q4 * 4 + 2], pd[q4 * 4 + 3]);
+        if constexpr (C::DS_TMEM) tmem_st_32x32b_x16(tDP + c * 16, pd);
+      }
+      if constexpr (C::DS_TMEM) tmem_st_wait();
       fence_proxy_async_smem();
       tc_fence_before_sync();
-      mbar_arrive(pds_ready);
-      if constexpr (C::PIPE) {
-        if (it > 0) drain(it - 1);   // its dq_full was waited for above
-      } else {
-        if (!wait_dq_full(it)) { ok = false; break; }
-        drain(it);
-      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_ready);
     }
-    if (C::PIPE && ok && n_it > 0) {   // the last pair's dQ; this wait also covers every MMA of the CTA
-      if (wait_dq_full(n_it - 1)) drain(n_it - 1);
-      else ok = false;
-    }
-    if (warp == FIRST_WORK_WARP && lane == 0) tma_store_wait_all0();
-    // epilogue: dK_j, dV_j (thread = key row). The last dq_full wait covered every MMA of this CTA.
+    // epilogue: dK_j, dV_j (thread = key row, this warp's half of the columns)
     if (ok && n_it > 0) {
+      const int last = n_it - 1;
+      ok = spin(dk_done, last & 1u, ERR_WAIT_AUX) && spin(&dv_done[last % NSB], (last / NSB) & 1u, ERR_WAIT_AUX) &&
+           spin(&dq_full[last % NSB], (last / NSB) & 1u, ERR_WAIT_AUX);   // dQ's MMAs have read K: its memory may be reused
+    }
+    if (ok && n_it > 0) {
+      tc_fence_after_sync();
       const int kvi = kv0 + r;
       const bool row_ok = kvi < p.L;
       const long long width = (long long)(p.H + 2 * p.Hkv) * D;
-      __nv_bfloat16* krow = p.dqkv + ((long long)b * p.L + kvi) * width + colK;
-      __nv_bfloat16* vrow = p.dqkv + ((long long)b * p.L + kvi) * width + colV;
+      __nv_bfloat16* row = p.dqkv + ((long long)b * p.L + kvi) * width;
 #pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        const uint32_t col = which == 0 ? C::DK_COL : C::DV_COL;
-        __nv_bfloat16* dst = which == 0 ? krow : vrow;
-        uint32_t v[DW];
-        if constexpr (DW == 32) tmem_ld_32x32b_x32(tmem_base + lane_addr + col + dc0, v);
-        else tmem_ld_32x32b_x16(tmem_base + lane_addr + col + dc0, v);
+      for (int c = 0; c < D / 32; ++c) {           // D / 64 blocks of 32 columns of dK, then of dV
+        const int which = c / (D / 64);
+        const int col = half * (D / 2) + (c % (D / 64)) * 32;
+        uint32_t v[32];
+        tmem_ld_32x32b_x32(tmem_base + lane_addr + (which == 0 ? C::DK_COL : C::DV_COL) + col, v);
         tmem_ld_wait();
-        if (row_ok) {
+        if (p.hsplit > 1) {
+          float* dst = reinterpret_cast<float*>(smem) + r * C::RED_PITCH + which * D + col;
 #pragma unroll
-          for (int q4 = 0; q4 < DW / 8; ++q4) {
+          for (int q4 = 0; q4 < 8; ++q4)
+            *reinterpret_cast<uint4*>(dst + q4 * 4) = make_uint4(v[q4 * 4], v[q4 * 4 + 1], v[q4 * 4 + 2], v[q4 * 4 + 3]);
+        } else if (row_ok) {
+          __nv_bfloat16* dst = row + (which == 0 ? colK : colV) + col;
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
             uint4 o;
             o.x = pack_bf16x2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
             o.y = pack_bf16x2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
             o.z = pack_bf16x2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
             o.w = pack_bf16x2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
-            *reinterpret_cast<uint4*>(dst + dc0 + q4 * 8) = o;
+            *reinterpret_cast<uint4*>(dst + q4 * 8) = o;
           }
         }
       }
@@ -481,6 +586,29 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
+  if (p.hsplit > 1) {
+    // the CTAs of the cluster each sum their share of dK | dV over all of them, in the order of the ranks
+    cluster_sync_all();
+    const uint32_t rank = cluster_ctarank(), n = (uint32_t)p.hsplit;
+    const uint32_t base = smem_u32(smem);
+    const long long width = (long long)(p.H + 2 * p.Hkv) * D;
+    constexpr int VPR = D / 2;                       // vectors of 4 in a key row: dK, then dV
+    const int rows = min(BN, p.L - kv0);
+    if (!*abort_flag) {
+      for (int i = (int)(rank * NTHREADS + threadIdx.x); i < rows * VPR; i += (int)(n * NTHREADS)) {
+        const int row = i / VPR, v = i - row * VPR;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (uint32_t j = 0; j < n; ++j) {
+          const float4 x = ld_cluster_f32x4(mapa_shared(base + (row * C::RED_PITCH + v * 4) * 4, j));
+          a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+        }
+        const int col = v * 4 < D ? colK + v * 4 : colV + v * 4 - D;
+        uint2 o = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
+        *reinterpret_cast<uint2*>(p.dqkv + ((long long)b * p.L + kv0 + row) * width + col) = o;
+      }
+    }
+    cluster_sync_all();    // nobody's shared memory goes away while a peer reads it
   }
 }
 
@@ -594,6 +722,34 @@ __global__ void dq_convert_rope_kernel(const float* __restrict__ acc, __nv_bfloa
   }
 }
 
+// CTAs that share the query heads of one (batch, kv head, key block). The kernel takes about as long as the longer of its
+// longest CTA (the first key block: every query block of its heads) and its whole work spread over the SMs, in pairs of
+// blocks with kOverhead for a CTA's start and end; the smallest split within 5 % of the best of that is taken, so a grid
+// that fills the GPU keeps one CTA per key block.
+static int head_split(int B, int L, int window, int H, int Hkv) {
+  constexpr double kOverhead = 3.0;
+  const int g = H / Hkv, nkb = ceil_div(L, BN);
+  long long pairs = 0;    // of one head
+  int longest = 0;
+  for (int j = 0; j < nkb; ++j) {
+    const long long q_end = window > 0 ? (long long)j * BN + BN - 1 + window : L;
+    const int n = (int)ceil_div_ll(q_end < L ? q_end : L, BM) - j;
+    pairs += n;
+    longest = n > longest ? n : longest;
+  }
+  const double sms = sm_count();
+  auto cost = [&](int hs) {
+    const double chain = (double)ceil_div(g, hs) * longest + kOverhead;
+    const double all = ((double)B * H * pairs + (double)B * Hkv * hs * nkb * kOverhead) / sms;
+    return chain > all ? chain : all;
+  };
+  double best = cost(1);
+  for (int hs = 2; hs <= g && hs <= 8; ++hs) best = cost(hs) < best ? cost(hs) : best;
+  int hs = 1;
+  while (cost(hs) > 1.05 * best) ++hs;
+  return hs;
+}
+
 template <int D>
 static int launch_bwd(const void* dout, const void* qkv, const void* out, const float* lse, float* delta, void* dqkv,
                       float* dq_acc, int B, int L, int window, int H, int Hkv, const int* pos,
@@ -609,9 +765,9 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
   rc = make_tmap_3d(&tmDO, dout, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)HD, (uint64_t)L, (uint64_t)B,
                     (uint64_t)HD * 2, (uint64_t)L * HD * 2, 64, 128, 1, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != B200_OK) return rc;
-  CUtensorMap tmDQ;
+  CUtensorMap tmDQ;   // one drain warp's 32 rows at a time
   rc = make_tmap_3d(&tmDQ, dq_acc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)HD, (uint64_t)L, (uint64_t)B,
-                    (uint64_t)HD * 4, (uint64_t)L * HD * 4, 32, 128, 1, CU_TENSOR_MAP_SWIZZLE_128B);
+                    (uint64_t)HD * 4, (uint64_t)L * HD * 4, 32, 32, 1, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc != B200_OK) return rc;
   {
     const long long threads = T * H * (D / 8);
@@ -625,9 +781,13 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
     B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     attr = true;
   }
-  BwdParams p{lse, delta, dq_acc, (__nv_bfloat16*)dqkv, B, L, H, Hkv, window, 1.0f / sqrtf((float)D)};
-  dim3 grid(Hkv * B, (L + BN - 1) / BN);
-  launch_pdl(kern, grid, NTHREADS, C::SMEM_BYTES, st, tmQKV, tmDO, tmDQ, p, device_err_word());
+  const int hs = head_split(B, L, window, H, Hkv);
+  BwdParams p{lse, delta, (__nv_bfloat16*)dqkv, B, L, H, Hkv, window, hs, 1.0f / sqrtf((float)D)};
+  dim3 grid(Hkv * B * hs, (L + BN - 1) / BN);
+  if (hs > 1)
+    launch_pdl_cluster(kern, grid, NTHREADS, C::SMEM_BYTES, st, hs, tmQKV, tmDO, tmDQ, p, device_err_word());
+  else
+    launch_pdl(kern, grid, NTHREADS, C::SMEM_BYTES, st, tmQKV, tmDO, tmDQ, p, device_err_word());
   B200_CUDA_CHECK(cudaGetLastError());
   {
     const bool rot = pos != nullptr;

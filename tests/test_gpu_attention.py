@@ -237,3 +237,26 @@ def test_scores_of_any_size(d, window):
     bad = out.isnan().any(1).cpu()
     assert torch.equal(bad, see[:, nan_at])                              # the rows that see the key, and no other
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("B,L,H,Hkv,d,window", [(1, 1, 8, 1, 64, None), (1, 127, 7, 1, 64, None), (1, 777, 14, 2, 64, None),
+                                                (2, 129, 16, 2, 64, 100), (1, 300, 5, 1, 128, None), (1, 257, 16, 2, 128, 200),
+                                                (1, 128, 24, 2, 64, None), (8, 1025, 16, 2, 64, None)])
+def test_query_heads_shared_by_a_cluster(B, L, H, Hkv, d, window):
+    """Groups of 5 to 12 query heads on grids that leave SMs idle: the heads of a group are shared by the CTAs of a cluster (also
+    a share that is not even, and more heads than a cluster has CTAs; the last case keeps one CTA per key block). Bound: as at the window edges, 2e-2 of the largest
+    gradient; key and value gradients repeat bit for bit."""
+    torch.manual_seed(L + H)
+    qkv = torch.randn(B * L, (H + 2 * Hkv) * d, device=DEV).bfloat16()
+    dout = torch.randn(B * L, H * d, device=DEV).bfloat16()
+    out, lse = attention.attention_fwd(qkv, B, L, H, Hkv, d, window)
+    got = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
+    again = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
+    if window is None:
+        ro, rl = attention.attention_reference_fwd(qkv.float(), B, L, H, Hkv, d)
+        want = attention.attention_reference_bwd(dout.float(), qkv.float(), ro, rl, B, L, H, Hkv, d)
+    else:
+        want = attention.windowed_bwd(dout.float(), qkv.float(), B, L, H, Hkv, d, window)
+    for cols in (slice(0, H * d), slice(H * d, (H + Hkv) * d), slice((H + Hkv) * d, None)):
+        assert (got[:, cols].float() - want[:, cols]).abs().max() <= 2e-2 * want[:, cols].abs().max() + 1e-6
+    assert torch.equal(got[:, H * d:], again[:, H * d:]) and _lib.take_device_error() == 0
