@@ -445,7 +445,8 @@ static int launch_rope_pair(const void* A, const void* W, int M, int N, int K, l
   const int tiles = ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, rp, device_err_word(), 1, nullptr, 0);
+  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, rp, device_err_word(), 1, nullptr, 0,
+               gemm::GroupArgs{});
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -573,7 +574,8 @@ static int launch_swiglu_bwd_pair(const void* dY, const void* Wd, int M, int f, 
   const int tiles = ceil_div(M, PAIR_BM) * ceil_div(f, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, f, K, 1, sp, device_err_word(), 1, nullptr, 0);
+  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, f, K, 1, sp, device_err_word(), 1, nullptr, 0,
+               gemm::GroupArgs{});
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -601,7 +603,8 @@ static int launch_swiglu_pair(const void* A, const void* Wgu, int M, int f, int 
   const int tiles = ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, sp, device_err_word(), 1, nullptr, f);
+  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, sp, device_err_word(), 1, nullptr, f,
+               gemm::GroupArgs{});
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -681,6 +684,38 @@ static int pair_k_splits(int tiles, int num_kb, int max_pairs, double* rounds) {
   return k_splits;
 }
 
+// The experts of a layer in one launch (gemm_pair.cuh, GROUPED): A [M, K] and the outputs are cut into n_groups runs of rows
+// whose lengths `counts` holds on the device, B is [n_groups * b_rows, K]. b_half: as in launch_swiglu_pair.
+template <class Epi>
+static int launch_grouped(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb,
+                          const typename Epi::Params& ep, const long long* counts, int n_groups, int b_rows, int b_half,
+                          cudaStream_t stream) {
+  constexpr int STAGES = 6;
+  using S = SmemPair<STAGES>;
+  CUtensorMap tmA, tmB;
+  int rc = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, BK, BM,
+                        CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc != B200_OK) return rc;
+  rc = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)K, (uint64_t)n_groups * b_rows,
+                    (uint64_t)ldb * 2, BK, PAIR_HALF_N, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc != B200_OK) return rc;
+  auto kern = gemm_pair_kernel<STAGES, false, false, Epi, true>;
+  const int smem_bytes = S::bytes(Epi::SMEM_BYTES, true);
+  static bool attr_set = false;
+  if (!attr_set) {
+    B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+    attr_set = true;
+  }
+  const int most = M / PAIR_BM + (n_groups < M ? n_groups : M);      // row tiles, however the rows are spread
+  const long long tiles = (long long)most * ceil_div(N, PAIR_BN);
+  const int max_pairs = sm_count() / 2;
+  const int pairs = tiles < max_pairs ? (int)tiles : max_pairs;
+  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, ep, device_err_word(), 1, nullptr, b_half,
+             GroupArgs{counts, n_groups, b_rows});
+  B200_CUDA_CHECK(cudaGetLastError());
+  return B200_OK;
+}
+
 // Two-SM (cta_group::2) launch: 256 x 256 tiles, one CTA pair per tile.
 template <bool A_MN, bool B_MN>
 static int launch_store_pair(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int fmt,
@@ -738,7 +773,8 @@ static int launch_store_pair(const void* A, const void* B, int M, int N, int K, 
   }
   const long long units = (long long)tiles * k_splits;
   const int pairs = units < max_pairs ? (int)units : max_pairs;
-  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, fmt, sp, device_err_word(), k_splits, sync, 0);
+  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, fmt, sp, device_err_word(), k_splits, sync, 0,
+               gemm::GroupArgs{});
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -1049,6 +1085,37 @@ int b200_gemm_swiglu(const void* x, const void* Wgu, void* gu, void* act, int M,
   const TilePlan plan = plan_tiles(M, 2 * f, K, false, split_k != 0);
   if (plan.bn) return launch_cluster_bn<false, false, ClusterSwiglu>(x, Wgu, M, 2 * f, K, ldx, ldw, 1, sp, plan, f, stream);
   return launch_swiglu_pair(x, Wgu, M, f, K, ldx, ldw, sp, stream);
+}
+
+static bool group_args_ok(const void* x, const void* W, const long long* counts, int M, int K, int n_groups, long long rows) {
+  using namespace b200::gemm;
+  return x && W && counts && M > 0 && K > 0 && !(K & 7) && n_groups > 0 && n_groups <= MAX_GROUPS &&
+         (long long)n_groups * rows <= 0x7fffffffLL &&
+         (long long)(M / PAIR_BM + n_groups) * b200::ceil_div_ll(rows, PAIR_BN) <= 0x7fffffffLL;
+}
+
+// The two GEMMs of a layer's experts. x [M, K] holds each expert's rows one run behind the other, counts int64 [E] their
+// lengths (on the device; they sum to M); Wgu [E, 2f, K], W [E, N, K], all dense. gu [M, 2f] and act [M, f] as in
+// b200_gemm_swiglu, y [M, N] = x W_e^T. bf16, E <= 128, f a multiple of 128, N and K of 8; else B200_ERR_ARG.
+int b200_gemm_grouped_swiglu(const void* x, const void* Wgu, const long long* counts, void* gu, void* act, int M, int f,
+                             int K, int E, cudaStream_t stream) {
+  using namespace b200;
+  using namespace b200::gemm;
+  if (!gu || !act || f <= 0 || (f % PAIR_HALF_N) || f > 0x3fffffff || !group_args_ok(x, Wgu, counts, M, K, E, 2LL * f) ||
+      (reinterpret_cast<uintptr_t>(gu) & 15) || (reinterpret_cast<uintptr_t>(act) & 15))
+    return B200_ERR_ARG;
+  SwigluParams sp{reinterpret_cast<__nv_bfloat16*>(gu), 2LL * f, reinterpret_cast<__nv_bfloat16*>(act), f, f};
+  return launch_grouped<EpiSwiglu>(x, Wgu, M, 2 * f, K, K, K, sp, counts, E, 2 * f, f, stream);
+}
+
+int b200_gemm_grouped(const void* x, const void* W, const long long* counts, void* y, int M, int N, int K, int E,
+                      cudaStream_t stream) {
+  using namespace b200;
+  using namespace b200::gemm;
+  if (!y || N <= 0 || (N & 7) || !group_args_ok(x, W, counts, M, K, E, N) || (reinterpret_cast<uintptr_t>(y) & 15))
+    return B200_ERR_ARG;
+  StoreParams sp{y, N, nullptr, 0, 1.f, 0, 0, 1};
+  return launch_grouped<EpiStore<PAIR_BN>>(x, W, M, N, K, K, K, sp, counts, E, N, 0, stream);
 }
 
 // qkv[M, N] = x[M, K] W[N, K]^T with the rotary embedding applied to the first n_rot_heads heads of every row in the

@@ -17,6 +17,13 @@
 // and releases the counter; the last slice sets it back to zero for the next launch. The order of the additions is
 // therefore fixed and the result repeats bit for bit, which atomic adds did not give. Units are handed out in
 // increasing order and all CTAs of the grid are resident, so the unit a slice waits for is always running or done.
+//
+// Grouped (GROUPED; the experts of a layer in ONE launch): the rows of A and C are cut into consecutive groups whose lengths
+// are on the device, and group e meets rows [e * b_rows, (e + 1) * b_rows) of B. Each CTA turns the lengths into tile
+// offsets itself, so the host need not know them; a tile belongs to one group, its rows past the group's end are computed
+// from the next group's rows and not stored. One launch fills its last round with tiles of every group (6124 tokens, two of 8
+// experts each, 2048 -> 5632 -> 2048: a down projection of one expert is 48 tiles for 74 pairs), and no read-back of the
+// lengths stands between the router and the experts: a collection batch of six such layers 9.13 / 8.13 ms.
 #pragma once
 #include "gemm_core.cuh"
 
@@ -27,6 +34,14 @@ constexpr int PAIR_BM = 256;  // rows per tile pair
 constexpr int PAIR_BN = 256;
 constexpr int PAIR_HALF_N = 128;
 
+constexpr int MAX_GROUPS = 128;
+
+struct GroupArgs {
+  const long long* counts;   // [n] rows of each group
+  int n;
+  int b_rows;                // rows of B per group
+};
+
 template <int STAGES>
 struct SmemPair {
   static constexpr int A_BYTES = BM * BK * 2;           // 128 x 64
@@ -34,14 +49,17 @@ struct SmemPair {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
   static constexpr int BAR_BYTES = 256;
-  static constexpr int bytes(int epi_bytes) { return RING_BYTES + BAR_BYTES + epi_bytes + 1024; }
+  static constexpr int GROUP_BYTES = 2 * (MAX_GROUPS + 1) * 4;   // first tile and first row of each group
+  static constexpr int bytes(int epi_bytes, bool grouped = false) {
+    return RING_BYTES + BAR_BYTES + epi_bytes + (grouped ? GROUP_BYTES : 0) + 1024;
+  }
 };
 
-template <int STAGES, bool A_MN, bool B_MN, class Epi>
+template <int STAGES, bool A_MN, bool B_MN, class Epi, bool GROUPED = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
                      int K, int fmt, typename Epi::Params ep, unsigned int* err_word, int k_splits,
-                     unsigned int* split_sync, int b_half_stride) {
+                     unsigned int* split_sync, int b_half_stride, GroupArgs grp) {
   using S = SmemPair<STAGES>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -84,8 +102,37 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   pdl_wait();
   pdl_trigger();
 
-  const int m_tiles = (M + PAIR_BM - 1) / PAIR_BM;
   const int n_tiles = (N + PAIR_BN - 1) / PAIR_BN;
+  int* g_tile = reinterpret_cast<int*>(epi_smem + Epi::SMEM_BYTES);   // GROUPED: row tiles in front of each group
+  int* g_row = g_tile + MAX_GROUPS + 1;                               //          and rows
+  int m_tiles = (M + PAIR_BM - 1) / PAIR_BM;
+  if constexpr (GROUPED) {
+    if (warp == 0) {
+      int tiles = 0, rows = 0;
+      if (lane == 0) g_tile[0] = g_row[0] = 0;
+      for (int e0 = 0; e0 < grp.n; e0 += 32) {
+        const int e = e0 + lane;
+        int r = e < grp.n ? (int)grp.counts[e] : 0;
+        int t = (r + PAIR_BM - 1) / PAIR_BM;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int ur = __shfl_up_sync(0xffffffffu, r, o), ut = __shfl_up_sync(0xffffffffu, t, o);
+          if (lane >= o) {
+            r += ur;
+            t += ut;
+          }
+        }
+        if (e < grp.n) {
+          g_tile[e + 1] = tiles + t;
+          g_row[e + 1] = rows + r;
+        }
+        tiles += __shfl_sync(0xffffffffu, t, 31);
+        rows += __shfl_sync(0xffffffffu, r, 31);
+      }
+    }
+    __syncthreads();
+    m_tiles = g_tile[grp.n];
+  }
   const int num_tiles = m_tiles * n_tiles;
   const int num_kb = (K + BK - 1) / BK;
   // split-K: a work unit is (slice of the K loop, tile), slice-major. k_splits = 1: one unit per tile.
@@ -99,13 +146,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   const int pair_id = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
   constexpr int GROUP_M = 8;
-  auto tile_coords = [&](int tile, int& m_blk, int& n_blk) {
+  // First row and column block of a tile, the first row of B that its columns count from, and the end of its rows. `e`:
+  // the group of the caller's tile before this one (tiles are visited in increasing order), 0 at first.
+  auto locate = [&](int tile, int& e, int& row, int& n_blk, int& b_row, int& row_end) {
+    int mt = m_tiles, base = 0;
+    row_end = M;
+    b_row = 0;
+    if constexpr (GROUPED) {
+      while (tile >= g_tile[e + 1] * n_tiles) ++e;
+      tile -= g_tile[e] * n_tiles;
+      mt = g_tile[e + 1] - g_tile[e];
+      base = g_row[e];
+      row_end = g_row[e + 1];
+      b_row = e * grp.b_rows;
+    }
     const int per_group = GROUP_M * n_tiles;
     const int g = tile / per_group;
     const int first_m = g * GROUP_M;
-    const int gsz = min(GROUP_M, m_tiles - first_m);
+    const int gsz = min(GROUP_M, mt - first_m);
     const int r = tile - g * per_group;
-    m_blk = first_m + (r % gsz);
+    row = base + (first_m + (r % gsz)) * PAIR_BM;
     n_blk = r / gsz;
   };
 
@@ -114,16 +174,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
+      int e = 0;
       for (int unit = pair_id; ok && unit < num_units; unit += num_pairs) {
-        int tile, kb0, kb1, m_blk, n_blk;
+        int tile, kb0, kb1, row, n_blk, b_row, row_end;
         unit_range(unit, tile, kb0, kb1);
-        tile_coords(tile, m_blk, n_blk);
-        const int m0 = m_blk * PAIR_BM + (int)cta * BM;
+        locate(tile, e, row, n_blk, b_row, row_end);
+        const int m0 = row + (int)cta * BM;
         // B rows of this CTA's half of the tile. b_half_stride > 0 (fused gate / up projection): the leader takes 128
         // rows of the first half of B and its peer the 128 rows that lie b_half_stride below them, so columns 0-127 of
         // the accumulator are the gate and columns 128-255 the up projection of the SAME 128 output features.
-        const int n0 = b_half_stride > 0 ? n_blk * PAIR_HALF_N + (int)cta * b_half_stride
-                                         : n_blk * PAIR_BN + (int)cta * PAIR_HALF_N;
+        const int n0 = b_row + (b_half_stride > 0 ? n_blk * PAIR_HALF_N + (int)cta * b_half_stride
+                                                  : n_blk * PAIR_BN + (int)cta * PAIR_HALF_N);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const uint32_t s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1u;
@@ -202,10 +263,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     const int quad = warp & 3;
     const uint32_t leader_tempty0 = mapa_shared(smem_u32(&tempty_bar[0]), 0);
     uint32_t tl = 0;
+    int e = 0;
     for (int unit = pair_id; unit < num_units; unit += num_pairs, ++tl) {
-      int tile, kb0, kb1, m_blk, n_blk;
+      int tile, kb0, kb1, row, n_blk, b_row, row_end;
       unit_range(unit, tile, kb0, kb1);
-      tile_coords(tile, m_blk, n_blk);
+      locate(tile, e, row, n_blk, b_row, row_end);
       const uint32_t acc = tl & 1u;
       const uint32_t aph = (tl >> 1) & 1u;
       int ok = mbar_wait_bounded(&tfull_bar[acc], aph, abort_flag, err_word, ERR_WAIT_TMEM_FULL) ? 1 : 0;
@@ -223,16 +285,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
             ok2 = __all_sync(0xffffffffu, ok2);
             if (!ok2) break;
           }
-          Epi::tile(Epi::slice_params(ep, sp), taddr, m_blk * PAIR_BM + (int)cta * BM, n_blk * PAIR_BN, M, N, quad,
+          Epi::tile(Epi::slice_params(ep, sp), taddr, row + (int)cta * BM, n_blk * PAIR_BN, row_end, N, quad,
                     lane, epi_smem);
           __threadfence();
           __syncwarp();
           if (lane == 0) st_release_gpu_u32(ctr, sp + 1 == k_splits ? 0u : (unsigned)(sp + 1));
         } else {
-          Epi::tile(ep, taddr, m_blk * PAIR_BM + (int)cta * BM, n_blk * PAIR_BN, M, N, quad, lane, epi_smem);
+          Epi::tile(ep, taddr, row + (int)cta * BM, n_blk * PAIR_BN, row_end, N, quad, lane, epi_smem);
         }
       } else {
-        Epi::tile(ep, taddr, m_blk * PAIR_BM + (int)cta * BM, n_blk * PAIR_BN, M, N, quad, lane, epi_smem);
+        Epi::tile(ep, taddr, row + (int)cta * BM, n_blk * PAIR_BN, row_end, N, quad, lane, epi_smem);
       }
       tc_fence_before_sync();
       __syncwarp();

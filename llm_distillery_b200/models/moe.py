@@ -5,11 +5,12 @@ both roles, student training and teacher inference.
 The reference loads such students through ``AutoModelForCausalLM`` (classes/student/model.py:194-201) and its shipped
 ``freeze_layers`` default names Mixtral's router (config.json: ``block_sparse_moe.gate``). Here a decoder layer with
 experts is two autograd nodes with explicit backward: ``AttnBlockFn`` (the attention half of the dense layer) and
-``MoEBlockFn``. The expert half sorts the (token, choice) pairs by expert once per layer, gathers the rows, runs every
-expert's two GEMMs on its contiguous slab of rows with the same tcgen05 GEMM kernels as the dense layers (the fused
-gate/up projection of all experts fills one buffer, so SwiGLU is one launch), and combines by GATHERING each token's k
-results - a fixed order of additions, no atomic scatter. Routing arithmetic ([T, E] tensors) is PyTorch in fp32.
-The number of rows per expert comes back to the host once per layer (the GEMM shapes depend on it).
+``MoEBlockFn``. The expert half sorts the (token, choice) pairs by expert once per layer, gathers the rows, runs each of
+the experts' two GEMMs as one launch over all experts' slabs of rows (SwiGLU in the epilogue of the first; a launch per
+expert for sizes and types that it does not take), and combines by GATHERING each token's k results - a fixed order of
+additions, no atomic scatter. Routing arithmetic ([T, E] tensors) is PyTorch in fp32. The number of rows per expert stays on
+the device in inference; a forward pass that a backward pass follows reads it back once per layer (the shapes of the weight
+gradients' GEMMs depend on it).
 No GEMM here cuts K (``basic.gemm``'s split_k), in inference either: behind a router a last bit can be another expert, and
 an expert's row count, which the cut would depend on, changes with every batch.
 """
@@ -23,6 +24,8 @@ from ..ops._lib import _F, _I, _LL, _VP
 from . import llama as _ll
 
 _lib.register("b200_expert_sort", [_VP, _LL, _I, _I, _VP, _VP, _VP, _VP, _VP])
+_lib.register("b200_gemm_grouped_swiglu", [_VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP])
+_lib.register("b200_gemm_grouped", [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP])
 _lib.register("b200_moe_combine", [_VP, _VP, _VP, _VP, _VP, _LL, _I, _I, _F, _VP])
 
 
@@ -48,6 +51,12 @@ def permutation(top_e: torch.Tensor, n_experts: int):
     keep their order inside an expert's slab), ``inverse`` undoes it, ``token`` is the token of each sorted pair,
     ``counts`` are the slab lengths as Python ints. One kernel on a GPU (csrc/ops/moe.cu) for up to 32 experts and
     ``SORT_MAX_PAIRS`` pairs; beyond them, and for indices that are not int64, the library's sort."""
+    order, inverse, token, counts = _sorted_pairs(top_e, n_experts)
+    return order, inverse, token, counts.tolist()
+
+
+def _sorted_pairs(top_e: torch.Tensor, n_experts: int):
+    """``permutation`` with the counts left where they are (int64 [n_experts])."""
     flat = top_e.reshape(-1)
     k = top_e.shape[1]
     if (flat.is_cuda and flat.dtype == torch.int64 and flat.is_contiguous() and n_experts <= 32
@@ -57,11 +66,11 @@ def permutation(top_e: torch.Tensor, n_experts: int):
         _lib.check(_lib.kernels().b200_expert_sort(_lib.ptr(flat), flat.numel(), n_experts, k, _lib.ptr(order),
                                                    _lib.ptr(inverse), _lib.ptr(token), _lib.ptr(counts), _lib.stream()),
                    "b200_expert_sort")
-        return order, inverse, token, counts.tolist()
+        return order, inverse, token, counts
     order = torch.argsort(flat, stable=True)
     inverse = torch.empty_like(order)
     inverse[order] = torch.arange(order.numel(), device=order.device)
-    counts = torch.bincount(flat, minlength=n_experts).tolist()
+    counts = torch.bincount(flat, minlength=n_experts)
     return order, inverse, torch.div(order, k, rounding_mode="floor"), counts
 
 
@@ -78,8 +87,33 @@ def combine(y: torch.Tensor, inverse: torch.Tensor, top_w: torch.Tensor, h1: tor
     return out
 
 
-def experts_forward(x_perm: torch.Tensor, counts: list[int], w_gu: torch.Tensor, w_d: torch.Tensor):
-    """x_perm [T*k, h] (rows grouped by expert) -> (gu [T*k, 2f], act [T*k, f], y [T*k, h])."""
+def _grouped(x_perm: torch.Tensor, counts: torch.Tensor, w_gu: torch.Tensor, w_d: torch.Tensor) -> bool:
+    """Whether the experts' GEMMs run as one launch each (b200_gemm_grouped*): dense bf16 operands on 16-byte boundaries, up
+    to 128 experts, whole 128-feature tiles of gate and up rows, row strides of whole 16 bytes."""
+    E, two_f, h = w_gu.shape
+    return (x_perm.is_cuda and x_perm.shape[0] > 0 and E <= 128 and two_f % 256 == 0 and h % 8 == 0
+            and tuple(w_d.shape) == (E, h, two_f // 2) and x_perm.shape[1] == h and counts.dtype == torch.int64
+            and counts.is_cuda and counts.is_contiguous()
+            and all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x_perm, w_gu, w_d)))
+
+
+def experts_forward(x_perm: torch.Tensor, counts: torch.Tensor, w_gu: torch.Tensor, w_d: torch.Tensor,
+                    host_counts: list[int] | None = None):
+    """x_perm [T*k, h] (rows grouped by expert, ``counts`` of them each) -> (gu [T*k, 2f], act [T*k, f], y [T*k, h]).
+    ``host_counts``: the counts where the host has them already."""
+    if _grouped(x_perm, counts, w_gu, w_d):
+        (n, h), (E, two_f, _), new = x_perm.shape, w_gu.shape, x_perm.new_empty
+        gu, act, y = new((n, two_f)), new((n, two_f // 2)), new((n, h))
+        lib, p = _lib.kernels(), _lib.ptr
+        _lib.check(lib.b200_gemm_grouped_swiglu(p(x_perm), p(w_gu), p(counts), p(gu), p(act), n, two_f // 2, h, E,
+                                                _lib.stream()), "b200_gemm_grouped_swiglu")
+        _lib.check(lib.b200_gemm_grouped(p(act), p(w_d), p(counts), p(y), n, h, two_f // 2, E, _lib.stream()),
+                   "b200_gemm_grouped")
+        return gu, act, y
+    return _experts_one_by_one(x_perm, counts.tolist() if host_counts is None else host_counts, w_gu, w_d)
+
+
+def _experts_one_by_one(x_perm: torch.Tensor, counts: list[int], w_gu: torch.Tensor, w_d: torch.Tensor):
     n, h = x_perm.shape
     two_f = w_gu.shape[1]
     gu = torch.empty((n, two_f), dtype=x_perm.dtype, device=x_perm.device)
@@ -126,7 +160,7 @@ def moe_mlp(n2: torch.Tensor, w_router: torch.Tensor, w_gu: torch.Tensor, w_d: t
     down matrix, gate vector) of a shared expert, or None."""
     T, h = n2.shape
     _, top_e, top_w = route(n2, w_router, k, renorm)
-    _, inverse, tok, counts = permutation(top_e, w_gu.shape[0])
+    _, inverse, tok, counts = _sorted_pairs(top_e, w_gu.shape[0])
     _, _, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d)
     if shared is None:
         out = combine(y, inverse, top_w, None)
@@ -265,8 +299,10 @@ class MoEBlockFn(torch.autograd.Function):
         T, hdim = h1.shape
         n2, _, rstd2 = basic.rmsnorm_fwd(h1, w_ln2, eps)
         probs, top_e, top_w = route(n2, w_router, k, renorm)
-        order, inverse, tok, counts = permutation(top_e, w_gu.shape[0])
-        gu, act, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d)
+        order, inverse, tok, counts = _sorted_pairs(top_e, w_gu.shape[0])
+        ctx.device_counts = counts
+        ctx.counts = counts.tolist() if any(ctx.needs_input_grad) else None      # only the backward pass reads them
+        gu, act, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d, ctx.counts)
         shared_saved = ()
         h2 = combine(y, inverse, top_w, h1, rmul) if w_sgu is None else None
         if h2 is None:
@@ -278,7 +314,6 @@ class MoEBlockFn(torch.autograd.Function):
                 shared_saved = (gu_s, act_s, y_s, gate)
             h2 = (h1.float() + (branch if rmul == 1.0 else branch * rmul)).to(h1.dtype)
         ctx.meta = meta
-        ctx.counts = counts
         ctx.weights = (w_ln2, w_router, w_gu, w_d)
         ctx.slots = tuple(_ll._slot(w) for w in ctx.weights)
         ctx.shared = (w_sgu, w_sd, w_sg)
@@ -308,7 +343,7 @@ class MoEBlockFn(torch.autograd.Function):
             top_p = probs.gather(1, top_e)
             top_w = top_p / top_p.sum(-1, keepdim=True) if renorm else top_p
             tok = torch.div(order, k, rounding_mode="floor")
-            gu, act, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d)
+            gu, act, y = experts_forward(n2.index_select(0, tok), ctx.device_counts, w_gu, w_d, counts)
             if w_sgu is not None:
                 gu_s, act_s, y_s, gate = shared_expert_forward(n2, w_sgu, w_sd, w_sg)
         else:

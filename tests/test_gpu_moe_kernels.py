@@ -75,3 +75,45 @@ def test_combine_passes_on_what_is_not_finite():
         ok = want.isfinite()
         assert ((got.float() - want).abs() <= 2 ** -8 * want.abs() + 1e-5)[ok].all() and not ok.all()
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("counts,h,f", [([1], 64, 128), ([0, 257, 0, 1, 255, 256], 128, 384), ([0] * 127 + [3], 64, 128),
+                                        ([5, 0, 130, 77, 1024, 512, 33, 0], 2048, 640), ([2000, 1], 264, 128), ([0, 7] * 64, 96, 256)])
+def test_experts_in_one_launch_match_a_launch_each(counts, h, f):
+    """Empty experts, one row, whole tiles and one row more, 128 experts, widths that are not whole tiles: the bits of the
+    launches per expert (one K slice each, the same order of additions)."""
+    g = torch.Generator("cuda").manual_seed(sum(counts) + h)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()  # noqa: E731
+    x, w_gu, w_d = rnd(sum(counts), h), rnd(len(counts), 2 * f, h) * 0.1, rnd(len(counts), h, f) * 0.1
+    dev = torch.tensor(counts, device="cuda")
+    assert moe._grouped(x, dev, w_gu, w_d)
+    for got, want in zip(moe.experts_forward(x, dev, w_gu, w_d), moe._experts_one_by_one(x, counts, w_gu, w_d)):
+        assert torch.equal(got, want)
+    assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("case", ["width", "strided", "offset", "fp16", "empty", "many"])
+def test_experts_that_one_launch_does_not_take(case):
+    """Operands outside the grouped launch keep the path they had (and what that refuses)."""
+    E, h, f = (129 if case == "many" else 4), 64, (192 if case == "width" else 128)
+    w_gu, w_d = torch.randn(E, 2 * f, h, device="cuda").bfloat16() * 0.1, torch.randn(E, h, f, device="cuda").bfloat16() * 0.1
+    counts = [0] * E if case == "empty" else [3, 0, 40, 7] + [0] * (E - 4)
+    x = torch.randn(sum(counts), h + 8, device="cuda").bfloat16()
+    if case == "offset":
+        x = torch.cat([x.new_zeros(4), x[:, 8:].reshape(-1)])[4:].view(-1, h)
+    else:
+        x = x[:, 8:] if case == "strided" else x[:, 8:].contiguous()
+    if case == "fp16":
+        x, w_gu, w_d = x.half(), w_gu.half(), w_d.half()
+    dev = torch.tensor(counts, device="cuda")
+    assert not moe._grouped(x, dev, w_gu, w_d)
+
+    def outcome(fn):
+        try:
+            return fn()
+        except Exception as e:  # noqa: BLE001
+            return type(e)
+    got = outcome(lambda: moe.experts_forward(x, dev, w_gu, w_d))
+    want = outcome(lambda: moe._experts_one_by_one(x, counts, w_gu, w_d))
+    assert got == want if isinstance(want, type) else all(torch.equal(a, b) for a, b in zip(got, want))
+    _lib.take_device_error()
