@@ -25,6 +25,10 @@ _lib.register("b200_lmhead_lse_gather", [_VP, _VP, _I, _I, _I, _LL, _LL, _VP, _I
 _lib.register("b200_distill_rows", [_VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _F, _VP])
 _lib.register("b200_lmhead_dlogits", [_VP, _VP, _I, _I, _I, _LL, _LL, _VP, _VP, _VP, _VP, _VP, _I, _F, _VP, _LL, _VP])
 
+_lib.register("b200_reference_loss", [_VP] * 9 + [_LL, _I, _I, _I, _F, _F, _VP])
+_lib.register("b200_reference_loss_grad", [_VP] * 11 + [_LL, _I, _I, _F, _VP])
+_lib.KERNELS_PER_CALL["b200_reference_loss"] = 2
+
 KIND_CODES = {"kl": 0, "rkl": 1, "jsd": 2, "jsd_renorm": 3, "none": 4}
 DZ_CHUNK_BYTES = 2 << 30  # bf16 dlogits materialised per backward chunk
 
@@ -177,6 +181,45 @@ def fused_distill_rows(Hc, W, ids, u, kind: str, temperature: float = 1.0, vocab
                                  1.0 / temperature, vocab)
 
 
+class _ReferenceLossFn(torch.autograd.Function):
+    """``divergence.reference_loss_segments`` on the statistics of the LM head (csrc/loss/reference.cu): the loss of each
+    conversation [n_seg] and the eight logged values [8, n_seg] in the order of ``divergence.LOSS_KEYS``."""
+
+    @staticmethod
+    def forward(ctx, lse, zk, u, ids, labels, avoid, seg, n_seg, temperature, vocab, alpha):
+        M, K = zk.shape
+        rows = torch.empty((10, M), dtype=torch.float32, device=zk.device)
+        out = torch.empty((8, n_seg), dtype=torch.float32, device=zk.device)
+        p = _lib.ptr
+        _lib.check(_lib.kernels().b200_reference_loss(p(zk), p(lse), p(u), p(ids), p(labels), p(avoid), p(seg), p(rows), p(out),
+                                                      M, K, vocab, n_seg, temperature, alpha, _lib.stream()),
+                   "b200_reference_loss")
+        ctx.save_for_backward(lse, zk, u, ids, labels, avoid, seg, rows)
+        ctx.temperature, ctx.vocab = temperature, vocab
+        ctx.mark_non_differentiable(out)
+        return out[0].clone(), out
+
+    @staticmethod
+    def backward(ctx, g, _):
+        lse, zk, u, ids, labels, avoid, seg, rows = ctx.saved_tensors
+        M, K = zk.shape
+        dzk, dlse = torch.empty_like(zk), torch.empty_like(lse)
+        p = _lib.ptr
+        g = g.float().contiguous()
+        _lib.check(_lib.kernels().b200_reference_loss_grad(p(zk), p(lse), p(u), p(ids), p(labels), p(avoid), p(seg), p(rows),
+                                                           p(g), p(dzk), p(dlse), M, K, ctx.vocab, ctx.temperature,
+                                                           _lib.stream()), "b200_reference_loss_grad")
+        return (dlse, dzk) + (None,) * 9
+
+
+def _native_reference_loss(zk, u, ids, labels, avoid, seg) -> bool:
+    """Whether the reference loss of these tensors runs in its kernels: what ``HostBatch`` holds, on a GPU."""
+    M = zk.shape[0]
+    return (zk.is_cuda and M > 0 and zk.shape[1] > 0 and u.shape == ids.shape == zk.shape
+            and all(t is not None and t.is_cuda and t.shape == (M,) and t.dtype == d
+                    for t, d in ((labels, torch.int64), (avoid, torch.bool), (seg, torch.int64))))
+
+
 def distill_head_loss(Hc, W, ids, u, *, kind: str, temperature: float, vocab: int | None, alpha: float = 2.0,
                       labels=None, avoid=None, seg=None, n_seg: int = 1, jsd_renorm: bool = False):
     """Loss of a micro-batch of content rows.
@@ -187,6 +230,11 @@ def distill_head_loss(Hc, W, ids, u, *, kind: str, temperature: float, vocab: in
     vocab = min(vocab or W.shape[0], W.shape[0])
     if kind == "reference":
         lse, zk = lmhead_stats(Hc, W, ids, temperature, vocab)
+        if _native_reference_loss(zk, u, ids, labels, avoid, seg):
+            custom, logs = _ReferenceLossFn.apply(lse.contiguous(), zk.contiguous(), u.float().contiguous(),
+                                                  ids.to(torch.int32).contiguous(), labels.contiguous(), avoid.contiguous(),
+                                                  seg.contiguous(), n_seg, float(temperature), vocab, float(alpha))
+            return custom.sum(), dict(zip(dv.LOSS_KEYS, logs.sum(1).unbind()))
         s, t = dv.student_teacher_logprobs(lse, zk, u.float(), ids.long() < vocab, temperature)
         custom, logs = dv.reference_loss_segments(s, t, ids.long(), labels, avoid, seg, n_seg, alpha)
         return custom.sum(), {k: v.detach().sum() for k, v in logs.items()}

@@ -80,3 +80,51 @@ def test_reference_loss_through_fused_stats():
     assert (Hg.grad.float().cpu() - Hr.grad).abs().max() <= 5e-2 * Hr.grad.abs().max()
     assert (Wg.grad.float().cpu() - Wr.grad).abs().max() <= 5e-2 * Wr.grad.abs().max()
     assert set(dv.LOSS_KEYS) <= set(logs)
+
+
+@pytest.mark.parametrize("M,K,Vc,T,lens", [(1, 2, 5000, 1.0, [1]), (7, 3, 5000, 1.0, [2, 5]), (65, 33, 900, 2.0, [64, 1]),
+                                           (700, 200, 4800, 1.0, [700]), (1601, 400, 5000, 2.0, [1, 511, 513, 576])])
+def test_reference_loss_kernels_against_fp64(M, K, Vc, T, lens):
+    """Loss, logged values and both gradients against the PyTorch form in fp64, with rows without a target, without a label, left
+    out of the cross-entropy and without a hit, and ids beyond the cropped vocabulary. Bound: sums of up to 400 fp32 terms, their
+    differences and a division by the largest of them: 2e-5 of the largest value (single values differ by 1e-6 of it)."""
+    g = torch.Generator().manual_seed(M)
+    V = 5000
+    z = torch.randn(M, V, generator=g) * 3
+    ids = torch.rand(M, V, generator=g).topk(K, -1).indices.sort(-1).values
+    u = (torch.randn(M, K, generator=g) * 3).log_softmax(-1)
+    zk, lse = z.gather(1, ids) / T, torch.logsumexp(z[:, :Vc] / T, -1)
+    labels = ids.gather(1, torch.randint(0, K, (M, 1), generator=g))[:, 0]
+    labels[torch.rand(M, generator=g) < 0.4] = 3                              # mostly outside the row's ids
+    labels[labels >= Vc] = 3
+    seg = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens))
+    last = torch.tensor(lens).cumsum(0) - 1
+    if M > 1:
+        labels[last] = -1
+    avoid = torch.rand(M, generator=g) < 0.1
+    if M > 10:
+        u[5], u[9, 1:] = float("-inf"), float("-inf")
+        labels[5] = labels[9] = -1
+    grads, outs = [], []
+    for dev, dt in ((DEV, torch.float32), ("cpu", torch.float64)):
+        a, b = (x.to(dev, dt).clone().requires_grad_() for x in (lse, zk))
+        args = [x.to(dev) for x in (ids.int(), labels, avoid, seg)]
+        if dev == DEV:
+            assert head._native_reference_loss(b, u.to(dev), *args)
+            custom, logs = head._ReferenceLossFn.apply(a, b, u.to(dev), *args, len(lens), T, Vc, 2.0)
+            logs = dict(zip(dv.LOSS_KEYS, logs))
+        else:
+            s, t = dv.student_teacher_logprobs(a, b, u.to(dt), args[0] < Vc, T)
+            custom, logs = dv.reference_loss_segments(s, t, args[0].long(), *args[1:], len(lens), 2.0)
+        (custom * torch.arange(1, len(lens) + 1, device=dev)).sum().backward()
+        grads.append([x.grad.double().cpu() for x in (a, b)])
+        outs.append({k: v.detach().double().cpu() for k, v in logs.items()})
+        assert torch.equal(logs["custom loss"].isnan(), custom.isnan())
+    for k in dv.LOSS_KEYS:
+        x, y = outs[0][k], outs[1][k]
+        assert torch.equal(x.isnan(), y.isnan()), k                           # no labelled row: 0 / 0 in both
+        assert ((x - y).abs().nan_to_num(0) <= 2e-5 * y.nan_to_num(0).abs().max() + 2e-6).all(), k
+    for x, y in zip(*grads):
+        assert torch.equal(x.isnan(), y.isnan())
+        assert (x - y).nan_to_num(0).abs().max() <= 2e-5 * y.nan_to_num(0).abs().max() + 1e-9
+    assert _lib.take_device_error() == 0
