@@ -521,7 +521,7 @@ class LlamaModel(nn.Module):
         """Inference-only forward in chunks of ``chunk_len`` positions against a key / value cache - the reference's
         long-context mechanism (classes/teacher/inference_worker.py:38-48: ``max_input_len = seq_chunk_len`` with an
         ExLlamaV2 cache). Per chunk the activations are [B*chunk_len, .] instead of [B*L, .]; every layer keeps its
-        rotated keys and its values for all positions seen so far ([B, L, Hkv*d] each, zero-filled beyond), and the
+        rotated keys and its values for all positions seen so far ([B, L, Hkv*d] each), and the
         chunk's queries attend to positions <= their own. Same result as ``hidden_states`` up to rounding."""
         cfg = self.cfg
         split = self.ordered_sums is False and not cfg.num_local_experts      # expert layers: see models/moe.py
@@ -532,8 +532,8 @@ class LlamaModel(nn.Module):
         H, Hkv, d = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         tables = self.layer_rope(*self.rope(dev, L))
         kv = Hkv * d
-        caches = [(torch.zeros((B, L, kv), dtype=self.embed_tokens.dtype, device=dev),
-                   torch.zeros((B, L, kv), dtype=self.embed_tokens.dtype, device=dev)) for _ in self.layers]
+        caches = [tuple(torch.empty((B, L, kv), dtype=self.embed_tokens.dtype, device=dev) for _ in range(2))
+                  for _ in self.layers]
         out = torch.empty((B, L, cfg.hidden_size), dtype=self.embed_tokens.dtype, device=dev)
         ids = input_ids.to(dev)
         for c0 in range(0, L, chunk_len):
@@ -553,8 +553,7 @@ class LlamaModel(nn.Module):
                         basic.rope_(qkv, pos, cos, sin, H + Hkv, d)
                         if after_rotation is not None:
                             qkv = after_rotation(qkv)
-                        kc[:, c0:c0 + n] = qkv[:, H * d:(H + Hkv) * d].reshape(B, n, kv)
-                        vc[:, c0:c0 + n] = qkv[:, (H + Hkv) * d:].reshape(B, n, kv)
+                        attention.cache_append(qkv, kc, vc, B, n, c0, H, Hkv, d)
                         return attention.attention_fwd_cached(qkv, kc, vc, B, n, c0, H, Hkv, d, window)
                     h = layer_inference(layer, cfg, h, attend, cfg.rms_norm_eps)
                     continue
@@ -571,8 +570,7 @@ class LlamaModel(nn.Module):
                     elif cfg.qk_norm:
                         qkv, _ = basic.headnorm_fwd(qkv, layer.q_norm, layer.k_norm, H, Hkv, d, cfg.rms_norm_eps)
                     basic.rope_(qkv, pos, cos, sin, H + Hkv, d)
-                kc[:, c0:c0 + n] = qkv[:, H * d:(H + Hkv) * d].reshape(B, n, kv)
-                vc[:, c0:c0 + n] = qkv[:, (H + Hkv) * d:].reshape(B, n, kv)
+                attention.cache_append(qkv, kc, vc, B, n, c0, H, Hkv, d)
                 att = attention.attention_fwd_cached(qkv, kc, vc, B, n, c0, H, Hkv, d, window)
                 rm = float(cfg.residual_multiplier)
                 h1 = basic.gemm(att, layer.o_proj, residual=h, alpha=rm, split_k=split)

@@ -183,6 +183,24 @@ def attention_cached_reference_fwd(qkv, k_cache, v_cache, B, L, q_off, H, Hkv, d
     return torch.einsum("bhlm,bmhd->blhd", p, v).reshape(B * L, H * d).to(qkv.dtype)
 
 
+def cache_append(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, B: int, n: int, c0: int, H: int, Hkv: int,
+                 d: int) -> None:
+    """The keys and values of a prefill chunk (positions c0 .. c0+n-1 of each of B sequences, packed in ``qkv``) into the
+    caches [B, rows, Hkv*d]. Rows behind them are zeroed up to the end of a tile of keys: the flash kernels load whole tiles
+    (64 keys), and the masked part must be finite. So a cache need not be zeroed when it is allocated."""
+    kv, rows = Hkv * d, k_cache.shape[1]
+    zero_end = min(rows, (c0 + n + 127) // 128 * 128)
+    if (qkv.is_cuda and kv % 8 == 0 and (H * d) % 8 == 0 and qkv.shape == (B * n, (H + 2 * Hkv) * d)
+            and k_cache.shape == v_cache.shape == (B, rows, kv)
+            and all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (qkv, k_cache, v_cache))):
+        from . import flash
+        flash.kv_append(qkv, k_cache, v_cache, B, n, zero_end, c0, H * d)
+        return
+    for cache, first in ((k_cache, H * d), (v_cache, (H + Hkv) * d)):
+        cache[:, c0:c0 + n] = qkv[:, first:first + kv].reshape(B, n, kv)
+        cache[:, c0 + n:zero_end] = 0
+
+
 def attention_fwd_cached(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, B: int, L: int, q_off: int,
                          H: int, Hkv: int, d: int, window: int | None = None) -> torch.Tensor:
     """Attention of one prefill chunk against the key / value caches (which already contain the chunk's own keys and

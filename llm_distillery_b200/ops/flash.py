@@ -9,6 +9,7 @@ from ._lib import _VP, _I, _LL
 _lib.register("b200_flash_attn_fwd", [_VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP])
 _lib.register("b200_flash_attn_fwd_cached", [_VP, _VP, _VP, _LL, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _VP])
 _lib.register("b200_flash_attn_bwd", [_VP, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP])
+_lib.register("b200_kv_append", [_VP, _VP, _VP, _I, _I, _I, _LL, _I, _I, _I, _LL, _VP])
 _lib.register("b200_dq_convert_rope", [_VP, _VP, _VP, _VP, _VP, _LL, _I, _I, _LL, _VP])
 _lib.register("b200_flash_attn_bwd_rope", [_VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP])
 
@@ -63,3 +64,10 @@ def flash_attn_fwd_cached(qkv, k_cache, v_cache, B, L, q_off, H, Hkv, d, window:
                                                    _lib.ptr(out), None, B, L, q_off, _window(window, q_off + L), H, Hkv, d, _lib.stream())
     _lib.check(rc, "b200_flash_attn_fwd_cached")
     return out
+
+
+def kv_append(qkv, k_cache, v_cache, B, n, zero_end, c0, col0):
+    """Columns col0 .. of the chunk's packed rows into rows c0 .. c0+n-1 of both caches; zeros up to row ``zero_end``."""
+    _lib.check(_lib.kernels().b200_kv_append(_lib.ptr(qkv), _lib.ptr(k_cache), _lib.ptr(v_cache), B, n, zero_end,
+                                             k_cache.shape[1], c0, col0, k_cache.shape[2], qkv.shape[1], _lib.stream()),
+               "b200_kv_append")

@@ -260,3 +260,23 @@ def test_query_heads_shared_by_a_cluster(B, L, H, Hkv, d, window):
     for cols in (slice(0, H * d), slice(H * d, (H + Hkv) * d), slice((H + Hkv) * d, None)):
         assert (got[:, cols].float() - want[:, cols]).abs().max() <= 2e-2 * want[:, cols].abs().max() + 1e-6
     assert torch.equal(got[:, H * d:], again[:, H * d:]) and _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("B,n,c0,rows,H,Hkv,d", [(1, 1, 0, 1, 2, 1, 64), (2, 100, 0, 777, 4, 2, 64), (3, 256, 512, 1000, 2, 2, 128),
+                                                 (2, 37, 100, 137, 3, 1, 64), (1, 65, 63, 4096, 8, 8, 128)])
+def test_cache_append_is_the_slice_assignment(B, n, c0, rows, H, Hkv, d):
+    """One launch for the keys and values of a chunk: the bits of the two slice assignments, zeros behind them up to a
+    multiple of 128 rows (or the cache's end), nothing else touched."""
+    torch.manual_seed(n)
+    qkv = torch.randn(B * n, (H + 2 * Hkv) * d, device=DEV).bfloat16()
+    caches = [torch.full((B, rows, Hkv * d), float("nan"), device=DEV, dtype=torch.bfloat16) for _ in range(4)]
+    attention.cache_append(qkv, caches[0], caches[1], B, n, c0, H, Hkv, d)
+    wide = torch.zeros(B * n, (H + 2 * Hkv) * d + 1, device=DEV, dtype=torch.bfloat16)
+    wide[:, 1:] = qkv
+    attention.cache_append(wide[:, 1:], caches[2], caches[3], B, n, c0, H, Hkv, d)        # strided rows: slice by slice
+    for i, first in ((0, H * d), (1, (H + Hkv) * d)):
+        want = torch.full_like(caches[i], float("nan"))
+        want[:, c0:c0 + n] = qkv[:, first:first + Hkv * d].reshape(B, n, -1)
+        want[:, c0 + n:(c0 + n + 127) // 128 * 128] = 0
+        for got in (caches[i], caches[i + 2]):
+            assert torch.equal(got.view(torch.int16), want.view(torch.int16))
