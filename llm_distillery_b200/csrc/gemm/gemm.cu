@@ -946,7 +946,7 @@ struct ClusterSwigluBwd {
 // BN/2 up rows: f = b_half > 0).
 template <int BN, bool DEEP, bool A_MN, bool B_MN, class Epi>
 static int launch_cluster(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int fmt,
-                          const typename Epi::Params& ep, int slices, int b_half, cudaStream_t stream) {
+                          const typename Epi::Params& ep, int slices, int b_half, int b_early, cudaStream_t stream) {
   using S = SmemCluster<BN, DEEP>;
   CUtensorMap tmA, tmB;
   const CUtensorMapDataType dt = fmt == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -970,7 +970,7 @@ static int launch_cluster(const void* A, const void* B, int M, int N, int K, lon
   }
   const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, BN);
   launch_pdl_cluster(kern, dim3((unsigned)(tiles * slices)), dim3(NUM_THREADS), S::BYTES, stream, slices, tmA, tmB, M, N, K,
-                     fmt, ep, device_err_word(), b_half);
+                     fmt, ep, device_err_word(), b_half, b_early);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -1009,7 +1009,10 @@ static bool use_pair(int M, int N, int K) {
 // resident CTAs. Examples, one CTA per tile before / cluster now: 93 x 2048 x 5632 37.8 / 11.0, 93 x 2560 x 2048 17.2 /
 // 7.4, 777 x 896 x 9728 59.3 / 21.4 (43.4 in one slice), 896 x 896 x 776 (weight gradient) 11.3 / 7.7; 2048 x 2048 x 2048
 // stays where it is (17.7, cluster 20.2: tiles of 128 x 128 read twice the operand bytes per product and are bound by the L2).
-struct TilePlan { int bn, slices; };
+struct TilePlan {
+  int bn, slices;
+  int b_early = 0;      // B may be loaded before the kernel in front of this one has completed
+};
 // A CTA may take the shared memory of two where the grid fits the SMs at one each; clusters only up to 3/4 of them (147
 // CTAs in clusters of 3 with an SM each ran as two rounds: 37.5 us, in shared SMs 30).
 static bool deep_ring(long long ctas, int slices) {
@@ -1047,12 +1050,12 @@ template <bool A_MN, bool B_MN, class Epi>
 static int launch_cluster_bn(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int fmt,
                              const typename Epi::Params& ep, TilePlan plan, int b_half, cudaStream_t stream) {
   const bool deep = deep_ring((long long)ceil_div(M, BM) * ceil_div(N, plan.bn) * plan.slices, plan.slices);
-  const int s = plan.slices;
+  const int s = plan.slices, e = plan.b_early;
   if (plan.bn == 64)
-    return deep ? launch_cluster<64, true, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, stream)
-                : launch_cluster<64, false, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, stream);
-  return deep ? launch_cluster<128, true, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, stream)
-              : launch_cluster<128, false, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, stream);
+    return deep ? launch_cluster<64, true, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, e, stream)
+                : launch_cluster<64, false, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, e, stream);
+  return deep ? launch_cluster<128, true, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, e, stream)
+              : launch_cluster<128, false, A_MN, B_MN, Epi>(A, B, M, N, K, lda, ldb, fmt, ep, s, b_half, e, stream);
 }
 
 }  // namespace gemm
@@ -1082,7 +1085,8 @@ int b200_gemm_swiglu(const void* x, const void* Wgu, void* gu, void* act, int M,
       (ld_gu & 7) || (ld_act & 7) || (reinterpret_cast<uintptr_t>(gu) & 15) || (reinterpret_cast<uintptr_t>(act) & 15))
     return B200_ERR_ARG;
   SwigluParams sp{reinterpret_cast<__nv_bfloat16*>(gu), ld_gu, reinterpret_cast<__nv_bfloat16*>(act), ld_act, f};
-  const TilePlan plan = plan_tiles(M, 2 * f, K, false, split_k != 0);
+  TilePlan plan = plan_tiles(M, 2 * f, K, false, split_k & 1);
+  plan.b_early = split_k & 2;
   if (plan.bn) return launch_cluster_bn<false, false, ClusterSwiglu>(x, Wgu, M, 2 * f, K, ldx, ldw, 1, sp, plan, f, stream);
   return launch_swiglu_pair(x, Wgu, M, f, K, ldx, ldw, sp, stream);
 }
@@ -1130,7 +1134,8 @@ int b200_gemm_rope(const void* x, const void* W, void* out, const int* pos, cons
       (reinterpret_cast<uintptr_t>(out) & 15))
     return B200_ERR_ARG;
   RopeParams rp{reinterpret_cast<__nv_bfloat16*>(out), ldo, pos, cos_tab, sin_tab, d, n_rot_heads * d};
-  TilePlan plan = plan_tiles(M, N, K, false, split_k != 0);
+  TilePlan plan = plan_tiles(M, N, K, false, split_k & 1);
+  plan.b_early = split_k & 2;
   if (plan.bn) {
     if (plan.bn < d) plan.bn = d;            // a tile holds whole heads
     return launch_cluster_bn<false, false, ClusterRope>(x, W, M, N, K, ldx, ldw, 1, rp, plan, 0, stream);
@@ -1148,7 +1153,8 @@ int b200_gemm_swiglu_bwd(const void* dy, const void* Wd, const void* gu, void* d
       (ld_gu & 7) || (ld_dgu & 7) || (reinterpret_cast<uintptr_t>(gu) & 15) || (reinterpret_cast<uintptr_t>(dgu) & 15))
     return B200_ERR_ARG;
   SwigluBwdParams sp{reinterpret_cast<const __nv_bfloat16*>(gu), ld_gu, reinterpret_cast<__nv_bfloat16*>(dgu), ld_dgu, f};
-  const TilePlan plan = plan_tiles(M, f, K, false, split_k != 0);
+  TilePlan plan = plan_tiles(M, f, K, false, split_k & 1);
+  plan.b_early = split_k & 2;
   if (plan.bn) return launch_cluster_bn<false, true, ClusterSwigluBwd>(dy, Wd, M, f, K, ld_dy, ldw, 1, sp, plan, 0, stream);
   return launch_swiglu_bwd_pair(dy, Wd, M, f, K, ld_dy, ldw, sp, stream);
 }
@@ -1158,7 +1164,8 @@ int b200_gemm_swiglu_bwd(const void* dy, const void* Wd, const void* gu, void* d
 //   b_mn = 0: B is [N,K] with row stride ldb;   b_mn = 1: B is stored [K,N] with row stride ldb
 //   fmt: 1 = bf16 operands, 0 = fp16.  out_f32: C is fp32, else the operand type.
 // Strides are in elements and must be multiples of 8 (16 bytes); base pointers 16-byte aligned.
-// split_k: K may be cut over the CTAs of a cluster (plan_tiles).
+// split_k: bit 0: K may be cut over the CTAs of a cluster (plan_tiles); bit 1: the kernel launched just before on the stream
+// does not write B, so that B may be read while that kernel still runs (gemm_cluster.cuh). The same in the fused forms above.
 // desc_cfg: optional 6 x uint32 override of the matrix-descriptor byte offsets (testing hook), else null.
 int b200_gemm(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
               long long ldc, int a_mn, int b_mn, int fmt, int out_f32, int accumulate, float alpha,
@@ -1184,7 +1191,8 @@ int b200_gemm(const void* A, const void* B, void* C, int M, int N, int K, long l
     dcp = &dco;
   }
   if (!dcp && pair_mode() < 0) {
-    const TilePlan plan = plan_tiles(M, N, K, out_f32 != 0, split_k != 0);
+    TilePlan plan = plan_tiles(M, N, K, out_f32 != 0, split_k & 1);
+    plan.b_early = split_k & 2;
     if (plan.bn) {
       if (!a_mn && !b_mn)
         return launch_cluster_bn<false, false, ClusterStore>(A, B, M, N, K, lda, ldb, fmt, sp, plan, 0, stream);

@@ -39,12 +39,6 @@ __device__ __forceinline__ uint32_t cluster_nctas() {
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr)
-               : "memory");
-  return v;
-}
 
 // Epi concept: Params; SPLIT_B (the tile's B rows are BN/2 rows at n and BN/2 rows b_half_stride below them);
 // items<BN>() work items per row; item<BN>(p, row, n0, N, it, get) with get(chunk) = the four accumulator columns
@@ -52,7 +46,7 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
 template <int BN, bool DEEP, bool A_MN, bool B_MN, class Epi>
 __global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
     gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
-                        int K, int fmt, typename Epi::Params ep, unsigned int* err_word, int b_half_stride) {
+                        int K, int fmt, typename Epi::Params ep, unsigned int* err_word, int b_half_stride, int b_early) {
   using S = SmemCluster<BN, DEEP>;
   constexpr int STAGES = S::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -87,9 +81,6 @@ __global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();
-  pdl_trigger();
-
   const int m_tiles = (M + BM - 1) / BM;
   const int tile = (int)blockIdx.x / n_slices;
   const int m0 = (tile % m_tiles) * BM;          // row tiles fastest: CTAs side by side read the same weights
@@ -99,28 +90,49 @@ __global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
   const int kb0 = (int)((long long)num_kb * slice / n_slices);
   const int kb1 = (int)((long long)num_kb * (slice + 1) / n_slices);
 
+  auto load_b = [&](int kb) {
+    const uint32_t st = (uint32_t)(kb - kb0) % STAGES;
+    uint8_t* sB = smem + st * S::STAGE_BYTES + S::A_BYTES;
+    if constexpr (B_MN) {
+#pragma unroll
+      for (int i = 0; i < BN / 64; ++i) tma_load_2d(sB + i * (BK * 128), &tmB, &full_bar[st], n0 + i * 64, kb * BK);
+    } else if constexpr (Epi::SPLIT_B) {
+      tma_load_2d(sB, &tmB, &full_bar[st], kb * BK, n_blk * (BN / 2));
+      tma_load_2d(sB + (BN / 2) * 128, &tmB, &full_bar[st], kb * BK, b_half_stride + n_blk * (BN / 2));
+    } else {
+      tma_load_2d(sB, &tmB, &full_bar[st], kb * BK, n0);
+    }
+  };
+  // B of the ring's first round in front of pdl_wait, where the caller says that the kernel before this one does not write
+  // it (a layer's weights): those bytes then arrive while that kernel drains. A grid starts early only when every CTA of the
+  // one before it is past its own wait, so whatever ran before THAT one is complete and visible here. Steps of 512 and of 777
+  // tokens 1.4 and 1.0 % shorter, a forward pass over 93 tokens 1.8 %.
+  const int early = b_early ? min(kb1 - kb0, STAGES) : 0;
+  if (warp == 0 && lane == 0) {
+    for (int i = 0; i < early; ++i) {
+      mbar_arrive_expect_tx(&full_bar[i], S::STAGE_BYTES);
+      load_b(kb0 + i);
+    }
+  }
+  __syncwarp();
+  pdl_wait();
+  pdl_trigger();
+
   if (warp == 0) {
     if (lane == 0) {
       for (int kb = kb0; kb < kb1; ++kb) {
         const uint32_t it = kb - kb0, s = it % STAGES, ph = (it / STAGES) & 1u;
         if (!mbar_wait_bounded(&empty_bar[s], ph ^ 1u, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
         uint8_t* sA = smem + s * S::STAGE_BYTES;
-        uint8_t* sB = sA + S::A_BYTES;
-        mbar_arrive_expect_tx(&full_bar[s], S::STAGE_BYTES);
+        if ((int)it >= early) {
+          mbar_arrive_expect_tx(&full_bar[s], S::STAGE_BYTES);
+          load_b(kb);
+        }
         if constexpr (!A_MN) {
           tma_load_2d(sA, &tmA, &full_bar[s], kb * BK, m0);
         } else {
 #pragma unroll
           for (int i = 0; i < BM / 64; ++i) tma_load_2d(sA + i * (BK * 128), &tmA, &full_bar[s], m0 + i * 64, kb * BK);
-        }
-        if constexpr (B_MN) {
-#pragma unroll
-          for (int i = 0; i < BN / 64; ++i) tma_load_2d(sB + i * (BK * 128), &tmB, &full_bar[s], n0 + i * 64, kb * BK);
-        } else if constexpr (Epi::SPLIT_B) {
-          tma_load_2d(sB, &tmB, &full_bar[s], kb * BK, n_blk * (BN / 2));
-          tma_load_2d(sB + (BN / 2) * 128, &tmB, &full_bar[s], kb * BK, b_half_stride + n_blk * (BN / 2));
-        } else {
-          tma_load_2d(sB, &tmB, &full_bar[s], kb * BK, n0);
         }
       }
     }

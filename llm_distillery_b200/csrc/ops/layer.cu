@@ -43,6 +43,11 @@ struct Dims {
   bool ok() const { return B > 0 && L > 0 && H > 0 && Hkv > 0 && (d == 64 || d == 128) && h > 0 && f > 0 && T <= 0x7fffffff; }
 };
 
+// A GEMM of this layer may start on its weights while the launch before it drains (bit 1 of split_k): that launch is one of
+// this layer's own, which write no weights. Not for the first launch of a call: what stands in front of it may expand or
+// update them.
+constexpr int kWeightsEarly = 2;
+
 // Carves 256-byte aligned pieces off a slab (base null: only sizes).
 struct Slab {
   uint8_t* base;
@@ -133,6 +138,7 @@ extern "C" int b200_layer_fwd(const void* x, const int* pos, const float* cos_ta
   const layer::Saved s(m, saved);
   const int T = (int)m.T, N = (int)m.N, A = (int)m.A;
   int launches = 0;
+  split_k |= layer::kWeightsEarly;
   RUN(b200_rmsnorm_fwd(x, nullptr, w_ln1, s.n1, nullptr, s.rstd1, T, h, eps, st));
   if (!b_qkv && N % 128 == 0) {
     RUN(b200_gemm_rope(s.n1, w_qkv, s.qkv, pos, cos_tab, sin_tab, T, N, h, H + Hkv, d, h, h, N, split_k, st));
@@ -170,13 +176,14 @@ extern "C" int b200_layer_bwd(const void* dh2, const void* x, const int* pos, co
   auto wgrad = [&](const void* dy, int n, const void* in, int k, float* g, int bit) {     // g[n, k] (+)= dy^T in
     return b200_gemm(dy, in, g, n, k, T, n, k, k, 1, 1, 1, 1, (acc >> bit) & 1, 1.f, nullptr, 0, nullptr, split_k, st);
   };
+  auto early = [&]() { return split_k | (launches > 0 ? layer::kWeightsEarly : 0); };
   auto dgrad = [&](const void* dy, int n, const void* w, int k, void* out) {              // out[T, k] = dy[T, n] w[n, k]
-    return b200_gemm(dy, w, out, T, k, n, n, k, k, 0, 1, 1, 0, 0, 1.f, nullptr, 0, nullptr, split_k, st);
+    return b200_gemm(dy, w, out, T, k, n, n, k, k, 0, 1, 1, 0, 0, 1.f, nullptr, 0, nullptr, early(), st);
   };
   // MLP branch
   if (g_d) RUN(wgrad(dh2, h, s.act, f, g_d, 5));
   if (f % 128 == 0) {
-    RUN(b200_gemm_swiglu_bwd(dh2, w_d, s.gu, t.dgu, T, f, h, h, f, 2LL * f, 2LL * f, split_k, st));
+    RUN(b200_gemm_swiglu_bwd(dh2, w_d, s.gu, t.dgu, T, f, h, h, f, 2LL * f, 2LL * f, early(), st));
   } else {
     RUN(dgrad(dh2, h, w_d, f, t.dact));
     RUN(b200_swiglu_bwd(s.gu, t.dact, t.dgu, T, f, st));
