@@ -85,40 +85,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
-// Non-suspending variant for the single threads that issue MMAs or TMA loads: mbarrier.test_wait returns at once, so
-// the waiter sees a completed phase within a few cycles (try_wait may park the thread, and waking it took 300+ cycles
-// in the attention kernels, where these hand-offs sit on the critical path). Same bound and abort protocol.
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_spin_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                                  unsigned int* err_word, unsigned int code) {
-  if (mbar_test_wait(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
-  uint32_t spins = 0;
-  while (true) {
-    if (mbar_test_wait(bar, parity)) return true;
-    if (((++spins) & 0xfffu) == 0u) {
-      if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > kWaitTimeoutNs) {
-        *abort_flag = 1;
-        if (err_word) atomicCAS(err_word, 0u, code);
-        return false;
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------- counters in global memory shared by the CTAs of a kernel
 __device__ __forceinline__ unsigned int ld_acquire_gpu_u32(const unsigned int* addr) {
   unsigned int v;
@@ -310,7 +276,18 @@ __device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&r)[32]) {
                :
                : "memory");
 }
-// registers -> TMEM (thread t writes lane base_lane + t, 16/32 consecutive columns)
+__device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+// registers -> TMEM (thread t writes lane base_lane + t, 8/16 consecutive columns)
+__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]));
+}
 __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "

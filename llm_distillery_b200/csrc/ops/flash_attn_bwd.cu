@@ -22,12 +22,13 @@
 // Order: S of the next pair is issued while the compute warps work on this one, so they go from dS_i straight to the
 // exponentials of pair i + 1 while dK_i, dP_{i+1} and dQ_i run. Head dim 64: two S buffers; P_i in the lower half of its
 // buffer, dQ_i in the upper half. Head dim 128 (S, dP, dV, dK take all 512 columns): one S buffer, dQ_i over dP_i.
-// The compute warps' fixed work is 16 K exponentials a pair (1024 clocks of the MUFU unit). Neither they (all of them taken
-// out: 7 % faster at head dim 64) nor the reduce-adds (2.5 %) bound the kernel, but the chain dS_i -> dK_i -> dP_{i+1} -> dS_{i+1}
-// with its barriers, about 3500 clocks a pair at head dim 64 and 4600 at 128.
-// All three kernels of a backward pass, B200, queries as rows and one S / dP buffer before / now: 8 x 2048, 32/4 heads of 64
-// 638 / 570 us; 4 x 4096, 32/8 of 64 1136 / 994; 2 x 4096, 32/8 of 128 1199 / 808; 1 x 777, 14/2 of 64 122 / 34.
-//
+// The compute warps' fixed work is 16 K exponentials a pair (1024 clocks of the MUFU unit). No single path bounds the kernel
+// (head dim 64, 523 us: without the reads of lse and delta 490, without those, exponentials, stores of dS and reduce-adds 408):
+// what remains is the chain dS_i -> dK_i -> dP_{i+1} -> dS_{i+1} with its barriers, about 2700 clocks a pair, with two compute
+// warps per scheduler to fill it. Four of them with 32 columns each measured the same (head dim 64) or slower (128: 80
+// registers a thread; 800 against 710 us).
+// All three kernels of a backward pass, B200, queries as rows and one S / dP buffer / now: 8 x 2048, 32/4 heads of 64
+// 638 / 521 us; 2 x 4000, 32/8 of 128 1191 / 710; 1 x 777, 14/2 of 64 122 / 33.
 // Few key blocks (short sequences, few kv heads) leave SMs idle while each CTA walks all query heads of its group: then a
 // cluster of up to 8 CTAs shares the heads, and the partial dK / dV meet through distributed shared memory, added in the
 // order of the CTAs' ranks (`head_split` below; results repeat bit for bit).
@@ -43,6 +44,10 @@ constexpr int NTHREADS = 512;
 constexpr int FIRST_DRAIN_WARP = 4;
 constexpr int FIRST_COMPUTE_WARP = 8;
 constexpr int NCOMPUTE_WARPS = 8;
+constexpr int CP = 64;   // query columns of a tile per compute warp; two warps share a TMEM lane quadrant
+// Registers a thread after setmaxnreg, of 128 at launch: the compute warps hold 64 probabilities, a drain warp whole rows of dQ
+constexpr int REGS_ISSUE = 64, REGS_DRAIN = 152, REGS_COMPUTE = 144;
+static_assert(REGS_ISSUE + REGS_DRAIN + 2 * REGS_COMPUTE <= 4 * 128, "registers of the block");
 constexpr int SUB = 128 * 128;   // bytes of a [128 rows x 64] bf16 sub-tile with 128-byte rows
 
 template <int D>
@@ -75,9 +80,9 @@ struct Cfg {
   static constexpr uint32_t DK_COL = DV_COL + D;
   static constexpr uint32_t TMEM_COLS = 512;
   static_assert(DK_COL + D == TMEM_COLS, "TMEM budget");
-  // P^T, 16 queries per 8 columns: at the start of the S buffer (64: dQ needs 64 whole columns behind it, so the second
-  // warp of a quadrant stores over scores of the first), or each warp's at the start of its own half (128)
-  static constexpr uint32_t P_HALF = (D == 64) ? 32 : 64;
+  // P^T, 16 queries per 8 columns: at the start of the S buffer (64: dQ needs 64 whole columns behind it, so a warp stores
+  // over scores of a warp before it), or each warp's at the start of its own columns (128)
+  static constexpr uint32_t P_PART = (D == 64) ? CP / 2 : CP;
   // dQ of a pair: the upper half of its S buffer (64), or over dP (128)
   static __device__ __forceinline__ uint32_t dq_col(int buf) { return D == 64 ? S_COL + buf * 128 + 64 : DP_COL; }
 };
@@ -115,7 +120,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   uint64_t* dp_full = bars + 21;
   uint64_t* ds_ready = bars + 22;   // compute warps
   uint64_t* dk_done = bars + 23;
-  uint64_t* s_read = bars + 24;     // [2][4] the first warp of a quadrant has read its half of S: the other may store P there
+  uint64_t* s_read = bars + 24;     // [2][4] a quadrant's first warp has read its scores: the second may store P there
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 32);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -181,14 +186,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
   const int colK = p.H * D + hkv * D;
   const int colV = (p.H + p.Hkv) * D + hkv * D;
-  auto spin = [&](uint64_t* bar, uint32_t parity, unsigned int code) {
-    return __all_sync(0xffffffffu, mbar_spin_bounded(bar, parity, abort_flag, err_word, code)) != 0;
+  // Suspending waits for all: 16 warps that poll take issue slots and shared-memory cycles from the compute warps (538 against
+  // 521 us a backward pass of 8 x 2048, 32/4 heads of 64).
+  auto wait = [&](uint64_t* bar, uint32_t parity, unsigned int code) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, err_word, code)) != 0;
   };
 
-  // Registers: 128 a thread at launch; the compute warps hold 64 probabilities and 64 scores. 4 x (64 + 104 + 2 x 168) x 32 =
-  // 64512 of the 65536 that the block was launched with.
   if (warp < FIRST_DRAIN_WARP) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_ISSUE));
     if (warp == 0) {
       // ---------------------------------------------------------------- loads
       if (elect_one()) {
@@ -216,7 +221,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       for (int it = 0; it < n_it; ++it) {
         const int qs = it % QS, os = it % OS;
         const int hq_now = hq, q0 = qb * BM;
-        if (it >= QS && !spin(&q_empty[qs], (it / QS - 1) & 1u, ERR_WAIT_EMPTY)) break;
+        if (it >= QS && !wait(&q_empty[qs], (it / QS - 1) & 1u, ERR_WAIT_EMPTY)) break;
         if (elect_one()) {
           uint8_t* sQ = smem + C::OFF_Q + qs * C::Q_BYTES;
           mbar_arrive_expect_tx(&q_full[qs], C::Q_BYTES);
@@ -237,7 +242,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           ++hq;
         }
         if (it + 1 < n_it) load_stats(hq, qb);
-        if (it >= OS && !spin(&do_empty[os], (it / OS - 1) & 1u, ERR_WAIT_EMPTY)) break;
+        if (it >= OS && !wait(&do_empty[os], (it / OS - 1) & 1u, ERR_WAIT_EMPTY)) break;
         if (elect_one()) {
           uint8_t* sDO = smem + C::OFF_DO + os * C::Q_BYTES;
           mbar_arrive_expect_tx(&do_full[os], C::Q_BYTES);
@@ -261,11 +266,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         const uint64_t kQ = make_smem_desc_sw128(sQ, 16, 1024), kDO = make_smem_desc_sw128(sDO, 16, 1024);
         const uint64_t kK = make_smem_desc_sw128(sK, 16, 1024), kV = make_smem_desc_sw128(sV, 16, 1024);
         auto issue_s = [&](int it) -> bool {
-          if (!spin(&q_full[it % QS], (it / QS) & 1u, ERR_WAIT_FULL)) return false;
+          if (!wait(&q_full[it % QS], (it / QS) & 1u, ERR_WAIT_FULL)) return false;
           if (it >= NSB) {      // the buffer held P (read by dV) and, head dim 64, dQ of pair it - NSB
             const int o = it - NSB;
-            if (!spin(&dv_done[o % NSB], (o / NSB) & 1u, ERR_WAIT_AUX)) return false;
-            if (D == 64 && !spin(&dq_empty[o % NSB], (o / NSB) & 1u, ERR_WAIT_AUX)) return false;
+            if (!wait(&dv_done[o % NSB], (o / NSB) & 1u, ERR_WAIT_AUX)) return false;
+            if (D == 64 && !wait(&dq_empty[o % NSB], (o / NSB) & 1u, ERR_WAIT_AUX)) return false;
           }
           tc_fence_after_sync();
           const uint64_t q = kQ + units(it % QS, C::Q_BYTES);
@@ -278,11 +283,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           __syncwarp();
           return true;
         };
-        bool ok = spin(kv_full, 0, ERR_WAIT_FULL) && issue_s(0);
+        bool ok = wait(kv_full, 0, ERR_WAIT_FULL) && issue_s(0);
         for (int it = 0; ok && it < n_it; ++it) {
-          if (!spin(&do_full[it % OS], (it / OS) & 1u, ERR_WAIT_FULL)) break;
+          if (!wait(&do_full[it % OS], (it / OS) & 1u, ERR_WAIT_FULL)) break;
           if (it > 0) {   // dP of pair it - 1 has been read, and what took its columns since: dS^T by dK (64), dQ by the drain (128)
-            if (D == 64 ? !spin(dk_done, (it - 1) & 1u, ERR_WAIT_AUX) : !spin(&dq_empty[0], (it - 1) & 1u, ERR_WAIT_AUX)) break;
+            if (D == 64 ? !wait(dk_done, (it - 1) & 1u, ERR_WAIT_AUX) : !wait(&dq_empty[0], (it - 1) & 1u, ERR_WAIT_AUX)) break;
           }
           tc_fence_after_sync();
           const uint64_t o = kDO + units(it % OS, C::Q_BYTES);
@@ -301,15 +306,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         const uint64_t tDO = make_smem_desc_sw128(sDO, SUB, 1024);
         for (int it = 0; it < n_it; ++it) {
           const int bf = it % NSB;
-          if (!spin(&p_ready[bf], (it / NSB) & 1u, ERR_WAIT_AUX)) break;
-          if (!spin(&do_full[it % OS], (it / OS) & 1u, ERR_WAIT_FULL)) break;
+          if (!wait(&p_ready[bf], (it / NSB) & 1u, ERR_WAIT_AUX)) break;
+          if (!wait(&do_full[it % OS], (it / OS) & 1u, ERR_WAIT_FULL)) break;
           tc_fence_after_sync();
           const uint64_t o = tDO + units(it % OS, C::Q_BYTES);
           const uint32_t pcol = tmem_base + C::S_COL + bf * 128;
           if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < BM / 16; ++k)
-              umma_f16_ts(tmem_base + C::DV_COL, pcol + (k >> 2) * C::P_HALF + (k & 3) * 8, o + (uint64_t)(k * 128), idesc,
+              umma_f16_ts(tmem_base + C::DV_COL, pcol + (k / (CP / 16)) * C::P_PART + (k % (CP / 16)) * 8, o + (uint64_t)(k * 128), idesc,
                           (it != 0 || k != 0) ? 1u : 0u);
             umma_commit(&dv_done[bf]);
             umma_commit(&do_empty[it % OS]);
@@ -321,9 +326,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         const uint32_t idesc_dq = make_idesc_f16(1, BM, D, 1, 1);
         const uint64_t tQ = make_smem_desc_sw128(sQ, SUB, 1024), tK = make_smem_desc_sw128(sK, SUB, 1024);
         const uint64_t kDS = make_smem_desc_sw128(sDS, 16, 1024), tDS = make_smem_desc_sw128(sDS, SUB, 1024);
-        bool ok = spin(kv_full, 0, ERR_WAIT_FULL);
+        bool ok = wait(kv_full, 0, ERR_WAIT_FULL);
         for (int it = 0; ok && it < n_it; ++it) {
-          if (!spin(ds_ready, it & 1u, ERR_WAIT_AUX)) break;
+          if (!wait(ds_ready, it & 1u, ERR_WAIT_AUX)) break;
           tc_fence_after_sync();
           const uint64_t q = tQ + units(it % QS, C::Q_BYTES);
           const uint64_t ds = units(it % C::NDS, C::P_BYTES);
@@ -333,8 +338,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
               for (int k = 0; k < BM / 16; ++k) {
                 const uint32_t acc = (it != 0 || k != 0) ? 1u : 0u;
-                if constexpr (C::DS_TMEM)   // a compute warp's 64 queries lie at the start of its own half of dP's columns
-                  umma_f16_ts(tmem_base + C::DK_COL, tmem_base + C::DP_COL + (k >> 2) * 64 + (k & 3) * 8,
+                if constexpr (C::DS_TMEM)   // a compute warp's queries lie at the start of its own columns of dP
+                  umma_f16_ts(tmem_base + C::DK_COL, tmem_base + C::DP_COL + (k / (CP / 16)) * CP + (k % (CP / 16)) * 8,
                               q + (uint64_t)(k * 128), idesc_dk, acc);
                 else
                   umma_f16_ss(tmem_base + C::DK_COL, kDS + ds + koff(k), q + (uint64_t)(k * 128), idesc_dk, acc);
@@ -363,36 +368,36 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
   } else if (warp < FIRST_COMPUTE_WARP) {
     // ------------------------------------------------------------------ dQ: TMEM -> staging -> TMA reduce-add
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_DRAIN));
     const int quad = warp & 3;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     uint8_t* stage = smem + C::OFF_DQS + quad * 8192;
     int hq = h_first, qb = i_start;
     for (int it = 0; it < n_it; ++it) {
       const int bf = it % NSB;
-      if (!spin(&dq_full[bf], (it / NSB) & 1u, ERR_WAIT_AUX)) break;
+      if (!wait(&dq_full[bf], (it / NSB) & 1u, ERR_WAIT_AUX)) break;
       tc_fence_after_sync();
       const uint32_t src = tmem_base + lane_addr + C::dq_col(bf);
+      constexpr int NR = D / 64;                 // 64 columns a round through the staging tiles
+      uint32_t v[2 * NR][32];
 #pragma unroll
-      for (int rr = 0; rr < D / 64; ++rr) {
-        uint32_t v0[32], v1[32];
-        tmem_ld_32x32b_x32(src + rr * 64, v0);
-        tmem_ld_32x32b_x32(src + rr * 64 + 32, v1);
-        tmem_ld_wait();
-        if (rr + 1 == D / 64) {
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&dq_empty[bf]);
-        }
+      for (int c = 0; c < 2 * NR; ++c) tmem_ld_32x32b_x32(src + c * 32, v[c]);
+#pragma unroll
+      for (int c = 0; c < 2 * NR; ++c) tmem_ld_wait_for(v[c]);
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&dq_empty[bf]);
+#pragma unroll
+      for (int rr = 0; rr < NR; ++rr) {
         if (lane == 0) tma_store_wait_read0();   // the reduce before this one has read the staging tiles
         __syncwarp();
         uint8_t* rowp = stage + lane * 128;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const int off = (c ^ (lane & 7)) * 16;
-          *reinterpret_cast<uint4*>(rowp + off) = make_uint4(v0[c * 4], v0[c * 4 + 1], v0[c * 4 + 2], v0[c * 4 + 3]);
-          *reinterpret_cast<uint4*>(rowp + 4096 + off) = make_uint4(v1[c * 4], v1[c * 4 + 1], v1[c * 4 + 2], v1[c * 4 + 3]);
-        }
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<uint4*>(rowp + h * 4096 + (c ^ (lane & 7)) * 16) =
+                make_uint4(v[2 * rr + h][c * 4], v[2 * rr + h][c * 4 + 1], v[2 * rr + h][c * 4 + 2], v[2 * rr + h][c * 4 + 3]);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
@@ -413,15 +418,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     if (lane == 0) tma_store_wait_all0();
   } else {
     // ------------------------------------------------------------------ softmax, dS and the epilogue
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_COMPUTE));
     const int quad = warp & 3;
-    const int half = (warp - FIRST_COMPUTE_WARP) >> 2;   // which 64 query columns of the tile
+    const int cpart = (warp - FIRST_COMPUTE_WARP) >> 2;  // which CP query columns of the tile
     const int r = quad * 32 + lane;                      // key row
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const float c2 = p.scale * 1.4426950408889634f;
     const uint64_t c2p = pack_f32x2(c2, c2), scp = pack_f32x2(p.scale, p.scale);
-    const uint32_t tS0 = tmem_base + lane_addr + C::S_COL + half * 64;
-    const uint32_t tDP = tmem_base + lane_addr + C::DP_COL + half * 64;
+    const uint32_t tS0 = tmem_base + lane_addr + C::S_COL + cpart * CP;
+    const uint32_t tDP = tmem_base + lane_addr + C::DP_COL + cpart * CP;
     bool ok = true;
     int qb = i_start;
     for (int it = 0; it < n_it; ++it) {
@@ -430,105 +435,104 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (++qb == nqb) qb = i_start;
       // tile columns lo .. hi (counted from this warp's first) are visible to this key; `masked`: not all of them to every key
       const bool masked = (kv0 + BN - 1) > q0 || (p.window > 0 && q0 + BM - p.window > kv0);
-      const int lo = kv0 + r - q0 - half * 64;
+      const int lo = kv0 + r - q0 - cpart * CP;
       const int hi = p.window > 0 ? lo + p.window - 1 : 0x3fffffff;
-      const float* stat = reinterpret_cast<const float*>(smem + C::OFF_STAT + qs * C::STAT_BYTES) + half * 64;
+      const float* stat = reinterpret_cast<const float*>(smem + C::OFF_STAT + qs * C::STAT_BYTES) + cpart * CP;
 
       // P = exp2(S * c - lse): S_it complete implies that the statistics of its queries are there
-      if (!spin(&s_full[bf], (it / NSB) & 1u, ERR_WAIT_TMEM_FULL) || !spin(&q_full[qs], (it / QS) & 1u, ERR_WAIT_FULL)) {
+      if (!wait(&s_full[bf], (it / NSB) & 1u, ERR_WAIT_TMEM_FULL) || !wait(&q_full[qs], (it / QS) & 1u, ERR_WAIT_FULL)) {
         ok = false;
         break;
       }
       tc_fence_after_sync();
-      uint32_t s[2][32];
-      tmem_ld_32x32b_x32(tS0 + bf * 128, s[0]);
-      tmem_ld_32x32b_x32(tS0 + bf * 128 + 32, s[1]);
-      tmem_ld_wait_for(s[0]);
-      tmem_ld_wait_for(s[1]);
-      if (D == 64 && half == 0) {
+      uint32_t s[CP / 32][32];
+#pragma unroll
+      for (int c = 0; c < CP / 32; ++c) tmem_ld_32x32b_x32(tS0 + bf * 128 + c * 32, s[c]);
+#pragma unroll
+      for (int c = 0; c < CP / 32; ++c) tmem_ld_wait_for(s[c]);
+      if (D == 64 && cpart == 0) {
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&s_read[bf * 4 + quad]);
       }
-      uint32_t pk[32];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < CP / 32; ++c) {
 #pragma unroll
         for (int e = 0; e < 32; e += 4) {
           const ulonglong2 nl = *reinterpret_cast<const ulonglong2*>(stat + c * 32 + e);
           float x0, x1, x2, x3;
           unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[c][e]), __uint_as_float(s[c][e + 1])), c2p, nl.x), x0, x1);
           unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[c][e + 2]), __uint_as_float(s[c][e + 3])), c2p, nl.y), x2, x3);
-          float y0 = fast_exp2(x0), y1 = fast_exp2(x1), y2 = fast_exp2(x2), y3 = fast_exp2(x3);
-          if (masked) {
-            const int q = c * 32 + e;
-            if (q < lo || q > hi) y0 = 0.f;
-            if (q + 1 < lo || q + 1 > hi) y1 = 0.f;
-            if (q + 2 < lo || q + 2 > hi) y2 = 0.f;
-            if (q + 3 < lo || q + 3 > hi) y3 = 0.f;
-          }
-          s[c][e] = __float_as_uint(y0);
-          s[c][e + 1] = __float_as_uint(y1);
-          s[c][e + 2] = __float_as_uint(y2);
-          s[c][e + 3] = __float_as_uint(y3);
-          pk[c * 16 + (e >> 1)] = pack_bf16x2(y0, y1);
-          pk[c * 16 + (e >> 1) + 1] = pack_bf16x2(y2, y3);
+          s[c][e] = __float_as_uint(fast_exp2(x0));
+          s[c][e + 1] = __float_as_uint(fast_exp2(x1));
+          s[c][e + 2] = __float_as_uint(fast_exp2(x2));
+          s[c][e + 3] = __float_as_uint(fast_exp2(x3));
         }
       }
-      if (D == 64 && half == 1) {    // these columns are the first warp's scores: long read by now
-        if (!spin(&s_read[bf * 4 + quad], (it / NSB) & 1u, ERR_WAIT_AUX)) {
+      if (masked) {
+#pragma unroll
+        for (int q = 0; q < CP; ++q)
+          if (q < lo || q > hi) s[q / 32][q % 32] = 0u;
+      }
+      uint32_t pk[CP / 32][16];
+#pragma unroll
+      for (int c = 0; c < CP / 32; ++c)
+#pragma unroll
+        for (int e = 0; e < 32; e += 2)
+          pk[c][e >> 1] = pack_bf16x2(__uint_as_float(s[c][e]), __uint_as_float(s[c][e + 1]));
+      if (D == 64 && cpart == 1) {   // these columns are the first warp's scores: long read by now
+        if (!wait(&s_read[bf * 4 + quad], (it / NSB) & 1u, ERR_WAIT_AUX)) {
           ok = false;
           break;
         }
         tc_fence_after_sync();
       }
-      {
-        const uint32_t dst = tmem_base + lane_addr + C::S_COL + bf * 128 + half * C::P_HALF;
-        tmem_st_32x32b_x16(dst, *reinterpret_cast<const uint32_t(*)[16]>(&pk[0]));
-        tmem_st_32x32b_x16(dst + 16, *reinterpret_cast<const uint32_t(*)[16]>(&pk[16]));
-        tmem_st_wait();
-      }
+#pragma unroll
+      for (int c = 0; c < CP / 32; ++c)
+        tmem_st_32x32b_x16(tmem_base + lane_addr + C::S_COL + bf * 128 + cpart * C::P_PART + c * 16, pk[c]);
+      tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[bf]);
 
       // dS = P * (dP - delta) * scale
-      if (!spin(dp_full, it & 1u, ERR_WAIT_TMEM_FULL)) {
+      if (!wait(dp_full, it & 1u, ERR_WAIT_TMEM_FULL)) {
         ok = false;
         break;
       }
       // the one dS tile of head dim 128 is read by dK of the pair before until that is done; with two tiles the drain of
       // dQ_{it-2}, which S_it waited for, has shown that theirs is free
-      if (C::NDS == 1 && it > 0 && !spin(dk_done, (it - 1) & 1u, ERR_WAIT_AUX)) {
+      if (C::NDS == 1 && it > 0 && !wait(dk_done, (it - 1) & 1u, ERR_WAIT_AUX)) {
         ok = false;
         break;
       }
       tc_fence_after_sync();
-      uint8_t* srow = smem + C::OFF_DS + (it % C::NDS) * C::P_BYTES + half * SUB + r * 128;
-      uint32_t dv[2][32];
-      tmem_ld_32x32b_x32(tDP, dv[0]);
-      tmem_ld_wait_for(dv[0]);
-      tmem_ld_32x32b_x32(tDP + 32, dv[1]);
+      uint8_t* srow = smem + C::OFF_DS + (it % C::NDS) * C::P_BYTES + cpart * SUB + r * 128;
+      uint32_t dv[2][16];                                 // dP, 16 columns at a time, one load ahead
+      tmem_ld_32x32b_x16(tDP, dv[0]);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        if (c == 1) tmem_ld_wait_for(dv[1]);
-        uint32_t pd[16];
+      for (int c = 0; c < CP / 16; ++c) {
+        tmem_ld_wait_for(dv[c & 1]);
+        if (c + 1 < CP / 16) tmem_ld_32x32b_x16(tDP + (c + 1) * 16, dv[(c + 1) & 1]);
+        const uint32_t(&pr)[32] = s[c / 2];
+        uint32_t pd[8];
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          const ulonglong2 nd = *reinterpret_cast<const ulonglong2*>(stat + BM + c * 32 + e);
-          const uint64_t t0 = fma_f32x2(pack_f32x2(__uint_as_float(dv[c][e]), __uint_as_float(dv[c][e + 1])), scp, nd.x);
-          const uint64_t t1 = fma_f32x2(pack_f32x2(__uint_as_float(dv[c][e + 2]), __uint_as_float(dv[c][e + 3])), scp, nd.y);
+        for (int e = 0; e < 16; e += 4) {
+          const ulonglong2 nd = *reinterpret_cast<const ulonglong2*>(stat + BM + c * 16 + e);
+          const int q = (c & 1) * 16 + e;
+          const uint64_t t0 = fma_f32x2(pack_f32x2(__uint_as_float(dv[c & 1][e]), __uint_as_float(dv[c & 1][e + 1])), scp, nd.x);
+          const uint64_t t1 = fma_f32x2(pack_f32x2(__uint_as_float(dv[c & 1][e + 2]), __uint_as_float(dv[c & 1][e + 3])), scp, nd.y);
           float y0, y1, y2, y3;
-          unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(s[c][e]), __uint_as_float(s[c][e + 1])), t0), y0, y1);
-          unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(s[c][e + 2]), __uint_as_float(s[c][e + 3])), t1), y2, y3);
+          unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(pr[q]), __uint_as_float(pr[q + 1])), t0), y0, y1);
+          unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(pr[q + 2]), __uint_as_float(pr[q + 3])), t1), y2, y3);
           pd[e >> 1] = pack_bf16x2(y0, y1);
           pd[(e >> 1) + 1] = pack_bf16x2(y2, y3);
         }
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4)
-          *reinterpret_cast<uint4*>(srow + ((c * 4 + q4) ^ (r & 7)) * 16) =
+        for (int q4 = 0; q4 < 2; ++q4)
+          *reinterpret_cast<uint4*>(srow + ((c * 2 + q4) ^ (r & 7)) * 16) =
               make_uint4(pd[q4 * 4], pd[q4 * 4 + 1], pd[q4 * 4 + 2], pd[q4 * 4 + 3]);
-        if constexpr (C::DS_TMEM) tmem_st_32x32b_x16(tDP + c * 16, pd);
+        if constexpr (C::DS_TMEM) tmem_st_32x32b_x8(tDP + c * 8, pd);
       }
       if constexpr (C::DS_TMEM) tmem_st_wait();
       fence_proxy_async_smem();
@@ -539,8 +543,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // epilogue: dK_j, dV_j (thread = key row, this warp's half of the columns)
     if (ok && n_it > 0) {
       const int last = n_it - 1;
-      ok = spin(dk_done, last & 1u, ERR_WAIT_AUX) && spin(&dv_done[last % NSB], (last / NSB) & 1u, ERR_WAIT_AUX) &&
-           spin(&dq_full[last % NSB], (last / NSB) & 1u, ERR_WAIT_AUX);   // dQ's MMAs have read K: its memory may be reused
+      ok = wait(dk_done, last & 1u, ERR_WAIT_AUX) && wait(&dv_done[last % NSB], (last / NSB) & 1u, ERR_WAIT_AUX) &&
+           wait(&dq_full[last % NSB], (last / NSB) & 1u, ERR_WAIT_AUX);   // dQ's MMAs have read K: its memory may be reused
     }
     if (ok && n_it > 0) {
       tc_fence_after_sync();
@@ -548,22 +552,24 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const bool row_ok = kvi < p.L;
       const long long width = (long long)(p.H + 2 * p.Hkv) * D;
       __nv_bfloat16* row = p.dqkv + ((long long)b * p.L + kvi) * width;
+      constexpr int W = 32;                           // columns at a time; D / 2 of dK and of dV per warp
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {           // D / 64 blocks of 32 columns of dK, then of dV
-        const int which = c / (D / 64);
-        const int col = half * (D / 2) + (c % (D / 64)) * 32;
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(tmem_base + lane_addr + (which == 0 ? C::DK_COL : C::DV_COL) + col, v);
-        tmem_ld_wait();
+      for (int c = 0; c < D / W; ++c) {
+        const int which = c / (D / 2 / W);              // 0: dK, 1: dV
+        const int col = cpart * (D / 2) + (c % (D / 2 / W)) * W;
+        const uint32_t src = tmem_base + lane_addr + (which == 0 ? C::DK_COL : C::DV_COL) + col;
+        uint32_t v[W];
+        tmem_ld_32x32b_x32(src, v);
+        tmem_ld_wait_for(v);
         if (p.hsplit > 1) {
           float* dst = reinterpret_cast<float*>(smem) + r * C::RED_PITCH + which * D + col;
 #pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4)
+          for (int q4 = 0; q4 < W / 4; ++q4)
             *reinterpret_cast<uint4*>(dst + q4 * 4) = make_uint4(v[q4 * 4], v[q4 * 4 + 1], v[q4 * 4 + 2], v[q4 * 4 + 3]);
         } else if (row_ok) {
           __nv_bfloat16* dst = row + (which == 0 ? colK : colV) + col;
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
+          for (int q4 = 0; q4 < W / 8; ++q4) {
             uint4 o;
             o.x = pack_bf16x2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
             o.y = pack_bf16x2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));

@@ -18,6 +18,8 @@
 // Sliding window: a block starts at the tile its first query's window reaches and masks the lower edge the way it masks
 // the diagonal; whole tiles in between take the unmasked path (7 B layer, 32 heads of 128, window 4096, 6001 positions:
 // about 0.5 ms; under a dense band mask in library attention 8.7 ms).
+// Every wait suspends its warp (mbarrier.try_wait): three roles that poll cost the softmax warps issue slots (8 x 2048, 32/4
+// heads of 64 270 / 265 us; 2 x 4000, 32/8 of 128 266 / 257).
 // P never touches shared memory: an N = D MMA fed from shared memory on both sides is bound by shared-memory
 // bandwidth, and the softmax warps issue no st.shared and no proxy fence.
 // TMEM: 2 x 64 score columns + D output columns (<= 256); shared memory 56 KB (D = 64) / 112 KB (D = 128): two CTAs
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
       for (int c = 0; c < D / 64; ++c) tma_load_3d(smem + c * (BM * 128), &tmQ, q_full, colQ + c * 64, q0, b);
       for (int j = 0; j < n_kv; ++j) {
         const int ks = j % KS;
-        if (!mbar_spin_bounded(&k_empty[ks], ((j / KS) & 1u) ^ 1u, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
+        if (!mbar_wait_bounded(&k_empty[ks], ((j / KS) & 1u) ^ 1u, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
         uint8_t* sK = smem + C::OFF_K + ks * C::T_BYTES;
         mbar_arrive_expect_tx(&k_full[ks], C::T_BYTES);
 #pragma unroll
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
       for (int j = 0; j < n_kv; ++j) {
         const int vs = j % VS;
         // V stage j % VS was read by P_{j-VS} V_{j-VS}
-        if (j >= VS && !mbar_spin_bounded(&pv_done[(j - VS) % NBUF], ((j - VS) / NBUF) & 1u, abort_flag, err_word,
+        if (j >= VS && !mbar_wait_bounded(&pv_done[(j - VS) % NBUF], ((j - VS) / NBUF) & 1u, abort_flag, err_word,
                                           ERR_WAIT_EMPTY))
           break;
         uint8_t* sV = smem + C::OFF_V + vs * C::T_BYTES;
@@ -204,8 +206,8 @@ __global__ void __launch_bounds__(NTHREADS, 2)
       for (int j = 0; j < n_kv; ++j) {
         const int bsel = j % NBUF, vs = j % VS;
         // P_j is in TMEM (over the first half of S_j) once the softmax warps have arrived
-        if (!__all_sync(0xffffffffu, mbar_spin_bounded(&p_ready[bsel], (j / NBUF) & 1u, abort_flag, err_word, ERR_WAIT_AUX) &&
-                                         mbar_spin_bounded(&v_full[vs], (j / VS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)))
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&p_ready[bsel], (j / NBUF) & 1u, abort_flag, err_word, ERR_WAIT_AUX) &&
+                                         mbar_wait_bounded(&v_full[vs], (j / VS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)))
           break;
         tc_fence_after_sync();
         const uint64_t stage = static_cast<uint64_t>((vs * C::T_BYTES) >> 4);
@@ -232,14 +234,14 @@ __global__ void __launch_bounds__(NTHREADS, 2)
         dQ[k] = make_smem_desc_sw128(smem_u32(smem) + sub * (BM * 128) + kk * 32, 16, 1024);
         dK[k] = make_smem_desc_sw128(smem_u32(smem + C::OFF_K) + sub * (BN * 128) + kk * 32, 16, 1024);
       }
-      const bool ok = __all_sync(0xffffffffu, mbar_spin_bounded(q_full, 0, abort_flag, err_word, ERR_WAIT_FULL));
+      const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(q_full, 0, abort_flag, err_word, ERR_WAIT_FULL));
       for (int t = 0; ok && t < n_kv; ++t) {
         const int ks = t % KS;
         // buffer t % NBUF held S_{t-NBUF} and then P_{t-NBUF}: it is free when that tile's P V has completed
         if (!__all_sync(0xffffffffu,
-                        (t < NBUF || mbar_spin_bounded(&pv_done[t % NBUF], ((t - NBUF) / NBUF) & 1u, abort_flag, err_word,
+                        (t < NBUF || mbar_wait_bounded(&pv_done[t % NBUF], ((t - NBUF) / NBUF) & 1u, abort_flag, err_word,
                                                        ERR_WAIT_AUX)) &&
-                            mbar_spin_bounded(&k_full[ks], (t / KS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)))
+                            mbar_wait_bounded(&k_full[ks], (t / KS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)))
           break;
         tc_fence_after_sync();
         const uint64_t stage = static_cast<uint64_t>((ks * C::T_BYTES) >> 4);
