@@ -204,3 +204,56 @@ extern "C" int b200_layer_bwd(const void* dh2, const void* x, const int* pos, co
   RUN(b200_rmsnorm_bwd(t.dn, x, w_ln1, s.rstd1, t.dh1, dx, t.partial, g_ln1 ? g_ln1 : t.dw, g_ln1 ? acc & 1 : 0, T, h, st));
   return launches + 4;     // the two norms launch a column sum besides, attention its row sums and its conversion
 }
+
+// Several layers in one call: where a batch is a few hundred tokens the host's way from one layer to the next (a foreign call,
+// a graph node, allocations: 45 us) is longer than the layer's kernels take. One record per layer, addresses as integers.
+struct B200StackLayer {
+  unsigned long long cos_tab, sin_tab, w_ln1, w_qkv, w_o, w_ln2, w_gu, w_d, b_qkv, saved, out;
+  long long window;
+};
+struct B200StackGrad {
+  unsigned long long x, g_ln1, g_qkv, g_o, g_ln2, g_gu, g_d, g_bqkv;   // the layer's input; gradients as in b200_layer_bwd
+  long long acc;
+};
+
+// out of the last layer = layers(x). Returns the number of launches, or a negative error code.
+extern "C" int b200_stack_fwd(const B200StackLayer* l, int n, const void* x, const int* pos, int B, int L, int H, int Hkv, int d,
+                              int h, int f, float eps, int split_k, cudaStream_t st) {
+  if (!l || n <= 0 || !x) return B200_ERR_ARG;
+  int launches = 0;
+  for (int i = 0; i < n; ++i) {
+    if (!l[i].out) return B200_ERR_ARG;
+    const int rc = b200_layer_fwd(x, pos, (const float*)l[i].cos_tab, (const float*)l[i].sin_tab, (const void*)l[i].w_ln1,
+                                  (const void*)l[i].w_qkv, (const void*)l[i].w_o, (const void*)l[i].w_ln2,
+                                  (const void*)l[i].w_gu, (const void*)l[i].w_d, (const void*)l[i].b_qkv, (void*)l[i].saved,
+                                  (void*)l[i].out, B, L, (int)l[i].window, H, Hkv, d, h, f, eps, split_k, st);
+    if (rc < 0) return rc;
+    launches += rc;
+    x = (const void*)l[i].out;
+  }
+  return launches;
+}
+
+// dx = gradient of the first layer's input; dx0 and dx1 [T, h] hold the gradients between layers in turn. `done` receives how
+// many layers, from the last on, have run (all of them unless an error code is returned).
+extern "C" int b200_stack_bwd(const B200StackLayer* l, const B200StackGrad* g, int n, const void* dout, const int* pos,
+                              void* scratch, void* dx, void* dx0, void* dx1, int B, int L, int H, int Hkv, int d, int h, int f,
+                              int split_k, int* done, cudaStream_t st) {
+  if (!l || !g || n <= 0 || !done || (n > 1 && (!dx0 || !dx1))) return B200_ERR_ARG;
+  int launches = 0;
+  *done = 0;
+  for (int i = n - 1; i >= 0; --i) {
+    void* to = i == 0 ? dx : (i & 1) ? dx1 : dx0;
+    const int rc = b200_layer_bwd(dout, (const void*)g[i].x, pos, (const float*)l[i].cos_tab, (const float*)l[i].sin_tab,
+                                  (const void*)l[i].w_ln1, (const void*)l[i].w_qkv, (const void*)l[i].w_o,
+                                  (const void*)l[i].w_ln2, (const void*)l[i].w_gu, (const void*)l[i].w_d, (void*)l[i].saved,
+                                  scratch, to, (float*)g[i].g_ln1, (float*)g[i].g_qkv, (float*)g[i].g_o, (float*)g[i].g_ln2,
+                                  (float*)g[i].g_gu, (float*)g[i].g_d, (float*)g[i].g_bqkv, (int)g[i].acc, B, L,
+                                  (int)l[i].window, H, Hkv, d, h, f, split_k, st);
+    if (rc < 0) return rc;
+    launches += rc;
+    ++*done;
+    dout = to;
+  }
+  return launches;
+}

@@ -6,8 +6,13 @@ take.
 ``fits`` says which layers run here: bf16 on a GPU, heads of 64 or 128 with a full rotation, no norms or biases besides the
 two RMSNorms and a q/k/v bias, and every weight either frozen or with a gradient slot to accumulate into. All others, and
 CPU tensors, keep ``DecoderLayerFn``.
+
+``run_stack`` runs all layers of a training pass over few tokens in one native call per direction, when nothing has to happen
+between them.
 """
 from __future__ import annotations
+
+import ctypes
 
 import torch
 
@@ -20,7 +25,9 @@ _lib.register("b200_layer_fwd", [_VP] * 13 + [_I] * 8 + [_F, _I, _VP])
 _lib.register("b200_layer_bwd", [_VP] * 21 + [_I] * 10 + [_VP])
 _lib.register("b200_layer_saved_bytes", [_I] * 7)
 _lib.register("b200_layer_scratch_bytes", [_I] * 7)
-for _n in ("b200_layer_fwd", "b200_layer_bwd", "b200_layer_saved_bytes", "b200_layer_scratch_bytes"):
+_lib.register("b200_stack_fwd", [_VP, _I, _VP, _VP] + [_I] * 7 + [_F, _I, _VP])
+_lib.register("b200_stack_bwd", [_VP, _VP, _I] + [_VP] * 6 + [_I] * 8 + [_VP, _VP])
+for _n in ("b200_layer_fwd", "b200_layer_bwd", "b200_stack_fwd", "b200_stack_bwd", "b200_layer_saved_bytes", "b200_layer_scratch_bytes"):
     _lib.KERNELS_PER_CALL[_n] = 0          # the calls return how many kernels they launched
 
 
@@ -122,3 +129,94 @@ class NativeLayerFn(torch.autograd.Function):
         if llama.LAYER_BACKWARD_DONE[0] is not None:
             llama.LAYER_BACKWARD_DONE[0](weights[0])
         return (dx,) + (None,) * 12
+
+
+# A training pass runs as one node up to this many tokens (a step of 512 tokens and four layers: 1.58 / 1.21 ms). Beyond, a
+# layer's kernels take longer than the host's way to the next layer, and a node per layer gives its activations back as the
+# backward pass moves on. Without gradients a layer's kernels take longer than that way at any size (93 tokens of a 1.1 B
+# teacher, one call per layer 1.67 ms); in one call they start only when all layers have been looked at (1.74).
+STACK_MAX_TOKENS = 2048
+
+
+def run_stack(x, pos, layers, meta, split):
+    """The layers one after the other. ``layers``: (six weights, q/k/v bias or None, cos, sin, window or None) of each, all of
+    which ``fits`` accepts. Same kernels, order and bits as a ``NativeLayerFn`` per layer."""
+    # one weight stands for all of them in the graph: their gradients go to their slots
+    anchor = next((w for ws, b, *_ in layers for w in ws + (b,) if w is not None and w.requires_grad), None)
+    return NativeStackFn.apply(x, anchor, pos, layers, meta, split)
+
+
+def _u64(values):
+    return (ctypes.c_uint64 * len(values))(*values)
+
+
+def _records(layers, L: int, saved: list[int], out: list[int]):
+    """B200StackLayer (csrc/ops/layer.cu) of each layer; ``saved`` and ``out``: addresses of its slab and its output."""
+    rows = []
+    for (ws, b, cos, sin, window), s, o in zip(layers, saved, out):
+        rows += [cos.data_ptr(), sin.data_ptr(), *(w.data_ptr() for w in ws), 0 if b is None else b.data_ptr(), s, o,
+                 0 if window is None or L <= window else window]
+    return _u64(rows)
+
+
+class NativeStackFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, anchor, pos, layers, meta, split):
+        B, L, H, Hkv, d, eps = meta[:6]
+        n, (T, h), f = len(layers), x.shape, layers[0][0][4].shape[0] // 2
+        lib, x = _lib.kernels(), x.contiguous()
+        size = lib.b200_layer_saved_bytes(B, L, H, Hkv, d, h, f)
+        saved = torch.empty(size * n, dtype=torch.uint8, device=x.device)
+        between = torch.empty((n - 1, T, h), dtype=x.dtype, device=x.device)         # the outputs of all layers but the last
+        out = torch.empty_like(x)
+        first, bytes_ = between.data_ptr(), T * h * x.element_size()
+        rows = _records(layers, L, [saved.data_ptr() + i * size for i in range(n)],
+                        [first + i * bytes_ for i in range(n - 1)] + [out.data_ptr()])
+        _launched(lib.b200_stack_fwd(rows, n, x.data_ptr(), pos.data_ptr(), B, L, H, Hkv, d, h, f, eps, int(split[0]),
+                                     _lib.stream()), "b200_stack_fwd")
+        ctx.layers, ctx.meta, ctx.split = layers, meta, split
+        ctx.save_for_backward(x, pos, saved, between)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        from . import llama
+        x, pos, saved, between = ctx.saved_tensors
+        B, L, H, Hkv, d, eps = ctx.meta[:6]
+        n, (T, h), f = len(ctx.layers), x.shape, ctx.layers[0][0][4].shape[0] // 2
+        lib, size, bytes_ = _lib.kernels(), saved.numel() // n, T * h * x.element_size()
+        grads, slots, written = [], [], set()
+        for i in range(n - 1, -1, -1):
+            ws, b, *_ = ctx.layers[i]
+            mine = [llama._slot(w) if w is not None else None for w in ws + (b,)]
+            acc = sum(1 << k for k, s in enumerate(mine) if s is not None and (not s.fresh or id(s) in written))
+            written.update(id(s) for s in mine)
+            slots.insert(0, mine)
+            grads[:0] = [x.data_ptr() if i == 0 else between.data_ptr() + (i - 1) * bytes_,
+                         *(0 if s is None else s.buf.data_ptr() for s in mine), acc]
+        rows, grads = _records(ctx.layers, L, [saved.data_ptr() + i * size for i in range(n)], [0] * n), _u64(grads)
+        dout = dout.contiguous()
+        scratch = torch.empty(lib.b200_layer_scratch_bytes(B, L, H, Hkv, d, h, f), dtype=torch.uint8, device=x.device)
+        turn = torch.empty((2, T, h), dtype=x.dtype, device=x.device)
+        dx, done, at = torch.empty_like(x), ctypes.c_int(0), ctypes.byref
+        hooks = llama.UNIT_PRE[0], llama.LAYER_WEIGHTS_PRE[0], llama.LAYER_BACKWARD_DONE[0]
+        each = any(k is not None for k in hooks)                 # something happens between layers: one at a time
+        for last in (range(n - 1, -1, -1) if each else (n - 1,)):
+            lo, w_ln1 = last if each else 0, ctx.layers[last][0][0]
+            if hooks[0] is not None:
+                hooks[0](w_ln1, True)
+            if hooks[1] is not None:
+                hooks[1](w_ln1)
+            to = dx if lo == 0 else turn[lo & 1]
+            rc = lib.b200_stack_bwd(at(rows, 96 * lo), at(grads, 72 * lo), last - lo + 1, dout.data_ptr(), pos.data_ptr(),
+                                    scratch.data_ptr(), to.data_ptr(), turn[0].data_ptr(), turn[1].data_ptr(), B, L, H, Hkv, d,
+                                    h, f, int(ctx.split[1]), at(done), _lib.stream())
+            for mine in slots[last + 1 - done.value:last + 1]:   # also of a call that failed: the layers that did run
+                for s in mine:
+                    if s is not None:
+                        s.fresh = False
+            _launched(rc, "b200_stack_bwd")
+            dout = to
+            if hooks[2] is not None:
+                hooks[2](w_ln1)
+        return (dx,) + (None,) * 5

@@ -466,6 +466,21 @@ class LlamaModel(nn.Module):
         meta7 = meta
         from . import layer_native
         checked, tables_ok = None, False
+        if (plain and pre is None and LAYER_WEIGHTS_PRE[0] is None and not meta[6] and not cfg.sandwich and not cfg.num_local_experts
+                and training and h.is_cuda and B * L <= layer_native.STACK_MAX_TOKENS):
+            stack = []         # nothing happens between the layers: all of them in one call, if each fits
+            for li, (layer, table) in enumerate(zip(self.layers, tables)):
+                b_qkv = getattr(layer, "qkv_bias", None)
+                w = (layer.input_layernorm, layer.qkv_proj, layer.o_proj, layer.post_attention_layernorm, layer.gate_up_proj,
+                     layer.down_proj)
+                if table is not checked:
+                    checked, tables_ok = table, layer_native.tables_fit(pos, *table, B * L, cfg.head_dim)
+                if not layer_native.fits(h, pos, *table, w, b_qkv, heads, training, tables_ok):
+                    break
+                stack.append((w, b_qkv, *table, cfg.layer_window(li, L)))
+            if stack and len(stack) == len(self.layers) and len({w[4].shape for w, *_ in stack}) == 1:
+                h = layer_native.run_stack(h, pos, stack, meta, split)
+                tables = []
         for li, (layer, table) in enumerate(zip(self.layers, tables)):
             cos, sin = table
             meta = meta7 + (cfg.layer_window(li, L),)       # the layer's sliding window when the sequence is longer

@@ -57,3 +57,38 @@ def test_native_layer_equals_the_layer_of_separate_calls(monkeypatch, bias, f, d
             else:
                 assert torch.equal(got, want), name
             assert want.norm() > 0 or name == "lm_head", name
+
+
+@pytest.mark.parametrize("between", ["nothing", "backward hook", "one layer"])
+def test_layers_in_one_call_equal_a_call_each(monkeypatch, between):
+    """All layers in one node (a few tokens, nothing between the layers) against a node per layer: outputs, gradients and those
+    of a second, accumulating pass bit for bit; a hook behind each layer's backward pass is called in order."""
+    cfg = llama.LlamaConfig(vocab_size=512, hidden_size=256, intermediate_size=640, num_hidden_layers=1 if between == "one layer" else 5,
+                            num_attention_heads=4, num_key_value_heads=2, max_position_embeddings=512, sliding_window=100,
+                            window_layers=None)
+    results, calls = [], []
+    for limit in (0, layer_native.STACK_MAX_TOKENS):
+        model = llama.build_model(cfg, dtype=torch.bfloat16, device="cuda", seed=3)
+        FlatParams([p for p in model.parameters() if p.requires_grad])
+        ids = torch.randint(0, 512, (2, 173), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+        monkeypatch.setattr(layer_native, "STACK_MAX_TOKENS", limit)
+        stacks, real = [], layer_native.run_stack
+        monkeypatch.setattr(layer_native, "run_stack", lambda *a: stacks.append(1) or real(*a))
+        order = []
+        if between == "backward hook":
+            monkeypatch.setattr(llama, "LAYER_BACKWARD_DONE", [lambda w: order.append(
+                [w is l.input_layernorm for l in model.layers].index(True))])
+        for _ in range(2):
+            y = model.hidden_states(ids)
+            y.backward(torch.randn(y.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(2)).to(y.dtype))
+        with torch.no_grad():
+            z = model.hidden_states(ids)
+        monkeypatch.undo()
+        assert len(stacks) == (2 if limit else 0)              # the passes with gradients
+        assert torch.equal(y, z) and _lib.take_device_error() == 0
+        results.append((y.detach(), {n: p.grad_slot.buf.clone() for n, p in model.named_parameters() if "embed" not in n}))
+        calls.append(order)
+    assert calls[0] == calls[1] and calls[1] == ([4, 3, 2, 1, 0] * 2 if between == "backward hook" else [])
+    assert torch.equal(results[0][0], results[1][0])
+    for name, want in results[0][1].items():
+        assert torch.equal(results[1][1][name], want), name

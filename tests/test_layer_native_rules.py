@@ -70,3 +70,41 @@ def test_gradient_slots_are_taken_as_written_only_by_a_call_that_ran(monkeypatch
     else:
         y.backward(torch.zeros_like(y))
     assert all(t.grad_slot.fresh == (rc < 0) for t in w)
+
+
+@pytest.mark.parametrize("ran", [0, 2, 3])
+def test_a_failing_call_over_several_layers_marks_those_that_ran(monkeypatch, ran):
+    """Three layers in one backward call: the slots of the last ``ran`` of them count as written, the others stay fresh."""
+    import ctypes
+
+    class Lib:
+        def b200_stack_bwd(self, *a):
+            ctypes.cast(a[-2], ctypes.POINTER(ctypes.c_int))[0] = ran
+            return 60 if ran == 3 else -2
+
+        def __getattr__(self, name):
+            return (lambda: b"") if name == "b200_last_cuda_error" else (lambda *a: 64)
+
+    class Slot:
+        def __init__(self, w):
+            self.buf, self.fresh = torch.zeros(w.shape), True
+    monkeypatch.setattr(layer_native._lib, "kernels", Lib)
+    monkeypatch.setattr(layer_native._lib, "stream", lambda: None)
+    n, layers = (H + 2 * HKV) * D, []
+    tables = torch.zeros(16, D // 2), torch.zeros(16, D // 2)
+    for _ in range(3):
+        w = tuple(torch.zeros(s, dtype=torch.bfloat16).requires_grad_() for s in ((W,), (n, W), (W, H * D), (W,), (2 * F, W), (W, F)))
+        for t in w:
+            t.grad_slot = Slot(t)
+        layers.append((w, None, *tables, None))
+    x = torch.zeros(T, W, dtype=torch.bfloat16)
+    y = layer_native.run_stack(x, torch.zeros(T, dtype=torch.int32), layers, (1, T, H, HKV, D, 1e-5, False, None),
+                               (False, False))
+    assert y.requires_grad                                   # by the weights alone
+    if ran < 3:
+        with pytest.raises(layer_native._lib.NativeError):
+            y.backward(torch.zeros_like(y))
+    else:
+        y.backward(torch.zeros_like(y))
+    assert [all(t.grad_slot.fresh for t in w) for w, *_ in layers] == [i < 3 - ran for i in range(3)]
+    assert not any(t.grad_slot.fresh for w, *_ in layers[3 - ran:] for t in w)
