@@ -337,26 +337,28 @@ __global__ void __launch_bounds__(128, 5) rmsnorm_bwd_warp_kernel(const __nv_bfl
   }
 }
 
-// out[j] (+)= sum_b partial[b][j]; block = 32 columns x 8 row groups, reduced through shared memory
-__global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ partial, float* __restrict__ out,
-                                                     int nblk, int h, int accumulate) {
+// out[j] (+)= sum_b partial[b][j]; block = 32 columns x 32 row groups, reduced through shared memory. There are only h / 32
+// blocks, so what bounds it is the chain of loads of a row group: 8 in flight, and 32 groups where 8 of them took 10 us for 777
+// rows of 896 and 12 us for 592 of 2048.
+constexpr int COLSUM_THREADS = 1024;
+__global__ void __launch_bounds__(COLSUM_THREADS) colsum_kernel(const float* __restrict__ partial, float* __restrict__ out,
+                                                                int nblk, int h, int accumulate) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float red[8][33];
+  constexpr int G = COLSUM_THREADS / 32;
+  __shared__ float red[G][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + tx;
   float s = 0.f;
   if (j < h)
-    // loads of 16 rows in flight (the additions keep their order): one at a time the chain of a few hundred rows was
-    // all this kernel did
-#pragma unroll 16
-    for (int b = ty; b < nblk; b += 8) s += partial[(size_t)b * h + j];
+#pragma unroll 8
+    for (int b = ty; b < nblk; b += G) s += partial[(size_t)b * h + j];
   red[ty][tx] = s;
   __syncthreads();
   if (ty == 0 && j < h) {
     float t = 0.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) t += red[k][tx];
+    for (int k = 0; k < G; ++k) t += red[k][tx];
     out[j] = accumulate ? out[j] + t : t;
   }
 }
@@ -571,6 +573,44 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const __nv_bfloat16* __r
       for (int k = 0; k < 8; ++k) s += red[k][cv][j];
       atomicAdd(out + v * 8 + j, s);
     }
+  }
+}
+
+// The same for few rows in one launch and a fixed order: block = 8 column vectors (64 columns) x 128 row lanes. For 777 rows of
+// 1152 the kernel above ran on 10 blocks, each thread 49 rows one after the other, behind a memset (18 us and 2).
+constexpr int BIAS_SMALL_ROWS = 2048;
+__global__ void __launch_bounds__(1024) bias_grad_small_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ out,
+                                                               int T, int N, long long ld, int accumulate) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ float red[32][65];
+  const int cv = threadIdx.x & 7, rl = threadIdx.x >> 3, warp = threadIdx.x >> 5;
+  const int v = blockIdx.x * 8 + cv;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (v * 8 < N) {
+#pragma unroll 4
+    for (int t = rl; t < T; t += 128) {
+      float a[8];
+      unpack8(reinterpret_cast<const uint4*>(dy + t * ld)[v], a);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += a[j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {                     // the warp's four row lanes
+    acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 8);
+    acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 16);
+  }
+  if ((threadIdx.x & 31) < 8)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) red[warp][cv * 8 + j] = acc[j];
+  __syncthreads();
+  const int col = blockIdx.x * 64 + threadIdx.x;
+  if (threadIdx.x < 64 && col < N) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) s += red[w][threadIdx.x];
+    out[col] = accumulate ? out[col] + s : s;
   }
 }
 
@@ -817,7 +857,7 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
 #undef B200_RMS_BWD_WARP
   B200_CUDA_CHECK(cudaGetLastError());
   const bool warp_kernel = h == 2048 || h == 1024 || h == 512 || h == 256;    // one partial row per 4-warp CTA there
-  launch_pdl(colsum_kernel, ceil_div(h, 32), 256, 0, st, dw_partial, dw_out, warp_kernel ? ceil_div(grid, 4) : grid, h,
+  launch_pdl(colsum_kernel, ceil_div(h, 32), COLSUM_THREADS, 0, st, dw_partial, dw_out, warp_kernel ? ceil_div(grid, 4) : grid, h,
                                                  dw_accumulate);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -864,7 +904,7 @@ int b200_headnorm_bwd(void* g, const void* x, const void* wq, const void* wk, co
     launch_pdl(headnorm_bwd_kernel<2>, grid, 256, 0, st, (__nv_bfloat16*)g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq,
                                                  (const __nv_bfloat16*)wk, rstd, dw_partial, T, H, Hkv, ld);
   B200_CUDA_CHECK(cudaGetLastError());
-  launch_pdl(colsum_kernel, ceil_div(2 * d, 32), 256, 0, st, dw_partial, dw_out, grid, 2 * d, dw_accumulate);
+  launch_pdl(colsum_kernel, ceil_div(2 * d, 32), COLSUM_THREADS, 0, st, dw_partial, dw_out, grid, 2 * d, dw_accumulate);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -897,6 +937,11 @@ int b200_bias_add(void* x, const void* bias, long long T, int N, long long ld, c
 // out[N] (fp32) (+)= column sums of dy[T, N] (bf16, row stride ld)
 int b200_bias_grad(const void* dy, float* out, long long T, int N, long long ld, int accumulate, cudaStream_t st) {
   if (!dy || !out || T <= 0 || N <= 0 || (N & 7) || (ld & 7)) return B200_ERR_ARG;
+  if (T <= BIAS_SMALL_ROWS) {      // beyond, N / 64 blocks are too few to read the rows
+    launch_pdl(bias_grad_small_kernel, ceil_div(N, 64), 1024, 0, st, (const __nv_bfloat16*)dy, out, (int)T, N, ld, accumulate);
+    B200_CUDA_CHECK(cudaGetLastError());
+    return B200_OK;
+  }
   if (!accumulate) B200_CUDA_CHECK(cudaMemsetAsync(out, 0, sizeof(float) * N, st));
   long long gy = (T + 511) / 512;
   if (gy > 64) gy = 64;
@@ -1038,7 +1083,7 @@ extern "C" int b200_rmsnorm_bwd_noalloc(const void* dy, const void* x, const voi
   B200_RMS_BY_WIDTH(rmsnorm_bwd_kernel, h, grid, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
                     (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, h);
   B200_CUDA_CHECK(cudaGetLastError());
-  launch_pdl(colsum_kernel, ceil_div(h, 32), 256, 0, st, scratch, dw_out, grid, h, dw_accumulate);
+  launch_pdl(colsum_kernel, ceil_div(h, 32), COLSUM_THREADS, 0, st, scratch, dw_out, grid, h, dw_accumulate);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

@@ -11,28 +11,40 @@ constexpr int SORT_MAX_EXPERTS = 32;
 
 // Counting sort of n expert indices (stable): order[p] = index of the pair at sorted position p, inverse[order[p]] = p,
 // token[p] = order[p] / k, counts[e] = pairs of expert e. ONE block: the keys of a layer are a few thousand to a few
-// hundred thousand small numbers that sit in L2, and the point is latency (the host waits for the counts): each thread
-// counts its contiguous run of keys per expert in shared memory, one scan over (expert, thread) turns the counts into
-// positions, and the same run is walked again in order. 12248 pairs of 8 experts: the ten launches of a library radix
-// sort, histogram, scatter and division that this replaces took about 90 us. The runs grow with the pairs and one block
-// does not: the caller goes to the library beyond 32768 of them (models/moe.py: SORT_MAX_PAIRS, with both sides' times).
+// hundred thousand small numbers that sit in L2, and the point is latency (the host or the experts' GEMMs wait for the counts).
+// The keys come in once, coalesced, as bytes into shared memory; each thread counts its contiguous run of them per expert there,
+// one scan over (expert, thread) turns the counts into positions, and the same run is walked again in order. 12248 pairs of 8
+// experts: the ten launches of a library radix sort, histogram, scatter and division that this replaces took about 90 us; with
+// each thread reading its run from global memory, one 8-byte key after the other, and writing all three lists from the one
+// block it took 33. The block writes `inverse` alone - stores of one SM to scattered sectors take a clock each - and a second
+// launch of many blocks makes the other two of it. The runs grow with the pairs and one block does not: the caller goes to the library beyond 32768 of them (models/moe.py: SORT_MAX_PAIRS, with both sides'
+// times); more than SORT_STAGED_PAIRS are walked in global memory.
+constexpr int SORT_STAGED_PAIRS = 65536;
 __global__ void __launch_bounds__(SORT_THREADS, 1)
-    expert_sort_kernel(const long long* __restrict__ experts, long long n, int E, int k, long long* __restrict__ order,
-                       long long* __restrict__ inverse, long long* __restrict__ token, long long* __restrict__ counts) {
+    expert_sort_kernel(const long long* __restrict__ experts, long long n, int E, long long* __restrict__ inverse,
+                       long long* __restrict__ counts) {
   pdl_wait();
   pdl_trigger();
-  extern __shared__ int slot[];                    // [E][SORT_THREADS]
-  __shared__ int warp_total[32];
+  extern __shared__ int slot[];                    // [E][SORT_THREADS], then the staged keys
+  __shared__ int warp_base[SORT_MAX_EXPERTS][33];  // pairs of an expert in the warps before each, then their position
+  uint8_t* key = reinterpret_cast<uint8_t*>(slot + E * SORT_THREADS);
+  const bool staged = n <= SORT_STAGED_PAIRS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long per = (n + SORT_THREADS - 1) / SORT_THREADS;
   const long long i0 = min(n, tid * per), i1 = min(n, i0 + per);
-  for (int e = 0; e < E; ++e) slot[e * SORT_THREADS + tid] = 0;
-  for (long long i = i0; i < i1; ++i) {
-    const long long e = experts[i];
-    if (e >= 0 && e < E) ++slot[(int)e * SORT_THREADS + tid];
+  auto valid = [&](long long e) { return e >= 0 && e < E ? (int)e : -1; };
+  auto expert = [&](long long i) { return staged ? (int)(int8_t)key[i] : valid(experts[i]); };
+  if (staged) {
+#pragma unroll 8
+    for (int i = tid; i < (int)n; i += SORT_THREADS) key[i] = (uint8_t)(int8_t)valid(experts[i]);
   }
-  int base = 0;
-  for (int e = 0; e < E; ++e) {                    // exclusive scan, expert-major
+  for (int e = 0; e < E; ++e) slot[e * SORT_THREADS + tid] = 0;
+  __syncthreads();
+  for (long long i = i0; i < i1; ++i) {
+    const int e = expert(i);
+    if (e >= 0) ++slot[e * SORT_THREADS + tid];
+  }
+  for (int e = 0; e < E; ++e) {                    // scan inside each warp, expert by expert
     const int mine = slot[e * SORT_THREADS + tid];
     int incl = mine;
 #pragma unroll
@@ -40,27 +52,49 @@ __global__ void __launch_bounds__(SORT_THREADS, 1)
       const int up = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += up;
     }
-    if (lane == 31) warp_total[warp] = incl;
-    __syncthreads();
-    int before = 0, total = 0;
-    for (int w = 0; w < 32; ++w) {
-      const int t = warp_total[w];
-      before += w < warp ? t : 0;
-      total += t;
+    if (lane == 31) warp_base[e][warp] = incl;
+    slot[e * SORT_THREADS + tid] = incl - mine;
+  }
+  __syncthreads();
+  for (int e = warp; e < E; e += 32) {             // then over the warps, one warp per expert
+    const int mine = warp_base[e][lane];
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
     }
-    slot[e * SORT_THREADS + tid] = base + before + incl - mine;
-    if (tid == 0) counts[e] = total;
-    base += total;
-    __syncthreads();
+    warp_base[e][lane] = incl - mine;
+    if (lane == 31) {
+      warp_base[e][32] = incl;
+      counts[e] = incl;
+    }
+  }
+  __syncthreads();
+  int base = 0;
+  for (int e = 0; e < E; ++e) {
+    slot[e * SORT_THREADS + tid] += base + warp_base[e][warp];
+    base += warp_base[e][32];
   }
   for (long long i = i0; i < i1; ++i) {
-    const long long e = experts[i];
-    if (e < 0 || e >= E) continue;
-    const int p = slot[(int)e * SORT_THREADS + tid]++;
-    order[p] = i;
-    inverse[i] = p;
-    token[p] = i / k;
+    const int e = expert(i);
+    if (e >= 0) inverse[i] = slot[e * SORT_THREADS + tid]++;
   }
+}
+
+// order and token of the sorted positions; pairs of no expert have none
+__global__ void __launch_bounds__(256)
+    expert_scatter_kernel(const long long* __restrict__ experts, const long long* __restrict__ inverse, int n, int E, int k,
+                          long long* __restrict__ order, long long* __restrict__ token) {
+  pdl_wait();
+  pdl_trigger();
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= n) return;
+  const long long e = experts[i];
+  if (e < 0 || e >= E) return;
+  const long long p = inverse[i];
+  order[p] = i;
+  token[p] = i / k;
 }
 
 // out[t] = (h1[t] +) scale * sum_j w[t, j] y[inverse[t k + j]], summed in fp32 in the order of the choices: one pass over
@@ -122,14 +156,16 @@ int b200_expert_sort(const long long* experts, long long n, int E, int k, long l
   if (!experts || !order || !inverse || !token || !counts || n <= 0 || n > 0x7fffffffLL || E <= 0 ||
       E > moe::SORT_MAX_EXPERTS || k <= 0)
     return B200_ERR_ARG;
-  const int smem = E * moe::SORT_THREADS * (int)sizeof(int);
+  const int smem = E * moe::SORT_THREADS * (int)sizeof(int) + (n <= moe::SORT_STAGED_PAIRS ? (int)n : 0);
   static bool attr = false;
   if (!attr) {
     B200_CUDA_CHECK(cudaFuncSetAttribute(moe::expert_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         moe::SORT_MAX_EXPERTS * moe::SORT_THREADS * (int)sizeof(int)));
+                                         moe::SORT_MAX_EXPERTS * moe::SORT_THREADS * (int)sizeof(int) + moe::SORT_STAGED_PAIRS));
     attr = true;
   }
-  launch_pdl(moe::expert_sort_kernel, 1, moe::SORT_THREADS, smem, st, experts, n, E, k, order, inverse, token, counts);
+  launch_pdl(moe::expert_sort_kernel, 1, moe::SORT_THREADS, smem, st, experts, n, E, inverse, counts);
+  B200_CUDA_CHECK(cudaGetLastError());
+  launch_pdl(moe::expert_scatter_kernel, (unsigned)ceil_div_ll(n, 256), 256, 0, st, experts, inverse, (int)n, E, k, order, token);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

@@ -24,6 +24,7 @@ from ..ops._lib import _F, _I, _LL, _VP
 from . import llama as _ll
 
 _lib.register("b200_expert_sort", [_VP, _LL, _I, _I, _VP, _VP, _VP, _VP, _VP])
+_lib.KERNELS_PER_CALL["b200_expert_sort"] = 2
 _lib.register("b200_gemm_grouped_swiglu", [_VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP])
 _lib.register("b200_gemm_grouped", [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP])
 _lib.register("b200_moe_combine", [_VP, _VP, _VP, _VP, _VP, _LL, _I, _I, _F, _VP])

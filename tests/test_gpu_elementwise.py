@@ -175,3 +175,17 @@ def test_rmsnorm_row_widths_of_the_block_kernels(h):
     assert torch.allclose(y.float(), ref, atol=1e-4, rtol=2 ** -8)
     assert torch.allclose(dx.float(), xf.grad + dres.float(), atol=1e-3, rtol=2 ** -7)
     assert torch.allclose(dw, wf.grad, atol=1e-3 * rows ** 0.5, rtol=1e-4)
+
+
+@pytest.mark.parametrize("T", [1, 127, 129, 777, 2048, 2049])
+@pytest.mark.parametrize("N,ld", [(8, 8), (72, 80), (1152, 1152)])
+def test_bias_gradient_of_few_and_many_rows(T, N, ld):
+    """Both sides of the row count at which the column sums take another kernel, odd remainders, padded rows, stored and added.
+    Bound: a sum of T fp32 terms (T 2^-24 of their absolute sum)."""
+    g = torch.Generator("cuda").manual_seed(T * N)
+    dy = torch.randn(T, ld, device="cuda", generator=g).bfloat16()[:, :N]
+    out = torch.full((N,), 3.0, device="cuda")
+    for add in (False, True):
+        basic.bias_grad(dy, out=out, accumulate=add)
+        want = dy.double().sum(0) * (2 if add else 1)
+        assert ((out.double() - want).abs() <= (T + 1) * 2 ** -23 * dy.double().abs().sum(0) + 1e-6).all()

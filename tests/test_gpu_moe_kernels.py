@@ -117,3 +117,19 @@ def test_experts_that_one_launch_does_not_take(case):
     want = outcome(lambda: moe._experts_one_by_one(x, counts, w_gu, w_d))
     assert got == want if isinstance(want, type) else all(torch.equal(a, b) for a, b in zip(got, want))
     _lib.take_device_error()
+
+
+@pytest.mark.parametrize("n,E", [(1023, 3), (65536, 32), (65537, 32), (200003, 5)])
+def test_expert_sort_of_any_number_of_pairs(n, E):
+    """The kernel itself around the number of pairs that it stages in shared memory, with indices out of range left out."""
+    e = torch.randint(-1, E + 1, (n,), device="cuda", generator=torch.Generator("cuda").manual_seed(n))
+    order, inverse, token = (torch.full((n,), -7, dtype=torch.int64, device="cuda") for _ in range(3))
+    counts = torch.empty(E, dtype=torch.int64, device="cuda")
+    p = _lib.ptr
+    _lib.check(_lib.kernels().b200_expert_sort(p(e), n, E, 3, p(order), p(inverse), p(token), p(counts), _lib.stream()), "sort")
+    ok = ((e >= 0) & (e < E)).nonzero()[:, 0]
+    want = ok[torch.argsort(e[ok], stable=True)]
+    m = want.numel()
+    assert torch.equal(order[:m], want) and torch.equal(token[:m], want // 3) and (order[m:] == -7).all()
+    assert torch.equal(inverse[want], torch.arange(m, device="cuda"))
+    assert torch.equal(counts, torch.bincount(e[ok], minlength=E))
