@@ -28,7 +28,8 @@
 // warps per scheduler to fill it. Four of them with 32 columns each measured the same (head dim 64) or slower (128: 80
 // registers a thread; 800 against 710 us).
 // All three kernels of a backward pass, B200, queries as rows and one S / dP buffer / now: 8 x 2048, 32/4 heads of 64
-// 638 / 521 us; 2 x 4000, 32/8 of 128 1191 / 710; 1 x 777, 14/2 of 64 122 / 33.
+// 638 / 521 us; 2 x 4000, 32/8 of 128 1191 / 710; 1 x 777, 14/2 of 64 122 / 33. The rotation of dK in the epilogue instead of a
+// launch behind it: 2 x 256, 8/2 of 64 21.0 / 16.0 us, 1 x 777, 14/2 34.2 / 32.0, large ones 4 to 10 us.
 // Few key blocks (short sequences, few kv heads) leave SMs idle while each CTA walks all query heads of its group: then a
 // cluster of up to 8 CTAs shares the heads, and the partial dK / dV meet through distributed shared memory, added in the
 // order of the CTAs' ranks (`head_split` below; results repeat bit for bit).
@@ -95,7 +96,38 @@ struct BwdParams {
   int window;          // > 0: the query at position i saw the keys j with i - window < j <= i; 0: all j <= i
   int hsplit;          // CTAs (one cluster) that share the query heads of a group
   float scale;
+  const int* pos;      // [T], with the tables below [max_pos, D / 2]: dK leaves with the inverse rotary embedding; null: as it is
+  const float* cs;
+  const float* sn;
 };
+
+// The inverse rotary embedding of N pairs of columns (j, j + D/2), from the values rounded to bf16, with the rope kernel's
+// expressions: what that kernel makes of stored gradients, bit for bit. `c`, `sg`: the pairs' entries of the tables.
+template <int N>
+__device__ __forceinline__ void load_table(const float* src, float (&v)[N]) {
+#pragma unroll
+  for (int j = 0; j < N; j += 4) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(src + j));
+    v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w;
+  }
+}
+template <int N>
+__device__ __forceinline__ void unrotate(float (&a)[N], float (&b)[N], const float (&c)[N], const float (&sg)[N]) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const float fa = __bfloat162float(__float2bfloat16(a[j])), fb = __bfloat162float(__float2bfloat16(b[j]));
+    const float sk = sg[j] * -1.f;
+    a[j] = __fmaf_rn(fa, c[j], -__fmul_rn(fb, sk));
+    b[j] = __fmaf_rn(fb, c[j], __fmul_rn(fa, sk));
+  }
+}
+template <int N>
+__device__ __forceinline__ void store_bf16(__nv_bfloat16* dst, const float (&v)[N]) {
+#pragma unroll
+  for (int j = 0; j < N; j += 8)
+    *reinterpret_cast<uint4*>(dst + j) = make_uint4(pack_bf16x2(v[j], v[j + 1]), pack_bf16x2(v[j + 2], v[j + 3]),
+                                                    pack_bf16x2(v[j + 4], v[j + 5]), pack_bf16x2(v[j + 6], v[j + 7]));
+}
 
 template <int D>
 __global__ void __launch_bounds__(NTHREADS, 1)
@@ -540,7 +572,18 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_ready);
     }
-    // epilogue: dK_j, dV_j (thread = key row, this warp's half of the columns)
+    // epilogue: dK_j, dV_j (thread = key row): W columns of the first half of the head and their partners of the second. The
+    // tables of the rotation are fetched while the last MMAs run.
+    constexpr int W = D / 4;
+    const int kvi = kv0 + r;
+    const bool row_ok = kvi < p.L;
+    const bool rotate = p.pos && row_ok && p.hsplit == 1;
+    float rc[W], rs[W];
+    if (rotate) {
+      const size_t e = (size_t)p.pos[(long long)b * p.L + kvi] * (D / 2) + cpart * W;
+      load_table(p.cs + e, rc);
+      load_table(p.sn + e, rs);
+    }
     if (ok && n_it > 0) {
       const int last = n_it - 1;
       ok = wait(dk_done, last & 1u, ERR_WAIT_AUX) && wait(&dv_done[last % NSB], (last / NSB) & 1u, ERR_WAIT_AUX) &&
@@ -548,35 +591,39 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
     if (ok && n_it > 0) {
       tc_fence_after_sync();
-      const int kvi = kv0 + r;
-      const bool row_ok = kvi < p.L;
       const long long width = (long long)(p.H + 2 * p.Hkv) * D;
       __nv_bfloat16* row = p.dqkv + ((long long)b * p.L + kvi) * width;
-      constexpr int W = 32;                           // columns at a time; D / 2 of dK and of dV per warp
 #pragma unroll
-      for (int c = 0; c < D / W; ++c) {
-        const int which = c / (D / 2 / W);              // 0: dK, 1: dV
-        const int col = cpart * (D / 2) + (c % (D / 2 / W)) * W;
-        const uint32_t src = tmem_base + lane_addr + (which == 0 ? C::DK_COL : C::DV_COL) + col;
-        uint32_t v[W];
-        tmem_ld_32x32b_x32(src, v);
-        tmem_ld_wait_for(v);
+      for (int which = 0; which < 2; ++which) {          // dK, dV
+        const uint32_t src = tmem_base + lane_addr + (which == 0 ? C::DK_COL : C::DV_COL) + cpart * W;
+        uint32_t ra[W], rb[W];
+        if constexpr (W == 32) {
+          tmem_ld_32x32b_x32(src, ra);
+          tmem_ld_32x32b_x32(src + D / 2, rb);
+        } else {
+          tmem_ld_32x32b_x16(src, ra);
+          tmem_ld_32x32b_x16(src + D / 2, rb);
+        }
+        tmem_ld_wait_for(ra);
+        tmem_ld_wait_for(rb);
         if (p.hsplit > 1) {
-          float* dst = reinterpret_cast<float*>(smem) + r * C::RED_PITCH + which * D + col;
+          float* dst = reinterpret_cast<float*>(smem) + r * C::RED_PITCH + which * D + cpart * W;
 #pragma unroll
-          for (int q4 = 0; q4 < W / 4; ++q4)
-            *reinterpret_cast<uint4*>(dst + q4 * 4) = make_uint4(v[q4 * 4], v[q4 * 4 + 1], v[q4 * 4 + 2], v[q4 * 4 + 3]);
-        } else if (row_ok) {
-          __nv_bfloat16* dst = row + (which == 0 ? colK : colV) + col;
-#pragma unroll
-          for (int q4 = 0; q4 < W / 8; ++q4) {
-            uint4 o;
-            o.x = pack_bf16x2(__uint_as_float(v[q4 * 8 + 0]), __uint_as_float(v[q4 * 8 + 1]));
-            o.y = pack_bf16x2(__uint_as_float(v[q4 * 8 + 2]), __uint_as_float(v[q4 * 8 + 3]));
-            o.z = pack_bf16x2(__uint_as_float(v[q4 * 8 + 4]), __uint_as_float(v[q4 * 8 + 5]));
-            o.w = pack_bf16x2(__uint_as_float(v[q4 * 8 + 6]), __uint_as_float(v[q4 * 8 + 7]));
-            *reinterpret_cast<uint4*>(dst + q4 * 8) = o;
+          for (int j = 0; j < W; j += 4) {
+            *reinterpret_cast<uint4*>(dst + j) = make_uint4(ra[j], ra[j + 1], ra[j + 2], ra[j + 3]);
+            *reinterpret_cast<uint4*>(dst + D / 2 + j) = make_uint4(rb[j], rb[j + 1], rb[j + 2], rb[j + 3]);
           }
+        } else if (row_ok) {
+          float fa[W], fb[W];
+#pragma unroll
+          for (int j = 0; j < W; ++j) {
+            fa[j] = __uint_as_float(ra[j]);
+            fb[j] = __uint_as_float(rb[j]);
+          }
+          if (which == 0 && rotate) unrotate(fa, fb, rc, rs);
+          __nv_bfloat16* dst = row + (which == 0 ? colK : colV) + cpart * W;
+          store_bf16(dst, fa);
+          store_bf16(dst + D / 2, fb);
         }
       }
     }
@@ -599,19 +646,30 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const uint32_t rank = cluster_ctarank(), n = (uint32_t)p.hsplit;
     const uint32_t base = smem_u32(smem);
     const long long width = (long long)(p.H + 2 * p.Hkv) * D;
-    constexpr int VPR = D / 2;                       // vectors of 4 in a key row: dK, then dV
+    constexpr int IPR = D / 4;                       // items of a key row: 4 columns and their partners, of dK, then of dV
     const int rows = min(BN, p.L - kv0);
     if (!*abort_flag) {
-      for (int i = (int)(rank * NTHREADS + threadIdx.x); i < rows * VPR; i += (int)(n * NTHREADS)) {
-        const int row = i / VPR, v = i - row * VPR;
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (uint32_t j = 0; j < n; ++j) {
-          const float4 x = ld_cluster_f32x4(mapa_shared(base + (row * C::RED_PITCH + v * 4) * 4, j));
-          a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+      for (int i = (int)(rank * NTHREADS + threadIdx.x); i < rows * IPR; i += (int)(n * NTHREADS)) {
+        const int row = i / IPR, which = (i - row * IPR) / (D / 8), j0 = (i - row * IPR) % (D / 8) * 4;
+        float fa[4] = {0.f, 0.f, 0.f, 0.f}, fb[4] = {0.f, 0.f, 0.f, 0.f};
+        const long long t = (long long)b * p.L + kv0 + row;
+        const bool rotate = which == 0 && p.pos;
+        float rc[4], rs[4];
+        if (rotate) {
+          const size_t e = (size_t)p.pos[t] * (D / 2) + j0;
+          load_table(p.cs + e, rc);
+          load_table(p.sn + e, rs);
         }
-        const int col = v * 4 < D ? colK + v * 4 : colV + v * 4 - D;
-        uint2 o = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
-        *reinterpret_cast<uint2*>(p.dqkv + ((long long)b * p.L + kv0 + row) * width + col) = o;
+        const uint32_t at = base + (row * C::RED_PITCH + which * D + j0) * 4;
+        for (uint32_t j = 0; j < n; ++j) {
+          const float4 x = ld_cluster_f32x4(mapa_shared(at, j)), y = ld_cluster_f32x4(mapa_shared(at + D * 2, j));
+          fa[0] += x.x; fa[1] += x.y; fa[2] += x.z; fa[3] += x.w;
+          fb[0] += y.x; fb[1] += y.y; fb[2] += y.z; fb[3] += y.w;
+        }
+        if (rotate) unrotate(fa, fb, rc, rs);
+        __nv_bfloat16* dst = p.dqkv + t * width + (which == 0 ? colK : colV) + j0;
+        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(fa[0], fa[1]), pack_bf16x2(fa[2], fa[3]));
+        *reinterpret_cast<uint2*>(dst + D / 2) = make_uint2(pack_bf16x2(fb[0], fb[1]), pack_bf16x2(fb[2], fb[3]));
       }
     }
     cluster_sync_all();    // nobody's shared memory goes away while a peer reads it
@@ -788,7 +846,7 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
     attr = true;
   }
   const int hs = head_split(B, L, window, H, Hkv);
-  BwdParams p{lse, delta, (__nv_bfloat16*)dqkv, B, L, H, Hkv, window, hs, 1.0f / sqrtf((float)D)};
+  BwdParams p{lse, delta, (__nv_bfloat16*)dqkv, B, L, H, Hkv, window, hs, 1.0f / sqrtf((float)D), pos, cos_tab, sin_tab};
   dim3 grid(Hkv * B * hs, (L + BN - 1) / BN);
   if (hs > 1)
     launch_pdl_cluster(kern, grid, NTHREADS, C::SMEM_BYTES, st, hs, tmQKV, tmDO, tmDQ, p, device_err_word());
@@ -829,9 +887,8 @@ extern "C" int b200_flash_attn_bwd(const void* dout, const void* qkv, const void
   return B200_ERR_ARG;
 }
 
-// The same, with the inverse rotary embedding of the QUERY heads applied where the fp32 dQ accumulator is converted to
-// bf16 (pos int32 [B*L]; cos / sin fp32 [max_pos, D/2]). The key heads' gradient comes out of the main kernel's epilogue
-// and is rotated by the caller.
+// The same with the inverse rotary embedding of the query and key heads (pos int32 [B*L]; cos / sin fp32 [max_pos, D/2]):
+// where the fp32 dQ accumulator is converted to bf16 and in the main kernel's epilogue.
 extern "C" int b200_flash_attn_bwd_rope(const void* dout, const void* qkv, const void* out, const float* lse,
                                         float* delta, void* dqkv, float* dq_acc, const int* pos, const float* cos_tab,
                                         const float* sin_tab, int B, int L, int window, int H, int Hkv, int D,

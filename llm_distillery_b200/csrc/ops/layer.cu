@@ -197,7 +197,6 @@ extern "C" int b200_layer_bwd(const void* dh2, const void* x, const int* pos, co
   RUN(dgrad(t.dh1, h, w_o, A, t.datt));
   RUN(b200_flash_attn_bwd_rope(t.datt, s.qkv, s.att, s.lse, t.delta, t.dqkv, t.dq_acc, pos, cos_tab, sin_tab, B, L, window, H,
                                Hkv, d, st));
-  RUN(b200_rope(static_cast<uint8_t*>(t.dqkv) + 2 * m.A, pos, cos_tab, sin_tab, T, Hkv, d, N, 1, st));   // the key heads
   if (g_bqkv) RUN(b200_bias_grad(t.dqkv, g_bqkv, T, N, N, (acc >> 6) & 1, st));
   if (g_qkv) RUN(wgrad(t.dqkv, N, s.n1, h, g_qkv, 1));
   RUN(dgrad(t.dqkv, N, w_qkv, h, t.dn));

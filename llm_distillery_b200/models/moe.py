@@ -30,9 +30,9 @@ _lib.register("b200_gemm_grouped", [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP])
 _lib.register("b200_moe_combine", [_VP, _VP, _VP, _VP, _VP, _LL, _I, _I, _F, _VP])
 
 
-# One block sorts in time that grows with the pairs, the library's ten launches in time that hardly does. With the counts
-# on the host, 8 / 32 experts: 2048 pairs 52 / 75 us against 140, 16 384 97 / 126 against 204, 32 768 150 / 187 against
-# 215, 65 536 262 / 300 against 229, 131 072 487 / 534 against 223.
+# One block sorts in time that grows with the pairs, the library's ten launches in time that hardly does: 8 / 32 experts, on the
+# device, 2048 pairs 6 / 12 us, 16 384 20 / 28, 32 768 41 / 54 (the block with one key in flight per thread 114 / 147). The
+# library took 140, 204, 215 and, for 65 536 and 131 072 pairs, 229 and 223 with the counts read back.
 SORT_MAX_PAIRS = 32768
 
 

@@ -150,8 +150,9 @@ def attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window: int | None = Non
 
 def attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin, window: int | None = None):
     """dqkv with respect to the projection's output BEFORE the rotary embedding: attention backward followed by the
-    inverse rotation of the query and key heads. On the GPU the query heads are rotated where their fp32 accumulator is
-    converted to bf16 (one pass less over 8/9 of the rotated columns); same values as ``attention_bwd`` + ``rope_``."""
+    inverse rotation of the query and key heads. On the GPU they are rotated where they are written: the query heads where
+    their fp32 accumulator is converted to bf16, the key heads in the kernel's epilogue; same values as ``attention_bwd`` +
+    ``rope_``."""
     from . import basic
     if window is not None and L <= window:
         window = None
@@ -161,9 +162,7 @@ def attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin,
     if (qkv.is_cuda and qkv.dtype == torch.bfloat16 and pos.dtype == torch.int32 and cos.is_contiguous()
             and sin.is_contiguous() and 2 * cos.shape[1] == d):      # partial rotary: the separate kernel below
         from . import flash
-        dqkv = flash.flash_attn_bwd(dout.to(qkv.dtype), qkv, out, lse, B, L, H, Hkv, d, rope=(pos, cos, sin), window=window)
-        basic.rope_(dqkv[:, H * d:], pos, cos, sin, Hkv, d, inverse=True)      # the key heads
-        return dqkv
+        return flash.flash_attn_bwd(dout.to(qkv.dtype), qkv, out, lse, B, L, H, Hkv, d, rope=(pos, cos, sin), window=window)
     dqkv = attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
     return basic.rope_(dqkv, pos, cos, sin, H + Hkv, d, inverse=True)
 

@@ -32,8 +32,8 @@ def flash_attn_fwd(qkv: torch.Tensor, B: int, L: int, H: int, Hkv: int, d: int, 
 
 
 def flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, rope=None, window: int | None = None):
-    """``rope = (pos, cos, sin)``: the inverse rotary embedding of the query heads' gradient is applied where the fp32
-    dQ accumulator is converted (the key heads' gradient is left to the caller)."""
+    """``rope = (pos, cos, sin)``: the inverse rotary embedding of the query and key heads' gradients is applied where they
+    are written."""
     if not dout.is_contiguous():
         dout = dout.contiguous()
     dqkv = torch.empty_like(qkv)

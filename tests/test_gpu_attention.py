@@ -280,3 +280,20 @@ def test_cache_append_is_the_slice_assignment(B, n, c0, rows, H, Hkv, d):
         want[:, c0 + n:(c0 + n + 127) // 128 * 128] = 0
         for got in (caches[i], caches[i + 2]):
             assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("B,L,H,Hkv,d", [(1, 777, 14, 2, 64), (2, 129, 8, 8, 64), (1, 1, 2, 1, 64), (1, 300, 12, 2, 128), (4, 1100, 32, 8, 128)])
+def test_key_gradients_are_rotated_back_where_they_are_written(B, L, H, Hkv, d):
+    """Key and value gradients of the backward pass that undoes the rotary embedding, written by one CTA or summed over a
+    cluster: the bits of the plain backward pass followed by the rope kernel (positions in any order)."""
+    from llm_distillery_b200.ops import basic
+    torch.manual_seed(L)
+    qkv = torch.randn(B * L, (H + 2 * Hkv) * d, device=DEV).bfloat16()
+    out, lse = attention.attention_fwd(qkv, B, L, H, Hkv, d)
+    dout = torch.randn_like(out)
+    pos = torch.randint(0, 2000, (B * L,), device=DEV, dtype=torch.int32)
+    cos, sin = basic.rope_tables(2000, d, 10000.0, DEV)
+    got = attention.attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin)
+    want = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d)
+    basic.rope_(want, pos, cos, sin, H + Hkv, d, inverse=True)
+    assert torch.equal(got[:, H * d:], want[:, H * d:]) and _lib.take_device_error() == 0
