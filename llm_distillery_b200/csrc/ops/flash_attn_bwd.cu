@@ -31,8 +31,9 @@
 // 638 / 521 us; 2 x 4000, 32/8 of 128 1191 / 710; 1 x 777, 14/2 of 64 122 / 33. The rotation of dK in the epilogue instead of a
 // launch behind it: 2 x 256, 8/2 of 64 21.0 / 16.0 us, 1 x 777, 14/2 34.2 / 32.0, large ones 4 to 10 us.
 // Few key blocks (short sequences, few kv heads) leave SMs idle while each CTA walks all query heads of its group: then a
-// cluster of up to 8 CTAs shares the heads, and the partial dK / dV meet through distributed shared memory, added in the
-// order of the CTAs' ranks (`head_split` below; results repeat bit for bit).
+// cluster of up to 8 CTAs may share the heads, and the partial dK / dV meet through distributed shared memory, added in the
+// order of the CTAs' ranks (`head_split` below; results repeat bit for bit). The caller has to allow it: under the reference
+// loss, whose value after the next update turned the other last bits into up to 0.8 % (777 tokens), the order stays.
 #include "../common/ptx.cuh"
 #include "../common/host.cuh"
 
@@ -817,7 +818,7 @@ static int head_split(int B, int L, int window, int H, int Hkv) {
 template <int D>
 static int launch_bwd(const void* dout, const void* qkv, const void* out, const float* lse, float* delta, void* dqkv,
                       float* dq_acc, int B, int L, int window, int H, int Hkv, const int* pos,
-                      const float* cos_tab, const float* sin_tab, cudaStream_t st) {
+                      const float* cos_tab, const float* sin_tab, int share_heads, cudaStream_t st) {
   using C = Cfg<D>;
   const long long width = (long long)(H + 2 * Hkv) * D;
   const long long T = (long long)B * L;
@@ -845,7 +846,7 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
     B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     attr = true;
   }
-  const int hs = head_split(B, L, window, H, Hkv);
+  const int hs = share_heads ? head_split(B, L, window, H, Hkv) : 1;
   BwdParams p{lse, delta, (__nv_bfloat16*)dqkv, B, L, H, Hkv, window, hs, 1.0f / sqrtf((float)D), pos, cos_tab, sin_tab};
   dim3 grid(Hkv * B * hs, (L + BN - 1) / BN);
   if (hs > 1)
@@ -881,26 +882,28 @@ extern "C" int b200_flash_attn_bwd(const void* dout, const void* qkv, const void
       Hkv <= 0 || (H % Hkv) != 0)
     return B200_ERR_ARG;
   if (window >= L) window = 0;      // causal; also keeps the sum of position and window inside 32 bits
-  if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, nullptr, nullptr, nullptr, st);
+  if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, nullptr, nullptr, nullptr, 0, st);
   if (D == 128)
-    return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, nullptr, nullptr, nullptr, st);
+    return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, nullptr, nullptr, nullptr, 0, st);
   return B200_ERR_ARG;
 }
 
-// The same with the inverse rotary embedding of the query and key heads (pos int32 [B*L]; cos / sin fp32 [max_pos, D/2]):
-// where the fp32 dQ accumulator is converted to bf16 and in the main kernel's epilogue.
+// The same with the inverse rotary embedding of the query and key heads (pos int32 [B*L]; cos / sin fp32 [max_pos, D/2]; pos
+// null: without): where the fp32 dQ accumulator is converted to bf16 and in the main kernel's epilogue. share_heads: the query
+// heads of a group may be shared by a cluster where that is faster; the order of the additions into dK and dV then depends on
+// the sizes. Without it the heads of a group are added one after the other at every size.
 extern "C" int b200_flash_attn_bwd_rope(const void* dout, const void* qkv, const void* out, const float* lse,
                                         float* delta, void* dqkv, float* dq_acc, const int* pos, const float* cos_tab,
-                                        const float* sin_tab, int B, int L, int window, int H, int Hkv, int D,
+                                        const float* sin_tab, int B, int L, int window, int H, int Hkv, int D, int share_heads,
                                         cudaStream_t st) {
   using namespace b200;
-  if (!dout || !qkv || !out || !lse || !delta || !dqkv || !dq_acc || !pos || !cos_tab || !sin_tab || B <= 0 || L <= 0 ||
+  if (!dout || !qkv || !out || !lse || !delta || !dqkv || !dq_acc || (pos && (!cos_tab || !sin_tab)) || B <= 0 || L <= 0 ||
       window < 0 || H <= 0 || Hkv <= 0 || (H % Hkv) != 0)
     return B200_ERR_ARG;
   if (window >= L) window = 0;      // causal; also keeps the sum of position and window inside 32 bits
-  if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, pos, cos_tab, sin_tab, st);
+  if (D == 64) return fab::launch_bwd<64>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, pos, cos_tab, sin_tab, share_heads, st);
   if (D == 128)
-    return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, pos, cos_tab, sin_tab, st);
+    return fab::launch_bwd<128>(dout, qkv, out, lse, delta, dqkv, dq_acc, B, L, window, H, Hkv, pos, cos_tab, sin_tab, share_heads, st);
   return B200_ERR_ARG;
 }
 

@@ -28,7 +28,7 @@ int b200_swiglu_fwd(const void*, void*, long long, int, cudaStream_t);
 int b200_swiglu_bwd(const void*, const void*, void*, long long, int, cudaStream_t);
 int b200_flash_attn_fwd(const void*, void*, float*, int, int, int, int, int, int, cudaStream_t);
 int b200_flash_attn_bwd_rope(const void*, const void*, const void*, const float*, float*, void*, float*, const int*,
-                             const float*, const float*, int, int, int, int, int, int, cudaStream_t);
+                             const float*, const float*, int, int, int, int, int, int, int, cudaStream_t);
 }
 
 namespace b200 {
@@ -196,7 +196,7 @@ extern "C" int b200_layer_bwd(const void* dh2, const void* x, const int* pos, co
   if (g_o) RUN(wgrad(t.dh1, h, s.att, A, g_o, 2));
   RUN(dgrad(t.dh1, h, w_o, A, t.datt));
   RUN(b200_flash_attn_bwd_rope(t.datt, s.qkv, s.att, s.lse, t.delta, t.dqkv, t.dq_acc, pos, cos_tab, sin_tab, B, L, window, H,
-                               Hkv, d, st));
+                               Hkv, d, split_k & 1, st));
   if (g_bqkv) RUN(b200_bias_grad(t.dqkv, g_bqkv, T, N, N, (acc >> 6) & 1, st));
   if (g_qkv) RUN(wgrad(t.dqkv, N, s.n1, h, g_qkv, 1));
   RUN(dgrad(t.dqkv, N, w_qkv, h, t.dn));

@@ -229,7 +229,7 @@ class DecoderLayerFn(torch.autograd.Function):
         g_o = _wgrad(db1, att, w_o, s_o, sp)
         datt = basic.linear_dgrad(db1, w_o, sp)
         del db1
-        dqkv = attention.attention_bwd_unrotated(datt, qkv, att, lse, B, L, H, Hkv, d, pos, cos, sin, window)
+        dqkv = attention.attention_bwd_unrotated(datt, qkv, att, lse, B, L, H, Hkv, d, pos, cos, sin, window, sp)
         del datt
         g_qn = g_kn = None
         if w_qn is not None:

@@ -148,11 +148,12 @@ def attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window: int | None = Non
     return flash.flash_attn_bwd(dout.to(qkv.dtype), qkv, out, lse, B, L, H, Hkv, d, window=window)
 
 
-def attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin, window: int | None = None):
+def attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin, window: int | None = None,
+                            share_heads: bool = False):
     """dqkv with respect to the projection's output BEFORE the rotary embedding: attention backward followed by the
     inverse rotation of the query and key heads. On the GPU they are rotated where they are written: the query heads where
     their fp32 accumulator is converted to bf16, the key heads in the kernel's epilogue; same values as ``attention_bwd`` +
-    ``rope_``."""
+    ``rope_``. ``share_heads``: see ``flash.flash_attn_bwd``."""
     from . import basic
     if window is not None and L <= window:
         window = None
@@ -162,7 +163,8 @@ def attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin,
     if (qkv.is_cuda and qkv.dtype == torch.bfloat16 and pos.dtype == torch.int32 and cos.is_contiguous()
             and sin.is_contiguous() and 2 * cos.shape[1] == d):      # partial rotary: the separate kernel below
         from . import flash
-        return flash.flash_attn_bwd(dout.to(qkv.dtype), qkv, out, lse, B, L, H, Hkv, d, rope=(pos, cos, sin), window=window)
+        return flash.flash_attn_bwd(dout.to(qkv.dtype), qkv, out, lse, B, L, H, Hkv, d, rope=(pos, cos, sin), window=window,
+                                    share_heads=share_heads)
     dqkv = attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
     return basic.rope_(dqkv, pos, cos, sin, H + Hkv, d, inverse=True)
 

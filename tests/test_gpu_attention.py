@@ -250,8 +250,9 @@ def test_query_heads_shared_by_a_cluster(B, L, H, Hkv, d, window):
     qkv = torch.randn(B * L, (H + 2 * Hkv) * d, device=DEV).bfloat16()
     dout = torch.randn(B * L, H * d, device=DEV).bfloat16()
     out, lse = attention.attention_fwd(qkv, B, L, H, Hkv, d, window)
-    got = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
-    again = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window)
+    from llm_distillery_b200.ops import flash
+    got = flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window=window, share_heads=True)
+    again = flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, window=window, share_heads=True)
     if window is None:
         ro, rl = attention.attention_reference_fwd(qkv.float(), B, L, H, Hkv, d)
         want = attention.attention_reference_bwd(dout.float(), qkv.float(), ro, rl, B, L, H, Hkv, d)
@@ -293,7 +294,9 @@ def test_key_gradients_are_rotated_back_where_they_are_written(B, L, H, Hkv, d):
     dout = torch.randn_like(out)
     pos = torch.randint(0, 2000, (B * L,), device=DEV, dtype=torch.int32)
     cos, sin = basic.rope_tables(2000, d, 10000.0, DEV)
-    got = attention.attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin)
-    want = attention.attention_bwd(dout, qkv, out, lse, B, L, H, Hkv, d)
-    basic.rope_(want, pos, cos, sin, H + Hkv, d, inverse=True)
-    assert torch.equal(got[:, H * d:], want[:, H * d:]) and _lib.take_device_error() == 0
+    from llm_distillery_b200.ops import flash
+    for share in (False, True):
+        got = attention.attention_bwd_unrotated(dout, qkv, out, lse, B, L, H, Hkv, d, pos, cos, sin, share_heads=share)
+        want = flash.flash_attn_bwd(dout, qkv, out, lse, B, L, H, Hkv, d, share_heads=share)
+        basic.rope_(want, pos, cos, sin, H + Hkv, d, inverse=True)
+        assert torch.equal(got[:, H * d:], want[:, H * d:]) and _lib.take_device_error() == 0

@@ -84,7 +84,7 @@ def test_reference_loss_through_fused_stats():
 
 @pytest.mark.parametrize("M,K,Vc,T,lens", [(1, 2, 5000, 1.0, [1]), (7, 3, 5000, 1.0, [2, 5]), (65, 33, 900, 2.0, [64, 1]),
                                            (700, 200, 4800, 1.0, [700]), (1601, 400, 5000, 2.0, [1, 511, 513, 576])])
-def test_reference_loss_kernels_against_fp64(M, K, Vc, T, lens):
+def test_reference_loss_kernels_against_fp64(monkeypatch, M, K, Vc, T, lens):
     """Loss, logged values and both gradients against the PyTorch form in fp64, with rows without a target, without a label, left
     out of the cross-entropy and without a hit, and ids beyond the cropped vocabulary. Bound: sums of up to 400 fp32 terms, their
     differences and a division by the largest of them: 2e-5 of the largest value (single values differ by 1e-6 of it)."""
@@ -106,6 +106,8 @@ def test_reference_loss_kernels_against_fp64(M, K, Vc, T, lens):
         u[5], u[9, 1:] = float("-inf"), float("-inf")
         labels[5] = labels[9] = -1
     grads, outs = [], []
+    assert not head._native_reference_loss(zk.to(DEV), u.to(DEV), *(x.to(DEV) for x in (ids, labels, avoid, seg)))      # few rows
+    monkeypatch.setattr(head, "NATIVE_REFERENCE_ROWS", 1)
     for dev, dt in ((DEV, torch.float32), ("cpu", torch.float64)):
         a, b = (x.to(dev, dt).clone().requires_grad_() for x in (lse, zk))
         args = [x.to(dev) for x in (ids.int(), labels, avoid, seg)]
