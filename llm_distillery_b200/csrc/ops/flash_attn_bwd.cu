@@ -28,7 +28,7 @@
 // warps per scheduler to fill it. Four of them with 32 columns each measured the same (head dim 64) or slower (128: 80
 // registers a thread; 800 against 710 us).
 // All three kernels of a backward pass, B200, queries as rows and one S / dP buffer / now: 8 x 2048, 32/4 heads of 64
-// 638 / 521 us; 2 x 4000, 32/8 of 128 1191 / 710; 1 x 777, 14/2 of 64 122 / 33. The rotation of dK in the epilogue instead of a
+// 638 / 521 us; 2 x 4000, 32/8 of 128 1191 / 710; 1 x 777, 14/2 of 64 122 / 33 with shared heads. The rotation of dK in the epilogue instead of a
 // launch behind it: 2 x 256, 8/2 of 64 21.0 / 16.0 us, 1 x 777, 14/2 34.2 / 32.0, large ones 4 to 10 us.
 // Few key blocks (short sequences, few kv heads) leave SMs idle while each CTA walks all query heads of its group: then a
 // cluster of up to 8 CTAs may share the heads, and the partial dK / dV meet through distributed shared memory, added in the

@@ -50,7 +50,7 @@ def route(n2: torch.Tensor, w_router: torch.Tensor, k: int, renorm: bool = True)
 def permutation(top_e: torch.Tensor, n_experts: int):
     """(order, inverse, token, counts): ``order`` lists the T*k (token, choice) pairs sorted by expert (stable, so tokens
     keep their order inside an expert's slab), ``inverse`` undoes it, ``token`` is the token of each sorted pair,
-    ``counts`` are the slab lengths as Python ints. One kernel on a GPU (csrc/ops/moe.cu) for up to 32 experts and
+    ``counts`` are the slab lengths as Python ints. Two launches on a GPU (csrc/ops/moe.cu) for up to 32 experts and
     ``SORT_MAX_PAIRS`` pairs; beyond them, and for indices that are not int64, the library's sort."""
     order, inverse, token, counts = _sorted_pairs(top_e, n_experts)
     return order, inverse, token, counts.tolist()
