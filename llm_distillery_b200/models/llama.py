@@ -465,11 +465,15 @@ class LlamaModel(nn.Module):
         tables = self.layer_rope(cos, sin)
         meta7 = meta
         from . import layer_native
-        checked, tables_ok = None, False
+        checked, tables_ok, first, stack = None, False, 0, []
         if (plain and pre is None and LAYER_WEIGHTS_PRE[0] is None and not meta[6] and not cfg.sandwich and not cfg.num_local_experts
                 and training and h.is_cuda and B * L <= layer_native.STACK_MAX_TOKENS):
-            stack = []         # nothing happens between the layers: all of them in one call, if each fits
-            for li, (layer, table) in enumerate(zip(self.layers, tables)):
+            # Nothing happens between the layers: one call for all of them, if each fits. Those that no gradient reaches stay in
+            # front of it: their backward pass is not run and their activations are given back.
+            first = 0 if h.requires_grad else next((i for i, layer in enumerate(self.layers)
+                                                    if any(p.requires_grad for p in layer.parameters())), len(self.layers))
+            for li in range(first, len(self.layers)):
+                layer, table = self.layers[li], tables[li]
                 b_qkv = getattr(layer, "qkv_bias", None)
                 w = (layer.input_layernorm, layer.qkv_proj, layer.o_proj, layer.post_attention_layernorm, layer.gate_up_proj,
                      layer.down_proj)
@@ -478,10 +482,12 @@ class LlamaModel(nn.Module):
                 if not layer_native.fits(h, pos, *table, w, b_qkv, heads, training, tables_ok):
                     break
                 stack.append((w, b_qkv, *table, cfg.layer_window(li, L)))
-            if stack and len(stack) == len(self.layers) and len({w[4].shape for w, *_ in stack}) == 1:
-                h = layer_native.run_stack(h, pos, stack, meta, split)
-                tables = []
+            if len(stack) < len(self.layers) - first or len({w[4].shape for w, *_ in stack}) > 1:
+                stack = []
         for li, (layer, table) in enumerate(zip(self.layers, tables)):
+            if stack and li == first:
+                h = layer_native.run_stack(h, pos, stack, meta7, split)
+                break
             cos, sin = table
             meta = meta7 + (cfg.layer_window(li, L),)       # the layer's sliding window when the sequence is longer
             if pre is not None:

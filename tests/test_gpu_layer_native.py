@@ -92,3 +92,36 @@ def test_layers_in_one_call_equal_a_call_each(monkeypatch, between):
     assert torch.equal(results[0][0], results[1][0])
     for name, want in results[0][1].items():
         assert torch.equal(results[1][1][name], want), name
+
+
+@pytest.mark.parametrize("embedding,layers,stacked", [(True, 0, 5), (True, 2, 3), (True, 5, 0), (False, 2, 5)])
+def test_layers_that_no_gradient_reaches_stay_out_of_the_one_call(monkeypatch, embedding, layers, stacked):
+    """Frozen embedding and first layers: outputs and gradients bit for bit those of a node per layer, whose backward pass ends at
+    the first layer with a trained weight - and no more launches and no more memory than it takes."""
+    cfg = llama.LlamaConfig(vocab_size=512, hidden_size=256, intermediate_size=640, num_hidden_layers=5, num_attention_heads=4,
+                            num_key_value_heads=2, max_position_embeddings=512)
+    results = []
+    for limit in (0, layer_native.STACK_MAX_TOKENS):
+        model = llama.build_model(cfg, dtype=torch.bfloat16, device="cuda", seed=3)
+        for w in [model.embed_tokens] * embedding + [p for l in model.layers[:layers] for p in l.parameters()]:
+            w.requires_grad_(False)
+        FlatParams([p for p in model.parameters() if p.requires_grad])
+        ids = torch.randint(0, 512, (2, 173), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+        monkeypatch.setattr(layer_native, "STACK_MAX_TOKENS", limit)
+        sizes, real = [], layer_native.run_stack
+        monkeypatch.setattr(layer_native, "run_stack", lambda x, pos, stack, *a: sizes.append(len(stack)) or real(x, pos, stack, *a))
+        before = torch.cuda.memory_allocated()
+        y = model.hidden_states(ids)
+        held = torch.cuda.memory_allocated() - before
+        launches = _lib.LAUNCH_COUNT[0]
+        y.backward(torch.randn(y.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(2)).to(y.dtype))
+        launches = _lib.LAUNCH_COUNT[0] - launches
+        monkeypatch.undo()
+        assert sizes == ([stacked] if limit and stacked else []) and _lib.take_device_error() == 0
+        results.append((y.detach(), {n: p.grad_slot.buf.clone() for n, p in model.named_parameters()
+                                     if p.requires_grad and "embed" not in n}, launches, held))
+    (want_y, want, launches_each, held_each), (got_y, got, launches, held) = results
+    assert torch.equal(got_y, want_y) and got.keys() == want.keys()
+    for name in want:
+        assert torch.equal(got[name], want[name]), name
+    assert launches <= launches_each and held <= 1.25 * held_each        # the allocator rounds blocks up; two layers more are 1.6
