@@ -19,7 +19,7 @@ namespace b200 {
 namespace refloss {
 
 // per-row values kept between the kernels, [ROWS][M]
-enum { R_KL, R_RKL, R_PS, R_PT, R_HIT, R_LS, R_LT, R_CKL, R_CRKL, R_CPICK, ROWS };
+enum { R_KL, R_RKL, R_PS, R_PT, R_HIT, R_MS, R_LS, R_MT, R_LT, R_CKL, R_CRKL, R_CPICK, ROWS };
 // per-conversation outputs, [OUTS][n_seg]
 enum { O_CUSTOM, O_CE, O_KL, O_RKL, O_WKL, O_WRKL, O_CET, O_DIFF, OUTS };
 
@@ -110,8 +110,11 @@ __global__ void __launch_bounds__(256) rows_kernel(RowArgs p, float* __restrict_
     o[R_PS * M] = ps;
     o[R_PT * M] = pt;
     o[R_HIT * M] = hit ? 1.f : 0.f;
-    o[R_LS * M] = any ? ms + ls : 0.f;
-    o[R_LT * M] = any ? mt + lt : 0.f;
+    // maximum and log of the sum apart: rounded into one number they would put its last bit, 5e-7 at 10, on every probability
+    o[R_MS * M] = any ? ms : 0.f;
+    o[R_LS * M] = ls;
+    o[R_MT * M] = any ? mt : 0.f;
+    o[R_LT * M] = lt;
   }
 }
 
@@ -252,7 +255,7 @@ __global__ void __launch_bounds__(256) grad_kernel(RowArgs p, const float* __res
   const long long M = p.M;
   const float* o = rows + r;
   const float gc = g[seg[r]], lse = p.lse[r];
-  const float rkl = o[R_RKL * M], ls = o[R_LS * M], lt = o[R_LT * M];
+  const float rkl = o[R_RKL * M], ms = o[R_MS * M], ls = o[R_LS * M], mt = o[R_MT * M], lt = o[R_LT * M];
   const float ck = gc * o[R_CKL * M], cr = gc * o[R_CRKL * M], cp = gc * o[R_CPICK * M];
   const long long label = p.labels[r];
   const bool wants = label >= 0 && !p.avoid[r];
@@ -261,7 +264,7 @@ __global__ void __launch_bounds__(256) grad_kernel(RowArgs p, const float* __res
     const Entry e = entry(p, r, k, lse);
     float d = 0.f;
     if (e.valid) {
-      const float t = e.t - lt, s1 = e.s - ls;
+      const float t = (e.t - mt) - lt, s1 = (e.s - ms) - ls;
       d = expf(s1) * (s1 - t - rkl) * cr - expf(t) * ck;
       if (wants && p.ids[r * p.K + k] == label) d += cp;
     }
@@ -282,7 +285,7 @@ static bool args_ok(const RowArgs& p) {
 extern "C" {
 using namespace b200;
 
-// rows: fp32 [10, M], kept for the gradient; out: fp32 [8, n_seg] (custom loss, CE, KL, reverse KL, weighted KL, weighted
+// rows: fp32 [12, M], kept for the gradient; out: fp32 [8, n_seg] (custom loss, CE, KL, reverse KL, weighted KL, weighted
 // reverse KL, teacher CE, CE difference of each conversation). seg int64 [M], non-decreasing in [0, n_seg).
 int b200_reference_loss(const float* zk, const float* lse, const float* u, const int* ids, const long long* labels,
                         const unsigned char* avoid, const long long* seg, float* rows, float* out, long long M, int K, int vocab,

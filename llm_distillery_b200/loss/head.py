@@ -192,7 +192,7 @@ class _ReferenceLossFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, lse, zk, u, ids, labels, avoid, seg, n_seg, temperature, vocab, alpha):
         M, K = zk.shape
-        rows = torch.empty((10, M), dtype=torch.float32, device=zk.device)
+        rows = torch.empty((12, M), dtype=torch.float32, device=zk.device)
         out = torch.empty((8, n_seg), dtype=torch.float32, device=zk.device)
         p = _lib.ptr
         _lib.check(_lib.kernels().b200_reference_loss(p(zk), p(lse), p(u), p(ids), p(labels), p(avoid), p(seg), p(rows), p(out),

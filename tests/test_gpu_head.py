@@ -130,3 +130,31 @@ def test_reference_loss_kernels_against_fp64(monkeypatch, M, K, Vc, T, lens):
         assert torch.equal(x.isnan(), y.isnan())
         assert (x - y).nan_to_num(0).abs().max() <= 2e-5 * y.nan_to_num(0).abs().max() + 1e-9
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("M,K", [(1, 2), (40, 33), (300, 200)])
+def test_reference_loss_gradient_of_far_log_probs(M, K):
+    """Values around -1000 (a temperature of 1/128) that fp32 holds exactly: the probabilities must not carry the last bit of a
+    maximum of that size (3e-5). Exact differences, exponentials and sums of up to 200 terms: 200 * 2^-24, 1.2e-5, at the very
+    worst; 5e-6 of the largest value stands for sums whose roundings do not all go one way."""
+    g = torch.Generator().manual_seed(M)
+    T, seg = 1 / 128, torch.zeros(M, dtype=torch.int64)
+    ids = torch.rand(M, 500, generator=g).topk(K, -1).indices.sort(-1).values
+    u = -8 - torch.randint(0, 9 * 2 ** 10, (M, K), generator=g) / 2 ** 17                      # u / T: -1024 .. -1033 in steps of 2^-10
+    lse = 1000 + torch.randint(0, 2 ** 10, (M,), generator=g) / 2 ** 10
+    zk = -torch.randint(0, 9 * 2 ** 10, (M, K), generator=g) / 2 ** 10                         # zk - lse: -1000 .. -1010
+    labels, avoid = ids[:, 0].clone(), torch.zeros(M, dtype=torch.bool)
+    grads = []
+    for dev, dt in ((DEV, torch.float32), ("cpu", torch.float64)):
+        a, b, t = lse.to(dev, dt).requires_grad_(), zk.to(dev, dt).requires_grad_(), u.to(dev, dt)
+        args = [x.to(dev) for x in (ids.int(), labels, avoid, seg)]
+        if dev == DEV:
+            custom, _ = head._ReferenceLossFn.apply(a, b, t, *args, 1, T, 500, 2.0)
+        else:
+            custom, _ = dv.reference_loss_segments(*dv.student_teacher_logprobs(a, b, t, args[0] < 500, T), args[0].long(),
+                                                   *args[1:], 1, 2.0)
+        custom.sum().backward()
+        grads.append([x.grad.double().cpu() for x in (a, b)])
+    for x, y in zip(*grads):
+        assert (x - y).abs().max() <= 5e-6 * y.abs().max()
+    assert _lib.take_device_error() == 0
