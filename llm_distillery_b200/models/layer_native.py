@@ -185,20 +185,10 @@ class NativeStackFn(torch.autograd.Function):
         B, L, H, Hkv, d, eps = ctx.meta[:6]
         n, (T, h), f = len(ctx.layers), x.shape, ctx.layers[0][0][4].shape[0] // 2
         lib, size, bytes_ = _lib.kernels(), saved.numel() // n, T * h * x.element_size()
-        grads, slots, written = [], [], set()
-        for i in range(n - 1, -1, -1):
-            ws, b, *_ = ctx.layers[i]
-            mine = [llama._slot(w) if w is not None else None for w in ws + (b,)]
-            acc = sum(1 << k for k, s in enumerate(mine) if s is not None and (not s.fresh or id(s) in written))
-            written.update(id(s) for s in mine)
-            slots.insert(0, mine)
-            grads[:0] = [x.data_ptr() if i == 0 else between.data_ptr() + (i - 1) * bytes_,
-                         *(0 if s is None else s.buf.data_ptr() for s in mine), acc]
-        rows, grads = _records(ctx.layers, L, [saved.data_ptr() + i * size for i in range(n)], [0] * n), _u64(grads)
         dout = dout.contiguous()
         scratch = torch.empty(lib.b200_layer_scratch_bytes(B, L, H, Hkv, d, h, f), dtype=torch.uint8, device=x.device)
         turn = torch.empty((2, T, h), dtype=x.dtype, device=x.device)
-        dx, done, at = torch.empty_like(x), ctypes.c_int(0), ctypes.byref
+        dx, done = torch.empty_like(x), ctypes.c_int(0)
         hooks = llama.UNIT_PRE[0], llama.LAYER_WEIGHTS_PRE[0], llama.LAYER_BACKWARD_DONE[0]
         each = any(k is not None for k in hooks)                 # something happens between layers: one at a time
         for last in (range(n - 1, -1, -1) if each else (n - 1,)):
@@ -207,11 +197,21 @@ class NativeStackFn(torch.autograd.Function):
                 hooks[0](w_ln1, True)
             if hooks[1] is not None:
                 hooks[1](w_ln1)
-            to = dx if lo == 0 else turn[lo & 1]
-            rc = lib.b200_stack_bwd(at(rows, 96 * lo), at(grads, 72 * lo), last - lo + 1, dout.data_ptr(), pos.data_ptr(),
-                                    scratch.data_ptr(), to.data_ptr(), turn[0].data_ptr(), turn[1].data_ptr(), B, L, H, Hkv, d,
-                                    h, f, int(ctx.split[1]), at(done), _lib.stream())
-            for mine in slots[last + 1 - done.value:last + 1]:   # also of a call that failed: the layers that did run
+            grads, slots, written = [], [], set()      # behind the hooks: they may have moved weights and slots
+            for i in range(last, lo - 1, -1):
+                ws, b, *_ = ctx.layers[i]
+                mine = [llama._slot(w) if w is not None else None for w in ws + (b,)]
+                acc = sum(1 << k for k, s in enumerate(mine) if s is not None and (not s.fresh or id(s) in written))
+                written.update(id(s) for s in mine)
+                slots.append(mine)
+                grads[:0] = [x.data_ptr() if i == 0 else between.data_ptr() + (i - 1) * bytes_,
+                             *(0 if s is None else s.buf.data_ptr() for s in mine), acc]
+            m, to = last + 1 - lo, dx if lo == 0 else turn[lo & 1]
+            rows = _records(ctx.layers[lo:last + 1], L, [saved.data_ptr() + i * size for i in range(lo, last + 1)], [0] * m)
+            rc = lib.b200_stack_bwd(rows, _u64(grads), m, dout.data_ptr(), pos.data_ptr(), scratch.data_ptr(), to.data_ptr(),
+                                    turn[0].data_ptr(), turn[1].data_ptr(), B, L, H, Hkv, d, h, f, int(ctx.split[1]),
+                                    ctypes.byref(done), _lib.stream())
+            for mine in slots[:done.value]:            # also of a call that failed: the layers that did run
                 for s in mine:
                     if s is not None:
                         s.fresh = False

@@ -108,3 +108,47 @@ def test_a_failing_call_over_several_layers_marks_those_that_ran(monkeypatch, ra
         y.backward(torch.zeros_like(y))
     assert [all(t.grad_slot.fresh for t in w) for w, *_ in layers] == [i < 3 - ran for i in range(3)]
     assert not any(t.grad_slot.fresh for w, *_ in layers[3 - ran:] for t in w)
+
+
+def test_what_a_hook_moves_is_read_where_it_then_lies(monkeypatch):
+    """A hook in front of a layer's backward pass (weights gathered, low-bit weights expanded) may put the layer's weights and
+    gradient slots elsewhere: the call takes their addresses behind it."""
+    import ctypes
+    from llm_distillery_b200.models import llama
+    got = []
+
+    class Lib:
+        def b200_stack_bwd(self, rows, grads, n, *a):
+            rows, grads = (ctypes.cast(r, ctypes.POINTER(ctypes.c_uint64)) for r in (rows, grads))
+            got.append((rows[3], grads[2]))                  # the q/k/v matrix and its gradient
+            ctypes.cast(a[-2], ctypes.POINTER(ctypes.c_int))[0] = n
+            return 20
+
+        def __getattr__(self, name):
+            return (lambda: b"") if name == "b200_last_cuda_error" else (lambda *a: 64)
+
+    class Slot:
+        def __init__(self, w):
+            self.buf, self.fresh = torch.zeros(w.shape), True
+    monkeypatch.setattr(layer_native._lib, "kernels", Lib)
+    monkeypatch.setattr(layer_native._lib, "stream", lambda: None)
+    n, layers = (H + 2 * HKV) * D, []
+    tables = torch.zeros(16, D // 2), torch.zeros(16, D // 2)
+    for _ in range(3):
+        w = tuple(torch.zeros(s, dtype=torch.bfloat16).requires_grad_() for s in ((W,), (n, W), (W, H * D), (W,), (2 * F, W), (W, F)))
+        for t in w:
+            t.grad_slot = Slot(t)
+        layers.append((w, None, *tables, None))
+    held = []
+
+    def gather(first, backward):
+        w = next(ws[1] for ws, *_ in layers if ws[0] is first)
+        held.append((w.data, w.grad_slot.buf))               # the old places stay taken: nothing else lands there
+        w.data = w.data.clone()
+        w.grad_slot = Slot(w)
+    y = layer_native.run_stack(torch.zeros(T, W, dtype=torch.bfloat16), torch.zeros(T, dtype=torch.int32), layers,
+                               (1, T, H, HKV, D, 1e-5, False, None), (False, False))
+    monkeypatch.setattr(llama, "UNIT_PRE", [gather])
+    y.backward(torch.zeros_like(y))
+    assert got == [(ws[1].data_ptr(), ws[1].grad_slot.buf.data_ptr()) for ws, *_ in reversed(layers)]
+    assert not any(t.grad_slot.fresh for ws, *_ in layers for t in ws)
