@@ -17,31 +17,29 @@ constexpr int SORT_MAX_EXPERTS = 32;
 // experts: the ten launches of a library radix sort, histogram, scatter and division that this replaces took about 90 us; with
 // each thread reading its run from global memory, one 8-byte key after the other, and writing all three lists from the one
 // block it took 33. The block writes `inverse` alone - stores of one SM to scattered sectors take a clock each - and a second
-// launch of many blocks makes the other two of it. The runs grow with the pairs and one block does not: the caller goes to the library beyond 32768 of them (models/moe.py: SORT_MAX_PAIRS, with both sides'
-// times); more than SORT_STAGED_PAIRS are walked in global memory.
-constexpr int SORT_STAGED_PAIRS = 65536;
+// launch of many blocks makes the other two of it. The runs grow with the pairs and one block does not: the library takes over
+// beyond SORT_MAX_PAIRS (models/moe.py has both sides' times), for which the keys still fit beside the counts.
+constexpr int SORT_MAX_PAIRS = 65536;
 __global__ void __launch_bounds__(SORT_THREADS, 1)
-    expert_sort_kernel(const long long* __restrict__ experts, long long n, int E, long long* __restrict__ inverse,
+    expert_sort_kernel(const long long* __restrict__ experts, int n, int E, long long* __restrict__ inverse,
                        long long* __restrict__ counts) {
   pdl_wait();
   pdl_trigger();
   extern __shared__ int slot[];                    // [E][SORT_THREADS], then the staged keys
   __shared__ int warp_base[SORT_MAX_EXPERTS][33];  // pairs of an expert in the warps before each, then their position
-  uint8_t* key = reinterpret_cast<uint8_t*>(slot + E * SORT_THREADS);
-  const bool staged = n <= SORT_STAGED_PAIRS;
+  int8_t* key = reinterpret_cast<int8_t*>(slot + E * SORT_THREADS);       // -1: of no expert
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long long per = (n + SORT_THREADS - 1) / SORT_THREADS;
-  const long long i0 = min(n, tid * per), i1 = min(n, i0 + per);
-  auto valid = [&](long long e) { return e >= 0 && e < E ? (int)e : -1; };
-  auto expert = [&](long long i) { return staged ? (int)(int8_t)key[i] : valid(experts[i]); };
-  if (staged) {
+  const int per = (n + SORT_THREADS - 1) / SORT_THREADS;
+  const int i0 = min(n, tid * per), i1 = min(n, i0 + per);
 #pragma unroll 8
-    for (int i = tid; i < (int)n; i += SORT_THREADS) key[i] = (uint8_t)(int8_t)valid(experts[i]);
+  for (int i = tid; i < n; i += SORT_THREADS) {
+    const long long e = experts[i];
+    key[i] = e >= 0 && e < E ? (int8_t)e : (int8_t)-1;
   }
   for (int e = 0; e < E; ++e) slot[e * SORT_THREADS + tid] = 0;
   __syncthreads();
-  for (long long i = i0; i < i1; ++i) {
-    const int e = expert(i);
+  for (int i = i0; i < i1; ++i) {
+    const int e = key[i];
     if (e >= 0) ++slot[e * SORT_THREADS + tid];
   }
   for (int e = 0; e < E; ++e) {                    // scan inside each warp, expert by expert
@@ -76,8 +74,8 @@ __global__ void __launch_bounds__(SORT_THREADS, 1)
     slot[e * SORT_THREADS + tid] += base + warp_base[e][warp];
     base += warp_base[e][32];
   }
-  for (long long i = i0; i < i1; ++i) {
-    const int e = expert(i);
+  for (int i = i0; i < i1; ++i) {
+    const int e = key[i];
     if (e >= 0) inverse[i] = slot[e * SORT_THREADS + tid]++;
   }
 }
@@ -150,20 +148,20 @@ __global__ void __launch_bounds__(256)
 extern "C" {
 using namespace b200;
 
-// experts int64 [n] in [0, E), E <= 32; order, inverse, token int64 [n], counts int64 [E]
+// experts int64 [n] in [0, E), n <= 65536, E <= 32; order, inverse, token int64 [n], counts int64 [E]
 int b200_expert_sort(const long long* experts, long long n, int E, int k, long long* order, long long* inverse,
                      long long* token, long long* counts, cudaStream_t st) {
-  if (!experts || !order || !inverse || !token || !counts || n <= 0 || n > 0x7fffffffLL || E <= 0 ||
+  if (!experts || !order || !inverse || !token || !counts || n <= 0 || n > moe::SORT_MAX_PAIRS || E <= 0 ||
       E > moe::SORT_MAX_EXPERTS || k <= 0)
     return B200_ERR_ARG;
-  const int smem = E * moe::SORT_THREADS * (int)sizeof(int) + (n <= moe::SORT_STAGED_PAIRS ? (int)n : 0);
+  const int smem = E * moe::SORT_THREADS * (int)sizeof(int) + (int)n;
   static bool attr = false;
   if (!attr) {
     B200_CUDA_CHECK(cudaFuncSetAttribute(moe::expert_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         moe::SORT_MAX_EXPERTS * moe::SORT_THREADS * (int)sizeof(int) + moe::SORT_STAGED_PAIRS));
+                                         moe::SORT_MAX_EXPERTS * moe::SORT_THREADS * (int)sizeof(int) + moe::SORT_MAX_PAIRS));
     attr = true;
   }
-  launch_pdl(moe::expert_sort_kernel, 1, moe::SORT_THREADS, smem, st, experts, n, E, inverse, counts);
+  launch_pdl(moe::expert_sort_kernel, 1, moe::SORT_THREADS, smem, st, experts, (int)n, E, inverse, counts);
   B200_CUDA_CHECK(cudaGetLastError());
   launch_pdl(moe::expert_scatter_kernel, (unsigned)ceil_div_ll(n, 256), 256, 0, st, experts, inverse, (int)n, E, k, order, token);
   B200_CUDA_CHECK(cudaGetLastError());

@@ -30,10 +30,11 @@ _lib.register("b200_gemm_grouped", [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP])
 _lib.register("b200_moe_combine", [_VP, _VP, _VP, _VP, _VP, _LL, _I, _I, _F, _VP])
 
 
-# One block sorts in time that grows with the pairs, the library's ten launches in time that hardly does: 8 / 32 experts, on the
-# device, 2048 pairs 6 / 12 us, 16 384 20 / 28, 32 768 41 / 54 (the block with one key in flight per thread 114 / 147). The
-# library took 140, 204, 215 and, for 65 536 and 131 072 pairs, 229 and 223 with the counts read back.
-SORT_MAX_PAIRS = 32768
+# One block sorts in time that grows with the pairs, the library's ten launches in time that hardly does. A call with the counts
+# read back, 8 / 32 experts, kernel against library: 2048 pairs 36 / 47 us against 137 / 134, 32 768 73 / 86 against 219 / 209,
+# 65 536 132 / 146 against 216 / 218; 131 072 276 / 296 against 210. With the counts left on the device 65 536 pairs take 99 / 112
+# against 199 / 200.
+SORT_MAX_PAIRS = 65536
 
 
 # ------------------------------------------------------------------------------------------------ routing

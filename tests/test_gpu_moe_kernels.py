@@ -20,8 +20,9 @@ def test_expert_sort_is_the_stable_sort(T, k, E):
     assert counts == torch.bincount(flat, minlength=E).tolist()
 
 
-@pytest.mark.parametrize("T,k,dtype,native", [(16384, 2, torch.int64, True), (16385, 2, torch.int64, False),
-                                              (4096, 8, torch.int64, True), (16384, 8, torch.int64, False),
+@pytest.mark.parametrize("T,k,dtype,native", [(16384, 2, torch.int64, True), (32768, 2, torch.int64, True),
+                                              (32769, 2, torch.int64, False), (4096, 8, torch.int64, True),
+                                              (16384, 8, torch.int64, False),
                                               (100, 2, torch.int32, False), (100, 2, torch.uint8, False)])
 def test_which_sort_takes_the_pairs(monkeypatch, T, k, dtype, native):
     """Many pairs are left to the library, whose sort is ahead there, and so are indices that the kernel would misread."""
@@ -119,9 +120,9 @@ def test_experts_that_one_launch_does_not_take(case):
     _lib.take_device_error()
 
 
-@pytest.mark.parametrize("n,E", [(1023, 3), (65536, 32), (65537, 32), (200003, 5)])
+@pytest.mark.parametrize("n,E", [(1, 1), (1023, 3), (1025, 32), (40001, 5), (65535, 1), (65536, 32)])
 def test_expert_sort_of_any_number_of_pairs(n, E):
-    """The kernel itself around the number of pairs that it stages in shared memory, with indices out of range left out."""
+    """The kernel itself up to the number of pairs that it takes, with indices out of range left out; one more is refused."""
     e = torch.randint(-1, E + 1, (n,), device="cuda", generator=torch.Generator("cuda").manual_seed(n))
     order, inverse, token = (torch.full((n,), -7, dtype=torch.int64, device="cuda") for _ in range(3))
     counts = torch.empty(E, dtype=torch.int64, device="cuda")
@@ -133,3 +134,5 @@ def test_expert_sort_of_any_number_of_pairs(n, E):
     assert torch.equal(order[:m], want) and torch.equal(token[:m], want // 3) and (order[m:] == -7).all()
     assert torch.equal(inverse[want], torch.arange(m, device="cuda"))
     assert torch.equal(counts, torch.bincount(e[ok], minlength=E))
+    rc = _lib.kernels().b200_expert_sort(p(e), 65537, E, 3, p(order), p(inverse), p(token), p(counts), _lib.stream())
+    assert rc < 0 and _lib.take_device_error() == 0
