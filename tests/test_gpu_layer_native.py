@@ -1,10 +1,12 @@
 """The native layer calls issue the launches of ``DecoderLayerFn``: same outputs and gradients, bit for bit."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
 from llm_distillery_b200.engine.optim import FlatParams
 from llm_distillery_b200.models import layer_native, llama
-from llm_distillery_b200.ops import _lib
+from llm_distillery_b200.ops import _lib, basic
 
 pytestmark = pytest.mark.gpu
 
@@ -125,3 +127,43 @@ def test_layers_that_no_gradient_reaches_stay_out_of_the_one_call(monkeypatch, e
     for name in want:
         assert torch.equal(got[name], want[name]), name
     assert launches <= launches_each and held <= 1.25 * held_each        # the allocator rounds blocks up; two layers more are 1.6
+
+
+@pytest.mark.parametrize("trained", [False, True])
+def test_a_layer_directly_behind_a_kernel_that_rewrites_its_weights(trained):
+    """The few-tile GEMMs of a layer ask for weights before the launch in front of them has ended: not for those that a kernel in
+    front of the whole call writes (an optimizer step, an expansion of low-bit weights). 46 M elements are rewritten right in
+    front of the forward and of the backward call, with other values each time; bit for bit what comes of waiting in between."""
+    T, H, Hkv, d, h, f = 93, 32, 4, 64, 2048, 5632
+    shapes = ((h,), ((H + 2 * Hkv) * d, h), (h, H * d), (h,), (2 * f, h), (h, f))
+    g = torch.Generator("cuda").manual_seed(0)
+    sizes = [torch.Size(s).numel() for s in shapes]
+    versions = [torch.randn(sum(sizes), device="cuda", generator=g) * 0.02 for _ in range(3)]
+    flat = torch.empty(sum(sizes), dtype=torch.bfloat16, device="cuda")
+    weights = [p.view(s).requires_grad_(trained) for p, s in zip(flat.split(sizes), shapes)]
+    if trained:
+        for w in weights:
+            w.grad_slot = SimpleNamespace(buf=torch.empty(w.shape, dtype=torch.float32, device="cuda"))
+    x = torch.randn(T, h, device="cuda", generator=g).bfloat16().requires_grad_()
+    dy = torch.randn(T, h, device="cuda", generator=g).bfloat16()
+    pos = torch.arange(T, dtype=torch.int32, device="cuda")
+    cos, sin = basic.rope_tables(T, d, 10000.0, "cuda")
+
+    def write(v, wait):
+        basic.cast_to_bf16(versions[v], flat)
+        if wait:
+            torch.cuda.synchronize()
+
+    def run(v, wait):
+        for w in weights if trained else []:
+            w.grad_slot.fresh = True
+        write(v, wait)
+        y = layer_native.NativeLayerFn.apply(x, pos, cos, sin, *weights, None, (1, T, H, Hkv, d, 1e-5, False, None), (not trained, True))
+        write((v + 1) % 3, wait)
+        dx, = torch.autograd.grad(y, x, dy)
+        return [y.detach(), dx] + ([w.grad_slot.buf.clone() for w in weights] if trained else [])
+    want = [run(v, True) for v in range(3)]
+    for i in range(12):
+        for got, ref in zip(run(i % 3, False), want[i % 3]):
+            assert torch.equal(got, ref)
+    assert _lib.take_device_error() == 0
