@@ -191,19 +191,18 @@ class NativeStackFn(torch.autograd.Function):
         dx, done = torch.empty_like(x), ctypes.c_int(0)
         hooks = llama.UNIT_PRE[0], llama.LAYER_WEIGHTS_PRE[0], llama.LAYER_BACKWARD_DONE[0]
         each = any(k is not None for k in hooks)                 # something happens between layers: one at a time
+        slots = [[llama._slot(w) if w is not None else None for w in ws + (b,)] for ws, b, *_ in ctx.layers]
         for last in (range(n - 1, -1, -1) if each else (n - 1,)):
             lo, w_ln1 = last if each else 0, ctx.layers[last][0][0]
             if hooks[0] is not None:
                 hooks[0](w_ln1, True)
             if hooks[1] is not None:
                 hooks[1](w_ln1)
-            grads, slots, written = [], [], set()      # behind the hooks: they may have moved weights and slots
+            grads, written = [], set()                 # addresses are read behind the hooks: they may have moved what lies there
             for i in range(last, lo - 1, -1):
-                ws, b, *_ = ctx.layers[i]
-                mine = [llama._slot(w) if w is not None else None for w in ws + (b,)]
+                mine = slots[i]
                 acc = sum(1 << k for k, s in enumerate(mine) if s is not None and (not s.fresh or id(s) in written))
                 written.update(id(s) for s in mine)
-                slots.append(mine)
                 grads[:0] = [x.data_ptr() if i == 0 else between.data_ptr() + (i - 1) * bytes_,
                              *(0 if s is None else s.buf.data_ptr() for s in mine), acc]
             m, to = last + 1 - lo, dx if lo == 0 else turn[lo & 1]
@@ -211,7 +210,7 @@ class NativeStackFn(torch.autograd.Function):
             rc = lib.b200_stack_bwd(rows, _u64(grads), m, dout.data_ptr(), pos.data_ptr(), scratch.data_ptr(), to.data_ptr(),
                                     turn[0].data_ptr(), turn[1].data_ptr(), B, L, H, Hkv, d, h, f, int(ctx.split[1]),
                                     ctypes.byref(done), _lib.stream())
-            for mine in slots[:done.value]:            # also of a call that failed: the layers that did run
+            for mine in slots[last + 1 - done.value:last + 1]:   # also of a call that failed: the layers that did run
                 for s in mine:
                     if s is not None:
                         s.fresh = False

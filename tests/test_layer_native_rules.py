@@ -112,7 +112,7 @@ def test_a_failing_call_over_several_layers_marks_those_that_ran(monkeypatch, ra
 
 def test_what_a_hook_moves_is_read_where_it_then_lies(monkeypatch):
     """A hook in front of a layer's backward pass (weights gathered, low-bit weights expanded) may put the layer's weights and
-    gradient slots elsewhere: the call takes their addresses behind it."""
+    gradient buffers elsewhere: the call takes their addresses behind it."""
     import ctypes
     from llm_distillery_b200.models import llama
     got = []
@@ -144,8 +144,7 @@ def test_what_a_hook_moves_is_read_where_it_then_lies(monkeypatch):
     def gather(first, backward):
         w = next(ws[1] for ws, *_ in layers if ws[0] is first)
         held.append((w.data, w.grad_slot.buf))               # the old places stay taken: nothing else lands there
-        w.data = w.data.clone()
-        w.grad_slot = Slot(w)
+        w.data, w.grad_slot.buf = w.data.clone(), w.grad_slot.buf.clone()
     y = layer_native.run_stack(torch.zeros(T, W, dtype=torch.bfloat16), torch.zeros(T, dtype=torch.int32), layers,
                                (1, T, H, HKV, D, 1e-5, False, None), (False, False))
     monkeypatch.setattr(llama, "UNIT_PRE", [gather])
