@@ -23,16 +23,17 @@
 // exponentials of pair i + 1 while dK_i, dP_{i+1} and dQ_i run. Head dim 64: two S buffers; P_i in the lower half of its
 // buffer, dQ_i in the upper half. Head dim 128 (S, dP, dV, dK take all 512 columns): one S buffer, dQ_i over dP_i.
 // The compute warps' fixed work is 16 K exponentials a pair (1024 clocks of the MUFU unit). No single path bounds the kernel
-// (head dim 64, 523 us: without the reads of lse and delta 490, without those, exponentials, stores of dS and reduce-adds 408):
-// what remains is the chain dS_i -> dK_i -> dP_{i+1} -> dS_{i+1} with its barriers, about 2700 clocks a pair, with two compute
-// warps per scheduler to fill it. Four of them with 32 columns each measured the same (head dim 64) or slower (128: 80
+// (head dim 64, 523 us in that run: without the reads of lse and delta 490, without those, exponentials, stores of dS and reduce-adds 408):
+// what remains is the chain dS_i -> dK_i -> dP_{i+1} -> dS_{i+1} with its barriers (3270 clocks a pair in all, the tensor pipe busy for 1360),
+// with two compute warps per scheduler to fill it. Four of them with 32 columns each measured the same (head dim 64) or slower (128: 80
 // registers a thread; 800 against 710 us).
 // All three kernels of a backward pass, B200, queries as rows and one S / dP buffer / now: 8 x 2048, 32/4 heads of 64
 // 638 / 521 us; 2 x 4000, 32/8 of 128 1191 / 710; 1 x 777, 14/2 of 64 122 / 33 with shared heads. The rotation of dK in the epilogue instead of a
 // launch behind it: 2 x 256, 8/2 of 64 21.0 / 16.0 us, 1 x 777, 14/2 34.2 / 32.0, large ones 4 to 10 us.
 // Few key blocks (short sequences, few kv heads) leave SMs idle while each CTA walks all query heads of its group: then a
 // cluster of up to 8 CTAs may share the heads, and the partial dK / dV meet through distributed shared memory, added in the
-// order of the CTAs' ranks (`head_split` below; results repeat bit for bit). The caller has to allow it: under the reference
+// order of the CTAs' ranks (`head_split` below; results repeat bit for bit). dK and dV are as far from fp64 either way (2.3 - 3.0e-3,
+// their rounding to bf16; within 0.05 % of each other). The caller has to allow it: under the reference
 // loss, whose value after the next update turned the other last bits into up to 0.8 % (777 tokens), the order stays.
 #include "../common/ptx.cuh"
 #include "../common/host.cuh"

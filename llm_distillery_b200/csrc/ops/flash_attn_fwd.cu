@@ -487,8 +487,9 @@ extern "C" int b200_flash_attn_fwd(const void* qkv, void* out, float* lse, int B
 
 // Chunked prefill against a key / value cache. qkv [B*L, (H + 2*Hkv)*D]: this chunk's projections (its K / V columns
 // are NOT read: the caller has copied them into the caches first). k_cache, v_cache [B, cache_rows, Hkv*D] bf16 with
-// row p = sequence position p, valid (and finite: allocate the caches zeroed) for p < q_off + L. The chunk's queries
-// are positions q_off .. q_off + L - 1 and see keys <= their own position. out [B*L, H*D], lse [H, B*L] (may be null).
+// row p = sequence position p, valid for p < q_off + L and finite up to the next multiple of 64 or the cache's end (whole tiles
+// are loaded, and a masked key times a NaN is NaN: b200_kv_append zeroes those rows). The chunk's queries are positions
+// q_off .. q_off + L - 1 and see keys <= their own position. out [B*L, H*D], lse [H, B*L] (may be null).
 extern "C" int b200_flash_attn_fwd_cached(const void* qkv, const void* k_cache, const void* v_cache, long long cache_rows,
                                           void* out, float* lse, int B, int L, int q_off, int window, int H, int Hkv,
                                           int D, cudaStream_t st) {

@@ -30,9 +30,12 @@ _lib.register("b200_reference_loss_grad", [_VP] * 11 + [_LL, _I, _I, _F, _VP])
 _lib.KERNELS_PER_CALL["b200_reference_loss"] = 2
 
 KIND_CODES = {"kl": 0, "rkl": 1, "jsd": 2, "jsd_renorm": 3, "none": 4}
-# The kernels of the reference loss add in another order than the library's reductions. Through the optimizer's first steps,
-# whose updates hardly depend on the size of a gradient, the next step's loss then differs: by up to 0.44 % over 12 batches of
-# 720 rows, by up to 0.05 % over 4 of 7000. Fewer rows keep the library's order.
+# The kernels of the reference loss add in another order than the library's reductions. Neither is nearer to fp64: gradients of 722
+# to 7000 rows are off by 0.7e-7 to 6.7e-7 here and by 1.1e-7 to 4.9e-7 there, most of it in the one row at a conversation's
+# maximum. But through the optimizer's first steps, whose updates hardly depend on the size of a gradient, other last bits become
+# another next loss: by up to 0.44 % over 8 batches of 751 rows, 0.12 % over 5 of 1492, 0.11 % of 2831, 0.06 % of 4385. So below
+# this line batches keep the library's order and with it the losses of earlier runs, for the price of about 250 launches (1.4 ms of
+# a step of 751 rows); four batches of about 7000 rows take 183.2 ms there, 180.0 here.
 NATIVE_REFERENCE_ROWS = 4096
 DZ_CHUNK_BYTES = 2 << 30  # bf16 dlogits materialised per backward chunk
 

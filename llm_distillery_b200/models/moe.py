@@ -9,7 +9,7 @@ experts is two autograd nodes with explicit backward: ``AttnBlockFn`` (the atten
 the experts' two GEMMs as one launch over all experts' slabs of rows (SwiGLU in the epilogue of the first; a launch per
 expert for sizes and types that it does not take), and combines by GATHERING each token's k results - a fixed order of
 additions, no atomic scatter. Routing arithmetic ([T, E] tensors) is PyTorch in fp32. The number of rows per expert stays on
-the device in inference; a forward pass that a backward pass follows reads it back once per layer (the shapes of the weight
+the device in inference (within the sizes of ``sorted_pairs``' kernel; the library's histogram waits for the device); a forward pass that a backward pass follows reads it back once per layer (the shapes of the weight
 gradients' GEMMs depend on it).
 No GEMM here cuts K (``basic.gemm``'s split_k), in inference either: behind a router a last bit can be another expert, and
 an expert's row count, which the cut would depend on, changes with every batch.
@@ -48,17 +48,12 @@ def route(n2: torch.Tensor, w_router: torch.Tensor, k: int, renorm: bool = True)
     return probs, top_e, (top_p / top_p.sum(-1, keepdim=True) if renorm else top_p)
 
 
-def permutation(top_e: torch.Tensor, n_experts: int):
+def sorted_pairs(top_e: torch.Tensor, n_experts: int):
     """(order, inverse, token, counts): ``order`` lists the T*k (token, choice) pairs sorted by expert (stable, so tokens
     keep their order inside an expert's slab), ``inverse`` undoes it, ``token`` is the token of each sorted pair,
-    ``counts`` are the slab lengths as Python ints. Two launches on a GPU (csrc/ops/moe.cu) for up to 32 experts and
-    ``SORT_MAX_PAIRS`` pairs; beyond them, and for indices that are not int64, the library's sort."""
-    order, inverse, token, counts = _sorted_pairs(top_e, n_experts)
-    return order, inverse, token, counts.tolist()
-
-
-def _sorted_pairs(top_e: torch.Tensor, n_experts: int):
-    """``permutation`` with the counts left where they are (int64 [n_experts])."""
+    ``counts`` are the slab lengths (int64 [n_experts], on the device of ``top_e``). Two launches on a GPU (csrc/ops/moe.cu) for
+    up to 32 experts and ``SORT_MAX_PAIRS`` pairs; beyond them, and for indices that are not int64, the library's sort, whose
+    histogram waits for the device."""
     flat = top_e.reshape(-1)
     k = top_e.shape[1]
     if (flat.is_cuda and flat.dtype == torch.int64 and flat.is_contiguous() and n_experts <= 32
@@ -162,7 +157,7 @@ def moe_mlp(n2: torch.Tensor, w_router: torch.Tensor, w_gu: torch.Tensor, w_d: t
     down matrix, gate vector) of a shared expert, or None."""
     T, h = n2.shape
     _, top_e, top_w = route(n2, w_router, k, renorm)
-    _, inverse, tok, counts = _sorted_pairs(top_e, w_gu.shape[0])
+    _, inverse, tok, counts = sorted_pairs(top_e, w_gu.shape[0])
     _, _, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d)
     if shared is None:
         out = combine(y, inverse, top_w, None)
@@ -301,7 +296,7 @@ class MoEBlockFn(torch.autograd.Function):
         T, hdim = h1.shape
         n2, _, rstd2 = basic.rmsnorm_fwd(h1, w_ln2, eps)
         probs, top_e, top_w = route(n2, w_router, k, renorm)
-        order, inverse, tok, counts = _sorted_pairs(top_e, w_gu.shape[0])
+        order, inverse, tok, counts = sorted_pairs(top_e, w_gu.shape[0])
         ctx.device_counts = counts
         ctx.counts = counts.tolist() if any(ctx.needs_input_grad) else None      # only the backward pass reads them
         gu, act, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d, ctx.counts)
