@@ -12,22 +12,6 @@ namespace ew {
 constexpr int NT = 256;
 constexpr int MAX_VEC = 4;  // 16-byte vectors cached per thread: rows up to NT*MAX_VEC*8 = 8192 elements
 
-template <int NTB = NT>
-__device__ __forceinline__ float block_sum(float v, float* red) {
-  v = warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  float t = (threadIdx.x < (NTB / 32)) ? red[threadIdx.x] : 0.f;
-  if (w == 0) {
-    t = warp_sum(t);
-    if (l == 0) red[0] = t;
-  }
-  __syncthreads();
-  return red[0];
-}
-
 __device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
@@ -46,9 +30,38 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return o;
 }
 
+// Sums of R values over a block of NTB threads, with one barrier: `red` holds two rounds in turn, so a fast warp's next round
+// does not meet a slow warp's reads of this one. The order of the additions is that of a butterfly over each warp and then
+// over the warps, whatever R is.
+template <int NTB, int R>
+__device__ __forceinline__ void block_sums(float (&v)[R], float (*red)[NTB / 32][R], int round) {
+  constexpr int NW = NTB / 32;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < R; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  float(*r)[R] = red[round & 1];
+  if (l == 0)
+#pragma unroll
+    for (int k = 0; k < R; ++k) r[w][k] = v[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    float t[NW];
+#pragma unroll
+    for (int i = 0; i < NW; ++i) t[i] = r[i][k];
+#pragma unroll
+    for (int o = NW / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < o; ++i) t[i] += t[i + o];
+    v[k] = t[0];
+  }
+}
+
 // y = rmsnorm(x (+ res)) * w ; if res != null also writes h = x + res to `hout`. rstd[row] saved for backward.
-// One block of NTB threads per row, NV vectors of 8 per thread (rows up to NV * NTB * 8 elements).
-template <int NV, int NTB>
+// One block of NTB threads takes R rows at a time, NV vectors of 8 per thread and row (rows up to NV * NTB * 8 elements).
+template <int NV, int NTB, int R>
 __global__ void __launch_bounds__(NTB) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                         const __nv_bfloat16* __restrict__ res,
                                                         const __nv_bfloat16* __restrict__ w,
@@ -56,46 +69,65 @@ __global__ void __launch_bounds__(NTB) rmsnorm_fwd_kernel(const __nv_bfloat16* _
                                                         float* __restrict__ rstd, int rows, int h, float eps) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float red[NTB / 32];
+  __shared__ float red[2][NTB / 32][R];
   const int nvec = h >> 3;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * h);
-    const uint4* rr = res ? reinterpret_cast<const uint4*>(res + (size_t)row * h) : nullptr;
-    float vals[NV][8];
-    float ss = 0.f;
+  int round = 0;
+  for (int row0 = blockIdx.x * R; row0 < rows; row0 += gridDim.x * R, ++round) {
+    uint4 q[R][NV];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int v = threadIdx.x + i * NTB;
-      if (v < nvec) {
-        unpack8(xr[v], vals[i]);
-        if (rr) {
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int v = threadIdx.x + i * NTB;
+        q[k][i] = (v < nvec && row0 + k < rows) ? reinterpret_cast<const uint4*>(x + (size_t)(row0 + k) * h)[v]
+                                                : make_uint4(0u, 0u, 0u, 0u);
+      }
+    float ss[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      ss[k] = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int v = threadIdx.x + i * NTB;
+        float a[8];
+        unpack8(q[k][i], a);
+        if (res && v < nvec && row0 + k < rows) {
           float r8[8];
-          unpack8(rr[v], r8);
+          unpack8(reinterpret_cast<const uint4*>(res + (size_t)(row0 + k) * h)[v], r8);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) vals[i][j] += r8[j];
-          if (hout) {
-            // the residual stream is stored in bf16: normalise what is stored, not the fp32 sum
-            uint4 hq = pack8(vals[i]);
-            reinterpret_cast<uint4*>(hout + (size_t)row * h)[v] = hq;
-            unpack8(hq, vals[i]);
-          }
+          for (int j = 0; j < 8; ++j) a[j] += r8[j];
+          // the residual stream is stored in bf16: normalise what is stored, not the fp32 sum
+          q[k][i] = pack8(a);
+          if (hout) reinterpret_cast<uint4*>(hout + (size_t)(row0 + k) * h)[v] = q[k][i];
+          unpack8(q[k][i], a);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss += vals[i][j] * vals[i][j];
+        for (int j = 0; j < 8; ++j) ss[k] = __fmaf_rn(a[j], a[j], ss[k]);
       }
     }
-    const float tot = block_sum<NTB>(ss, red);
-    const float rs = rsqrtf(tot / (float)h + eps);
-    if (threadIdx.x == 0 && rstd) rstd[row] = rs;
+    block_sums<NTB, R>(ss, red, round);
+    uint4 wq[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * NTB;
-      if (v < nvec) {
-        float w8[8], o[8];
-        unpack8(reinterpret_cast<const uint4*>(w)[v], w8);
+      if (v < nvec) wq[i] = reinterpret_cast<const uint4*>(w)[v];
+    }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = vals[i][j] * rs * w8[j];
-        reinterpret_cast<uint4*>(y + (size_t)row * h)[v] = pack8(o);
+    for (int k = 0; k < R; ++k) {
+      if (row0 + k >= rows) break;
+      const float rs = rsqrtf(ss[k] / (float)h + eps);
+      if (threadIdx.x == 0 && rstd) rstd[row0 + k] = rs;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int v = threadIdx.x + i * NTB;
+        if (v < nvec) {
+          float a[8], w8[8], o[8];
+          unpack8(q[k][i], a);
+          unpack8(wq[i], w8);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = a[j] * rs * w8[j];
+          reinterpret_cast<uint4*>(y + (size_t)(row0 + k) * h)[v] = pack8(o);
+        }
       }
     }
   }
@@ -167,10 +199,20 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_warp_kernel(const __nv_bfloat
   }
 }
 
-// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres) ; dw partial sums per block in fp32.
-// NV and NTB as in the forward kernel: with arrays for the longest row (NV = 4) a thread held 157 registers and an SM one
-// block, 8000 rows of 4096 took 210 us; sized for the row (NV = 2) several blocks share it.
-template <int NV, int NTB>
+// 16-byte copies into shared memory that run behind the arithmetic, and the wait for all but the last N groups of them.
+__device__ __forceinline__ void copy16_async(uint32_t dst, const uint4* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres) ; dw partial sums per block in fp32, each thread's in its registers.
+// R rows at a time, as in the forward kernel. STAGES > 0: the rows come through a ring of that many rounds in shared memory;
+// a thread copies and reads its own 16-byte pieces only, so the ring needs no barrier.
+template <int NV, int NTB, int R, int STAGES>
 __global__ void __launch_bounds__(NTB) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                         const __nv_bfloat16* __restrict__ x,
                                                         const __nv_bfloat16* __restrict__ w,
@@ -180,55 +222,106 @@ __global__ void __launch_bounds__(NTB) rmsnorm_bwd_kernel(const __nv_bfloat16* _
                                                         int rows, int h) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float red[NTB / 32];
+  __shared__ float red[2][NTB / 32][R];
+  extern __shared__ uint4 ring[];                    // [STAGES][R][NV][x, dy, dres][NTB]
   const int nvec = h >> 3;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   float dwacc[NV][8];
-  float w8[NV][8];
+  uint4 wq[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int v = threadIdx.x + i * NTB;
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
-    if (v < nvec) unpack8(reinterpret_cast<const uint4*>(w)[v], w8[i]);
+    wq[i] = v < nvec ? reinterpret_cast<const uint4*>(w)[v] : zero;
   }
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const float rs = rstd[row];
-    float xh[NV][8], g[NV][8];
-    float dot = 0.f;
+  const int step = gridDim.x * R;
+  auto slot = [&](int stage, int k, int i, int which) { return (((stage * R + k) * NV + i) * 3 + which) * NTB + (int)threadIdx.x; };
+  auto fetch = [&](int stage, int row0) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int v = threadIdx.x + i * NTB;
-      if (v < nvec) {
-        float d8[8];
-        unpack8(reinterpret_cast<const uint4*>(x + (size_t)row * h)[v], xh[i]);
-        unpack8(reinterpret_cast<const uint4*>(dy + (size_t)row * h)[v], d8);
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int v = threadIdx.x + i * NTB;
+        if (v < nvec && row0 + k < rows) {
+          const size_t at = (size_t)(row0 + k) * h;
+          copy16_async(smem_u32(ring + slot(stage, k, i, 0)), reinterpret_cast<const uint4*>(x + at) + v);
+          copy16_async(smem_u32(ring + slot(stage, k, i, 1)), reinterpret_cast<const uint4*>(dy + at) + v);
+          if (dres) copy16_async(smem_u32(ring + slot(stage, k, i, 2)), reinterpret_cast<const uint4*>(dres + at) + v);
+        }
+      }
+    copy_commit();
+  };
+  const int first = blockIdx.x * R;
+#pragma unroll
+  for (int s = 0; s < STAGES; ++s) fetch(s, first + s * step);
+  int round = 0, stage = 0;
+  for (int row0 = first; row0 < rows; row0 += step, ++round) {
+    uint4 xq[R][NV], dq[R][NV], rq[R][NV];
+    float rs[R], dot[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) rs[k] = row0 + k < rows ? rstd[row0 + k] : 0.f;
+    if constexpr (STAGES > 0) copy_wait<STAGES - 1>();
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int v = threadIdx.x + i * NTB;
+        const bool ok = v < nvec && row0 + k < rows;
+        if constexpr (STAGES > 0) {
+          xq[k][i] = ok ? ring[slot(stage, k, i, 0)] : zero;
+          dq[k][i] = ok ? ring[slot(stage, k, i, 1)] : zero;
+          rq[k][i] = ok && dres ? ring[slot(stage, k, i, 2)] : zero;
+        } else {
+          const size_t at = (size_t)(row0 + k) * h;
+          xq[k][i] = ok ? reinterpret_cast<const uint4*>(x + at)[v] : zero;
+          dq[k][i] = ok ? reinterpret_cast<const uint4*>(dy + at)[v] : zero;
+          rq[k][i] = ok && dres ? reinterpret_cast<const uint4*>(dres + at)[v] : zero;
+        }
+      }
+    if constexpr (STAGES > 0) {
+      fetch(stage, row0 + STAGES * step);
+      stage = stage + 1 == STAGES ? 0 : stage + 1;
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      dot[k] = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        float xf[8], df[8], wf[8];
+        unpack8(xq[k][i], xf);
+        unpack8(dq[k][i], df);
+        unpack8(wq[i], wf);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          xh[i][j] *= rs;
-          dwacc[i][j] += d8[j] * xh[i][j];
-          g[i][j] = d8[j] * w8[i][j];
-          dot += g[i][j] * xh[i][j];
+          const float xh = xf[j] * rs[k];
+          dwacc[i][j] = __fmaf_rn(df[j], xh, dwacc[i][j]);
+          dot[k] = __fmaf_rn(df[j] * wf[j], xh, dot[k]);
         }
       }
     }
-    const float c = block_sum<NTB>(dot, red) / (float)h;
+    block_sums<NTB, R>(dot, red, round);
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int v = threadIdx.x + i * NTB;
-      if (v < nvec) {
-        float o[8];
+    for (int k = 0; k < R; ++k) {
+      if (row0 + k >= rows) break;
+      const float c = dot[k] / (float)h;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = __fmaf_rn(-xh[i][j], c, g[i][j]);
-        if (dres) {         // fused multiply-adds by name: every instantiation rounds alike
-          float r8[8];
-          unpack8(reinterpret_cast<const uint4*>(dres + (size_t)row * h)[v], r8);
+      for (int i = 0; i < NV; ++i) {
+        const int v = threadIdx.x + i * NTB;
+        if (v < nvec) {
+          float xf[8], df[8], wf[8], r8[8], o[8];
+          unpack8(xq[k][i], xf);
+          unpack8(dq[k][i], df);
+          unpack8(wq[i], wf);
+          unpack8(rq[k][i], r8);
+          // fused multiply-adds by name: every instantiation rounds alike
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = __fmaf_rn(rs, o[j], r8[j]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] *= rs;
+          for (int j = 0; j < 8; ++j) {
+            const float t = __fmaf_rn(-(xf[j] * rs[k]), c, df[j] * wf[j]);
+            o[j] = dres ? __fmaf_rn(rs[k], t, r8[j]) : rs[k] * t;
+          }
+          reinterpret_cast<uint4*>(dx + (size_t)(row0 + k) * h)[v] = pack8(o);
         }
-        reinterpret_cast<uint4*>(dx + (size_t)row * h)[v] = pack8(o);
       }
     }
   }
@@ -795,16 +888,39 @@ static inline int grid_for(long long work_items, int threads, int per_sm = 8) {
 }  // namespace ew
 }  // namespace b200
 
-// The block-per-row kernels in the size that holds a row of h elements (h <= NT * MAX_VEC * 8): half a block for rows
+// The block kernels in the size that holds a row of h elements (h <= NT * MAX_VEC * 8): half a block for rows
 // that half a block covers, else as many vectors per thread as the row needs. The sums do not depend on it.
-#define B200_RMS_BY_WIDTH(KERNEL, h, grid, st, ...)                                        \
-  do {                                                                                     \
-    if ((h) <= NT / 2 * 8) launch_pdl(KERNEL<1, NT / 2>, grid, NT / 2, 0, st, __VA_ARGS__); \
-    else if ((h) <= NT * 8) launch_pdl(KERNEL<1, NT>, grid, NT, 0, st, __VA_ARGS__);       \
-    else if ((h) <= NT * 16) launch_pdl(KERNEL<2, NT>, grid, NT, 0, st, __VA_ARGS__);      \
-    else if ((h) <= NT * 24) launch_pdl(KERNEL<3, NT>, grid, NT, 0, st, __VA_ARGS__);      \
-    else launch_pdl(KERNEL<MAX_VEC, NT>, grid, NT, 0, st, __VA_ARGS__);                    \
+#define B200_RMS_BY_WIDTH(GO, h)            \
+  do {                                      \
+    if ((h) <= NT / 2 * 8) GO(1, NT / 2);   \
+    else if ((h) <= NT * 8) GO(1, NT);      \
+    else if ((h) <= NT * 16) GO(2, NT);     \
+    else if ((h) <= NT * 24) GO(3, NT);     \
+    else GO(MAX_VEC, NT);                   \
   } while (0)
+
+namespace b200 {
+namespace ew {
+
+// Launch of the backward kernel over `grid` blocks.
+template <int NV, int NTB, int R, int STAGES>
+static int launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
+                              float* dw_partial, int rows, int h, int grid, cudaStream_t st) {
+  auto kern = rmsnorm_bwd_kernel<NV, NTB, R, STAGES>;
+  constexpr int smem = STAGES * R * NV * 3 * 16 * NTB;
+  static bool attr_set = false;
+  if (smem > 48 * 1024 && !attr_set) {
+    B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    attr_set = true;
+  }
+  launch_pdl(kern, grid, NTB, smem, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
+             (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, rows, h);
+  B200_CUDA_CHECK(cudaGetLastError());
+  return B200_OK;
+}
+
+}  // namespace ew
+}  // namespace b200
 
 extern "C" {
 using namespace b200;
@@ -819,7 +935,6 @@ int b200_rmsnorm_bwd_blocks(int rows) {
 int b200_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* hout, float* rstd, int rows, int h,
                      float eps, cudaStream_t st) {
   if (!x || !w || !y || rows <= 0 || (h & 7) || h > NT * MAX_VEC * 8) return B200_ERR_ARG;
-  const int grid = rows < sm_count() * 8 ? rows : sm_count() * 8;
   const int wblocks = ceil_div(rows, 4) < sm_count() * 5 ? ceil_div(rows, 4) : sm_count() * 5;  // 4 rows per 128-thread CTA
 #define B200_RMS_FWD_WARP(VPL)                                                                                        \
   launch_pdl(rmsnorm_fwd_warp_kernel<VPL>, wblocks, 128, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,            \
@@ -829,9 +944,23 @@ int b200_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, voi
   else if (h == 1024) B200_RMS_FWD_WARP(4);
   else if (h == 512) B200_RMS_FWD_WARP(2);
   else if (h == 256) B200_RMS_FWD_WARP(1);
-  else
-    B200_RMS_BY_WIDTH(rmsnorm_fwd_kernel, h, grid, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,
-                      (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)hout, rstd, rows, h, eps);
+  else {
+    // Two rows at a time where a thread has several vectors of each and there are many rows: 8000 x 4096 35.3 us (one row,
+    // three barriers) / 25.5 (one row, one barrier) / 23.2, 5.65 TB/s; 2048 x 4096 10.1 / 7.7 / 7.8. With one vector a thread
+    // more blocks on an SM do as well (12000 x 1536: 18.1 / 20.4).
+    const bool two = h > NT * 8 && rows >= 4096;
+    const int blocks = two ? ceil_div(rows, 2) : rows, cap = sm_count() * (two ? 4 : 8), grid = blocks < cap ? blocks : cap;
+#define B200_RMS_FWD(NV, NTB, R)                                                                                      \
+  launch_pdl(rmsnorm_fwd_kernel<NV, NTB, R>, grid, NTB, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,    \
+             (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)hout, rstd, rows, h, eps)
+#define B200_RMS_FWD_ONE(NV, NTB) B200_RMS_FWD(NV, NTB, 1)
+#define B200_RMS_FWD_TWO(NV, NTB) B200_RMS_FWD(NV, NTB, (NV > 1 ? 2 : 1))
+    if (two) B200_RMS_BY_WIDTH(B200_RMS_FWD_TWO, h);
+    else B200_RMS_BY_WIDTH(B200_RMS_FWD_ONE, h);
+#undef B200_RMS_FWD_TWO
+#undef B200_RMS_FWD_ONE
+#undef B200_RMS_FWD
+  }
 #undef B200_RMS_FWD_WARP
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -842,23 +971,42 @@ int b200_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* 
                      float* dw_partial, float* dw_out, int dw_accumulate, int rows, int h, cudaStream_t st) {
   if (!dy || !x || !w || !rstd || !dx || !dw_partial || !dw_out || rows <= 0 || (h & 7) || h > NT * MAX_VEC * 8)
     return B200_ERR_ARG;
-  const int grid = b200_rmsnorm_bwd_blocks(rows);  // partial rows: one per block, or one per warp in the warp kernels
+  int grid = b200_rmsnorm_bwd_blocks(rows);  // partial rows: one per block of the block kernels
+  int rc = B200_OK;
+#define B200_RMS_BWD(NV, NTB, R, STAGES) \
+  rc = launch_rmsnorm_bwd<NV, NTB, R, STAGES>(dy, x, w, rstd, dres, dx, dw_partial, rows, h, grid, st)
+#define B200_RMS_BWD_PLAIN(NV, NTB) B200_RMS_BWD(NV, NTB, 1, 0)
+#define B200_RMS_BWD_RING(NV, NTB) B200_RMS_BWD(NV, NTB, (NV > 1 ? 1 : 2), 3)
 #define B200_RMS_BWD_WARP(VPL)                                                                                       \
-  launch_pdl(rmsnorm_bwd_warp_kernel<VPL>, ceil_div(grid, 4), 128, 4 * (VPL) * 256 * 4, st,                                                    \
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,   \
-      (__nv_bfloat16*)dx, dw_partial, rows, grid)
-  if (h == 2048) B200_RMS_BWD_WARP(8);
-  else if (h == 1024) B200_RMS_BWD_WARP(4);
-  else if (h == 512) B200_RMS_BWD_WARP(2);
-  else if (h == 256) B200_RMS_BWD_WARP(1);
-  else
-    B200_RMS_BY_WIDTH(rmsnorm_bwd_kernel, h, grid, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
-                      (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, rows, h);
+  grid = ceil_div(grid, 4);              /* four rows, and one partial row, per CTA */                               \
+  launch_pdl(rmsnorm_bwd_warp_kernel<VPL>, grid, 128, 4 * (VPL) * 256 * 4, st,                                       \
+      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,  \
+      (__nv_bfloat16*)dx, dw_partial, rows, b200_rmsnorm_bwd_blocks(rows))
+  // The ring from 2048 rows on, where HBM is the bound, for rows that keep a block's threads busy and fit its ring. All times
+  // with the column sum, the kernels before / the ring: 16384 x 2048 68.3 / 46.9 us (5.73 TB/s), 7572 x 2048 39.6 / 26.7,
+  // 8000 x 4096 110 / 44.6, 2048 x 4096 38.7 / 17.0, 12000 x 1536 55.0 / 30.8, 4000 x 896 16.4 / 12.8. Fewer rows are a chain of
+  // latencies either way (777 x 896: 6.8 / 6.5) and keep the order of the additions into dw.
+  if (rows >= 2048 && h > 512 && h <= NT * 16) {
+    const int per_sm = h > NT * 8 ? 2 : 3;
+    const int blocks = h > NT * 8 ? rows : ceil_div(rows, 2);
+    grid = blocks < sm_count() * per_sm ? blocks : sm_count() * per_sm;
+    if (h <= NT / 2 * 8) B200_RMS_BWD_RING(1, NT / 2);
+    else if (h <= NT * 8) B200_RMS_BWD_RING(1, NT);
+    else B200_RMS_BWD_RING(2, NT);
+  } else if (h == 2048) { B200_RMS_BWD_WARP(8);
+  } else if (h == 1024) { B200_RMS_BWD_WARP(4);
+  } else if (h == 512) { B200_RMS_BWD_WARP(2);
+  } else if (h == 256) { B200_RMS_BWD_WARP(1);
+  } else {
+    B200_RMS_BY_WIDTH(B200_RMS_BWD_PLAIN, h);
+  }
 #undef B200_RMS_BWD_WARP
+#undef B200_RMS_BWD_RING
+#undef B200_RMS_BWD_PLAIN
+#undef B200_RMS_BWD
+  if (rc != B200_OK) return rc;
   B200_CUDA_CHECK(cudaGetLastError());
-  const bool warp_kernel = h == 2048 || h == 1024 || h == 512 || h == 256;    // one partial row per 4-warp CTA there
-  launch_pdl(colsum_kernel, ceil_div(h, 32), COLSUM_THREADS, 0, st, dw_partial, dw_out, warp_kernel ? ceil_div(grid, 4) : grid, h,
-                                                 dw_accumulate);
+  launch_pdl(colsum_kernel, ceil_div(h, 32), COLSUM_THREADS, 0, st, dw_partial, dw_out, grid, h, dw_accumulate);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -1080,9 +1228,12 @@ extern "C" int b200_rmsnorm_bwd_noalloc(const void* dy, const void* x, const voi
   const int grid = rows < B200_RMSNORM_NOALLOC_MAX_BLOCKS ? rows : B200_RMSNORM_NOALLOC_MAX_BLOCKS;
   // every block writes its own partial row (all h columns) before the column sum reads rows [0, grid):
   // nothing left over from an earlier call is ever read
-  B200_RMS_BY_WIDTH(rmsnorm_bwd_kernel, h, grid, st, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
-                    (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, h);
-  B200_CUDA_CHECK(cudaGetLastError());
+  int launched = B200_OK;
+#define B200_RMS_BWD_PLAIN(NV, NTB) \
+  launched = launch_rmsnorm_bwd<NV, NTB, 1, 0>(dy, x, w, rstd, dres, dx, scratch, rows, h, grid, st)
+  B200_RMS_BY_WIDTH(B200_RMS_BWD_PLAIN, h);
+#undef B200_RMS_BWD_PLAIN
+  if (launched != B200_OK) return launched;
   launch_pdl(colsum_kernel, ceil_div(h, 32), COLSUM_THREADS, 0, st, scratch, dw_out, grid, h, dw_accumulate);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;

@@ -177,6 +177,39 @@ def test_rmsnorm_row_widths_of_the_block_kernels(h):
     assert torch.allclose(dw, wf.grad, atol=1e-3 * rows ** 0.5, rtol=1e-4)
 
 
+@pytest.mark.parametrize("rows,h", [(2047, 1032), (2048, 520), (2049, 1024), (2051, 1032), (2048, 2048), (2049, 2056),
+                                    (2500, 4096), (2048, 4104), (4095, 4096), (4097, 2056), (4099, 6152), (4096, 8192)])
+def test_rmsnorm_of_many_rows(rows, h):
+    """Both sides of the row counts at which blocks take several rows at a time or bring them through a ring in shared memory,
+    with and without a residual, against fp32 (bounds as above; the weight gradient a sum of `rows` fp32 terms). The block
+    kernels add a row's terms in one order: its values do not depend on how many rows there are."""
+    gen = torch.Generator("cuda").manual_seed(rows + h)
+    x, dy, dres = (torch.randn(rows, h, device=DEV, generator=gen).bfloat16() for _ in range(3))
+    w = (1 + 0.1 * torch.randn(h, device=DEV, generator=gen)).bfloat16()
+    y, _, rstd = basic.rmsnorm_fwd(x, w, 1e-5)
+    ys, hs, _ = basic.rmsnorm_fwd(x, w, 1e-5, dres)
+    assert torch.equal(hs, (x.float() + dres.float()).bfloat16())
+    assert torch.equal(ys, basic.rmsnorm_fwd(hs, w, 1e-5)[0])
+    xf, wf = x.float().requires_grad_(), w.float().requires_grad_()
+    ref = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-5) * wf
+    ref.backward(dy.float())
+    assert torch.allclose(y.float(), ref, atol=1e-4, rtol=2 ** -8)
+    xh = (x.double() * rstd.double()[:, None])
+    terms = dy.double() * xh
+    for res in (None, dres):
+        dw = torch.full((h,), 3.0, device=DEV)
+        dx, _ = basic.rmsnorm_bwd(dy, x, w, rstd, dres=res, dw_out=dw, dw_accumulate=True)
+        want = xf.grad + (res.float() if res is not None else 0)
+        assert torch.allclose(dx.float(), want, atol=1e-3, rtol=2 ** -7)
+        assert ((dw - 3.0 - terms.sum(0)).abs() <= (rows + 4) * 2 ** -24 * terms.abs().sum(0) + 1e-5).all()
+        if h not in (256, 512, 1024, 2048):
+            few, _ = basic.rmsnorm_bwd(dy[-37:].contiguous(), x[-37:].contiguous(), w, rstd[-37:].contiguous(),
+                                       dres=res if res is None else res[-37:].contiguous())
+            assert torch.equal(dx[-37:], few)
+    assert torch.equal(y[-37:], basic.rmsnorm_fwd(x[-37:].contiguous(), w, 1e-5)[0])
+    assert _lib.take_device_error() == 0
+
+
 @pytest.mark.parametrize("T", [1, 127, 129, 777, 2048, 2049])
 @pytest.mark.parametrize("N,ld", [(8, 8), (72, 80), (1152, 1152)])
 def test_bias_gradient_of_few_and_many_rows(T, N, ld):
