@@ -95,8 +95,7 @@ class TeacherCollector:
             else:
                 lg.copy_(Hc[r0:r1].float() @ W.float().t())
             if self.enable_topk:
-                v, i = topk_ops.topk_logprob(lg, self.vocab, self.K)
-                out_v[r0:r1], out_i[r0:r1] = v, i
+                topk_ops.topk_logprob(lg, self.vocab, self.K, out=(out_v[r0:r1], out_i[r0:r1]))
             else:
                 out_v[r0:r1] = topk_ops.logprob_full(lg, self.vocab)
         return self._to_host(out_v, out_i, counts)

@@ -1,16 +1,22 @@
 // Exact per-row top-K of log_softmax(logits[:, :V]) for teacher collection, and the multi-teacher top-K merge.
 //
-// topk_logprob: one CTA per row over fp32 logits (the row chunk just written by the LM-head GEMM, L2 resident):
-//   1. one read: max, sum-exp -> lse, and a histogram of the upper 11 bits of the order-preserving keys
-//   2. second read: everything above the K-th element's bin is selected, the bin itself becomes a candidate list in
-//      shared memory, which three small radix passes narrow to the exact K-th value and the number of ties to keep
-//   3. the lowest-index ties complete the selection
-//   4. bitonic sort in shared memory by (value desc, index asc) - the order torch.topk users expect
-//   5. write fp16 log-probs (value - lse) and int32 ids
+// topk_logprob: one CTA per row over fp32 logits (the row chunk just written by the LM-head GEMM, L2 resident), one read:
+//   1. maxima of groups of 16 elements (4 for short rows or many K), and the log-sum-exp with them. The K-th largest of two
+//      thousand or more maxima bounds the row's K-th largest from below (K elements are no smaller), and closely: of 32000
+//      elements and K = 200 about 220 reach it
+//   2. the groups that reach the bound are read again, and their elements that do become a list in shared memory
+//   3. the list is sorted by (value desc, index asc) - the order torch.topk users expect - in registers, and K of it are
+//      written as fp16 log-probs (value - lse) and int32 ids
+// That is about five instructions an element and leaves the read of the chunk; a histogram of all keys and a second read, with
+// key arithmetic and branches an element, took 73. Before / now, 1024 rows of 32000, K 200: 92 / 45 us (29 of it the read),
+// 4096 rows 315 / 136, 1024 rows K 400 110 / 56, 512 rows of 128 256, K 128 204 / 58, 93 rows 40 / 18.
+// A row whose list overflows (ties, masked or equal entries) or whose sum is no finite number takes `select_by_radix`: a
+// histogram of the upper key bits, radix passes over the bin of the K-th element, then everything above it.
 // Output layout matches the HDF5 datasets: [rows, K] fp16 + [rows, K] int32.
 //
 // topk_merge: per row, union of two top-K lists with probabilities of equal ids summed, best K kept, log stored
 // (the multi-teacher rule of the data store), sorted by value.
+#include <float.h>
 #include "../common/ptx.cuh"
 #include "../common/host.cuh"
 
@@ -42,6 +48,46 @@ __device__ void bitonic_desc(unsigned long long* s, int n) {
         }
       }
       __syncthreads();
+    }
+  }
+}
+
+// Descending sort of NT * E 64-bit keys, E consecutive ones in each thread's registers (key e of thread t: place t * E + e).
+// Exchanges stay in the thread or, over shuffles, in the warp; only those across warps go through `scratch` [NT * E], whose
+// contents have been read by all threads before the call or are of no use. 256 keys: 6 of 36 steps.
+template <int E>
+__device__ __forceinline__ void sort_desc(unsigned long long (&key)[E], unsigned long long* scratch) {
+  const int base = threadIdx.x * E;
+#pragma unroll
+  for (int k = 2; k <= NT * E; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j < E) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          if (e & j) continue;
+          const int f = e ^ j;
+          const unsigned long long a = key[e], b = key[f];
+          const bool swap = (((base + e) & k) == 0) ? a < b : a > b;
+          key[e] = swap ? b : a;
+          key[f] = swap ? a : b;
+        }
+      } else {
+        if (j >= 32 * E) {
+          __syncthreads();
+#pragma unroll
+          for (int e = 0; e < E; ++e) scratch[e * NT + threadIdx.x] = key[e];
+          __syncthreads();
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const unsigned long long a = key[e];
+          const unsigned long long b = j >= 32 * E ? scratch[e * NT + (threadIdx.x ^ (j / E))]
+                                                   : __shfl_xor_sync(0xffffffffu, a, (j / E) & 31);
+          const bool keep_larger = (((base + e) & j) == 0) == (((base + e) & k) == 0);
+          key[e] = (a > b) == keep_larger ? a : b;
+        }
+      }
     }
   }
 }
@@ -101,147 +147,100 @@ __device__ __forceinline__ void for_row(const float* __restrict__ x, int lo, int
 
 constexpr int HB = 11;               // bits of the first histogram: sign, exponent, two bits of the mantissa
 constexpr int NBIN = 1 << HB;        // = NT * 8
-constexpr int CAND_CAP = 1024;       // elements of the threshold bin that are kept in shared memory
-constexpr int SAMPLE = 4096;         // leading elements whose K-th largest bounds the row's K-th largest from below
+static_assert(NBIN == NT * 8, "find_kth_bin<8> covers the first histogram");
 
-// Two reads of the row. Read 1: running (max, sum-exp) per thread and a histogram of the upper 11 key bits; the first
-// 4096 elements go first, and since the K-th largest of a subset is a lower bound of the K-th largest of the row, the
-// rest of the row only enters the histogram from that bin up (a few per cent of it: the shared-memory atomics were
-// the cost of the one-pass histogram). The histogram gives the bin b of the K-th largest element. Read 2: elements of
-// higher bins are selected, those of bin b (typically 100-200) become candidates in shared memory, and three small
-// radix passes over the candidates' remaining 21 key bits give the exact threshold and the number of ties to keep.
-// A bin with more than CAND_CAP elements falls back to radix passes over the row.
-//
-// Vocabulary-shard mode (out_raw != null): the row is one rank's slice of the vocabulary; the kernel writes the raw
-// fp32 logits of the slice's top K, their GLOBAL ids (index + id_offset) and the slice's log-sum-exp, which
-// topk_combine_kernel turns into the exact top-K log-probs of the whole vocabulary.
-__global__ void __launch_bounds__(NT) topk_logprob_kernel(const float* __restrict__ logits, long long ld, int V, int K,
-                                                         __half* __restrict__ out_logp, int* __restrict__ out_idx,
-                                                         float* __restrict__ out_raw, float* __restrict__ out_lse,
-                                                         int id_offset) {
-  static_assert(NBIN == NT * 8, "find_kth_bin<8> covers the first histogram");
-  __shared__ unsigned long long sel[MAX_K];
-  __shared__ unsigned long long cand[CAND_CAP];
-  __shared__ unsigned int hist[NBIN];
-  __shared__ unsigned int ties[TIE_CAP];
-  __shared__ float redm[NT / 32], reds[NT / 32];
-  __shared__ unsigned int redu[NT / 32];
-  __shared__ unsigned int s_bin, s_above, s_inbin, s_nsel, s_ncand, s_nties;
-  __shared__ float s_lse;
-  const long long row = blockIdx.x;
-  const float* x = logits + row * ld;
+// KCAP: the largest K
+template <int KCAP>
+struct TopkSmem {
+  static constexpr int CAP = KCAP + TIE_CAP / 2;     // candidates; the radix selection's K elements and 32-bit ties
+  unsigned long long cand[CAP];
+  union {
+    unsigned int hist[NBIN];
+    unsigned long long kept[NBIN / 2];
+  };
+  float redm[NT / 32], reds[NT / 32];
+  unsigned int redu[NT / 32];
+  unsigned int bin, above, inbin, nsel, ncand, nties;
+  float stat;
+};
+
+__device__ __forceinline__ unsigned long long entry(float v, int i) {
+  return ((unsigned long long)fkey(v) << 32) | (0xffffffffu - (uint32_t)i);
+}
+
+// Leaves the row's K largest in sm.cand[0 .. K-1], in any order, and returns the log-sum-exp (elements that are no number
+// take no part in that). Read 1: running (max, sum-exp) per thread and a histogram of the upper 11 key bits, which gives the
+// bin of the K-th largest element. Read 2: elements of higher bins are selected; three small radix passes over the bin's
+// remaining 21 key bits, reading the row, give the exact threshold and the number of ties to keep, lowest indices first.
+template <int KCAP>
+__device__ __noinline__ float select_by_radix(TopkSmem<KCAP>& sm, const float* __restrict__ x, int V, int K) {
+  unsigned long long* sel = sm.cand;                                          // K entries
+  unsigned int* ties = reinterpret_cast<unsigned int*>(sm.cand + KCAP);       // TIE_CAP entries
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-
-  for (int i = tid; i < NBIN; i += NT) hist[i] = 0;
-  if (tid == 0) { s_nsel = 0; s_ncand = 0; s_nties = 0; }
   __syncthreads();
-
-  // ---- read 1: max, sum-exp, histogram
+  for (int i = tid; i < NBIN; i += NT) sm.hist[i] = 0;
+  if (tid == 0) { sm.nsel = 0; sm.nties = 0; }
+  __syncthreads();
   float m = -INFINITY, sum = 0.f;
-  auto stat = [&](float v) {
+  for_row(x, 0, V, [&](float v, int) {
     if (v > m) { sum *= __expf(m - v); m = v; }
     if (v > -INFINITY) sum += __expf(v - m);
-  };
-  const int n_sample = V >= 4 * SAMPLE ? SAMPLE : 0;
-  unsigned lb_bin = 0;
-  if (n_sample) {
-    for_row(x, 0, n_sample, [&](float v, int) {
-      stat(v);
-      atomicAdd(&hist[fkey(v) >> (32 - HB)], 1u);
-    });
-    __syncthreads();
-    find_kth_bin<8>(hist, (unsigned)K, redu, &s_bin, &s_above, &s_inbin);
-    lb_bin = s_bin;
-    __syncthreads();
-  }
-  for_row(x, n_sample, V, [&](float v, int) {
-    stat(v);
-    const unsigned bin = fkey(v) >> (32 - HB);
-    if (bin >= lb_bin) atomicAdd(&hist[bin], 1u);
+    atomicAdd(&sm.hist[fkey(v) >> (32 - HB)], 1u);
   });
   {
     const float wm = warp_max(m);
     const float part = (m > -INFINITY) ? sum * __expf(m - wm) : 0.f;
     const float ws = warp_sum(part);
-    if (lane == 0) { redm[warp] = wm; reds[warp] = ws; }
+    if (lane == 0) { sm.redm[warp] = wm; sm.reds[warp] = ws; }
   }
   __syncthreads();
   if (tid == 0) {
-    float M = redm[0];
-    for (int w = 1; w < NT / 32; ++w) M = fmaxf(M, redm[w]);
+    float M = sm.redm[0];
+    for (int w = 1; w < NT / 32; ++w) M = fmaxf(M, sm.redm[w]);
     float t = 0.f;
     for (int w = 0; w < NT / 32; ++w)
-      if (redm[w] > -INFINITY) t += reds[w] * __expf(redm[w] - M);
-    s_lse = M + __logf(t);
+      if (sm.redm[w] > -INFINITY) t += sm.reds[w] * __expf(sm.redm[w] - M);
+    sm.stat = M + __logf(t);
   }
-  find_kth_bin<8>(hist, (unsigned)K, redu, &s_bin, &s_above, &s_inbin);
-  const unsigned bstar = s_bin;
-  const unsigned n_inbin = s_inbin;
-  unsigned remaining = (unsigned)K - s_above;       // how many elements of bin bstar belong to the top K (>= 1)
-  const bool in_smem = n_inbin <= (unsigned)CAND_CAP;
-
-  // ---- read 2: higher bins are in; bin bstar becomes the candidate list
-  for_row(x, 0, V, [&](float v, int i) {
-    const uint32_t k = fkey(v);
-    const unsigned bin = k >> (32 - HB);
-    if (bin > bstar) {
-      sel[atomicAdd(&s_nsel, 1u)] = ((unsigned long long)k << 32) | (0xffffffffu - (uint32_t)i);
-    } else if (bin == bstar && in_smem) {
-      cand[atomicAdd(&s_ncand, 1u)] = ((unsigned long long)k << 32) | (0xffffffffu - (uint32_t)i);
-    }
-  });
+  find_kth_bin<8>(sm.hist, (unsigned)K, sm.redu, &sm.bin, &sm.above, &sm.inbin);
+  const unsigned bstar = sm.bin;
+  unsigned remaining = (unsigned)K - sm.above;       // how many elements of bin bstar belong to the top K (>= 1)
   __syncthreads();
-
-  // f(key, index) for every element of bin bstar
-  auto for_bin = [&](auto f) {
-    if (in_smem) {
-      for (unsigned c = tid; c < n_inbin; c += NT) {
-        const unsigned long long e = cand[c];
-        f((uint32_t)(e >> 32), 0xffffffffu - (uint32_t)(e & 0xffffffffu));
-      }
-    } else {
-      for_row(x, 0, V, [&](float v, int i) {
-        const uint32_t k = fkey(v);
-        if ((k >> (32 - HB)) == bstar) f(k, (uint32_t)i);
-      });
-    }
-  };
-
-  // ---- the remaining 21 key bits: 8 + 8 + 5
+  // the remaining 21 key bits: 8 + 8 + 5
   uint32_t prefix = bstar << (32 - HB), mask = 0xffffffffu << (32 - HB);
 #pragma unroll 1
   for (int pass = 0; pass < 3; ++pass) {
     const int shift = pass == 0 ? 13 : (pass == 1 ? 5 : 0);
     const uint32_t digit = pass == 2 ? 0x1fu : 0xffu;
-    hist[tid] = 0;
+    sm.hist[tid] = 0;
     __syncthreads();
-    for_bin([&](uint32_t k, uint32_t) {
-      if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & digit], 1u);
+    for_row(x, 0, V, [&](float v, int) {
+      const uint32_t k = fkey(v);
+      if ((k & mask) == prefix) atomicAdd(&sm.hist[(k >> shift) & digit], 1u);
     });
     __syncthreads();
-    find_kth_bin<1>(hist, remaining, redu, &s_bin, &s_above, &s_inbin);
-    prefix |= s_bin << shift;
+    find_kth_bin<1>(sm.hist, remaining, sm.redu, &sm.bin, &sm.above, &sm.inbin);
+    prefix |= sm.bin << shift;
     mask |= digit << shift;
-    remaining -= s_above;
+    remaining -= sm.above;
     __syncthreads();
   }
   const uint32_t thr = prefix;            // key of the K-th largest element
   const unsigned need_eq = remaining;     // how many elements equal to it belong to the top K
-
-  // ---- gather from bin bstar
-  for_bin([&](uint32_t k, uint32_t i) {
+  for_row(x, 0, V, [&](float v, int i) {
+    const uint32_t k = fkey(v);
     if (k > thr) {
-      sel[atomicAdd(&s_nsel, 1u)] = ((unsigned long long)k << 32) | (0xffffffffu - i);
+      sel[atomicAdd(&sm.nsel, 1u)] = entry(v, i);
     } else if (k == thr) {
-      const unsigned p = atomicAdd(&s_nties, 1u);
-      if (p < TIE_CAP) ties[p] = i;
+      const unsigned p = atomicAdd(&sm.nties, 1u);
+      if (p < TIE_CAP) ties[p] = (unsigned)i;
     }
   });
   __syncthreads();
-  const unsigned ngt = s_nsel;
-  const unsigned nt = s_nties;
+  const unsigned ngt = sm.nsel;
+  const unsigned nt = sm.nties;
   if (nt > TIE_CAP) {
-    // pathological row (more than TIE_CAP equal values at the threshold): ordered sequential pick
+    // more than TIE_CAP equal values at the threshold: ordered sequential pick
     if (tid == 0) {
       unsigned got = 0;
       for (int i = 0; i < V && got < need_eq; ++i)
@@ -257,22 +256,217 @@ __global__ void __launch_bounds__(NT) topk_logprob_kernel(const float* __restric
     }
   }
   __syncthreads();
+  return sm.stat;
+}
 
-  // ---- sort (pad to a power of two with zeros, which sort last) and write
-  int n2 = 1;
-  while (n2 < K) n2 <<= 1;
-  for (int i = K + tid; i < n2; i += NT) sel[i] = 0ull;
-  __syncthreads();
-  bitonic_desc(sel, n2);
-
-  const float lse = s_lse;
-  for (int i = tid; i < K; i += NT) {
-    const unsigned long long e = sel[i];
-    const float z = kfloat((uint32_t)(e >> 32));
+// Sorts sm.cand[0 .. n-1] and writes the K largest of them (K <= n, K <= NT * E). More of them than the sort takes are thinned
+// first: by a histogram over [bound, mx], and inside the bin of the K-th by counting larger entries (no two are equal).
+template <int E, int KCAP>
+__device__ __forceinline__ void sort_and_write(TopkSmem<KCAP>& sm, unsigned n, int K, float lse, float mx, float bound,
+                                               long long row, __half* __restrict__ out_logp, int* __restrict__ out_idx,
+                                               float* __restrict__ out_raw, int id_offset) {
+  static_assert(NT * E <= NBIN / 2 && NT * E <= TopkSmem<KCAP>::CAP, "the list of those kept, and the sort's scratch");
+  const int tid = threadIdx.x;
+  const unsigned long long* from = sm.cand;
+  if (n > (unsigned)(NT * E)) {
+    const float scale = (float)NBIN / (mx - bound);
+    auto bin_of = [&](unsigned long long e) {
+      return (unsigned)min(NBIN - 1, max(0, (int)((kfloat((uint32_t)(e >> 32)) - bound) * scale)));
+    };
+    for (int i = tid; i < NBIN; i += NT) sm.hist[i] = 0;
+    if (tid == 0) sm.nsel = 0;
+    __syncthreads();
+    for (unsigned c = tid; c < n; c += NT) atomicAdd(&sm.hist[bin_of(sm.cand[c])], 1u);
+    __syncthreads();
+    find_kth_bin<8>(sm.hist, (unsigned)K, sm.redu, &sm.bin, &sm.above, &sm.inbin);
+    const unsigned at = sm.bin;
+    for (unsigned c = tid; c < n; c += NT) {
+      const unsigned long long e = sm.cand[c];
+      const unsigned bin = bin_of(e);
+      bool keep = bin > at;
+      if (bin == at) {
+        unsigned larger = 0;
+        for (unsigned u = 0; u < n; ++u) larger += sm.cand[u] > e ? 1u : 0u;
+        keep = larger < (unsigned)K;
+      }
+      if (keep) sm.kept[atomicAdd(&sm.nsel, 1u)] = e;      // K of them
+    }
+    __syncthreads();
+    from = sm.kept;
+    n = (unsigned)K;
+  }
+  unsigned long long key[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const unsigned i = (unsigned)(e * NT + tid);
+    key[e] = i < n ? from[i] : 0ull;      // zeros sort last
+  }
+  sort_desc<E>(key, sm.cand);
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = tid * E + e;
+    if (i >= K) break;
+    const float z = kfloat((uint32_t)(key[e] >> 32));
     if (out_raw) out_raw[row * K + i] = z;
     else out_logp[row * K + i] = __float2half(z - lse);
-    out_idx[row * K + i] = (int)(0xffffffffu - (uint32_t)(e & 0xffffffffu)) + id_offset;
+    out_idx[row * K + i] = (int)(0xffffffffu - (uint32_t)(key[e] & 0xffffffffu)) + id_offset;
   }
+}
+
+// Four elements of a row from index 4 q on; those past its end are -inf.
+template <bool ALIGNED>
+__device__ __forceinline__ float4 quad(const float* __restrict__ x, int q, int V) {
+  const int i = 4 * q;
+  if (i + 3 < V) {
+    if (ALIGNED) return *reinterpret_cast<const float4*>(x + i);
+    return make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+  }
+  return make_float4(i < V ? x[i] : -INFINITY, i + 1 < V ? x[i + 1] : -INFINITY, i + 2 < V ? x[i + 2] : -INFINITY, -INFINITY);
+}
+
+// A round is UNROLL quads of every thread, NT quads apart, and a group what a thread sees in `per_group` rounds (one, unless
+// a row has more than MAX_GROUPS of them). The maxima of the groups stay in shared memory as the upper 16 bits of their keys,
+// rounded up. The bound comes from CLASSES classes of each thread's groups. One quad a round where rows are short or K is
+// large: more and smaller groups, so that a few more than K elements reach the bound.
+constexpr int MAX_GROUPS = 64;
+
+// Vocabulary-shard mode (out_raw != null): the row is one rank's slice of the vocabulary; the kernel writes the raw
+// fp32 logits of the slice's top K, their GLOBAL ids (index + id_offset) and the slice's log-sum-exp, which
+// topk_combine_kernel turns into the exact top-K log-probs of the whole vocabulary.
+template <int UNROLL, int KCAP, bool ALIGNED>
+__global__ void __launch_bounds__(NT, 5) topk_logprob_kernel(const float* __restrict__ logits, long long ld, int V, int K,
+                                                         __half* __restrict__ out_logp, int* __restrict__ out_idx,
+                                                         float* __restrict__ out_raw, float* __restrict__ out_lse,
+                                                         int id_offset, int per_group) {
+  using Smem = TopkSmem<KCAP>;
+  constexpr int CLASSES = KCAP / 64;                     // NT * CLASSES maxima are four times K or more
+  __shared__ Smem sm;
+  extern __shared__ uint16_t gmax[];                     // [groups][NT]
+  const long long row = blockIdx.x;
+  const float* x = logits + row * ld;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int quads = (V + 3) >> 2;
+  const int rounds = (quads + UNROLL * NT - 1) / (UNROLL * NT);
+  const int groups = (rounds + per_group - 1) / per_group;             // of each thread
+  for (int i = tid; i < NBIN; i += NT) sm.hist[i] = 0;
+  if (tid == 0) { sm.ncand = 0; sm.nsel = 0; }
+
+  // ---- the row: maxima of the groups, and the sum of exponentials against the maximum so far
+  float m = -FLT_MAX;          // lowest finite value: nothing below is ever inf - inf
+  float sum = 0.f;
+  const uint64_t l2e = pack_f32x2(1.4426950408889634f, 1.4426950408889634f);
+  for (int g = 0, r = 0; g < groups; ++g) {
+    float gm = -INFINITY;
+    for (const int r1 = min(rounds, r + per_group); r < r1; ++r) {
+      const int q0 = r * UNROLL * NT + tid;
+      float4 v[UNROLL];
+      if (q0 + (UNROLL - 1) * NT < (V >> 2)) {
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) v[u] = quad<ALIGNED>(x, q0 + u * NT, 0x7fffffff);
+      } else {
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) v[u] = quad<ALIGNED>(x, q0 + u * NT, V);
+      }
+      float rm = -INFINITY;
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) rm = fmax3(fmax3(rm, v[u].x, v[u].y), v[u].z, v[u].w);
+      gm = fmaxf(gm, rm);
+      if (rm > m) {
+        sum *= __expf(m - rm);
+        m = rm;
+      }
+      const uint64_t nm = pack_f32x2(-m, -m);
+      uint64_t s2 = 0ull;
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        float e0, e1, e2, e3;
+        unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[u].x, v[u].y), nm), l2e), e0, e1);
+        unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(v[u].z, v[u].w), nm), l2e), e2, e3);
+        s2 = add_f32x2(s2, pack_f32x2(fast_exp2(e0), fast_exp2(e1)));
+        s2 = add_f32x2(s2, pack_f32x2(fast_exp2(e2), fast_exp2(e3)));
+      }
+      float s0, s1;
+      unpack_f32x2(s2, s0, s1);
+      sum += s0 + s1;
+    }
+    gmax[g * NT + tid] = (uint16_t)((fkey(gm) + 0xffffu) >> 16);
+  }
+  {
+    const float wm = warp_max(m);
+    const float ws = warp_sum(sum * __expf(m - wm));
+    if (lane == 0) { sm.redm[warp] = wm; sm.reds[warp] = ws; }
+  }
+  __syncthreads();
+  float mx = sm.redm[0];
+#pragma unroll
+  for (int w = 1; w < NT / 32; ++w) mx = fmaxf(mx, sm.redm[w]);
+  sum = 0.f;
+#pragma unroll
+  for (int w = 0; w < NT / 32; ++w) sum += sm.reds[w] * __expf(sm.redm[w] - mx);
+  float lse = mx + __logf(sum);
+
+  // ---- the K-th largest maximum of the classes: K groups hold an element above (kth - 1) << 16
+  unsigned kth = 0;
+  float bound = -INFINITY;
+  const int classes = min(CLASSES, groups);
+  if (classes * NT >= K) {
+    unsigned cm[CLASSES];
+#pragma unroll
+    for (int c = 0; c < CLASSES; ++c) {
+      if (c >= classes) break;
+      cm[c] = 0;
+      for (int g = c; g < groups; g += CLASSES) cm[c] = max(cm[c], (unsigned)gmax[g * NT + tid]);
+      atomicAdd(&sm.hist[cm[c] >> (16 - HB)], 1u);
+    }
+    __syncthreads();
+    find_kth_bin<8>(sm.hist, (unsigned)K, sm.redu, &sm.bin, &sm.above, &sm.inbin);
+    const unsigned top = sm.bin, want = (unsigned)K - sm.above;
+    sm.hist[tid] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < CLASSES; ++c)
+      if (c < classes && (cm[c] >> (16 - HB)) == top) atomicAdd(&sm.hist[cm[c] & ((1u << (16 - HB)) - 1)], 1u);
+    __syncthreads();
+    find_kth_bin<1>(sm.hist, want, sm.redu, &sm.bin, &sm.above, &sm.inbin);
+    kth = (top << (16 - HB)) | sm.bin;
+    if (kth > 0) bound = kfloat((kth - 1) << 16);      // K-th of -inf: no number, which all elements reach
+  }
+
+  // ---- the groups that reach it, then their elements that do
+  unsigned int* list = sm.hist;
+  for (int g = 0; g < groups; ++g)
+    if (gmax[g * NT + tid] >= kth) {
+      const unsigned p = atomicAdd(&sm.nsel, 1u);
+      if (p < (unsigned)NBIN) list[p] = (unsigned)(g * NT + tid);
+    }
+  __syncthreads();
+  const unsigned nlist = sm.nsel;
+  if (nlist <= (unsigned)NBIN) {
+    const int per = per_group * UNROLL;                      // quads of a group
+    for (int w = tid; w < (int)nlist * per; w += NT) {
+      const int at = w / per, j = w - at * per;
+      const int g = (int)list[at] / NT, t = (int)list[at] % NT;
+      const int q = (g * per + j) * NT + t;
+      if (q >= quads) continue;
+      const float4 v = quad<ALIGNED>(x, q, V);
+      const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (!(f[e] < bound) && 4 * q + e < V) {
+          const unsigned p = atomicAdd(&sm.ncand, 1u);
+          if (p < (unsigned)Smem::CAP) sm.cand[p] = entry(f[e], 4 * q + e);
+        }
+    }
+  }
+  __syncthreads();
+  unsigned n = sm.ncand;
+  if (nlist > (unsigned)NBIN || n > (unsigned)Smem::CAP || n < (unsigned)K || !(sum > 0.f && sum < INFINITY)) {
+    lse = select_by_radix<KCAP>(sm, x, V, K);
+    n = (unsigned)K;
+  }
+  if (K <= NT) sort_and_write<1, KCAP>(sm, n, K, lse, mx, bound, row, out_logp, out_idx, out_raw, id_offset);
+  else if (KCAP <= 2 * NT || K <= 2 * NT) sort_and_write<2, KCAP>(sm, n, K, lse, mx, bound, row, out_logp, out_idx, out_raw, id_offset);
+  else sort_and_write<KCAP / NT, KCAP>(sm, n, K, lse, mx, bound, row, out_logp, out_idx, out_raw, id_offset);
   if (out_lse && tid == 0) out_lse[row] = lse;
 }
 
@@ -376,7 +570,15 @@ __global__ void __launch_bounds__(NT) topk_merge_kernel(const float* __restrict_
 
 static int launch_topk(const float* logits, long long ld, int rows, int V, int K, __half* out_logp, int* out_idx,
                        float* out_raw, float* out_lse, int id_offset, cudaStream_t st) {
-  topk_logprob_kernel<<<rows, NT, 0, st>>>(logits, ld, V, K, out_logp, out_idx, out_raw, out_lse, id_offset);
+  const bool aligned = !(reinterpret_cast<uintptr_t>(logits) & 15) && !(ld & 3), wide = V >= 16 * 1024 && K <= 512;
+  const int rounds = ceil_div(ceil_div(V, 4), (wide ? 4 : 1) * NT);
+  const int per_group = ceil_div(rounds, MAX_GROUPS);
+  const int smem = ceil_div(rounds, per_group) * NT * 2;
+  auto kern = wide ? (aligned ? topk_logprob_kernel<4, 512, true> : topk_logprob_kernel<4, 512, false>)
+                   : (aligned ? topk_logprob_kernel<1, MAX_K, true> : topk_logprob_kernel<1, MAX_K, false>);
+  if (smem > 16 * 1024)    // with the static part more than a launch may have unasked
+    B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_GROUPS * NT * 2));
+  kern<<<rows, NT, smem, st>>>(logits, ld, V, K, out_logp, out_idx, out_raw, out_lse, id_offset, per_group);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

@@ -13,19 +13,28 @@ _lib.register("b200_trie_walk", [_VP, _VP, _VP, _VP, _I, _VP, _VP, _I, _VP, _VP,
 _lib.register("b200_logprob_full", [_VP, _LL, _I, _I, _VP, _LL, _VP])
 
 
-def topk_logprob(logits: torch.Tensor, vocab: int, k: int):
-    """(fp16 log-probs [rows, k] sorted descending, int32 ids [rows, k]) of log_softmax(logits[:, :vocab])."""
+def topk_logprob(logits: torch.Tensor, vocab: int, k: int, out=None):
+    """(fp16 log-probs [rows, k] sorted descending, int32 ids [rows, k]) of log_softmax(logits[:, :vocab]). ``out``: a pair of
+    contiguous tensors of these shapes and types that receive them."""
     rows = logits.shape[0]
     if not logits.is_cuda:
         z = logits[:, :vocab].float()
         _, i = torch.sort(z, dim=-1, descending=True, stable=True)   # rank on the logits: subtraction can merge values
         i = i[:, :k]
         lp = torch.gather(z, 1, i) - torch.logsumexp(z, dim=-1, keepdim=True)
+        if out is not None:
+            out[0].copy_(lp), out[1].copy_(i)
+            return out
         return lp.to(torch.float16), i.to(torch.int32)
     if logits.dtype != torch.float32 or logits.stride(-1) != 1:
         raise TypeError("topk_logprob: logits must be fp32 with contiguous rows")
-    out_lp = torch.empty((rows, k), dtype=torch.float16, device=logits.device)
-    out_ix = torch.empty((rows, k), dtype=torch.int32, device=logits.device)
+    if out is None:
+        out = (torch.empty((rows, k), dtype=torch.float16, device=logits.device),
+               torch.empty((rows, k), dtype=torch.int32, device=logits.device))
+    out_lp, out_ix = out
+    for t, dtype in ((out_lp, torch.float16), (out_ix, torch.int32)):
+        if t.shape != (rows, k) or t.dtype != dtype or t.device != logits.device or not t.is_contiguous():
+            raise ValueError("topk_logprob: out must be contiguous fp16 and int32 tensors of [rows, k] beside the logits")
     _lib.check(_lib.kernels().b200_topk_logprob(_lib.ptr(logits), logits.stride(0), rows, vocab, k, _lib.ptr(out_lp),
                                                 _lib.ptr(out_ix), _lib.stream()), "b200_topk_logprob")
     return out_lp, out_ix

@@ -54,6 +54,49 @@ def test_topk_logprob_rows_that_defeat_the_histogram(case):
     assert torch.allclose(got[finite], want[finite], atol=2e-3, rtol=1e-3)
 
 
+@pytest.mark.parametrize("V,K", [(1, 1), (3, 2), (255, 255), (1021, 200), (4096, 513), (16383, 400), (16384, 512), (16387, 257), (32000, 513),
+                                 (32001, 1024), (40000, 256), (300001, 128)])
+@pytest.mark.parametrize("layout", ["plain", "off 16 bytes", "ascending", "descending"])
+def test_topk_logprob_over_group_sizes(V, K, layout):
+    """Both group sizes and all sort widths, rows that are no multiple of a quad or of a round, rows off 16-byte boundaries, and rows
+    whose largest elements lie side by side; the same as one vocabulary shard."""
+    rows, ld = 5, V + 5
+    g = torch.Generator("cuda").manual_seed(V + K)
+    buf = torch.full((rows, ld + 3), 1e9, device=DEV)                    # what lies beside a row must not be read as its own
+    x = buf[:, 3 if layout == "off 16 bytes" else 0:][:, :V]
+    x.copy_(torch.randn(rows, V, device=DEV, generator=g) * 3)
+    if "scending" in layout:
+        x.copy_(x.sort(-1, descending=layout == "descending").values)
+    lp, ix = topk.topk_logprob(x, V, K)
+    ref_lp, ref_ix = topk.topk_logprob(x.cpu(), V, K)
+    assert torch.equal(ix.cpu(), ref_ix)
+    # fp16 of a log-probability; exp and log in fp32 add 1e-6
+    assert torch.allclose(lp.float().cpu(), ref_lp.float(), atol=2e-6, rtol=2 ** -10)
+    lib = _lib.kernels()
+    raw, lse = torch.empty((rows, K), device=DEV), torch.empty(rows, device=DEV)
+    ids = torch.empty((rows, K), dtype=torch.int32, device=DEV)
+    from llm_distillery_b200.parallel import tp  # noqa: F401  (declares the signature)
+    assert lib.b200_topk_partial(_lib.ptr(x), x.stride(0), rows, V, K, 1000, _lib.ptr(raw), _lib.ptr(ids), _lib.ptr(lse),
+                                 _lib.stream()) == 0
+    assert torch.equal(ids - 1000, ix) and torch.equal(raw, x.gather(1, ix.long()))
+    assert torch.allclose(lse, x.double().logsumexp(-1).float(), atol=2e-6, rtol=1e-6)
+    assert _lib.take_device_error() == 0
+
+
+def test_topk_logprob_rows_with_infinities():
+    """+inf and NaN rank above all finite values, as keys; the log-sum-exp of such a row is no finite number where an inf takes
+    part, and passes over NaN."""
+    V, K = 20000, 200
+    x = torch.randn(4, V, device=DEV) * 3
+    x[1, 777], x[2, 5], x[3, :] = float("inf"), float("nan"), float("-inf")
+    lp, ix = topk.topk_logprob(x, V, K)
+    assert torch.equal(ix[:1].cpu(), topk.topk_logprob(x[:1].cpu(), V, K)[1])
+    assert ix[1, 0] == 777 and ix[2, 0] == 5 and torch.equal(ix[3].cpu(), torch.arange(K, dtype=torch.int32))
+    rest = torch.cat([x[2, :5], x[2, 6:]]).double()
+    assert torch.allclose(lp[2, 1:].double(), rest.topk(K - 1).values - rest.logsumexp(-1), atol=2e-6, rtol=2 ** -10)
+    assert lp[2, 0].isnan() and lp[3].isnan().all()
+
+
 def test_logprob_full_and_merge():
     torch.manual_seed(0)
     x = torch.randn(50, 777, device=DEV) * 3
