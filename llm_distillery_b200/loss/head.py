@@ -25,6 +25,9 @@ _lib.register("b200_lmhead_lse_gather", [_VP, _VP, _I, _I, _I, _LL, _LL, _VP, _I
 _lib.register("b200_distill_rows", [_VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _F, _VP])
 _lib.register("b200_lmhead_dlogits", [_VP, _VP, _I, _I, _I, _LL, _LL, _VP, _VP, _VP, _VP, _VP, _I, _F, _VP, _LL, _VP])
 
+_lib.register("b200_mean_loss", [_VP] * 4 + [_LL, _I, _VP])
+_lib.register("b200_mean_loss_grad", [_VP] * 4 + [_LL, _I, _VP])
+
 _lib.register("b200_reference_loss", [_VP] * 9 + [_LL, _I, _I, _I, _F, _F, _VP])
 _lib.register("b200_reference_loss_grad", [_VP] * 11 + [_LL, _I, _I, _F, _VP])
 _lib.KERNELS_PER_CALL["b200_reference_loss"] = 2
@@ -155,6 +158,34 @@ class _FusedDistillFn(torch.autograd.Function):
         return dH, dW, None, None, None, None, None
 
 
+class _FusedDistillLossFn(torch.autograd.Function):
+    """The rows of ``_FusedDistillFn`` and the loss of the micro-batch (the sum over its conversations of the mean of their
+    rows) as one node."""
+
+    @staticmethod
+    def forward(ctx, Hc, W, ids, u, seg, n_seg, kind, inv_T, vocab):
+        M, K = ids.shape
+        zk, pmax, psum, nt = _pass1(Hc, W, ids, inv_T, vocab)
+        lse, rows, a, A = _rows(pmax, psum, zk, u, ids, M, K, nt, vocab, kind, inv_T)
+        loss = torch.empty((), dtype=torch.float32, device=Hc.device)
+        count = torch.empty(n_seg, dtype=torch.float32, device=Hc.device)
+        _lib.check(_lib.kernels().b200_mean_loss(_lib.ptr(rows), _lib.ptr(seg), _lib.ptr(loss), _lib.ptr(count), M, n_seg,
+                                                 _lib.stream()), "b200_mean_loss")
+        ctx.save_for_backward(Hc, ids, lse, a, A, seg, count)
+        ctx.W, ctx.slot, ctx.inv_T, ctx.vocab = W, _slot(W), inv_T, vocab
+        return loss
+
+    @staticmethod
+    def backward(ctx, dloss):
+        Hc, ids, lse, a, A, seg, count = ctx.saved_tensors
+        g, dloss = torch.empty_like(lse), dloss.float()
+        _lib.check(_lib.kernels().b200_mean_loss_grad(_lib.ptr(seg), _lib.ptr(count), _lib.ptr(dloss), _lib.ptr(g), lse.numel(),
+                                                      count.numel(), _lib.stream()), "b200_mean_loss_grad")
+        dH, dW = _backward_chunks(Hc, ctx.W, ids, a, A, lse, g, ctx.inv_T, ctx.vocab, ctx.slot, ctx.needs_input_grad[0],
+                                  split_k=True)
+        return (dH, dW) + (None,) * 7
+
+
 def _torch_stats(Hc, W, ids, inv_T, vocab):
     z = (Hc.float() @ W[:vocab].float().t()) * inv_T
     lse = torch.logsumexp(z, dim=-1)
@@ -246,7 +277,12 @@ def distill_head_loss(Hc, W, ids, u, *, kind: str, temperature: float, vocab: in
         s, t = dv.student_teacher_logprobs(lse, zk, u.float(), ids.long() < vocab, temperature)
         custom, logs = dv.reference_loss_segments(s, t, ids.long(), labels, avoid, seg, n_seg, alpha)
         return custom.sum(), {k: v.detach().sum() for k, v in logs.items()}
+    key = {"kl": "kl_div", "rkl": "reverse kl_div", "jsd": "jsd"}[kind]
+    if Hc.is_cuda and ids.shape[0] > 0 and seg is not None and seg.is_cuda and seg.dtype == torch.int64 and seg.shape == ids.shape[:1]:
+        code = KIND_CODES["jsd_renorm" if kind == "jsd" and jsd_renorm else kind]
+        loss = _FusedDistillLossFn.apply(Hc.contiguous(), W, ids.contiguous(), u.float().contiguous(), seg.contiguous(), n_seg,
+                                         code, 1.0 / temperature, vocab)
+        return loss, {key: loss.detach(), "custom loss": loss.detach()}
     rows = fused_distill_rows(Hc, W, ids, u, kind, temperature, vocab, jsd_renorm)
     per_convo = dv._seg_sum(rows, seg, n_seg) / dv.seg_count(seg, n_seg, rows.dtype)
-    key = {"kl": "kl_div", "rkl": "reverse kl_div", "jsd": "jsd"}[kind]
     return per_convo.sum(), {key: per_convo.detach().sum(), "custom loss": per_convo.detach().sum()}

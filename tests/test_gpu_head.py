@@ -57,6 +57,34 @@ def test_fused_loss_and_gradients(kind, M, h, V, K, Vc, T):
     assert gW[Vc:].abs().max() == 0 if Vc < V else True
 
 
+@pytest.mark.parametrize("lens", [[1], [31, 1], [257, 3], [40, 300, 256, 1], [3] * 70])
+@pytest.mark.parametrize("kind", ["kl", "rkl", "jsd", "jsd_renorm"])
+def test_mean_loss_of_conversations(kind, lens):
+    """The loss of a batch as one node against its rows averaged in fp64, and its gradients against those of the rows with the
+    weights that the averages give them (bound: one fp32 sum of up to 300 terms, the weights rounded once)."""
+    M, h, V, K, T = sum(lens), 256, 2000, 40, 2.0
+    Hc, W, ids, u = _setup(M, h, V, K, seed=len(lens))
+    seg = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).to(DEV)
+    grads = []
+    for whole in (True, False):
+        Hg, Wg = Hc.clone().requires_grad_(), W.clone().requires_grad_()
+        if whole:
+            loss, logs = head.distill_head_loss(Hg, Wg, ids, u, kind=kind.removesuffix("_renorm"), temperature=T, vocab=V, seg=seg,
+                                                n_seg=len(lens), jsd_renorm=kind == "jsd_renorm")
+            assert all(torch.equal(v, loss) and not v.requires_grad for v in logs.values()) and "custom loss" in logs
+            (loss * 0.5).backward()
+        else:
+            rows = head.fused_distill_rows(Hg, Wg, ids, u, kind.removesuffix("_renorm"), T, V, jsd_renorm=kind == "jsd_renorm")
+            weight = (1.0 / torch.tensor(lens, dtype=torch.float64, device=DEV))[seg]
+            want = (rows.detach().double() * weight).sum()
+            assert abs(loss.item() - want.item()) <= 300 * 2 ** -23 * (rows.detach().double().abs() * weight).sum().item()
+            (rows * (0.5 * weight).float()).sum().backward()
+        grads.append((Hg.grad.float(), Wg.grad.float()))
+    for a, b in zip(*grads):
+        assert (a - b).abs().max() <= 2 ** -7 * b.abs().max()
+    assert _lib.take_device_error() == 0
+
+
 def test_reference_loss_through_fused_stats():
     M, h, V, K, Vc, T = 400, 256, 2000, 64, 2000, 1.0
     Hc, W, ids, u = _setup(M, h, V, K, seed=2)
