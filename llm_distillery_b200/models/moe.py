@@ -8,9 +8,10 @@ experts is two autograd nodes with explicit backward: ``AttnBlockFn`` (the atten
 ``MoEBlockFn``. The expert half sorts the (token, choice) pairs by expert once per layer, gathers the rows, runs each of
 the experts' two GEMMs as one launch over all experts' slabs of rows (SwiGLU in the epilogue of the first; a launch per
 expert for sizes and types that it does not take), and combines by GATHERING each token's k results - a fixed order of
-additions, no atomic scatter. Routing arithmetic ([T, E] tensors) is PyTorch in fp32. The number of rows per expert stays on
-the device in inference (within the sizes of ``sorted_pairs``' kernel; the library's histogram waits for the device); a forward pass that a backward pass follows reads it back once per layer (the shapes of the weight
-gradients' GEMMs depend on it).
+additions, no atomic scatter. The router is a kernel of its own in the forward pass, the rest of the routing arithmetic
+([T, E] tensors) PyTorch in fp32. The number of rows per expert stays on the device in inference (within the sizes of
+``sorted_pairs``' kernel; the library's histogram waits for the device); a forward pass that a backward pass follows reads it
+back once per layer (the shapes of the weight gradients' GEMMs depend on it).
 No GEMM here cuts K (``basic.gemm``'s split_k), in inference either: behind a router a last bit can be another expert, and
 an expert's row count, which the cut would depend on, changes with every batch.
 """
@@ -24,16 +25,14 @@ from ..ops._lib import _F, _I, _LL, _VP
 from . import llama as _ll
 
 _lib.register("b200_expert_sort", [_VP, _LL, _I, _I, _VP, _VP, _VP, _VP, _VP])
-_lib.KERNELS_PER_CALL["b200_expert_sort"] = 2
+_lib.register("b200_moe_route", [_VP, _VP, _LL, _I, _I, _I, _I, _VP, _VP, _VP, _VP])
 _lib.register("b200_gemm_grouped_swiglu", [_VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP])
 _lib.register("b200_gemm_grouped", [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP])
 _lib.register("b200_moe_combine", [_VP, _VP, _VP, _VP, _VP, _LL, _I, _I, _F, _VP])
 
 
-# One block sorts in time that grows with the pairs, the library's ten launches in time that hardly does. A call with the counts
-# read back, 8 / 32 experts, kernel against library: 2048 pairs 36 / 47 us against 137 / 134, 32 768 73 / 86 against 219 / 209,
-# 65 536 132 / 146 against 216 / 218; 131 072 276 / 296 against 210. With the counts left on the device 65 536 pairs take 99 / 112
-# against 199 / 200.
+# The sort kernel's time grows with the pairs, that of the library's ten launches hardly does. With the counts left on the device,
+# 8 / 32 experts, kernel against library: 65 536 pairs take 27 / 50 us against 199 / 200 (2000 pairs 2.6).
 SORT_MAX_PAIRS = 65536
 
 
@@ -41,7 +40,18 @@ SORT_MAX_PAIRS = 65536
 def route(n2: torch.Tensor, w_router: torch.Tensor, k: int, renorm: bool = True):
     """Router of one layer: (probs [T,E] fp32, chosen experts [T,k] int64, their weights [T,k] fp32 - renormalised
     over the chosen experts (Mixtral; Qwen3-MoE with ``norm_topk_prob``) or the plain softmax values).
-    Logits are computed in the model's dtype and the softmax in fp32, as HuggingFace's blocks do."""
+    Logits are computed in the model's dtype and the softmax in fp32, as HuggingFace's blocks do. One launch on a GPU
+    (csrc/ops/moe.cu) for bf16 and up to 16 experts."""
+    (T, h), E = n2.shape, w_router.shape[0]
+    graph = torch.is_grad_enabled() and (n2.requires_grad or w_router.requires_grad)
+    if (n2.is_cuda and not graph and T and E <= 16 and 0 < k <= E and h % 8 == 0 and w_router.shape == (E, h) and w_router.device == n2.device
+            and all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (n2, w_router))):
+        probs = torch.empty((T, E), dtype=torch.float32, device=n2.device)
+        top_e = torch.empty((T, k), dtype=torch.int64, device=n2.device)
+        top_w = torch.empty((T, k), dtype=torch.float32, device=n2.device)
+        _lib.check(_lib.kernels().b200_moe_route(_lib.ptr(n2), _lib.ptr(w_router), T, h, E, k, int(renorm), _lib.ptr(probs),
+                                                 _lib.ptr(top_e), _lib.ptr(top_w), _lib.stream()), "b200_moe_route")
+        return probs, top_e, top_w
     logits = F.linear(n2, w_router)
     probs = torch.softmax(logits.float(), dim=-1)
     top_p, top_e = torch.topk(probs, k, dim=-1)
@@ -51,7 +61,7 @@ def route(n2: torch.Tensor, w_router: torch.Tensor, k: int, renorm: bool = True)
 def sorted_pairs(top_e: torch.Tensor, n_experts: int):
     """(order, inverse, token, counts): ``order`` lists the T*k (token, choice) pairs sorted by expert (stable, so tokens
     keep their order inside an expert's slab), ``inverse`` undoes it, ``token`` is the token of each sorted pair,
-    ``counts`` are the slab lengths (int64 [n_experts], on the device of ``top_e``). Two launches on a GPU (csrc/ops/moe.cu) for
+    ``counts`` are the slab lengths (int64 [n_experts], on the device of ``top_e``). One launch on a GPU (csrc/ops/moe.cu) for
     up to 32 experts and ``SORT_MAX_PAIRS`` pairs; beyond them, and for indices that are not int64, the library's sort, whose
     histogram waits for the device."""
     flat = top_e.reshape(-1)
@@ -336,7 +346,7 @@ class MoEBlockFn(torch.autograd.Function):
         if recompute:
             h1, top_e, order, inverse = ctx.saved_tensors
             n2, _, rstd2 = basic.rmsnorm_fwd(h1, w_ln2, eps)
-            probs = torch.softmax(F.linear(n2, w_router).float(), dim=-1)
+            probs = route(n2, w_router, k, renorm)[0]
             top_p = probs.gather(1, top_e)
             top_w = top_p / top_p.sum(-1, keepdim=True) if renorm else top_p
             tok = torch.div(order, k, rounding_mode="floor")

@@ -42,6 +42,30 @@ def test_which_sort_takes_the_pairs(monkeypatch, T, k, dtype, native):
     assert torch.equal(order[inverse], torch.arange(T * k, device="cuda"))
 
 
+@pytest.mark.parametrize("T,h,E,k", [(1, 8, 1, 1), (3, 264, 8, 2), (4, 256, 7, 7), (1531, 2048, 8, 2), (5, 520, 9, 4), (33, 2048, 16, 4),
+                                     (2, 8, 15, 8), (257, 1024, 16, 16)])
+@pytest.mark.parametrize("renorm", [True, False])
+def test_route_is_the_softmax_of_the_rounded_logits(T, h, E, k, renorm):
+    """Probabilities against fp64 within one rounding of the logits to bf16 either way (2^-8 of each), choices and weights against
+    the probabilities: the k largest, of equal ones (experts 0 and 1 have the same weights) the lower first."""
+    g = torch.Generator("cuda").manual_seed(T + E)
+    x = torch.randn(T, h, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(E, h, device="cuda", generator=g) * 3 / h ** 0.5).bfloat16()
+    if E > 1:
+        w[1] = w[0]
+    probs, top_e, top_w = moe.route(x, w, k, renorm)
+    logits = x.double() @ w.double().t()
+    want = logits.softmax(-1)
+    assert ((probs.double() / want).log().abs() <= 2 ** -8 * 2 * logits.abs().amax(-1, keepdim=True) + 1e-5).all()
+    assert torch.equal(top_e, probs.sort(dim=-1, descending=True, stable=True).indices[:, :k])
+    top_p = probs.gather(1, top_e)
+    assert torch.allclose(top_w, top_p / top_p.sum(-1, keepdim=True) if renorm else top_p, rtol=1e-6, atol=0)
+    # a caller that differentiates through it keeps the library's operators
+    xr = x.clone().requires_grad_()
+    assert moe.route(xr, w, k, renorm)[2].requires_grad
+    assert _lib.take_device_error() == 0
+
+
 @pytest.mark.parametrize("T,k,h,resid,rmul", [(1, 1, 8, True, 1.0), (257, 2, 2048, True, 1.0), (33, 8, 264, False, 1.0),
                                               (100, 4, 512, True, 0.25)])
 def test_combine_matches_the_gathered_sum(T, k, h, resid, rmul):
