@@ -177,11 +177,12 @@ __device__ __forceinline__ void tma_store_wait_read0() {
 __device__ __forceinline__ void tma_store_wait_all0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---------------------------------------------------------------- one thread of a converged warp
-// The warps that issue tcgen05 instructions in the few-tile and the CTA-pair GEMM and in flash attention run their loops -
-// waits, counters, descriptors - with all 32 lanes and let one elected lane issue: the operands are then warp-uniform
-// values. In a loop that only lane 0 runs they are not, and each instruction paid for moving them (a K block of 64 in the
-// few-tile GEMM: 0.30 us, elected 0.25 us). The one-SM GEMM of 128 x 256 tiles (gemm_core.cuh, comm/tp_gemm.cu) still
-// issues from lane 0.
+// The warps that issue TMA loads and tcgen05 instructions let the lane that this names run their loops, and the others wait
+// behind them. In a branch on `lane == 0` the operands of those instructions - descriptors, addresses, barriers - are no
+// warp-uniform values and each instruction pays for moving them; behind elect.sync they are. A K block of 64 of the few-tile
+// GEMM, loads and products both issued from lane 0: 0.30 us, products issued by the elected lane with all lanes in the loop
+// 0.25, both loops run by the elected lane 0.16 (777 x 896 x 9728 45.0 / 29.0 us, 777 x 896 x 896 7.7 / 6.2).
+// The one-SM GEMM of 128 x 256 tiles (gemm_core.cuh, comm/tp_gemm.cu) still issues from lane 0.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile(

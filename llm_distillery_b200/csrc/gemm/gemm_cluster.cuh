@@ -90,8 +90,7 @@ __global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
   const int kb0 = (int)((long long)num_kb * slice / n_slices);
   const int kb1 = (int)((long long)num_kb * (slice + 1) / n_slices);
 
-  auto load_b = [&](int kb) {
-    const uint32_t st = (uint32_t)(kb - kb0) % STAGES;
+  auto load_b = [&](int kb, uint32_t st) {
     uint8_t* sB = smem + st * S::STAGE_BYTES + S::A_BYTES;
     if constexpr (B_MN) {
 #pragma unroll
@@ -108,56 +107,65 @@ __global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
   // one before it is past its own wait, so whatever ran before THAT one is complete and visible here. Steps of 512 and of 777
   // tokens 1.4 and 1.0 % shorter, a forward pass over 93 tokens 1.8 %.
   const int early = b_early ? min(kb1 - kb0, STAGES) : 0;
-  if (warp == 0 && lane == 0) {
-    for (int i = 0; i < early; ++i) {
-      mbar_arrive_expect_tx(&full_bar[i], S::STAGE_BYTES);
-      load_b(kb0 + i);
+  if (warp == 0) {
+    if (elect_one()) {
+      for (int i = 0; i < early; ++i) {
+        mbar_arrive_expect_tx(&full_bar[i], S::STAGE_BYTES);
+        load_b(kb0 + i, i);
+      }
     }
+    __syncwarp();
   }
-  __syncwarp();
   pdl_wait();
   pdl_trigger();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
+      uint32_t st = 0, ph = 1u;
       for (int kb = kb0; kb < kb1; ++kb) {
-        const uint32_t it = kb - kb0, s = it % STAGES, ph = (it / STAGES) & 1u;
-        if (!mbar_wait_bounded(&empty_bar[s], ph ^ 1u, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
-        uint8_t* sA = smem + s * S::STAGE_BYTES;
-        if ((int)it >= early) {
-          mbar_arrive_expect_tx(&full_bar[s], S::STAGE_BYTES);
-          load_b(kb);
+        if (!mbar_wait_bounded(&empty_bar[st], ph, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
+        uint8_t* sA = smem + st * S::STAGE_BYTES;
+        if (kb - kb0 >= early) {
+          mbar_arrive_expect_tx(&full_bar[st], S::STAGE_BYTES);
+          load_b(kb, st);
         }
         if constexpr (!A_MN) {
-          tma_load_2d(sA, &tmA, &full_bar[s], kb * BK, m0);
+          tma_load_2d(sA, &tmA, &full_bar[st], kb * BK, m0);
         } else {
 #pragma unroll
-          for (int i = 0; i < BM / 64; ++i) tma_load_2d(sA + i * (BK * 128), &tmA, &full_bar[s], m0 + i * 64, kb * BK);
+          for (int i = 0; i < BM / 64; ++i) tma_load_2d(sA + i * (BK * 128), &tmA, &full_bar[st], m0 + i * 64, kb * BK);
+        }
+        if (++st == STAGES) {
+          st = 0;
+          ph ^= 1u;
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     const uint32_t idesc = make_idesc_f16(fmt, BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
     constexpr DescCfg dc = default_desc_cfg<BN, A_MN, B_MN>();
-    for (int kb = kb0; kb < kb1; ++kb) {
-      const uint32_t it = kb - kb0, s = it % STAGES, ph = (it / STAGES) & 1u;
-      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[s], ph, abort_flag, err_word, ERR_WAIT_FULL)))
-        break;
-      tc_fence_after_sync();
-      const uint32_t a_base = smem_u32(smem + s * S::STAGE_BYTES);
-      const uint32_t b_base = a_base + S::A_BYTES;
-      if (elect_one()) {
+    const uint64_t da0 = make_smem_desc_sw128(smem_u32(smem), dc.a_lbo, dc.a_sbo);
+    const uint64_t db0 = make_smem_desc_sw128(smem_u32(smem) + S::A_BYTES, dc.b_lbo, dc.b_sbo);
+    if (elect_one()) {
+      uint32_t st = 0, ph = 0u;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait_bounded(&full_bar[st], ph, abort_flag, err_word, ERR_WAIT_FULL)) break;
+        tc_fence_after_sync();
+        const uint64_t off = static_cast<uint64_t>((st * S::STAGE_BYTES) >> 4);
 #pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k) {
-          const uint64_t da = make_smem_desc_sw128(a_base + k * dc.a_kadv, dc.a_lbo, dc.a_sbo);
-          const uint64_t db = make_smem_desc_sw128(b_base + k * dc.b_kadv, dc.b_lbo, dc.b_sbo);
-          umma_f16_ss(tmem_base, da, db, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
-        }
-        umma_commit(&empty_bar[s]);
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          umma_f16_ss(tmem_base, da0 + off + static_cast<uint64_t>((k * dc.a_kadv) >> 4),
+                      db0 + off + static_cast<uint64_t>((k * dc.b_kadv) >> 4), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+        umma_commit(&empty_bar[st]);
         if (kb + 1 == kb1) umma_commit(done_bar);
+        if (++st == STAGES) {
+          st = 0;
+          ph ^= 1u;
+        }
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else {
     // accumulator -> shared memory. done_bar means every MMA has read its stage, so the ring is free.
     const int quad = warp & 3;

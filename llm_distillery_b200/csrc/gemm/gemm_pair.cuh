@@ -171,8 +171,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      uint32_t it = 0;
+    if (elect_one()) {
+      uint32_t it = 0, s = 0, ph = 1u;
       bool ok = true;
       int e = 0;
       for (int unit = pair_id; ok && unit < num_units; unit += num_pairs) {
@@ -186,9 +186,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         const int n0 = b_row + (b_half_stride > 0 ? n_blk * PAIR_HALF_N + (int)cta * b_half_stride
                                                   : n_blk * PAIR_BN + (int)cta * PAIR_HALF_N);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const uint32_t s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1u;
-          if (!mbar_wait_bounded(&empty_bar[s], ph ^ 1u, abort_flag, err_word, ERR_WAIT_EMPTY)) {
+          if (!mbar_wait_bounded(&empty_bar[s], ph, abort_flag, err_word, ERR_WAIT_EMPTY)) {
             ok = false;
             break;
           }
@@ -209,6 +207,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
             for (int i = 0; i < PAIR_HALF_N / 64; ++i)
               tma_load_2d_pair(sB + i * (BK * 128), &tmB, &full_bar[s], n0 + i * 64, kb * BK);
           }
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
       }
       // drain: the last commits must have released every stage before this CTA's shared memory goes away
@@ -217,46 +219,47 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         if (!mbar_wait_bounded(&empty_bar[j % STAGES], (j / STAGES) & 1u, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
     if (cta == 0) {
       const uint32_t idesc = make_idesc_f16(fmt, PAIR_BM, PAIR_BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       constexpr uint32_t a_lbo = A_MN ? BK * 128 : 16, a_kadv = A_MN ? UMMA_K * 128 : UMMA_K * 2;
       constexpr uint32_t b_lbo = B_MN ? BK * 128 : 16, b_kadv = B_MN ? UMMA_K * 128 : UMMA_K * 2;
-      uint32_t it = 0, tl = 0;
-      bool ok = true;
-      for (int unit = pair_id; ok && unit < num_units; unit += num_pairs, ++tl) {
-        int tile, kb0, kb1;
-        unit_range(unit, tile, kb0, kb1);
-        const uint32_t acc = tl & 1u;
-        const uint32_t aph = (tl >> 1) & 1u;
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&tempty_bar[acc], aph ^ 1u, abort_flag, err_word, ERR_WAIT_TMEM_EMPTY)))
-          break;
-        tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * PAIR_BN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const uint32_t s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1u;
-          if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full_bar[s], ph, abort_flag, err_word, ERR_WAIT_FULL))) {
-            ok = false;
-            break;
-          }
+      const uint64_t da0 = make_smem_desc_sw128(smem_u32(smem), a_lbo, 1024);
+      const uint64_t db0 = make_smem_desc_sw128(smem_u32(smem) + S::A_BYTES, b_lbo, 1024);
+      if (elect_one()) {
+        uint32_t s = 0, ph = 0u, tl = 0;
+        bool ok = true;
+        for (int unit = pair_id; ok && unit < num_units; unit += num_pairs, ++tl) {
+          int tile, kb0, kb1;
+          unit_range(unit, tile, kb0, kb1);
+          const uint32_t acc = tl & 1u;
+          const uint32_t aph = (tl >> 1) & 1u;
+          if (!mbar_wait_bounded(&tempty_bar[acc], aph ^ 1u, abort_flag, err_word, ERR_WAIT_TMEM_EMPTY)) break;
           tc_fence_after_sync();
-          const uint32_t a_base = smem_u32(smem + s * S::STAGE_BYTES);
-          const uint32_t b_base = a_base + S::A_BYTES;
-          if (elect_one()) {
-#pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k) {
-              const uint64_t da = make_smem_desc_sw128(a_base + k * a_kadv, a_lbo, 1024);
-              const uint64_t db = make_smem_desc_sw128(b_base + k * b_kadv, b_lbo, 1024);
-              umma_f16_ss_pair(d_tmem, da, db, idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+          const uint32_t d_tmem = tmem_base + acc * PAIR_BN;
+          for (int kb = kb0; kb < kb1; ++kb) {
+            if (!mbar_wait_bounded(&full_bar[s], ph, abort_flag, err_word, ERR_WAIT_FULL)) {
+              ok = false;
+              break;
             }
+            tc_fence_after_sync();
+            const uint64_t off = static_cast<uint64_t>((s * S::STAGE_BYTES) >> 4);
+#pragma unroll
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_f16_ss_pair(d_tmem, da0 + off + static_cast<uint64_t>((k * a_kadv) >> 4),
+                               db0 + off + static_cast<uint64_t>((k * b_kadv) >> 4), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
             umma_commit_pair(&empty_bar[s], 0x3);
             if (kb + 1 == kb1) umma_commit_pair(&tfull_bar[acc], 0x3);
+            if (++s == STAGES) {
+              s = 0;
+              ph ^= 1u;
+            }
           }
-          __syncwarp();
         }
       }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ epilogue warps (both CTAs)
