@@ -26,6 +26,7 @@ template <int BN>
 struct EpiStore {
   using Params = StoreParams;
   static constexpr bool SPLIT_K = true;   // the pair kernel may cut the K loop into slices that are added in order
+  static constexpr bool PREFETCH = false;
   // slice 0 of a tile stores (or adds to what C held, if the caller accumulates); every later slice adds
   static __device__ __forceinline__ Params slice_params(const Params& p, int slice) {
     Params q = p;
@@ -263,6 +264,7 @@ struct SwigluParams {
 struct EpiSwiglu {
   using Params = SwigluParams;
   static constexpr bool SPLIT_K = false;
+  static constexpr bool PREFETCH = false;
   static constexpr int STAGE_BYTES = 32 * 256;
   static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;
 
@@ -355,6 +357,7 @@ struct RopeParams {
 struct EpiRope {
   using Params = RopeParams;
   static constexpr bool SPLIT_K = false;
+  static constexpr bool PREFETCH = false;
   static constexpr int STAGE_BYTES = 32 * 256;
   static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;
 
@@ -452,10 +455,13 @@ static int launch_rope_pair(const void* A, const void* W, int M, int N, int K, l
 }
 
 // Backward of SwiGLU in the epilogue of the down projection's dgrad GEMM: the accumulator tile is d(act) for 256 tokens
-// x 256 features; the warp pulls the matching gate and up values (32 rows x 128 columns each, coalesced 256-byte row
-// segments) into two swizzled stages, every lane then works on its own row - d(act) rounded to bf16 first, so that the
-// result equals GEMM + stand-alone kernel bit for bit - and overwrites the stages with d(gate) and d(up), which leave
-// as whole row segments. d(act) itself is never written.
+// x 256 features. A warp takes its 32 rows in quarters of 64 columns: the matching gate and up values come by asynchronous
+// copies of whole 128-byte row segments into one of two swizzled stages while it works on the quarter before (the first one's
+// while the main loop still runs), every lane then works on its own row - d(act) rounded to bf16 first, so that the
+// result equals GEMM + stand-alone kernel bit for bit - and overwrites the stage with d(gate) and d(up), which leave
+// as whole row segments. d(act) itself is never written. With the loads in front of each half, through registers, a tile's
+// epilogue took longer than its main loop: 16384 x 2048 -> 5632 379 us,
+// now 321 (under the power cap 470 / 342).
 struct SwigluBwdParams {
   const __nv_bfloat16* gu;   // [M, 2f] saved by the forward pass
   long long ld_gu;
@@ -467,56 +473,61 @@ struct SwigluBwdParams {
 struct EpiSwigluBwd {
   using Params = SwigluBwdParams;
   static constexpr bool SPLIT_K = false;
-  static constexpr int STAGE_BYTES = 2 * 32 * 256;     // gate and up stage per epilogue warp
+  static constexpr bool PREFETCH = true;
+  static constexpr int QUARTER = 32 * 128;               // gate or up values of a quarter
+  static constexpr int STAGE_BYTES = 2 * 2 * QUARTER;    // two stages of both per epilogue warp
   static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;
+
+  static __device__ __forceinline__ int rows_of(int m0, int M, int quad) { return min(32, M - (m0 + quad * 32)); }
+
+  // gate and up values of quarter q into its stage, as one group of copies (empty where the quarter lies beyond N)
+  static __device__ __forceinline__ void fetch(const Params& p, int q, int m0, int n0, int M, int N, int quad, int lane,
+                                               uint8_t* epi_smem) {
+    const int rows = rows_of(m0, M, quad), col = n0 + q * 64 + (lane & 7) * 8;
+    if (n0 + q * 64 < N) {
+      const uint32_t sg = smem_u32(epi_smem + quad * STAGE_BYTES + (q & 1) * 2 * QUARTER);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int row = 4 * j + (lane >> 3);
+        if (row < rows) {
+          const __nv_bfloat16* src = p.gu + (long long)(m0 + quad * 32 + row) * p.ld_gu + col;
+          const uint32_t dst = sg + row * 128 + (((lane & 7) ^ (row & 7)) << 4);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + QUARTER), "l"(src + p.f) : "memory");
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+
+  static __device__ __forceinline__ void prefetch(const Params& p, int m0, int n0, int M, int N, int quad, int lane,
+                                                  uint8_t* epi_smem) {
+    fetch(p, 0, m0, n0, M, N, quad, lane, epi_smem);
+  }
 
   static __device__ __forceinline__ void tile(const Params& p, uint32_t taddr, int m0, int n0, int M, int N, int quad,
                                               int lane, uint8_t* epi_smem) {
-    uint8_t* sg = epi_smem + quad * STAGE_BYTES;
-    uint8_t* su = sg + 32 * 256;
-    const int row0 = m0 + quad * 32;
-    const int rows_valid = min(32, M - row0);
-    const int chunk = lane & 15;
+    const int rows = rows_of(m0, M, quad), row0 = m0 + quad * 32;
 #pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      const int col0 = n0 + half * 128;
-      if (col0 >= N) break;                              // N is a multiple of 128: a half is whole or absent
-      const int col = col0 + chunk * 8;
-      {
-        uint4 t[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int row = 2 * j + (lane >> 4);
-          t[j] = row < rows_valid ? __ldg(reinterpret_cast<const uint4*>(p.gu + (long long)(row0 + row) * p.ld_gu + col))
-                                  : make_uint4(0u, 0u, 0u, 0u);
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int row = 2 * j + (lane >> 4);
-          *reinterpret_cast<uint4*>(sg + row * 256 + ((chunk ^ (row & 15)) << 4)) = t[j];
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int row = 2 * j + (lane >> 4);
-          t[j] = row < rows_valid
-                     ? __ldg(reinterpret_cast<const uint4*>(p.gu + (long long)(row0 + row) * p.ld_gu + p.f + col))
-                     : make_uint4(0u, 0u, 0u, 0u);
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int row = 2 * j + (lane >> 4);
-          *reinterpret_cast<uint4*>(su + row * 256 + ((chunk ^ (row & 15)) << 4)) = t[j];
-        }
+    for (int q = 0; q < 4; ++q) {
+      if (q < 3) {
+        fetch(p, q + 1, m0, n0, M, N, quad, lane, epi_smem);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
       __syncwarp();
-#pragma unroll 1
-      for (int c4 = 0; c4 < 4; ++c4) {
+      if (n0 + q * 64 >= N) continue;                    // N is a multiple of 128
+      uint8_t* sg = epi_smem + quad * STAGE_BYTES + (q & 1) * 2 * QUARTER;
+      uint8_t* su = sg + QUARTER;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
         uint32_t r[32];
-        tmem_ld_32x32b_x32(taddr + half * 128 + c4 * 32, r);
+        tmem_ld_32x32b_x32(taddr + q * 64 + c * 32, r);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int off = lane * 256 + (((c4 * 4 + j) ^ (lane & 15)) << 4);
+          const int off = lane * 128 + (((c * 4 + j) ^ (lane & 7)) << 4);
           const uint4 qg = *reinterpret_cast<const uint4*>(sg + off);
           const uint4 qu = *reinterpret_cast<const uint4*>(su + off);
           const __nv_bfloat162* hg = reinterpret_cast<const __nv_bfloat162*>(&qg);
@@ -545,8 +556,18 @@ struct EpiSwigluBwd {
           *reinterpret_cast<uint4*>(su + off) = ou;
         }
       }
-      EpiSwiglu::flush(sg, p.dgu, p.ld_dgu, row0, rows_valid, col0, p.f, lane);
-      EpiSwiglu::flush(su, p.dgu + p.f, p.ld_dgu, row0, rows_valid, col0, p.f, lane);
+      __syncwarp();
+      __nv_bfloat16* dst = p.dgu + (long long)row0 * p.ld_dgu + n0 + q * 64 + (lane & 7) * 8;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int row = 4 * j + (lane >> 3);
+        const int off = row * 128 + (((lane & 7) ^ (row & 7)) << 4);
+        if (row < rows) {
+          *reinterpret_cast<uint4*>(dst + (long long)row * p.ld_dgu) = *reinterpret_cast<const uint4*>(sg + off);
+          *reinterpret_cast<uint4*>(dst + (long long)row * p.ld_dgu + p.f) = *reinterpret_cast<const uint4*>(su + off);
+        }
+      }
+      __syncwarp();                                      // the stage may be filled again
     }
   }
 };

@@ -273,6 +273,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       locate(tile, e, row, n_blk, b_row, row_end);
       const uint32_t acc = tl & 1u;
       const uint32_t aph = (tl >> 1) & 1u;
+      if constexpr (Epi::PREFETCH)      // operands from global memory, while the main loop runs
+        Epi::prefetch(ep, row + (int)cta * BM, n_blk * PAIR_BN, row_end, N, quad, lane, epi_smem);
       int ok = mbar_wait_bounded(&tfull_bar[acc], aph, abort_flag, err_word, ERR_WAIT_TMEM_FULL) ? 1 : 0;
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
@@ -303,6 +305,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(leader_tempty0 + acc * 8);
     }
+    if constexpr (Epi::PREFETCH) asm volatile("cp.async.wait_all;" ::: "memory");   // of a loop that was given up
   }
 
   __syncwarp();

@@ -35,6 +35,7 @@ struct LseParams {
 
 struct EpiLse {
   static constexpr bool SPLIT_K = false;
+  static constexpr bool PREFETCH = false;
   using Params = LseParams;
   static constexpr int SMEM_BYTES = 0;
   static __device__ __forceinline__ void tile(const Params& p, uint32_t taddr, int m0, int n0, int M, int N, int quad,
@@ -115,6 +116,7 @@ struct DzParams {
 
 struct EpiDz {
   static constexpr bool SPLIT_K = false;
+  static constexpr bool PREFETCH = false;
   using Params = DzParams;
   static constexpr int STAGE_BYTES = 32 * 256;   // per epilogue warp: 32 rows x 128 bf16 columns, chunks XOR-swizzled
   static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;

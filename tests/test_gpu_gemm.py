@@ -213,6 +213,20 @@ def test_one_slice_keeps_the_order_of_the_pair_kernel(T):
     assert _lib.take_device_error() == 0
 
 
+@pytest.mark.parametrize("T,f,h", [(5003, 1408, 520), (4737, 1152, 264), (18945, 128, 256), (4865, 1280, 2048)])
+def test_swiglu_backward_epilogue_of_ragged_pair_tiles(T, f, h):
+    """Rows that end inside a warp's 32 and features that end in the middle of a 256 x 256 tile: the bits of GEMM + separate
+    kernel, and nothing written behind the last row."""
+    g = torch.Generator("cuda").manual_seed(T)
+    dy = torch.randn(T, h, device=DEV, generator=g).bfloat16()
+    w_d = (torch.randn(h, f, device=DEV, generator=g) * 0.05).bfloat16()
+    gu = torch.randn(T, 2 * f, device=DEV, generator=g).bfloat16()
+    out = torch.full((T + 40, 2 * f), 7.0, device=DEV, dtype=torch.bfloat16)
+    dgu = basic.linear_dgrad_swiglu_bwd(dy, w_d, gu, out=out[:T])
+    assert torch.equal(dgu, basic.swiglu_bwd(gu, basic.linear_dgrad(dy, w_d)))
+    assert (out[T:] == 7.0).all() and _lib.take_device_error() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(8, 64, 64), (128, 128, 512), (136, 72, 200), (304, 1152, 896)])
 @pytest.mark.parametrize("layout,dtype", [("nt", torch.float16), ("nn", torch.float16), ("tn", torch.float16),
                                           ("tt", torch.float16), ("tt", torch.bfloat16)])
