@@ -1,7 +1,8 @@
 // Causal GQA flash-attention forward for sm_100a on tcgen05 tensor cores.
 //
-// One CTA = one (batch, q-head, 128-query block); keys are walked in tiles of BN = 64. Roles (224 threads):
-//   warp 0    TMA producer : Q once, then K tiles through a 3-stage ring and V tiles through a 2-stage ring (3D tensor
+// One CTA = one (batch, q-head, 128-query block); keys are walked in tiles of BN = 64. Roles (256 threads; of warps 0, 1, 2 and 7 the elected
+// lane, which in place of loops on lane 0, or with all lanes in them, made calls of one to a few blocks 4 % shorter):
+//   warps 0, 7 TMA producers: Q once, then K tiles through a 3-stage ring; V tiles through a 2-stage ring (3D tensor
 //                            map [B][L][width], so rows past the sequence end read zeros; no multicast)
 //   warp 1    P V issuer   : O += P_j V_j with A = P_j read from TMEM and V_j as MN-major B from shared memory
 //   warp 2    S issuer     : S_j = Q K_j^T (tcgen05.mma, both operands K-major) into one of TWO score buffers in TMEM
@@ -35,7 +36,7 @@ namespace fa {
 
 constexpr int BM = 128;
 constexpr int BN = 64;
-constexpr int NTHREADS = 224;
+constexpr int NTHREADS = 256;
 constexpr int VS = 2;  // V ring
 constexpr float kRescaleThreshold = 8.0f;  // in log2 units
 // Measured (B200, 1965 MHz): 0.254 ms / 0.264 ms (head dim 64, batch 8 x 2048 / head dim 128, batch 2 x 4096) with every
@@ -167,94 +168,114 @@ __global__ void __launch_bounds__(NTHREADS, 2)
   const int colV = p.colV0 + hkv * D;
 
   if (warp == 0) {
-    // two producer threads: K runs NBUF tiles ahead of the softmax and must not queue behind the V loads, which are
-    // gated by the P V MMAs two tiles back
-    if (lane == 0) {
+    // K runs NBUF tiles ahead of the softmax and must not queue behind the V loads, which are gated by the P V MMAs two
+    // tiles back: another warp's (below)
+    if (elect_one()) {
       mbar_arrive_expect_tx(q_full, C::Q_BYTES);
 #pragma unroll
       for (int c = 0; c < D / 64; ++c) tma_load_3d(smem + c * (BM * 128), &tmQ, q_full, colQ + c * 64, q0, b);
+      int ks = 0;
+      uint32_t ph = 1u;
       for (int j = 0; j < n_kv; ++j) {
-        const int ks = j % KS;
-        if (!mbar_wait_bounded(&k_empty[ks], ((j / KS) & 1u) ^ 1u, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
+        if (!mbar_wait_bounded(&k_empty[ks], ph, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
         uint8_t* sK = smem + C::OFF_K + ks * C::T_BYTES;
         mbar_arrive_expect_tx(&k_full[ks], C::T_BYTES);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) tma_load_3d(sK + c * (BN * 128), &tmK, &k_full[ks], colK + c * 64, (tile0 + j) * BN, b);
+        if (++ks == KS) {
+          ks = 0;
+          ph ^= 1u;
+        }
       }
-    } else if (lane == 1) {
+    }
+    __syncwarp();
+  } else if (warp == NTHREADS / 32 - 1) {
+    if (elect_one()) {
+      int pb = 0;                                   // barrier and parity of P V of tile j - VS
+      uint32_t pph = 0u;
       for (int j = 0; j < n_kv; ++j) {
         const int vs = j % VS;
         // V stage j % VS was read by P_{j-VS} V_{j-VS}
-        if (j >= VS && !mbar_wait_bounded(&pv_done[(j - VS) % NBUF], ((j - VS) / NBUF) & 1u, abort_flag, err_word,
-                                          ERR_WAIT_EMPTY))
-          break;
+        if (j >= VS) {
+          if (!mbar_wait_bounded(&pv_done[pb], pph, abort_flag, err_word, ERR_WAIT_EMPTY)) break;
+          if (++pb == NBUF) {
+            pb = 0;
+            pph ^= 1u;
+          }
+        }
         uint8_t* sV = smem + C::OFF_V + vs * C::T_BYTES;
         mbar_arrive_expect_tx(&v_full[vs], C::T_BYTES);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) tma_load_3d(sV + c * (BN * 128), &tmV, &v_full[vs], colV + c * 64, (tile0 + j) * BN, b);
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ O += P_j V_j
-    {
-      const uint32_t idesc_o = make_idesc_f16(1, BM, D, 0, 1);
-      // descriptors are constants plus a stage offset (the address field counts 16-byte units): built once
-      uint64_t dV[BN / 16];
-#pragma unroll
-      for (int k = 0; k < BN / 16; ++k)   // V is MN-major (D contiguous), 64-wide D chunks BN*128 bytes apart
-        dV[k] = make_smem_desc_sw128(smem_u32(smem + C::OFF_V) + k * (16 * 128), BN * 128, 1024);
+    const uint32_t idesc_o = make_idesc_f16(1, BM, D, 0, 1);
+    // descriptors are a constant plus a stage offset (the address field counts 16-byte units); V is MN-major (D contiguous),
+    // 64-wide D chunks BN*128 bytes apart
+    const uint64_t dV = make_smem_desc_sw128(smem_u32(smem + C::OFF_V), BN * 128, 1024);
+    if (elect_one()) {
+      int bsel = 0;
+      uint32_t ph = 0u;
       for (int j = 0; j < n_kv; ++j) {
-        const int bsel = j % NBUF, vs = j % VS;
+        const int vs = j % VS;
         // P_j is in TMEM (over the first half of S_j) once the softmax warps have arrived
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&p_ready[bsel], (j / NBUF) & 1u, abort_flag, err_word, ERR_WAIT_AUX) &&
-                                         mbar_wait_bounded(&v_full[vs], (j / VS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)))
+        if (!mbar_wait_bounded(&v_full[vs], (j / VS) & 1u, abort_flag, err_word, ERR_WAIT_FULL) ||
+            !mbar_wait_bounded(&p_ready[bsel], ph, abort_flag, err_word, ERR_WAIT_AUX))
           break;
         tc_fence_after_sync();
-        const uint64_t stage = static_cast<uint64_t>((vs * C::T_BYTES) >> 4);
-        const uint32_t pcol = tmem_base + C::S_COL + bsel * BN;   // bsel = j % NBUF
+        const uint64_t v = dV + static_cast<uint64_t>((vs * C::T_BYTES) >> 4);
+        const uint32_t pcol = tmem_base + C::S_COL + bsel * BN;
         // BN/16 k-steps over keys. A = P from TMEM (16 bf16 of a row = 8 columns per step)
-        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BN / 16; ++k)
-            umma_f16_ts(tmem_base + C::O_COL, pcol + k * 8, dV[k] + stage, idesc_o, (j != 0 || k != 0) ? 1u : 0u);
-          umma_commit(&pv_done[bsel]);
-          if (j + 1 == n_kv) umma_commit(o_final);   // a barrier of its own for the last tile: the epilogue waits on nothing else
+        for (int k = 0; k < BN / 16; ++k)
+          umma_f16_ts(tmem_base + C::O_COL, pcol + k * 8, v + static_cast<uint64_t>((k * 16 * 128) >> 4), idesc_o,
+                      (j != 0 || k != 0) ? 1u : 0u);
+        umma_commit(&pv_done[bsel]);
+        if (j + 1 == n_kv) umma_commit(o_final);   // a barrier of its own for the last tile: the epilogue waits on nothing else
+        if (++bsel == NBUF) {
+          bsel = 0;
+          ph ^= 1u;
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else if (warp == 2) {
     // ------------------------------------------------------------------ S_t = Q K_t^T
-    {
-      const uint32_t idesc_s = make_idesc_f16(1, BM, BN, 0, 0);
-      uint64_t dQ[D / 16], dK[D / 16];
-#pragma unroll
-      for (int k = 0; k < D / 16; ++k) {
-        const uint32_t sub = k >> 2, kk = k & 3;   // 64-column sub-tiles are BM*128 (Q) / BN*128 (K) bytes apart
-        dQ[k] = make_smem_desc_sw128(smem_u32(smem) + sub * (BM * 128) + kk * 32, 16, 1024);
-        dK[k] = make_smem_desc_sw128(smem_u32(smem + C::OFF_K) + sub * (BN * 128) + kk * 32, 16, 1024);
-      }
-      const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(q_full, 0, abort_flag, err_word, ERR_WAIT_FULL));
+    const uint32_t idesc_s = make_idesc_f16(1, BM, BN, 0, 0);
+    const uint64_t dQ = make_smem_desc_sw128(smem_u32(smem), 16, 1024), dK = make_smem_desc_sw128(smem_u32(smem + C::OFF_K), 16, 1024);
+    if (elect_one()) {
+      const bool ok = mbar_wait_bounded(q_full, 0, abort_flag, err_word, ERR_WAIT_FULL);
+      int ks = 0, bsel = 0;
+      uint32_t kph = 0u, ph = 1u;        // ph: parity of P V of tile t - NBUF
       for (int t = 0; ok && t < n_kv; ++t) {
-        const int ks = t % KS;
         // buffer t % NBUF held S_{t-NBUF} and then P_{t-NBUF}: it is free when that tile's P V has completed
-        if (!__all_sync(0xffffffffu,
-                        (t < NBUF || mbar_wait_bounded(&pv_done[t % NBUF], ((t - NBUF) / NBUF) & 1u, abort_flag, err_word,
-                                                       ERR_WAIT_AUX)) &&
-                            mbar_wait_bounded(&k_full[ks], (t / KS) & 1u, abort_flag, err_word, ERR_WAIT_FULL)))
+        if (!mbar_wait_bounded(&k_full[ks], kph, abort_flag, err_word, ERR_WAIT_FULL) ||
+            (t >= NBUF && !mbar_wait_bounded(&pv_done[bsel], ph, abort_flag, err_word, ERR_WAIT_AUX)))
           break;
         tc_fence_after_sync();
-        const uint64_t stage = static_cast<uint64_t>((ks * C::T_BYTES) >> 4);
-        const uint32_t dcol = tmem_base + C::S_COL + (t % NBUF) * BN;
-        if (elect_one()) {
+        const uint64_t kd = dK + static_cast<uint64_t>((ks * C::T_BYTES) >> 4);
 #pragma unroll
-          for (int k = 0; k < D / 16; ++k) umma_f16_ss(dcol, dQ[k], dK[k] + stage, idesc_s, k != 0 ? 1u : 0u);
-          umma_commit(&s_full[t % NBUF]);
-          umma_commit(&k_empty[ks]);
+        for (int k = 0; k < D / 16; ++k) {   // 64-column sub-tiles are BM*128 (Q) / BN*128 (K) bytes apart
+          const uint64_t oq = static_cast<uint64_t>(((k >> 2) * (BM * 128) + (k & 3) * 32) >> 4);
+          const uint64_t okk = static_cast<uint64_t>(((k >> 2) * (BN * 128) + (k & 3) * 32) >> 4);
+          umma_f16_ss(tmem_base + C::S_COL + bsel * BN, dQ + oq, kd + okk, idesc_s, k != 0 ? 1u : 0u);
         }
-        __syncwarp();
+        umma_commit(&s_full[bsel]);
+        umma_commit(&k_empty[ks]);
+        if (++ks == KS) {
+          ks = 0;
+          kph ^= 1u;
+        }
+        if (++bsel == NBUF) {
+          bsel = 0;
+          ph ^= 1u;
+        }
       }
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------ softmax / epilogue
     const int quad = warp & 3;
