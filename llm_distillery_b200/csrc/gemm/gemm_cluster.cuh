@@ -42,7 +42,8 @@ __device__ __forceinline__ uint32_t cluster_nctas() {
 
 // Epi concept: Params; SPLIT_B (the tile's B rows are BN/2 rows at n and BN/2 rows b_half_stride below them);
 // items<BN>() work items per row; item<BN>(p, row, n0, N, it, get) with get(chunk) = the four accumulator columns
-// 4 * chunk .. 4 * chunk + 3 of the row.
+// 4 * chunk .. 4 * chunk + 3 of the row. AHEAD > 0: operands from global memory, Pre, are loaded for that many of a thread's
+// items at a time by load<BN>(p, row, n0, it, pre) - the first of them while the main loop runs - and item takes one more argument.
 template <int BN, bool DEEP, bool A_MN, bool B_MN, class Epi>
 __global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
     gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
@@ -119,6 +120,19 @@ __global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
   pdl_wait();
   pdl_trigger();
 
+  constexpr int IPR = Epi::template items<BN>(), AHEAD = Epi::AHEAD > 0 ? Epi::AHEAD : 1;
+  const int r0 = BM * slice / n_slices, r1 = min(BM * (slice + 1) / n_slices, M - m0);
+  const int n_items = max(r1 - r0, 0) * IPR, col0 = Epi::SPLIT_B ? n_blk * (BN / 2) : n0;
+  typename Epi::Pre pre[AHEAD];
+  auto load_ahead = [&](int first) {
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int i = first + u * NUM_THREADS;
+      if (i < n_items) Epi::template load<BN>(ep, m0 + r0 + i / IPR, col0, i % IPR, pre[u]);
+    }
+  };
+  if (Epi::AHEAD > 0 && warp >= 2) load_ahead(threadIdx.x);
+
   if (warp == 0) {
     if (elect_one()) {
       uint32_t st = 0, ph = 1u;
@@ -191,12 +205,9 @@ __global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
   if (n_slices > 1) cluster_sync_all(); else __syncthreads();
 
   {
-    const int r0 = BM * slice / n_slices, r1 = min(BM * (slice + 1) / n_slices, M - m0);
-    constexpr int IPR = Epi::template items<BN>();
     const uint32_t part = smem_u32(smem);
-    for (int i = threadIdx.x; i < (r1 - r0) * IPR; i += NUM_THREADS) {
-      const int row = r0 + i / IPR, it = i % IPR;
-      auto get = [&](int chunk) {
+    auto sum_of = [&](int row) {
+      return [=](int chunk) {
         const uint32_t off = part + row * (BN * 4) + ((chunk ^ (row & 15)) << 4);
         float4 a;
         if (n_slices == 1) {
@@ -213,7 +224,22 @@ __global__ void __launch_bounds__(NUM_THREADS, DEEP ? 1 : 2)
         }
         return a;
       };
-      Epi::template item<BN>(ep, m0 + row, Epi::SPLIT_B ? n_blk * (BN / 2) : n0, N, it, get);
+    };
+    if constexpr (Epi::AHEAD > 0) {
+      if (warp < 2) load_ahead(threadIdx.x);
+      for (int first = threadIdx.x; first < n_items; first += AHEAD * NUM_THREADS) {
+        if (first != (int)threadIdx.x) load_ahead(first);
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+          const int i = first + u * NUM_THREADS, row = r0 + i / IPR;
+          if (i < n_items) Epi::template item<BN>(ep, m0 + row, col0, N, i % IPR, sum_of(row), pre[u]);
+        }
+      }
+    } else {
+      for (int i = threadIdx.x; i < n_items; i += NUM_THREADS) {
+        const int row = r0 + i / IPR;
+        Epi::template item<BN>(ep, m0 + row, col0, N, i % IPR, sum_of(row));
+      }
     }
   }
 

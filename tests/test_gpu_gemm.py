@@ -213,6 +213,33 @@ def test_one_slice_keeps_the_order_of_the_pair_kernel(T):
     assert _lib.take_device_error() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 4, 64), (31, 68, 200), (93, 2048, 1024), (130, 132, 896), (777, 896, 264)])
+@pytest.mark.parametrize("split", [False, True])
+def test_few_tile_stores_of_both_forms(M, N, K, split):
+    """Outputs whose rows start on boundaries of four columns and outputs that are off them hold the same bits: plain, with a
+    residual, and fp32 stored and added."""
+    g = torch.Generator("cuda").manual_seed(M + N)
+    x, w = (torch.randn(n, K, device=DEV, generator=g).bfloat16() for n in (M, N))
+    res = torch.randn(M, N, device=DEV, generator=g).bfloat16()
+
+    def off(t):
+        o = torch.zeros(M, N + 1, device=DEV, dtype=t.dtype)[:, :N]
+        return o.copy_(t)
+    for b_mn in (False, True)[:1 + (N % 8 == 0)]:
+        b = w.t().contiguous() if b_mn else w
+        a = basic.gemm(x, b, b_mn=b_mn, split_k=split)
+        assert torch.equal(a, basic.gemm(x, b, b_mn=b_mn, out=off(a * 0), split_k=split))
+        r = basic.gemm(x, b, b_mn=b_mn, residual=res, split_k=split)
+        assert torch.equal(r, basic.gemm(x, b, b_mn=b_mn, residual=res, out=off(a * 0), split_k=split))
+    dy, xt = torch.randn(K, 8 * M, device=DEV, generator=g).bfloat16(), torch.randn(K, N + (-N) % 8, device=DEV, generator=g).bfloat16()
+    f = basic.gemm(dy, xt, a_mn=True, b_mn=True, out_dtype=torch.float32, split_k=split)
+    o = torch.zeros(f.shape[0], f.shape[1] + 1, device=DEV)[:, :-1]
+    assert torch.equal(f, basic.gemm(dy, xt, a_mn=True, b_mn=True, out=o, split_k=split))
+    twice = basic.gemm(dy, xt, a_mn=True, b_mn=True, out=f.clone(), accumulate=True, split_k=split)
+    assert torch.equal(twice, basic.gemm(dy, xt, a_mn=True, b_mn=True, out=o, accumulate=True, split_k=split))
+    assert _lib.take_device_error() == 0
+
+
 @pytest.mark.parametrize("T,f,h", [(5003, 1408, 520), (4737, 1152, 264), (18945, 128, 256), (4865, 1280, 2048)])
 def test_swiglu_backward_epilogue_of_ragged_pair_tiles(T, f, h):
     """Rows that end inside a warp's 32 and features that end in the middle of a 256 x 256 tile: the bits of GEMM + separate
