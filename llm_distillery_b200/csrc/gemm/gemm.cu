@@ -1095,13 +1095,14 @@ static bool use_pair(int M, int N, int K) {
 // cross-entropies, and turned a last bit of an activation into 0.1 to 0.7 % of its value (38 runs of five students, 200
 // to 1100 tokens; the KL losses: 0.001 %), so that the loss of a conversation would depend on the batch that it is in.
 //
-// Times in microseconds, least squares over sizes from 93 to 3000 tokens on layers of 256 to 14336 (B200, weights from
-// HBM; within 4 - 8 %): a cluster CTA costs a fixed part (launch, first loads, exchange, epilogue) and a part per K
+// Times in microseconds, least squares over 296 sizes from 40 to 2048 tokens on layers of 256 to 28672 (B200, weights from
+// HBM; within 5 - 9 %), then moved a little towards the choices that were measured best: the chosen form takes 0.2 % longer than
+// the best one on average, with the constants of the kernel before its issuing loops were the elected lane's 2.2 % (single sizes
+// 25 %). A cluster CTA costs a fixed part (launch, first loads, exchange, epilogue) and a part per K
 // block, more of both when two share an SM; the 256 x 256 kernel pays per round of its SM pairs. Clusters do not pack
 // onto the last SMs of the chip (294 CTAs in clusters of 3 or 6 ran as two rounds), so split tiles stop at 7/8 of the
-// resident CTAs. Examples, one CTA per tile before / cluster now: 93 x 2048 x 5632 37.8 / 11.0, 93 x 2560 x 2048 17.2 /
-// 7.4, 777 x 896 x 9728 59.3 / 21.4 (43.4 in one slice), 896 x 896 x 776 (weight gradient) 11.3 / 7.7; 2048 x 2048 x 2048
-// stays where it is (17.7, cluster 20.2: tiles of 128 x 128 read twice the operand bytes per product and are bound by the L2).
+// resident CTAs. Examples, 128 x 256 tiles of one CTA / cluster: 93 x 2048 x 5632 37.8 / 10.2, 93 x 2560 x 2048 17.2 /
+// 7.4, 777 x 896 x 4864 32.7 / 18.6 in one slice, 1100 x 512 x 512 8.1 / 4.2; 2048 x 2048 x 2048 17.7, cluster 18.0.
 struct TilePlan {
   int bn, slices;
   int b_early = 0;      // B may be loaded before the kernel in front of this one has completed
@@ -1114,8 +1115,9 @@ static bool deep_ring(long long ctas, int slices) {
 static TilePlan plan_tiles(int M, int N, int K, bool f32, bool split) {
   // [bn = 64, 128][deep ring, one CTA per SM, two]: fixed, per K block, split, per slice
   static const double kCost[2][3][4] = {
-      {{4.33, 0.256, 0.78, -0.081}, {4.73, 0.295, 0.0, 0.064}, {4.05, 0.331, 1.34, 0.134}},
-      {{6.04, 0.275, 1.20, -0.249}, {6.56, 0.396, 0.0, 0.055}, {6.05, 0.457, 0.89, 0.219}}};
+      {{2.66, 0.181, 1.39, -0.030}, {1.99, 0.252, 2.12, 0.002}, {2.57, 0.279, 1.52, 0.141}},
+      {{3.79, 0.200, 2.15, -0.147}, {2.64, 0.366, 2.64, 0.045}, {3.47, 0.398, 2.26, 0.183}}};
+  static const double kUneven = 0.2;      // slices that are no power of two: rows and clusters do not divide evenly
   const int sms = sm_count(), num_kb = ceil_div(K, BK);
   const long long pair_tiles = (long long)ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
   TilePlan plan{0, 1};
@@ -1124,7 +1126,7 @@ static TilePlan plan_tiles(int M, int N, int K, bool f32, bool split) {
     const int s = pair_k_splits((int)pair_tiles, num_kb, sms / 2, &rounds);
     if (!split && s > 1 && use_pair(M, N, K)) return plan;      // that order of additions stays
   }
-  double least = 0.95 * (4.8 + rounds * (0.328 * num_kb + (f32 ? 3.2 : 1.3)));
+  double least = 6.0 + rounds * (0.344 * num_kb + (f32 ? 2.7 : 0.76));
   for (int w = 0; w < 2; ++w) {
     const int bn = w ? 128 : 64;
     const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, bn);
@@ -1132,7 +1134,7 @@ static TilePlan plan_tiles(int M, int N, int K, bool f32, bool split) {
       const long long ctas = tiles * s;
       if (ctas > (s > 1 ? 2LL * sms * 7 / 8 : 2LL * sms)) break;
       const double* c = kCost[w][deep_ring(ctas, s) ? 0 : ctas > sms ? 2 : 1];
-      const double us = c[0] + c[1] * ceil_div(num_kb, s) + (s > 1 ? c[2] : 0.0) + c[3] * s;
+      const double us = c[0] + c[1] * ceil_div(num_kb, s) + (s > 1 ? c[2] : 0.0) + c[3] * s + (s & (s - 1) ? kUneven : 0.0);
       if (us < least) { least = us; plan = TilePlan{bn, s}; }
     }
   }
