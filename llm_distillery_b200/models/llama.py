@@ -486,7 +486,25 @@ class LlamaModel(nn.Module):
                 stack.append((w, b_qkv, *table, cfg.layer_window(li, L)))
             if len(stack) < len(self.layers) - first or len({w[4].shape for w, *_ in stack}) > 1:
                 stack = []
+        ahead = 0
+        if (plain and pre is None and LAYER_WEIGHTS_PRE[0] is None and not cfg.sandwich and not cfg.num_local_experts
+                and not training and h.is_cuda and B * L <= layer_native.STACK_MAX_TOKENS):
+            fitting = {}       # of each table, looked at once
+
+            def entry(i):
+                layer, table = self.layers[i], tables[i]
+                b_qkv = getattr(layer, "qkv_bias", None)
+                w = (layer.input_layernorm, layer.qkv_proj, layer.o_proj, layer.post_attention_layernorm, layer.gate_up_proj,
+                     layer.down_proj)
+                if id(table) not in fitting:
+                    fitting[id(table)] = layer_native.tables_fit(pos, *table, B * L, cfg.head_dim)
+                if not layer_native.fits(h, pos, *table, w, b_qkv, heads, False, fitting[id(table)]):
+                    return None
+                return w, b_qkv, *table, cfg.layer_window(i, L)
+            h, ahead = layer_native.run_inference(h, pos, entry, len(self.layers), meta7, split[0])
         for li, (layer, table) in enumerate(zip(self.layers, tables)):
+            if li < ahead:
+                continue
             if stack and li == first:
                 h = layer_native.run_stack(h, pos, stack, meta7, split)
                 break

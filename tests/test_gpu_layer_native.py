@@ -96,6 +96,41 @@ def test_layers_in_one_call_equal_a_call_each(monkeypatch, between):
         assert torch.equal(results[1][1][name], want), name
 
 
+@pytest.mark.parametrize("layers", [1, 2, 9])
+@pytest.mark.parametrize("refused", [None, 0, 3])
+def test_inference_in_calls_of_several_layers_equals_a_call_each(monkeypatch, layers, refused):
+    """Passes without gradients run 1, 1, 2, 4, ... layers a call, up to a layer that does not fit; the bits of a call per
+    layer, with windows that differ from layer to layer, in plain and in K-cutting GEMMs."""
+    cfg = llama.LlamaConfig(vocab_size=512, hidden_size=256, intermediate_size=640, num_hidden_layers=layers, num_attention_heads=4,
+                            num_key_value_heads=2, max_position_embeddings=512, attention_bias=True, sliding_window=50,
+                            window_layers=[i % 2 == 0 for i in range(layers)])
+    model = llama.build_model(cfg, dtype=torch.bfloat16, device="cuda", seed=3)
+    ids = torch.randint(0, 512, (2, 173), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    weight = model.layers[refused].qkv_proj if refused is not None and refused < layers else None
+    real, lib, calls = layer_native.fits, _lib.kernels(), []
+    monkeypatch.setattr(layer_native, "fits", lambda *a: a[4][1] is not weight and real(*a))
+
+    class Recorder:
+        def __getattr__(self, name):
+            fn = getattr(lib, name)
+            if name != "b200_stack_fwd":
+                return fn
+            return lambda rows, n, *a: calls.append(n) or fn(rows, n, *a)
+    monkeypatch.setattr(_lib, "kernels", Recorder)
+    for ordered in (True, False):
+        model.ordered_sums = ordered
+        got = []
+        for limit in (0, layer_native.STACK_MAX_TOKENS):
+            monkeypatch.setattr(layer_native, "STACK_MAX_TOKENS", limit)
+            with torch.no_grad():
+                got.append(model.hidden_states(ids))
+        assert torch.equal(*got)
+    fit = layers if weight is None else refused
+    sizes = [n for n in (1, 1, 2, 4, 8)]
+    want = [min(n, fit - sum(sizes[:i])) for i, n in enumerate(sizes) if sum(sizes[:i]) < fit]
+    assert calls == want * 2 and _lib.take_device_error() == 0
+
+
 @pytest.mark.parametrize("embedding,layers,stacked", [(True, 0, 5), (True, 2, 3), (True, 5, 0), (False, 2, 5)])
 def test_layers_that_no_gradient_reaches_stay_out_of_the_one_call(monkeypatch, embedding, layers, stacked):
     """Frozen embedding and first layers: outputs and gradients bit for bit those of a node per layer, whose backward pass ends at
