@@ -354,6 +354,7 @@ struct RopeParams {
   int n_rot;            // first n_rot columns are rotated ((H + Hkv) * d)
 };
 
+template <int D>
 struct EpiRope {
   using Params = RopeParams;
   static constexpr bool SPLIT_K = false;
@@ -379,9 +380,22 @@ struct EpiRope {
     uint8_t* stage = epi_smem + quad * STAGE_BYTES;
     const int row0 = m0 + quad * 32;
     const int rows_valid = min(32, M - row0);
-    const int half_d = p.d >> 1;
+    constexpr int half_d = D >> 1;
     const long long tpos = lane < rows_valid ? (long long)p.pos[row0 + lane] : 0;
-    const int step = p.d == 64 ? 1 : 2;                   // distance, in chunks, between the two halves of a pair
+    // heads of 64: all pairs of a row take the same 32 entries, fetched once for the tile (once per pair: 16384 x 2560 x 2048
+    // 130 us, now 116)
+    float cc[32], ss[32];
+    auto entries = [&](int j0) {
+      const float* cp = p.cs + tpos * half_d + j0;
+      const float* sp = p.sn + tpos * half_d + j0;
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) {
+        const float4 c4 = *reinterpret_cast<const float4*>(cp + j), s4 = *reinterpret_cast<const float4*>(sp + j);
+        cc[j] = c4.x; cc[j + 1] = c4.y; cc[j + 2] = c4.z; cc[j + 3] = c4.w;
+        ss[j] = s4.x; ss[j + 1] = s4.y; ss[j + 2] = s4.z; ss[j + 3] = s4.w;
+      }
+    };
+    if (D == 64 && n0 < p.n_rot) entries(0);
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
       const int colh = n0 + half * 128;
@@ -389,33 +403,27 @@ struct EpiRope {
 #pragma unroll 1
       for (int k = 0; k < 2; ++k) {
         // d = 64: pair (0,1) then (2,3); d = 128: pair (0,2) then (1,3)
-        const int ca = p.d == 64 ? 2 * k : k;
-        const int cb = ca + step;
+        const int ca = D == 64 ? 2 * k : k;
+        const int cb = ca + (D == 64 ? 1 : 2);
         uint32_t ra[32], rb[32];
         tmem_ld_32x32b_x32(taddr + half * 128 + ca * 32, ra);
         tmem_ld_32x32b_x32(taddr + half * 128 + cb * 32, rb);
-        tmem_ld_wait();
+        const bool rotate = colh + ca * 32 < p.n_rot;
+        if (D == 128 && rotate) entries(k * 32);
+        tmem_ld_wait_for(ra);
+        tmem_ld_wait_for(rb);
         float a[32], b[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           a[j] = __bfloat162float(__float2bfloat16(__uint_as_float(ra[j])));
           b[j] = __bfloat162float(__float2bfloat16(__uint_as_float(rb[j])));
         }
-        if (colh + ca * 32 < p.n_rot) {
-          const int j0 = p.d == 64 ? 0 : k * 32;          // first cos / sin entry of chunk ca
-          const float* cp = p.cs + tpos * half_d + j0;
-          const float* sp = p.sn + tpos * half_d + j0;
+        if (rotate) {
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const float4 c4v = *reinterpret_cast<const float4*>(cp + j);
-            const float4 s4v = *reinterpret_cast<const float4*>(sp + j);
-            const float cc[4] = {c4v.x, c4v.y, c4v.z, c4v.w}, ss[4] = {s4v.x, s4v.y, s4v.z, s4v.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float fa = a[j + e], fb = b[j + e];
-              a[j + e] = __fmaf_rn(fa, cc[e], -__fmul_rn(fb, ss[e]));
-              b[j + e] = __fmaf_rn(fb, cc[e], __fmul_rn(fa, ss[e]));
-            }
+          for (int j = 0; j < 32; ++j) {
+            const float fa = a[j], fb = b[j];
+            a[j] = __fmaf_rn(fa, cc[j], -__fmul_rn(fb, ss[j]));
+            b[j] = __fmaf_rn(fb, cc[j], __fmul_rn(fa, ss[j]));
           }
         }
         put(stage, lane, ca, a);
@@ -426,9 +434,10 @@ struct EpiRope {
   }
 };
 
+template <int D>
 static int launch_rope_pair(const void* A, const void* W, int M, int N, int K, long long lda, long long ldb,
                             const RopeParams& rp, cudaStream_t stream) {
-  using Epi = EpiRope;
+  using Epi = EpiRope<D>;
   constexpr int STAGES = 6;
   using S = SmemPair<STAGES>;
   CUtensorMap tmA, tmB;
@@ -566,6 +575,93 @@ struct EpiSwigluBwd {
           *reinterpret_cast<uint4*>(dst + (long long)row * p.ld_dgu) = *reinterpret_cast<const uint4*>(sg + off);
           *reinterpret_cast<uint4*>(dst + (long long)row * p.ld_dgu + p.f) = *reinterpret_cast<const uint4*>(su + off);
         }
+      }
+      __syncwarp();                                      // the stage may be filled again
+    }
+  }
+};
+
+// bf16 output with a residual, whole groups of eight columns on 16-byte boundaries: the residual's quarters of 64 columns arrive
+// like the gate values above, every lane adds its row's sums to them (scaled and added in fp32, rounded once, as EpiStore does)
+// and the stage leaves as whole row segments. Loaded by each lane from its own row behind the accumulator, the residual cost
+// 16384 x 2048 x 2048 100 us where it is 93 now.
+struct EpiResidual {
+  using Params = StoreParams;
+  static constexpr bool SPLIT_K = false;
+  static constexpr bool PREFETCH = true;
+  static constexpr int QUARTER = 32 * 128;
+  static constexpr int STAGE_BYTES = 2 * QUARTER;
+  static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;
+
+  static bool fits(const Params& p, int N) {
+    return p.resid && !p.out_f32 && p.fmt == 1 && !p.accumulate && !(N & 7) && !(p.ldc & 7) && !(p.ldr & 7) &&
+           !(reinterpret_cast<uintptr_t>(p.C) & 15) && !(reinterpret_cast<uintptr_t>(p.resid) & 15);
+  }
+
+  static __device__ __forceinline__ void fetch(const Params& p, int q, int m0, int n0, int M, int N, int quad, int lane,
+                                               uint8_t* epi_smem) {
+    const int row0 = m0 + quad * 32, col = n0 + q * 64 + (lane & 7) * 8;
+    if (col < N) {
+      const uint32_t dst = smem_u32(epi_smem + quad * STAGE_BYTES + (q & 1) * QUARTER);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int row = 4 * j + (lane >> 3);
+        if (row0 + row < M)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + row * 128 + (((lane & 7) ^ (row & 7)) << 4)),
+                       "l"(p.resid + (long long)(row0 + row) * p.ldr + col)
+                       : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+
+  static __device__ __forceinline__ void prefetch(const Params& p, int m0, int n0, int M, int N, int quad, int lane,
+                                                  uint8_t* epi_smem) {
+    fetch(p, 0, m0, n0, M, N, quad, lane, epi_smem);
+  }
+
+  static __device__ __forceinline__ void tile(const Params& p, uint32_t taddr, int m0, int n0, int M, int N, int quad,
+                                              int lane, uint8_t* epi_smem) {
+    const int row0 = m0 + quad * 32;
+    __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C);
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+      if (q < 3) {
+        fetch(p, q + 1, m0, n0, M, N, quad, lane, epi_smem);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      __syncwarp();
+      if (n0 + q * 64 >= N) continue;
+      uint8_t* stage = epi_smem + quad * STAGE_BYTES + (q & 1) * QUARTER;
+      uint32_t r[2][32];
+      tmem_ld_32x32b_x32(taddr + q * 64, r[0]);
+      tmem_ld_32x32b_x32(taddr + q * 64 + 32, r[1]);
+      tmem_ld_wait_for(r[0]);
+      tmem_ld_wait_for(r[1]);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        uint4* at = reinterpret_cast<uint4*>(stage + lane * 128 + ((c ^ (lane & 7)) << 4));
+        uint4 o = *at;
+        uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const float2 f = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w[t]));
+          const uint32_t* v = &r[c >> 2][(c & 3) * 8 + 2 * t];
+          w[t] = pack_bf16x2(__fadd_rn(__fmul_rn(__uint_as_float(v[0]), p.alpha), f.x),
+                             __fadd_rn(__fmul_rn(__uint_as_float(v[1]), p.alpha), f.y));
+        }
+        *at = o;
+      }
+      __syncwarp();
+      const int col = n0 + q * 64 + (lane & 7) * 8;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int row = 4 * j + (lane >> 3);
+        if (row0 + row < M && col < N)
+          *reinterpret_cast<uint4*>(C + (long long)(row0 + row) * p.ldc + col) =
+              *reinterpret_cast<const uint4*>(stage + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
       }
       __syncwarp();                                      // the stage may be filled again
     }
@@ -738,10 +834,9 @@ static int launch_grouped(const void* A, const void* B, int M, int N, int K, lon
 }
 
 // Two-SM (cta_group::2) launch: 256 x 256 tiles, one CTA pair per tile.
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, class Epi = EpiStore<PAIR_BN>>
 static int launch_store_pair(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int fmt,
                              const StoreParams& sp, cudaStream_t stream) {
-  using Epi = EpiStore<PAIR_BN>;
   constexpr int STAGES = 6;
   using S = SmemPair<STAGES>;
   CUtensorMap tmA, tmB;
@@ -1236,7 +1331,8 @@ int b200_gemm_rope(const void* x, const void* W, void* out, const int* pos, cons
     return d == 64 ? launch_cluster_bn<false, false, ClusterRope<64>>(x, W, M, N, K, ldx, ldw, 1, rp, plan, 0, stream)
                    : launch_cluster_bn<false, false, ClusterRope<128>>(x, W, M, N, K, ldx, ldw, 1, rp, plan, 0, stream);
   }
-  return launch_rope_pair(x, W, M, N, K, ldx, ldw, rp, stream);
+  return d == 64 ? launch_rope_pair<64>(x, W, M, N, K, ldx, ldw, rp, stream)
+                 : launch_rope_pair<128>(x, W, M, N, K, ldx, ldw, rp, stream);
 }
 
 // dgu[M, 2f] = SwiGLU backward of (gu, d(act)) with d(act) = dy[M, K] Wd[K, f] taken straight from the accumulator
@@ -1308,6 +1404,8 @@ int b200_gemm(const void* A, const void* B, void* C, int M, int N, int K, long l
     }
   }
   if (!dcp && use_pair(M, N, K)) {
+    if (!a_mn && !b_mn && EpiResidual::fits(sp, N))
+      return launch_store_pair<false, false, EpiResidual>(A, B, M, N, K, lda, ldb, fmt, sp, stream);
     if (!a_mn && !b_mn) return launch_store_pair<false, false>(A, B, M, N, K, lda, ldb, fmt, sp, stream);
     if (!a_mn && b_mn) return launch_store_pair<false, true>(A, B, M, N, K, lda, ldb, fmt, sp, stream);
     if (a_mn && b_mn) return launch_store_pair<true, true>(A, B, M, N, K, lda, ldb, fmt, sp, stream);

@@ -254,6 +254,21 @@ def test_swiglu_backward_epilogue_of_ragged_pair_tiles(T, f, h):
     assert (out[T:] == 7.0).all() and _lib.take_device_error() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(5003, 1416, 520), (4737, 1160, 264), (18945, 200, 256), (8200, 2048, 2048)])
+def test_residual_epilogue_of_ragged_pair_tiles(M, N, K):
+    """Rows that end inside a warp's 32 and columns that end inside a quarter of a 256 x 256 tile: the bits of the general
+    epilogue (an output off the 16-byte boundaries takes it), in place too, and nothing written outside the output."""
+    g = torch.Generator("cuda").manual_seed(M)
+    x, w = (torch.randn(n, K, device=DEV, generator=g).bfloat16() for n in (M, N))
+    res = torch.randn(M, N, device=DEV, generator=g).bfloat16()
+    plain = torch.zeros(M, N + 1, device=DEV, dtype=torch.bfloat16)[:, :N]
+    basic.gemm(x, w, residual=res, alpha=0.37, out=plain)
+    out = torch.full((M + 40, N + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    basic.gemm(x, w, residual=res, alpha=0.37, out=out[:M, :N])
+    assert torch.equal(out[:M, :N], plain) and (out[M:] == 7.0).all() and (out[:, N:] == 7.0).all()
+    assert torch.equal(basic.gemm(x, w, residual=res, alpha=0.37, out=res), plain) and _lib.take_device_error() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(8, 64, 64), (128, 128, 512), (136, 72, 200), (304, 1152, 896)])
 @pytest.mark.parametrize("layout,dtype", [("nt", torch.float16), ("nn", torch.float16), ("tn", torch.float16),
                                           ("tt", torch.float16), ("tt", torch.bfloat16)])
