@@ -180,3 +180,33 @@ def test_optimizer_kernels_match_torch_restatement(name):
     tol = 3e-2 if name == "adamw8bit" else 1e-4
     assert torch.allclose(fg.master.cpu(), fc.master, atol=tol, rtol=tol), (fg.master.cpu() - fc.master).abs().max()
     assert torch.allclose(w.detach().float().cpu(), fg.master.cpu()[: w.numel()].view(300, 70), atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("n", [1, 6, 255, 256, 260, 2047, 70001])
+@pytest.mark.parametrize("decoupled", [0, 1])
+def test_8bit_adam_of_aligned_and_unaligned_shards(n, decoupled):
+    """Blocks cut short, and buffers off the 16-byte boundaries: the same bits on both paths, nothing written behind the last
+    value, and after the first step every block's scales are the maxima of its moments ((1 - beta) g, sqrt((1 - beta2) g^2):
+    three roundings each)."""
+    gen = torch.Generator("cuda").manual_seed(n)
+    w0, g = (torch.randn(n, device=DEV, generator=gen) for _ in range(2))
+    nb = (n + 255) // 256
+
+    def run(off):
+        f = [torch.full((n + off + 8,), 7.0, device=DEV, dtype=d) for d in (torch.float32, torch.bfloat16, torch.float32)]
+        c = [torch.full((n + off + 8,), 7, device=DEV, dtype=d) for d in (torch.int8, torch.uint8)]
+        s = torch.zeros(2, nb, device=DEV)
+        w, m, gr, mq, vq = (t[off:off + n] for t in (f[0], f[1], f[2], *c))
+        w.copy_(w0), gr.copy_(g), mq.zero_(), vq.zero_()
+        scales = []
+        for step in (1, 2):
+            _lib.check(_lib.kernels().b200_adam8_step(
+                _lib.ptr(w), _lib.ptr(m), _lib.ptr(gr), _lib.ptr(mq), _lib.ptr(vq), _lib.ptr(s[0]), _lib.ptr(s[1]), n, 1e-3, 0.9,
+                0.99, 1e-8, 0.01, step, 1.0, decoupled, _lib.stream()), "adam step")
+            scales.append(s.clone())
+        assert all((t[:off] == 7).all() and (t[off + n:] == 7).all() for t in (*f, *c))
+        return w, m, mq, vq, *scales
+    got, off1 = run(0), run(1)
+    assert all(torch.equal(a, b) for a, b in zip(got, off1)) and _lib.take_device_error() == 0
+    ge = torch.nn.functional.pad((g if decoupled else g + 0.01 * w0).double(), (0, nb * 256 - n)).view(nb, 256).abs().amax(1)
+    assert torch.allclose(got[4][0].double(), 0.1 * ge, rtol=4e-7) and torch.allclose(got[4][1].double(), 0.1 * ge, rtol=4e-6)
