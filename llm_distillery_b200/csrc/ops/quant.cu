@@ -21,9 +21,8 @@ __constant__ float kNF4[16] = {-1.0f, -0.6961928009986877f, -0.5250730514526367f
                                0.07958029955625534f, 0.16093020141124725f, 0.24611230194568634f, 0.33791524171829224f,
                                0.44070982933044434f, 0.5626170039176941f, 0.7229568362236023f, 1.0f};
 
-// One launch expands up to MAX_PARTS matrices (the four of a decoder layer): their 16-value groups form one index space,
-// so that the short ones fill the tail of the long one. A TinyLlama layer (44 M values) took 34 us as four launches, each
-// with its own ramp and tail; its bytes need 17.
+// One launch expands up to MAX_PARTS matrices (the four of a decoder layer): their blocks form one index space, so that the
+// short ones fill the tail of the long one, where four launches would each have their own ramp and tail.
 constexpr int MAX_PARTS = 4;
 struct Nf4Part {
   const uint8_t* packed;
@@ -31,76 +30,109 @@ struct Nf4Part {
   const float* absmax_scale;
   __nv_bfloat16* out;
   float offset;
-  long long end;        // groups of this part and those before it
+  long long units;      // groups of eight values
+  int end;              // blocks of this part and those before it
 };
 struct Nf4Parts { Nf4Part part[MAX_PARTS]; int n; };
 struct Int8Part {
   const int8_t* code;
   const float* row_scale;
   __nv_bfloat16* out;
-  int groups_per_row;
-  long long end;
+  int units_per_row;    // groups of eight values
+  long long units;
+  int end;
 };
 struct Int8Parts { Int8Part part[MAX_PARTS]; int n; };
 
-// 16 values (8 packed bytes) per thread; sizes are multiples of 64, so a thread never straddles a block.
+// Bound by HBM and L2: 2.5 bytes a value. A thread takes four groups of eight values (4 packed bytes, 16 bytes of output), a
+// block apart, so that every access of a warp is one run, and all of its loads are under way before the first is used; the
+// blocks cover each part in order and none straddles two. Issue slots come next (two thirds of them at 10 instructions a value),
+// so the table is indexed in bytes and a block holds one second-level scale. A TinyLlama layer (44 M values) 21.1 us alone and
+// 24.6 behind large GEMMs, 218 M values 86 (5.3 / 6.3 TB/s); groups of 16 in two stores 32 bytes apart, walked by a resident
+// grid: 23.8, 33.4, 107.
+constexpr int UNITS = 4;
 __global__ void __launch_bounds__(256) dequant_nf4_kernel(const __grid_constant__ Nf4Parts ps) {
   pdl_wait();
   pdl_trigger();
   __shared__ float lut[16];
   if (threadIdx.x < 16) lut[threadIdx.x] = kNF4[threadIdx.x];
-  __syncthreads();
-  const long long total = ps.part[ps.n - 1].end;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    int m = 0;
-    while (i >= ps.part[m].end) ++m;
-    const Nf4Part& p = ps.part[m];
-    const long long g = m ? i - ps.part[m - 1].end : i;
-    const long long blk = g >> 2;  // 64-value block
-    const float am = (float)p.absmax_code[blk] * p.absmax_scale[blk >> 8] + p.offset;
-    const uint2 q = reinterpret_cast<const uint2*>(p.packed)[g];
-    uint32_t w[8];
+  int m = 0;
+  while ((int)blockIdx.x >= ps.part[m].end) ++m;
+  const Nf4Part& p = ps.part[m];
+  const long long base = (long long)(blockIdx.x - (m ? ps.part[m - 1].end : 0)) * (256 * UNITS);
+  const int left = (int)min(p.units - base, (long long)(256 * UNITS));
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(p.packed) + base;
+  const int8_t* code = p.absmax_code + (base >> 3);      // 64-value blocks,
+  const float scale = p.absmax_scale[base >> 11], offset = p.offset;               // 256 of them a scale
+  uint4* out = reinterpret_cast<uint4*>(p.out) + base;
+  uint32_t q[UNITS];
+  float am[UNITS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t byte = ((j < 4 ? q.x : q.y) >> (8 * (j & 3))) & 0xffu;
-      w[j] = pack_bf16x2(lut[byte >> 4] * am, lut[byte & 15u] * am);
+  for (int k = 0; k < UNITS; ++k) {
+    const int u = threadIdx.x + k * 256;
+    if (u >= left) continue;
+    q[k] = src[u];
+    am[k] = (float)code[u >> 3];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < UNITS; ++k) {
+    const int u = threadIdx.x + k * 256;
+    if (u >= left) continue;
+    const float a = am[k] * scale + offset;
+    auto value = [&](uint32_t byte_offset) { return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(lut) + byte_offset); };
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {                        // of byte j the high half first
+      const uint32_t hi = (q[k] >> (8 * j + 2)) & 0x3cu, lo = (j ? q[k] >> (8 * j - 2) : q[k] << 2) & 0x3cu;
+      w[j] = pack_bf16x2(value(hi) * a, value(lo) * a);
     }
-    uint4* o = reinterpret_cast<uint4*>(p.out + (g << 4));
-    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    out[u] = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
-// 16 values per thread; row lengths are multiples of 16.
+// As above, from 8 codes to 16 bytes a group; the row of a group is found from the block's first one. 44 M values 28 us, 218 M 112
+// (groups of 16 in a resident grid, a 64-bit division each: 42, 173).
 __global__ void __launch_bounds__(256) dequant_int8_kernel(const __grid_constant__ Int8Parts ps) {
   pdl_wait();
   pdl_trigger();
-  const long long total = ps.part[ps.n - 1].end;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    int m = 0;
-    while (i >= ps.part[m].end) ++m;
-    const Int8Part& p = ps.part[m];
-    const long long g = m ? i - ps.part[m - 1].end : i;
-    const float sc = p.row_scale[g / p.groups_per_row];
-    const uint4 q = reinterpret_cast<const uint4*>(p.code)[g];
-    const uint32_t words[4] = {q.x, q.y, q.z, q.w};
-    uint32_t w[8];
+  int m = 0;
+  while ((int)blockIdx.x >= ps.part[m].end) ++m;
+  const Int8Part& p = ps.part[m];
+  const long long base = (long long)(blockIdx.x - (m ? ps.part[m - 1].end : 0)) * (256 * UNITS);
+  const int left = (int)min(p.units - base, (long long)(256 * UNITS));
+  const uint2* src = reinterpret_cast<const uint2*>(p.code) + base;
+  uint4* out = reinterpret_cast<uint4*>(p.out) + base;
+  const long long row = base / p.units_per_row;
+  const uint32_t first = (uint32_t)(base - row * p.units_per_row), per_row = p.units_per_row;
+  const float* scale = p.row_scale + row;
+  uint2 q[UNITS];
+  float sc[UNITS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t two = words[j >> 1] >> (16 * (j & 1));
-      w[j] = pack_bf16x2((float)(int8_t)(two & 0xffu) * sc, (float)(int8_t)((two >> 8) & 0xffu) * sc);
+  for (int k = 0; k < UNITS; ++k) {
+    const int u = threadIdx.x + k * 256;
+    if (u >= left) continue;
+    q[k] = src[u];
+    sc[k] = scale[(first + u) / per_row];
+  }
+#pragma unroll
+  for (int k = 0; k < UNITS; ++k) {
+    const int u = threadIdx.x + k * 256;
+    if (u >= left) continue;
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t two = (j < 2 ? q[k].x : q[k].y) >> (16 * (j & 1));
+      w[j] = pack_bf16x2((float)(int8_t)(two & 0xffu) * sc[k], (float)(int8_t)((two >> 8) & 0xffu) * sc[k]);
     }
-    uint4* o = reinterpret_cast<uint4*>(p.out + (g << 4));
-    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    out[u] = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
-static int grid_for(long long items) {
-  long long b = (items + 255) / 256;
-  const long long cap = (long long)sm_count() * 8;
-  if (b > cap) b = cap;
-  return (int)(b < 1 ? 1 : b);
+// blocks of a part and those before it; 0: beyond a grid
+static int blocks_to(long long end, long long units) {
+  end += (units + 256 * UNITS - 1) / (256 * UNITS);
+  return end > 0x7fffffffll ? 0 : (int)end;
 }
 
 }  // namespace quant
@@ -116,16 +148,16 @@ int b200_dequant_nf4(const void* const* packed, const void* const* absmax_code, 
     return B200_ERR_ARG;
   quant::Nf4Parts ps{};
   ps.n = n_parts;
-  long long end = 0;
+  int end = 0;
   for (int i = 0; i < n_parts; ++i) {
     if (!packed[i] || !absmax_code[i] || !absmax_scale[i] || !out[i] || counts[i] <= 0 || (counts[i] & 63) ||
         (reinterpret_cast<uintptr_t>(packed[i]) & 7) || (reinterpret_cast<uintptr_t>(out[i]) & 15))
       return B200_ERR_ARG;
-    end += counts[i] >> 4;
+    if (!(end = quant::blocks_to(end, counts[i] >> 3))) return B200_ERR_ARG;
     ps.part[i] = quant::Nf4Part{(const uint8_t*)packed[i], (const int8_t*)absmax_code[i], absmax_scale[i],
-                                (__nv_bfloat16*)out[i], offset[i], end};
+                                (__nv_bfloat16*)out[i], offset[i], counts[i] >> 3, end};
   }
-  launch_pdl(quant::dequant_nf4_kernel, quant::grid_for(end), 256, 0, st, ps);
+  launch_pdl(quant::dequant_nf4_kernel, end, 256, 0, st, ps);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
@@ -135,15 +167,16 @@ int b200_dequant_int8(const void* const* code, const float* const* row_scale, vo
   if (!code || !row_scale || !out || !rows || !cols || n_parts < 1 || n_parts > quant::MAX_PARTS) return B200_ERR_ARG;
   quant::Int8Parts ps{};
   ps.n = n_parts;
-  long long end = 0;
+  int end = 0;
   for (int i = 0; i < n_parts; ++i) {
     if (!code[i] || !row_scale[i] || !out[i] || rows[i] <= 0 || cols[i] <= 0 || (cols[i] & 15) ||
         (reinterpret_cast<uintptr_t>(code[i]) & 15) || (reinterpret_cast<uintptr_t>(out[i]) & 15))
       return B200_ERR_ARG;
-    end += rows[i] * (cols[i] >> 4);
-    ps.part[i] = quant::Int8Part{(const int8_t*)code[i], row_scale[i], (__nv_bfloat16*)out[i], cols[i] >> 4, end};
+    const long long units = rows[i] * (cols[i] >> 3);
+    if (!(end = quant::blocks_to(end, units))) return B200_ERR_ARG;
+    ps.part[i] = quant::Int8Part{(const int8_t*)code[i], row_scale[i], (__nv_bfloat16*)out[i], cols[i] >> 3, units, end};
   }
-  launch_pdl(quant::dequant_int8_kernel, quant::grid_for(end), 256, 0, st, ps);
+  launch_pdl(quant::dequant_int8_kernel, end, 256, 0, st, ps);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

@@ -107,3 +107,20 @@ def test_matrices_of_a_layer_in_one_launch(kind):
         quant.dequantize_all(qs, outs)
         for q, o, b in zip(qs, outs, buf):
             assert torch.equal(o, quant.dequantize_reference(q, torch.float32).bfloat16()) and (b[-64:] == 7).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["nf4", "int8"])
+@pytest.mark.parametrize("shape", [(128, 64), (129, 64), (255, 64), (300, 208), (7, 16384), (2051, 192)])
+def test_dequant_over_blocks_of_8192_values(kind, shape):
+    """One block of the kernel, one more group, several with a rest, rows longer than a block: bit for bit, between two others."""
+    if kind == "nf4" and shape[0] * shape[1] % 64:
+        shape = (shape[0] + 4 - shape[0] % 4, shape[1])
+    quantize = quant.quantize_nf4 if kind == "nf4" else quant.quantize_int8
+    g = torch.Generator("cuda").manual_seed(shape[0])
+    qs = [quantize(torch.randn(*s, device="cuda", generator=g)) for s in (shape, (131, 64), shape)]
+    buf = [torch.full((q_n + 64,), 7.0, dtype=torch.bfloat16, device="cuda") for q_n in (shape[0] * shape[1], 131 * 64, shape[0] * shape[1])]
+    outs = [b[:-64].view(s) for b, s in zip(buf, (shape, (131, 64), shape))]
+    quant.dequantize_all(qs, outs)
+    for q, o, b in zip(qs, outs, buf):
+        assert torch.equal(o, quant.dequantize_reference(q, torch.float32).bfloat16()) and (b[-64:] == 7).all()
