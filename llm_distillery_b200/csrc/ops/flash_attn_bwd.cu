@@ -681,27 +681,21 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // delta[h, t] = sum_d dout[t, h*D + d] * out[t, h*D + d]; one group of D/8 lanes per (t, h). Also zeroes the fp32 dQ
 // accumulator: a memset of its own costs a launch and keeps the kernels on both sides of it from overlapping (16 384
 // tokens of 32 heads of 64: 35 + 29 us apart, 42 together).
+// Bound by HBM: 8 bytes an element. A thread takes 8 elements (they lie in the order of the threads, so only the lane that
+// stores a sum needs its token and head), and zeroes two pieces of 16 bytes that lie in runs over the warp. Inside a training
+// step of 16 384 x 2048: 51 us (every lane its own 64-bit division, 32 bytes zeroed a lane: 56).
 template <int D>
-__global__ void delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
-                             float* __restrict__ delta, float* __restrict__ dq_acc, long long T, int H) {
+__global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
+                                                    float* __restrict__ delta, float* __restrict__ dq_acc, long long T, int H) {
   pdl_wait();
   pdl_trigger();
   constexpr int LPG = D / 8;  // lanes per (t,h)
-  const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x);
-  const long long grp = gid / LPG;
-  const int sub = (int)(gid % LPG);
+  const long long total = T * H * LPG, gid = blockIdx.x * 256ll + threadIdx.x;
   float s = 0.f;
-  const bool ok = grp < T * H;
-  long long t = 0;
-  int h = 0;
+  const bool ok = gid < total;
   if (ok) {
-    t = grp / H;
-    h = (int)(grp - t * H);
-    const size_t off = (size_t)t * H * D + (size_t)h * D + sub * 8;
-    uint4 a = *reinterpret_cast<const uint4*>(dout + off);
-    uint4 b = *reinterpret_cast<const uint4*>(out + off);
-    reinterpret_cast<float4*>(dq_acc + off)[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-    reinterpret_cast<float4*>(dq_acc + off)[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint4 a = reinterpret_cast<const uint4*>(dout)[gid];
+    const uint4 b = reinterpret_cast<const uint4*>(out)[gid];
     const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
     const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
 #pragma unroll
@@ -711,8 +705,17 @@ __global__ void delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_
     }
   }
 #pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const long long z = blockIdx.x * 512ll + k * 256 + threadIdx.x;
+    if (z < 2 * total) reinterpret_cast<float4*>(dq_acc)[z] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
   for (int o = LPG / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (ok && sub == 0) delta[(size_t)h * T + t] = s;
+  if (ok && threadIdx.x % LPG == 0) {
+    const long long grp = gid / LPG;
+    const long long t = grp < 0x7fffffffll ? (uint32_t)grp / (uint32_t)H : grp / H;
+    delta[(grp - t * H) * T + t] = s;
+  }
 }
 
 // dqkv[t, 0:H*D] = bf16(dq_acc[t, :])
@@ -737,55 +740,64 @@ __global__ void dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* 
   }
 }
 
-// The same with the inverse rotary embedding of the query heads applied on the way: one thread takes the two 8-element
+// The same with the inverse rotary embedding of the query heads applied on the way: one thread takes the two 4-element
 // vectors that the rotation pairs (i and i + D/2 of a head), rounds them to bf16 first - what the stand-alone rope
 // kernel would read back - and rotates with that kernel's expressions, so the result is bit-identical to convert + rope.
-__global__ void dq_convert_rope_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dqkv,
-                                       const int* __restrict__ pos, const float* __restrict__ cs,
-                                       const float* __restrict__ sn, long long T, int H, int D, long long width) {
+// Bound by HBM: 6 bytes an element. A block takes TOKENS tokens, a thread's loads of two items are under way together, and
+// the grid covers all tokens. Inside a training step of 16 384 x 2048: 44.5 us (two 8-element vectors a thread, 64-bit
+// divisions, a resident grid: 56).
+constexpr int TOKENS = 4;
+template <int D>
+__global__ void __launch_bounds__(256) dq_convert_rope_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dqkv,
+                                                              const int* __restrict__ pos, const float* __restrict__ cs,
+                                                              const float* __restrict__ sn, long long T, int H, long long width) {
   pdl_wait();
   pdl_trigger();
-  const int half = D >> 1;
-  const int vph = half >> 3;                 // vector pairs per head
-  const int vpt = H * vph;
-  const long long total = T * vpt;
-  const int HD = H * D;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / vpt;
-    const int r = (int)(i - t * vpt);
-    const int hd = r / vph;
-    const int j = (r - hd * vph) * 8;
-    const float* a = acc + t * HD + (long long)hd * D + j;
-    const float4 a0 = reinterpret_cast<const float4*>(a)[0], a1 = reinterpret_cast<const float4*>(a)[1];
-    const float4 b0 = reinterpret_cast<const float4*>(a + half)[0], b1 = reinterpret_cast<const float4*>(a + half)[1];
-    const float fa_in[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-    const float fb_in[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-    const int p = pos[t];
-    const float4 c0 = *reinterpret_cast<const float4*>(cs + (size_t)p * half + j);
-    const float4 c1 = *reinterpret_cast<const float4*>(cs + (size_t)p * half + j + 4);
-    const float4 s0 = *reinterpret_cast<const float4*>(sn + (size_t)p * half + j);
-    const float4 s1 = *reinterpret_cast<const float4*>(sn + (size_t)p * half + j + 4);
-    const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-    const float sg[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-    float oa[8], ob[8];
+  constexpr int HALF = D / 2, VPH = HALF / 4;                  // vector pairs per head
+  const uint32_t vpt = H * VPH;
+  const long long t0 = blockIdx.x * (long long)TOKENS;
+  const uint32_t items = (uint32_t)min(T - t0, (long long)TOKENS) * vpt;
+  for (uint32_t first = threadIdx.x; first < items; first += 512) {
+    float4 a[2], b[2], c[2], g[2];
+    long long dst[2];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float fa = __bfloat162float(__float2bfloat16(fa_in[k]));
-      const float fb = __bfloat162float(__float2bfloat16(fb_in[k]));
-      const float sk = sg[k] * -1.f;                       // the transposed rotation
-      oa[k] = __fmaf_rn(fa, c[k], -__fmul_rn(fb, sk));
-      ob[k] = __fmaf_rn(fb, c[k], __fmul_rn(fa, sk));
+    for (int u = 0; u < 2; ++u) {
+      const uint32_t i = first + u * 256;
+      if (i >= items) continue;
+      const uint32_t t = i / vpt, r = i - t * vpt, hd = r / VPH, j = (r - hd * VPH) * 4;
+      const float* src = acc + (t0 + t) * (H * D) + hd * D + j;
+      a[u] = *reinterpret_cast<const float4*>(src);
+      b[u] = *reinterpret_cast<const float4*>(src + HALF);
+      const size_t tab = (size_t)pos[t0 + t] * HALF + j;
+      c[u] = *reinterpret_cast<const float4*>(cs + tab);
+      g[u] = *reinterpret_cast<const float4*>(sn + tab);
+      dst[u] = (t0 + t) * width + hd * D + j;
     }
-    uint4 o1, o2;
-    o1.x = pack_bf16x2(oa[0], oa[1]); o1.y = pack_bf16x2(oa[2], oa[3]);
-    o1.z = pack_bf16x2(oa[4], oa[5]); o1.w = pack_bf16x2(oa[6], oa[7]);
-    o2.x = pack_bf16x2(ob[0], ob[1]); o2.y = pack_bf16x2(ob[2], ob[3]);
-    o2.z = pack_bf16x2(ob[4], ob[5]); o2.w = pack_bf16x2(ob[6], ob[7]);
-    __nv_bfloat16* dst = dqkv + t * width + (long long)hd * D + j;
-    *reinterpret_cast<uint4*>(dst) = o1;
-    *reinterpret_cast<uint4*>(dst + half) = o2;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (first + u * 256 >= items) continue;
+      const float *pa = &a[u].x, *pb = &b[u].x, *pc = &c[u].x, *pg = &g[u].x;
+      float oa[4], ob[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float fa = __bfloat162float(__float2bfloat16(pa[k]));
+        const float fb = __bfloat162float(__float2bfloat16(pb[k]));
+        const float sk = pg[k] * -1.f;                         // the transposed rotation
+        oa[k] = __fmaf_rn(fa, pc[k], -__fmul_rn(fb, sk));
+        ob[k] = __fmaf_rn(fb, pc[k], __fmul_rn(fa, sk));
+      }
+      *reinterpret_cast<uint2*>(dqkv + dst[u]) = make_uint2(pack_bf16x2(oa[0], oa[1]), pack_bf16x2(oa[2], oa[3]));
+      *reinterpret_cast<uint2*>(dqkv + dst[u] + HALF) = make_uint2(pack_bf16x2(ob[0], ob[1]), pack_bf16x2(ob[2], ob[3]));
+    }
   }
+}
+
+template <int D>
+static int launch_dq_convert_rope(const float* acc, __nv_bfloat16* dqkv, const int* pos, const float* cs, const float* sn,
+                                  long long T, int H, long long width, cudaStream_t st) {
+  launch_pdl(dq_convert_rope_kernel<D>, (unsigned)((T + TOKENS - 1) / TOKENS), 256, 0, st, acc, dqkv, pos, cs, sn, T, H, width);
+  B200_CUDA_CHECK(cudaGetLastError());
+  return B200_OK;
 }
 
 // CTAs that share the query heads of one (batch, kv head, key block). The kernel takes about as long as the longer of its
@@ -855,19 +867,11 @@ static int launch_bwd(const void* dout, const void* qkv, const void* out, const 
   else
     launch_pdl(kern, grid, NTHREADS, C::SMEM_BYTES, st, tmQKV, tmDO, tmDQ, p, device_err_word());
   B200_CUDA_CHECK(cudaGetLastError());
-  {
-    const bool rot = pos != nullptr;
-    long long work = rot ? T * (HD >> 4) : T * (HD >> 3);
-    long long blocks = (work + 255) / 256;
-    const long long cap = (long long)sm_count() * 8;
-    if (blocks > cap) blocks = cap;
-    if (rot)
-      launch_pdl(dq_convert_rope_kernel, (unsigned)blocks, 256, 0, st, dq_acc, (__nv_bfloat16*)dqkv, pos, cos_tab, sin_tab, T, H,
-                                                              D, width);
-    else
-      launch_pdl(dq_convert_kernel, (unsigned)blocks, 256, 0, st, dq_acc, (__nv_bfloat16*)dqkv, T, (int)HD, width);
-    B200_CUDA_CHECK(cudaGetLastError());
-  }
+  if (pos) return launch_dq_convert_rope<D>(dq_acc, (__nv_bfloat16*)dqkv, pos, cos_tab, sin_tab, T, H, width, st);
+  const long long blocks = (T * (HD >> 3) + 255) / 256;
+  launch_pdl(dq_convert_kernel, (unsigned)(blocks < 0x7fffffffll ? blocks : 0x7fffffffll), 256, 0, st, dq_acc,
+             (__nv_bfloat16*)dqkv, T, (int)HD, width);
+  B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }
 
@@ -914,12 +918,6 @@ extern "C" int b200_dq_convert_rope(const float* acc, void* dqkv, const int* pos
                                     const float* sin_tab, long long T, int H, int D, long long width, cudaStream_t st) {
   using namespace b200;
   if (!acc || !dqkv || !pos || !cos_tab || !sin_tab || T <= 0 || H <= 0 || (D != 64 && D != 128)) return B200_ERR_ARG;
-  long long work = T * ((long long)H * D >> 4);
-  long long blocks = (work + 255) / 256;
-  const long long cap = (long long)sm_count() * 8;
-  if (blocks > cap) blocks = cap;
-  launch_pdl(fab::dq_convert_rope_kernel, (unsigned)blocks, 256, 0, st, acc, (__nv_bfloat16*)dqkv, pos, cos_tab, sin_tab, T, H, D,
-                                                              width);
-  B200_CUDA_CHECK(cudaGetLastError());
-  return B200_OK;
+  return D == 64 ? fab::launch_dq_convert_rope<64>(acc, (__nv_bfloat16*)dqkv, pos, cos_tab, sin_tab, T, H, width, st)
+                 : fab::launch_dq_convert_rope<128>(acc, (__nv_bfloat16*)dqkv, pos, cos_tab, sin_tab, T, H, width, st);
 }
