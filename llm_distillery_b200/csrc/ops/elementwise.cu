@@ -935,7 +935,7 @@ int b200_rmsnorm_bwd_blocks(int rows) {
 int b200_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* hout, float* rstd, int rows, int h,
                      float eps, cudaStream_t st) {
   if (!x || !w || !y || rows <= 0 || (h & 7) || h > NT * MAX_VEC * 8) return B200_ERR_ARG;
-  const int wblocks = ceil_div(rows, 4) < sm_count() * 5 ? ceil_div(rows, 4) : sm_count() * 5;  // 4 rows per 128-thread CTA
+  const int wblocks = ceil_div(rows, 4);  // 4 rows per 128-thread CTA; 16384 x 2048 21.5 us (a resident grid of 5 an SM: 23.9)
 #define B200_RMS_FWD_WARP(VPL)                                                                                        \
   launch_pdl(rmsnorm_fwd_warp_kernel<VPL>, wblocks, 128, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,            \
                                                         (const __nv_bfloat16*)w, (__nv_bfloat16*)y,                   \
@@ -947,9 +947,10 @@ int b200_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, voi
   else {
     // Two rows at a time where a thread has several vectors of each and there are many rows: 8000 x 4096 35.3 us (one row,
     // three barriers) / 25.5 (one row, one barrier) / 23.2, 5.65 TB/s; 2048 x 4096 10.1 / 7.7 / 7.8. With one vector a thread
-    // more blocks on an SM do as well (12000 x 1536: 18.1 / 20.4).
+    // more blocks on an SM do as well (12000 x 1536: 18.1 / 20.4),
+    // and 128 threads take 16 blocks an SM (4000 x 896 4.6; 8: 6.0).
     const bool two = h > NT * 8 && rows >= 4096;
-    const int blocks = two ? ceil_div(rows, 2) : rows, cap = sm_count() * (two ? 4 : 8), grid = blocks < cap ? blocks : cap;
+    const int blocks = two ? ceil_div(rows, 2) : rows, cap = sm_count() * (two ? 4 : h <= 1024 ? 16 : 8), grid = blocks < cap ? blocks : cap;
 #define B200_RMS_FWD(NV, NTB, R)                                                                                      \
   launch_pdl(rmsnorm_fwd_kernel<NV, NTB, R>, grid, NTB, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,    \
              (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)hout, rstd, rows, h, eps)
