@@ -773,24 +773,31 @@ __global__ void embed_fwd_kernel(const long long* __restrict__ ids, const __nv_b
   }
 }
 
-// dW[ids[t], :] += dout[t, :]   (fp32 gradient buffer, atomics: rows repeat)
-__global__ void embed_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dout,
-                                 float* __restrict__ dW, long long T, int h, int vocab) {
+// dW[ids[t], :] += dout[t, :]   (fp32 gradient buffer, atomics: rows repeat). A block per token, four elements a thread in one
+// 16-byte reduction (VEC: dW on a 16-byte boundary). Bound by HBM: 10 bytes an element. 16384 x 2048 49 us;
+// eight scalar atomics a thread, 32 bytes apart over the warp, took 205 (a quarter of the tokens alike: 85, was 656).
+template <bool VEC>
+__global__ void __launch_bounds__(256) embed_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dout,
+                                                        float* __restrict__ dW, long long T, int h, int vocab) {
   pdl_wait();
   pdl_trigger();
-  const int hv = h >> 3;
-  const long long total = T * hv;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / hv;
-    const int v = (int)(i - t * hv);
-    long long id = ids[t];
+  for (long long t = blockIdx.x; t < T; t += gridDim.x) {
+    const long long id = ids[t];
     if (id < 0 || id >= vocab) continue;
-    float d[8];
-    unpack8(reinterpret_cast<const uint4*>(dout + t * h)[v], d);
-    float* dst = dW + id * h + (long long)v * 8;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(dst + j, d[j]);
+    for (int v = threadIdx.x * 4; v < h; v += 1024) {
+      const uint2 q = *reinterpret_cast<const uint2*>(dout + t * h + v);
+      const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x));
+      const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
+      float* dst = dW + id * h + v;
+      if (VEC) {
+        atomicAdd(reinterpret_cast<float4*>(dst), make_float4(a.x, a.y, b.x, b.y));
+      } else {
+        atomicAdd(dst, a.x);
+        atomicAdd(dst + 1, a.y);
+        atomicAdd(dst + 2, b.x);
+        atomicAdd(dst + 3, b.y);
+      }
+    }
   }
 }
 
@@ -1126,7 +1133,8 @@ int b200_embed_fwd(const long long* ids, const void* W, void* out, long long T, 
 
 int b200_embed_bwd(const long long* ids, const void* dout, float* dW, long long T, int h, int vocab, cudaStream_t st) {
   if (!ids || !dout || !dW || T <= 0 || (h & 7)) return B200_ERR_ARG;
-  launch_pdl(embed_bwd_kernel, grid_for(T * (h >> 3), 256), 256, 0, st, ids, (const __nv_bfloat16*)dout, dW, T, h, vocab);
+  auto kern = reinterpret_cast<uintptr_t>(dW) & 15 ? embed_bwd_kernel<false> : embed_bwd_kernel<true>;
+  launch_pdl(kern, (unsigned)(T < 0x7fffffffll ? T : 0x7fffffffll), 256, 0, st, ids, (const __nv_bfloat16*)dout, dW, T, h, vocab);
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
 }

@@ -222,3 +222,25 @@ def test_bias_gradient_of_few_and_many_rows(T, N, ld):
         basic.bias_grad(dy, out=out, accumulate=add)
         want = dy.double().sum(0) * (2 if add else 1)
         assert ((out.double() - want).abs() <= (T + 1) * 2 ** -23 * dy.double().abs().sum(0) + 1e-6).all()
+
+
+@pytest.mark.parametrize("T,h,vocab", [(1, 8, 3), (37, 896, 11), (300, 1024, 5000), (129, 1032, 7), (2050, 2056, 64)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_embedding_gradient_of_repeated_tokens(T, h, vocab, off):
+    """Rows that end at, before and behind a block's 1024 columns, ids out of range skipped, a gradient on and off a 16-byte
+    boundary. Bound: each of a row's additions rounds a partial sum, which is at most the sum of the absolute values."""
+    g = torch.Generator("cuda").manual_seed(T)
+    ids = torch.randint(0, vocab, (T,), device=DEV, generator=g)
+    ids[::5] = vocab // 2
+    if T > 3:
+        ids[1], ids[2] = -1, vocab
+    dout = torch.randn(T, h, device=DEV, generator=g).bfloat16()
+    buf = torch.ones(vocab * h + 8, device=DEV)
+    dW = buf[off:off + vocab * h]
+    rc = _lib.kernels().b200_embed_bwd(_lib.ptr(ids), _lib.ptr(dout), _lib.ptr(dW), T, h, vocab, _lib.stream())
+    ok = (ids >= 0) & (ids < vocab)
+    ref, size = (torch.ones(vocab, h, device=DEV, dtype=torch.float64).index_add_(0, ids[ok], d[ok].double())
+                 for d in (dout, dout.abs()))
+    n = torch.bincount(ids[ok], minlength=vocab).max().item()
+    assert rc == 0 and ((dW.view(vocab, h).double() - ref).abs() <= n * 2.0 ** -24 * size).all()
+    assert (buf[:off] == 1).all() and (buf[off + vocab * h:] == 1).all() and _lib.take_device_error() == 0
