@@ -27,6 +27,7 @@ struct EpiStore {
   using Params = StoreParams;
   static constexpr bool SPLIT_K = true;   // the pair kernel may cut the K loop into slices that are added in order
   static constexpr bool PREFETCH = false;
+  static constexpr int WARPS = NUM_EPI_WARPS;
   // slice 0 of a tile stores (or adds to what C held, if the caller accumulates); every later slice adds
   static __device__ __forceinline__ Params slice_params(const Params& p, int slice) {
     Params q = p;
@@ -265,6 +266,7 @@ struct EpiSwiglu {
   using Params = SwigluParams;
   static constexpr bool SPLIT_K = false;
   static constexpr bool PREFETCH = false;
+  static constexpr int WARPS = NUM_EPI_WARPS;
   static constexpr int STAGE_BYTES = 32 * 256;
   static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;
 
@@ -359,6 +361,7 @@ struct EpiRope {
   using Params = RopeParams;
   static constexpr bool SPLIT_K = false;
   static constexpr bool PREFETCH = false;
+  static constexpr int WARPS = NUM_EPI_WARPS;
   static constexpr int STAGE_BYTES = 32 * 256;
   static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;
 
@@ -457,7 +460,7 @@ static int launch_rope_pair(const void* A, const void* W, int M, int N, int K, l
   const int tiles = ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, rp, device_err_word(), 1, nullptr, 0,
+  launch_pdl(kern, 2 * pairs, pair_threads<Epi>(), smem_bytes, stream, tmA, tmB, M, N, K, 1, rp, device_err_word(), 1, nullptr, 0,
                gemm::GroupArgs{});
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -483,6 +486,7 @@ struct EpiSwigluBwd {
   using Params = SwigluBwdParams;
   static constexpr bool SPLIT_K = false;
   static constexpr bool PREFETCH = true;
+  static constexpr int WARPS = NUM_EPI_WARPS;
   static constexpr int QUARTER = 32 * 128;               // gate or up values of a quarter
   static constexpr int STAGE_BYTES = 2 * 2 * QUARTER;    // two stages of both per epilogue warp
   static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;
@@ -589,6 +593,7 @@ struct EpiResidual {
   using Params = StoreParams;
   static constexpr bool SPLIT_K = false;
   static constexpr bool PREFETCH = true;
+  static constexpr int WARPS = NUM_EPI_WARPS;
   static constexpr int QUARTER = 32 * 128;
   static constexpr int STAGE_BYTES = 2 * QUARTER;
   static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;
@@ -691,7 +696,7 @@ static int launch_swiglu_bwd_pair(const void* dY, const void* Wd, int M, int f, 
   const int tiles = ceil_div(M, PAIR_BM) * ceil_div(f, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, f, K, 1, sp, device_err_word(), 1, nullptr, 0,
+  launch_pdl(kern, 2 * pairs, pair_threads<Epi>(), smem_bytes, stream, tmA, tmB, M, f, K, 1, sp, device_err_word(), 1, nullptr, 0,
                gemm::GroupArgs{});
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -720,7 +725,7 @@ static int launch_swiglu_pair(const void* A, const void* Wgu, int M, int f, int 
   const int tiles = ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, sp, device_err_word(), 1, nullptr, f,
+  launch_pdl(kern, 2 * pairs, pair_threads<Epi>(), smem_bytes, stream, tmA, tmB, M, N, K, 1, sp, device_err_word(), 1, nullptr, f,
                gemm::GroupArgs{});
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -827,7 +832,7 @@ static int launch_grouped(const void* A, const void* B, int M, int N, int K, lon
   const long long tiles = (long long)most * ceil_div(N, PAIR_BN);
   const int max_pairs = sm_count() / 2;
   const int pairs = tiles < max_pairs ? (int)tiles : max_pairs;
-  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, 1, ep, device_err_word(), 1, nullptr, b_half,
+  launch_pdl(kern, 2 * pairs, pair_threads<Epi>(), smem_bytes, stream, tmA, tmB, M, N, K, 1, ep, device_err_word(), 1, nullptr, b_half,
              GroupArgs{counts, n_groups, b_rows});
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;
@@ -889,7 +894,7 @@ static int launch_store_pair(const void* A, const void* B, int M, int N, int K, 
   }
   const long long units = (long long)tiles * k_splits;
   const int pairs = units < max_pairs ? (int)units : max_pairs;
-  launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, K, fmt, sp, device_err_word(), k_splits, sync, 0,
+  launch_pdl(kern, 2 * pairs, pair_threads<Epi>(), smem_bytes, stream, tmA, tmB, M, N, K, fmt, sp, device_err_word(), k_splits, sync, 0,
                gemm::GroupArgs{});
   B200_CUDA_CHECK(cudaGetLastError());
   return B200_OK;

@@ -55,8 +55,15 @@ struct SmemPair {
   }
 };
 
+// An epilogue of 8 warps gives each quadrant of TMEM two of them: the second takes the tile's columns from 128 on. For
+// epilogues whose arithmetic on 4 warps outlasts the main loop.
+template <class Epi>
+constexpr int pair_threads() {
+  return 64 + 32 * Epi::WARPS;
+}
+
 template <int STAGES, bool A_MN, bool B_MN, class Epi, bool GROUPED = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<Epi>(), 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
                      int K, int fmt, typename Epi::Params ep, unsigned int* err_word, int k_splits,
                      unsigned int* split_sync, int b_half_stride, GroupArgs grp) {
@@ -85,7 +92,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 2 * NUM_EPI_WARPS);
+      mbar_init(&tempty_bar[a], 2 * Epi::WARPS);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -264,6 +271,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
   } else {
     // ------------------------------------------------------------ epilogue warps (both CTAs)
     const int quad = warp & 3;
+    static_assert(Epi::WARPS == NUM_EPI_WARPS || (Epi::WARPS == 2 * NUM_EPI_WARPS && !Epi::SPLIT_K && !GROUPED));
+    const int col0 = Epi::WARPS == NUM_EPI_WARPS ? 0 : (warp - 2) / NUM_EPI_WARPS * PAIR_HALF_N;
+    if (col0) epi_smem += Epi::SMEM_BYTES / 2;
     const uint32_t leader_tempty0 = mapa_shared(smem_u32(&tempty_bar[0]), 0);
     uint32_t tl = 0;
     int e = 0;
@@ -274,12 +284,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
       const uint32_t acc = tl & 1u;
       const uint32_t aph = (tl >> 1) & 1u;
       if constexpr (Epi::PREFETCH)      // operands from global memory, while the main loop runs
-        Epi::prefetch(ep, row + (int)cta * BM, n_blk * PAIR_BN, row_end, N, quad, lane, epi_smem);
+        Epi::prefetch(ep, row + (int)cta * BM, n_blk * PAIR_BN + col0, row_end, N, quad, lane, epi_smem);
       int ok = mbar_wait_bounded(&tfull_bar[acc], aph, abort_flag, err_word, ERR_WAIT_TMEM_FULL) ? 1 : 0;
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + acc * PAIR_BN + (static_cast<uint32_t>(quad * 32) << 16);
+      const uint32_t taddr = tmem_base + acc * PAIR_BN + col0 + (static_cast<uint32_t>(quad * 32) << 16);
       if constexpr (Epi::SPLIT_K) {
         if (k_splits > 1) {
           const int sp = unit / num_tiles;
@@ -290,16 +300,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
             ok2 = __all_sync(0xffffffffu, ok2);
             if (!ok2) break;
           }
-          Epi::tile(Epi::slice_params(ep, sp), taddr, row + (int)cta * BM, n_blk * PAIR_BN, row_end, N, quad,
+          Epi::tile(Epi::slice_params(ep, sp), taddr, row + (int)cta * BM, n_blk * PAIR_BN + col0, row_end, N, quad,
                     lane, epi_smem);
           __threadfence();
           __syncwarp();
           if (lane == 0) st_release_gpu_u32(ctr, sp + 1 == k_splits ? 0u : (unsigned)(sp + 1));
         } else {
-          Epi::tile(ep, taddr, row + (int)cta * BM, n_blk * PAIR_BN, row_end, N, quad, lane, epi_smem);
+          Epi::tile(ep, taddr, row + (int)cta * BM, n_blk * PAIR_BN + col0, row_end, N, quad, lane, epi_smem);
         }
       } else {
-        Epi::tile(ep, taddr, row + (int)cta * BM, n_blk * PAIR_BN, row_end, N, quad, lane, epi_smem);
+        Epi::tile(ep, taddr, row + (int)cta * BM, n_blk * PAIR_BN + col0, row_end, N, quad, lane, epi_smem);
       }
       tc_fence_before_sync();
       __syncwarp();

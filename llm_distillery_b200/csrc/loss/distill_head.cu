@@ -36,6 +36,7 @@ struct LseParams {
 struct EpiLse {
   static constexpr bool SPLIT_K = false;
   static constexpr bool PREFETCH = false;
+  static constexpr int WARPS = NUM_EPI_WARPS;
   using Params = LseParams;
   static constexpr int SMEM_BYTES = 0;
   static __device__ __forceinline__ void tile(const Params& p, uint32_t taddr, int m0, int n0, int M, int N, int quad,
@@ -114,15 +115,21 @@ struct DzParams {
   int id_off;          // see LseParams
 };
 
+// A warp takes COLS columns of its rows. On CTA pairs two warps share a quadrant's 256: the searches, gathers and exponentials of
+// four warps outlasted a main loop of 2048 (16384 x 32000, 200 ids a row: 1615 us, now 1463;
+// 7000 rows, 400 ids 755 / 635; 777 x 151936 x 896 331 / 267).
+template <int COLS>
 struct EpiDz {
   static constexpr bool SPLIT_K = false;
   static constexpr bool PREFETCH = false;
+  static constexpr int WARPS = NUM_EPI_WARPS * (BN / COLS);
   using Params = DzParams;
-  static constexpr int STAGE_BYTES = 32 * 256;   // per epilogue warp: 32 rows x 128 bf16 columns, chunks XOR-swizzled
-  static constexpr int SMEM_BYTES = NUM_EPI_WARPS * STAGE_BYTES;
+  static constexpr int STAGE_BYTES = 32 * 128;   // per epilogue warp: 32 rows x 64 bf16 columns, chunks XOR-swizzled
+  static constexpr int SMEM_BYTES = WARPS * STAGE_BYTES;
   static __device__ __forceinline__ void tile(const Params& p, uint32_t taddr, int m0, int n0, int M, int N, int quad,
                                               int lane, uint8_t* epi_smem) {
-    // bf16 dlogits leave through a shared-memory stage as whole 256-byte row segments when the layout allows it
+    if (n0 >= N) return;
+    // bf16 dlogits leave through a shared-memory stage as whole 128-byte row segments when the layout allows it
     const bool staged = !(N & 7) && !(p.ldz & 7) && !(reinterpret_cast<uintptr_t>(p.dz) & 15);
     uint8_t* stage = epi_smem + quad * STAGE_BYTES;
     const int row0 = m0 + quad * 32;
@@ -143,10 +150,20 @@ struct EpiDz {
       coef = -gs * p.A[row];
       lse2 = p.lse[row] * LOG2E;
     }
-    int next_id = (row_ok && pos < p.K) ? __ldg(ids + pos) - p.id_off : 0x7fffffff;
+    const float* as = p.a + (long long)row * p.K;
+    int next_id = 0x7fffffff;      // the next teacher id and its coefficient, fetched together
+    float next_a = 0.f;
+    auto fetch = [&]() {
+      next_id = 0x7fffffff;
+      if (row_ok && pos < p.K) {
+        next_id = __ldg(ids + pos) - p.id_off;
+        next_a = __ldg(as + pos);
+      }
+    };
+    fetch();
     const float c2 = p.inv_T * LOG2E;
 #pragma unroll 1
-    for (int c = 0; c < BN / 32; ++c) {
+    for (int c = 0; c < COLS / 32; ++c) {
       uint32_t r[32];
       __syncwarp();  // lanes may have diverged in the previous chunk; tcgen05.ld is warp-collective
       tmem_ld_32x32b_x32(taddr + c * 32, r);
@@ -159,11 +176,11 @@ struct EpiDz {
       if (active) {
         while (next_id < col0 + 32) {
           const int sel = next_id - col0;
-          const float add = gs * __ldg(p.a + (long long)row * p.K + pos);
+          const float add = gs * next_a;
+          ++pos;
+          fetch();
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] += (sel == j) ? add : 0.f;
-          ++pos;
-          next_id = pos < p.K ? __ldg(ids + pos) - p.id_off : 0x7fffffff;
         }
       }
       if (staged) {
@@ -174,17 +191,17 @@ struct EpiDz {
           o.y = pack_bf16x2(v[q4 * 8 + 2], v[q4 * 8 + 3]);
           o.z = pack_bf16x2(v[q4 * 8 + 4], v[q4 * 8 + 5]);
           o.w = pack_bf16x2(v[q4 * 8 + 6], v[q4 * 8 + 7]);
-          const int chunk = (c & 3) * 4 + q4;
-          *reinterpret_cast<uint4*>(stage + lane * 256 + ((chunk ^ (lane & 15)) << 4)) = o;
+          const int chunk = (c & 1) * 4 + q4;
+          *reinterpret_cast<uint4*>(stage + lane * 128 + ((chunk ^ (lane & 7)) << 4)) = o;
         }
-        if ((c & 3) == 3) {  // 128 columns staged: write them out, two 256-byte row segments per instruction
+        if (c & 1) {  // 64 columns staged: write them out, four 128-byte row segments per instruction
           __syncwarp();
-          const int chunk = lane & 15;
-          const int col = n0 + (c >> 2) * 128 + chunk * 8;
+          const int chunk = lane & 7;
+          const int col = n0 + (c >> 1) * 64 + chunk * 8;
 #pragma unroll 4
-          for (int j = 0; j < 16; ++j) {
-            const int rr = 2 * j + (lane >> 4);
-            const uint4 o = *reinterpret_cast<const uint4*>(stage + rr * 256 + ((chunk ^ (rr & 15)) << 4));
+          for (int j = 0; j < 8; ++j) {
+            const int rr = 4 * j + (lane >> 3);
+            const uint4 o = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((chunk ^ (rr & 7)) << 4));
             if (rr < rows_valid && col < N)
               *reinterpret_cast<uint4*>(p.dz + (long long)(row0 + rr) * p.ldz + col) = o;
           }
@@ -214,7 +231,7 @@ struct EpiDz {
   }
 };
 
-template <class Epi>
+template <class Epi, class PairEpi = Epi>
 static int launch_head(const void* Hc, const void* W, int M, int N, int Kdim, long long ldh, long long ldw,
                        const typename Epi::Params& ep, cudaStream_t stream) {
   // enough 256 x 256 tiles: run on SM pairs (cta_group::2), else one CTA per 128 x 256 tile
@@ -228,8 +245,8 @@ static int launch_head(const void* Hc, const void* W, int M, int N, int Kdim, lo
   if (rc != B200_OK) return rc;
   if (pair) {
     constexpr int PSTAGES = 6;
-    auto kern = gemm_pair_kernel<PSTAGES, false, false, Epi>;
-    const int smem_bytes = SmemPair<PSTAGES>::bytes(Epi::SMEM_BYTES);
+    auto kern = gemm_pair_kernel<PSTAGES, false, false, PairEpi>;
+    const int smem_bytes = SmemPair<PSTAGES>::bytes(PairEpi::SMEM_BYTES);
     static bool attr = false;
     if (!attr) {
       B200_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
@@ -237,8 +254,8 @@ static int launch_head(const void* Hc, const void* W, int M, int N, int Kdim, lo
     }
     const int tiles = ceil_div(M, PAIR_BM) * ceil_div(N, PAIR_BN);
     const int pairs = tiles < sm_count() / 2 ? tiles : sm_count() / 2;
-    launch_pdl(kern, 2 * pairs, NUM_THREADS, smem_bytes, stream, tmA, tmB, M, N, Kdim, 1, ep, device_err_word(), 1, nullptr, 0,
-               GroupArgs{});
+    launch_pdl(kern, 2 * pairs, pair_threads<PairEpi>(), smem_bytes, stream, tmA, tmB, M, N, Kdim, 1, ep, device_err_word(), 1, nullptr,
+               0, GroupArgs{});
     B200_CUDA_CHECK(cudaGetLastError());
     return B200_OK;
   }
@@ -492,7 +509,7 @@ int b200_lmhead_dlogits(const void* Hc, const void* W, int M, int N, int h, long
       (ldw & 7))
     return B200_ERR_ARG;
   DzParams ep{ids, a, A, lse, g, (__nv_bfloat16*)dz, ldz, K, inv_T, 0};
-  return launch_head<EpiDz>(Hc, W, M, N, h, ldh, ldw, ep, st);
+  return launch_head<EpiDz<BN>, EpiDz<BN / 2>>(Hc, W, M, N, h, ldh, ldw, ep, st);
 }
 
 // Pass 2 on one vocabulary slice (see b200_lmhead_lse_gather_shard).
@@ -503,6 +520,6 @@ int b200_lmhead_dlogits_shard(const void* Hc, const void* W, int M, int N, int h
       (ldw & 7))
     return B200_ERR_ARG;
   DzParams ep{ids, a, A, lse, g, (__nv_bfloat16*)dz, ldz, K, inv_T, id_off};
-  return launch_head<EpiDz>(Hc, W, M, N, h, ldh, ldw, ep, st);
+  return launch_head<EpiDz<BN>, EpiDz<BN / 2>>(Hc, W, M, N, h, ldh, ldw, ep, st);
 }
 }

@@ -186,3 +186,35 @@ def test_reference_loss_gradient_of_far_log_probs(M, K):
     for x, y in zip(*grads):
         assert (x - y).abs().max() <= 5e-6 * y.abs().max()
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,h,K", [(2500, 2000, 256, 9), (2401, 1800, 264, 33), (257, 9610, 320, 64), (5000, 1284, 256, 1)])
+@pytest.mark.parametrize("ld", [0, 3])
+def test_dlogits_of_ragged_pair_tiles(M, N, h, K, ld):
+    """256 x 256 tiles whose last columns end in either half, ids on the halves' edges and behind the vocabulary, rows of the
+    result on and off 16-byte boundaries. Bound: the result's rounding to bf16 (2^-8), and of the exponential the error of its
+    argument: products of bf16 summed in fp32 (below 1e-5 sqrt(h)) and three roundings of numbers up to 40."""
+    g = torch.Generator("cuda").manual_seed(M)
+    x, w = (torch.randn(n, h, device=DEV, generator=g).bfloat16() * s for n, s in ((M, 1.0), (N, 0.1)))
+    ids = torch.stack([torch.randperm(N, device=DEV, generator=g)[:K] for _ in range(M)]).int()
+    edges = torch.tensor([0, 127, 128, 255, 256, 383, 384, N - 1], device=DEV, dtype=torch.int32)[:K]
+    ids[::2, :len(edges)] = edges
+    ids[1::3, -1] = N + 2
+    ids = ids.sort(1).values
+    ok = (ids[:, 1:] != ids[:, :-1]).all(1) if K > 1 else torch.ones(M, dtype=torch.bool, device=DEV)     # rows without a repeated id
+    a = torch.randn(M, K, device=DEV, generator=g)
+    A, gr = torch.randn(M, device=DEV, generator=g), torch.rand(M, device=DEV, generator=g)
+    z = (x.double() @ w.double().t()) * 0.5
+    lse = z.logsumexp(1)
+    p = torch.exp(z - lse[:, None])
+    ref = torch.zeros(M, N + 8, device=DEV, dtype=torch.float64).scatter_add_(1, ids.long(), a.double())[:, :N] - A.double()[:, None] * p
+    scale = gr.double()[:, None] * 0.5
+    width = (N + 7) // 8 * 8 + 8 + ld
+    buf = torch.full((M + 1, width), 7.0, device=DEV, dtype=torch.bfloat16)
+    lse32 = lse.float()
+    rc = _lib.kernels().b200_lmhead_dlogits(_lib.ptr(x), _lib.ptr(w), M, N, h, h, h, _lib.ptr(ids), _lib.ptr(a), _lib.ptr(A),
+                                            _lib.ptr(lse32), _lib.ptr(gr), K, 0.5, _lib.ptr(buf), width, _lib.stream())
+    err = (buf[:M, :N].double() - ref * scale).abs()
+    bound = 2.0 ** -8 * (ref * scale).abs() + scale * (A.double().abs()[:, None] * p * (1e-5 * h ** 0.5 + 1e-4) + 1e-6)
+    assert rc == 0 and (err <= bound)[ok].all() and ok.float().mean() > 0.3
+    assert (buf[:M, N:] == 7).all() and (buf[M:] == 7).all() and _lib.take_device_error() == 0
