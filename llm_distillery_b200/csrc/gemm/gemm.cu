@@ -251,11 +251,12 @@ struct EpiStore {
 // Fused gate / up projection + SwiGLU on the CTA-pair kernel. The accumulator of a tile holds, for 256 rows, the gate
 // (columns 0-127) and the up projection (columns 128-255) of the same 128 features (the B halves come from rows
 // j*128 and f + j*128 of the fused weight, gemm_pair.cuh). The epilogue writes three things per row: gate and up,
-// rounded to bf16, into gu [M, 2f] (the backward pass reads them), and act = silu(gate) * up computed from the ROUNDED
+// rounded to bf16, into gu [M, 2f] (the backward pass reads them; without one, two thirds of the output and of the epilogue
+// go: 16384 x 2048 -> 5632 510 us, then 475), and act = silu(gate) * up computed from the ROUNDED
 // values, so that it equals what the stand-alone SwiGLU kernel makes of gu bit for bit. Each leaves through the
 // swizzled stage as 256-byte row segments.
 struct SwigluParams {
-  __nv_bfloat16* gu;    // [M, 2f]
+  __nv_bfloat16* gu;    // [M, 2f]; null: not written
   long long ld_gu;
   __nv_bfloat16* act;   // [M, f]
   long long ld_act;
@@ -292,7 +293,7 @@ struct EpiSwiglu {
     const int col0 = (n0 / PAIR_BN) * PAIR_HALF_N;       // first of the tile's 128 features
     // gate, then up: rounded copies into gu
 #pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
+    for (int half = p.gu ? 0 : 2; half < 2; ++half) {
 #pragma unroll 1
       for (int c4 = 0; c4 < 4; ++c4) {
         uint32_t r[32];
@@ -1046,9 +1047,11 @@ struct ClusterSwiglu {
     unpack_bf16x4(qu, ur);
 #pragma unroll
     for (int j = 0; j < 4; ++j) a[j] = __fdividef(gr[j], 1.f + __expf(-gr[j])) * ur[j];
-    __nv_bfloat16* gp = p.gu + (long long)row * p.ld_gu + col;
-    *reinterpret_cast<uint2*>(gp) = qg;
-    *reinterpret_cast<uint2*>(gp + p.f) = qu;
+    if (p.gu) {
+      __nv_bfloat16* gp = p.gu + (long long)row * p.ld_gu + col;
+      *reinterpret_cast<uint2*>(gp) = qg;
+      *reinterpret_cast<uint2*>(gp + p.f) = qu;
+    }
     *reinterpret_cast<uint2*>(p.act + (long long)row * p.ld_act + col) = pack_bf16x4(a);
   }
 };
@@ -1276,7 +1279,7 @@ int b200_gemm_swiglu(const void* x, const void* Wgu, void* gu, void* act, int M,
                      long long ldw, long long ld_gu, long long ld_act, int split_k, cudaStream_t stream) {
   using namespace b200;
   using namespace b200::gemm;
-  if (!x || !Wgu || !gu || !act || M <= 0 || f <= 0 || K <= 0 || (f % PAIR_HALF_N) || (ldx & 7) || (ldw & 7) ||
+  if (!x || !Wgu || !act || M <= 0 || f <= 0 || K <= 0 || (f % PAIR_HALF_N) || (ldx & 7) || (ldw & 7) ||
       (ld_gu & 7) || (ld_act & 7) || (reinterpret_cast<uintptr_t>(gu) & 15) || (reinterpret_cast<uintptr_t>(act) & 15))
     return B200_ERR_ARG;
   SwigluParams sp{reinterpret_cast<__nv_bfloat16*>(gu), ld_gu, reinterpret_cast<__nv_bfloat16*>(act), ld_act, f};
@@ -1300,7 +1303,7 @@ int b200_gemm_grouped_swiglu(const void* x, const void* Wgu, const long long* co
                              int K, int E, cudaStream_t stream) {
   using namespace b200;
   using namespace b200::gemm;
-  if (!gu || !act || f <= 0 || (f % PAIR_HALF_N) || f > 0x3fffffff || !group_args_ok(x, Wgu, counts, M, K, E, 2LL * f) ||
+  if (!act || f <= 0 || (f % PAIR_HALF_N) || f > 0x3fffffff || !group_args_ok(x, Wgu, counts, M, K, E, 2LL * f) ||
       (reinterpret_cast<uintptr_t>(gu) & 15) || (reinterpret_cast<uintptr_t>(act) & 15))
     return B200_ERR_ARG;
   SwigluParams sp{reinterpret_cast<__nv_bfloat16*>(gu), 2LL * f, reinterpret_cast<__nv_bfloat16*>(act), f, f};

@@ -47,6 +47,9 @@ struct Dims {
 // this layer's own, which write no weights. Not for the first launch of a call: what stands in front of it may expand or
 // update them.
 constexpr int kWeightsEarly = 2;
+// Bit 2 of a forward call's split_k: no backward pass will read its slab (or it will be filled again first), so the gate and up
+// values need not be written where the activation comes with their GEMM.
+constexpr int kActOnly = 4;
 
 // Carves 256-byte aligned pieces off a slab (base null: only sizes).
 struct Slab {
@@ -138,7 +141,8 @@ extern "C" int b200_layer_fwd(const void* x, const int* pos, const float* cos_ta
   const layer::Saved s(m, saved);
   const int T = (int)m.T, N = (int)m.N, A = (int)m.A;
   int launches = 0;
-  split_k |= layer::kWeightsEarly;
+  void* gu = (split_k & layer::kActOnly) ? nullptr : s.gu;
+  split_k = (split_k & ~layer::kActOnly) | layer::kWeightsEarly;
   RUN(b200_rmsnorm_fwd(x, nullptr, w_ln1, s.n1, nullptr, s.rstd1, T, h, eps, st));
   if (!b_qkv && N % 128 == 0) {
     RUN(b200_gemm_rope(s.n1, w_qkv, s.qkv, pos, cos_tab, sin_tab, T, N, h, H + Hkv, d, h, h, N, split_k, st));
@@ -151,7 +155,7 @@ extern "C" int b200_layer_fwd(const void* x, const int* pos, const float* cos_ta
   RUN(b200_gemm(s.att, w_o, s.h1, T, h, A, A, A, h, 0, 0, 1, 0, 0, 1.f, x, h, nullptr, split_k, st));
   RUN(b200_rmsnorm_fwd(s.h1, nullptr, w_ln2, s.n2, nullptr, s.rstd2, T, h, eps, st));
   if (f % 128 == 0) {
-    RUN(b200_gemm_swiglu(s.n2, w_gu, s.gu, s.act, T, f, h, h, h, 2LL * f, f, split_k, st));
+    RUN(b200_gemm_swiglu(s.n2, w_gu, gu, s.act, T, f, h, h, h, 2LL * f, f, split_k, st));
   } else {
     RUN(b200_gemm(s.n2, w_gu, s.gu, T, 2 * f, h, h, h, 2LL * f, 0, 0, 1, 0, 0, 1.f, nullptr, 0, nullptr, split_k, st));
     RUN(b200_swiglu_fwd(s.gu, s.act, T, f, st));

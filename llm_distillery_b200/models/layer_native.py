@@ -64,7 +64,10 @@ def _launched(rc: int, what: str) -> None:
     _lib.LAUNCH_COUNT[0] += rc
 
 
-def _forward(x, pos, cos, sin, weights, b_qkv, meta, split, with_output: bool):
+ACT_ONLY = 4       # bit of a forward call's split: nothing will read the gate and up values (csrc/ops/layer.cu)
+
+
+def _forward(x, pos, cos, sin, weights, b_qkv, meta, split, with_output: bool, act_only: bool = False):
     B, L, H, Hkv, d, eps, _, window = meta
     h, f = x.shape[1], weights[4].shape[0] // 2
     lib = _lib.kernels()
@@ -75,19 +78,19 @@ def _forward(x, pos, cos, sin, weights, b_qkv, meta, split, with_output: bool):
     _launched(lib.b200_layer_fwd(x.data_ptr(), pos.data_ptr(), cos.data_ptr(), sin.data_ptr(), w1.data_ptr(), wq.data_ptr(),
                                  wo.data_ptr(), w2.data_ptr(), wg.data_ptr(), wd.data_ptr(),
                                  0 if b_qkv is None else b_qkv.data_ptr(), saved.data_ptr(),
-                                 out.data_ptr() if with_output else 0, B, L, window, H, Hkv, d, h, f, eps, int(split),
-                                 _lib.stream()), "b200_layer_fwd")
+                                 out.data_ptr() if with_output else 0, B, L, window, H, Hkv, d, h, f, eps,
+                                 int(split) | (ACT_ONLY if act_only else 0), _lib.stream()), "b200_layer_fwd")
     return saved, out
 
 
 class NativeLayerFn(torch.autograd.Function):
-    """``llama.DecoderLayerFn`` for layers that ``fits`` accepts."""
+    """``llama.DecoderLayerFn`` for layers that ``fits`` accepts. A third entry of ``split``: no gradient will be asked for."""
 
     @staticmethod
     def forward(ctx, x, pos, cos, sin, w_ln1, w_qkv, w_o, w_ln2, w_gu, w_d, b_qkv, meta, split):
         weights = (w_ln1, w_qkv, w_o, w_ln2, w_gu, w_d)
         x = x.contiguous()
-        saved, out = _forward(x, pos, cos, sin, weights, b_qkv, meta, split[0], True)
+        saved, out = _forward(x, pos, cos, sin, weights, b_qkv, meta, split[0], True, meta[6] or (len(split) > 2 and split[2]))
         ctx.meta, ctx.split, ctx.weights, ctx.b_qkv = meta, split, weights, b_qkv
         if meta[6]:        # gradient checkpointing: keep only the layer input
             ctx.save_for_backward(x, pos, cos, sin)
@@ -164,7 +167,7 @@ def run_inference(x, pos, entry, count: int, meta, split: bool):
         out = torch.empty_like(x)
         to = [turn[i & 1].data_ptr() for i in range(n - 1)] + [out.data_ptr()]
         _launched(lib.b200_stack_fwd(_records(some, L, [slab.data_ptr()] * n, to), n, x.data_ptr(), pos.data_ptr(), B, L, H, Hkv, d,
-                                     h, f, eps, int(split), _lib.stream()), "b200_stack_fwd")
+                                     h, f, eps, int(split) | ACT_ONLY, _lib.stream()), "b200_stack_fwd")
         x, done = out, done + n
     return x, done
 

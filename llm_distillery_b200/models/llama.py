@@ -543,7 +543,7 @@ class LlamaModel(nn.Module):
                 if table is not checked:
                     checked, tables_ok = table, layer_native.tables_fit(pos, cos, sin, B * L, cfg.head_dim)
                 if layer_native.fits(h, pos, cos, sin, w, b_qkv, heads, training, tables_ok):
-                    h = layer_native.NativeLayerFn.apply(h, pos, cos, sin, *w, b_qkv, meta, split)
+                    h = layer_native.NativeLayerFn.apply(h, pos, cos, sin, *w, b_qkv, meta, split + (not torch.is_grad_enabled(),))
                     continue
             h = DecoderLayerFn.apply(h, pos, cos, sin, layer.input_layernorm, layer.qkv_proj, layer.o_proj,
                                      layer.post_attention_layernorm, layer.gate_up_proj, layer.down_proj, meta,
@@ -631,7 +631,7 @@ class LlamaModel(nn.Module):
                     h = basic.bias_add_(basic.gemm(act, layer.down_proj, residual=h1, alpha=rm),
                                         layer.down_bias if rm == 1.0 else layer.down_bias * rm)
                     continue
-                _, act = basic.linear_swiglu_fwd(n2, layer.gate_up_proj, split_k=split)
+                _, act = basic.linear_swiglu_fwd(n2, layer.gate_up_proj, split_k=split, keep_gu=False)
                 h = basic.gemm(act, layer.down_proj, residual=h1, alpha=rm, split_k=split)
             y, _, _ = basic.rmsnorm_fwd(h, self.norm, cfg.rms_norm_eps)
             if cfg.logits_scaling != 1.0:

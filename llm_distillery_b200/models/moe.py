@@ -105,12 +105,12 @@ def _grouped(x_perm: torch.Tensor, counts: torch.Tensor, w_gu: torch.Tensor, w_d
 
 
 def experts_forward(x_perm: torch.Tensor, counts: torch.Tensor, w_gu: torch.Tensor, w_d: torch.Tensor,
-                    host_counts: list[int] | None = None):
+                    host_counts: list[int] | None = None, keep_gu: bool = True):
     """x_perm [T*k, h] (rows grouped by expert, ``counts`` of them each) -> (gu [T*k, 2f], act [T*k, f], y [T*k, h]).
-    ``host_counts``: the counts where the host has them already."""
+    ``host_counts``: the counts where the host has them already. Without ``keep_gu`` gu may be None: only a backward pass reads it."""
     if _grouped(x_perm, counts, w_gu, w_d):
         (n, h), (E, two_f, _), new = x_perm.shape, w_gu.shape, x_perm.new_empty
-        gu, act, y = new((n, two_f)), new((n, two_f // 2)), new((n, h))
+        gu, act, y = new((n, two_f)) if keep_gu else None, new((n, two_f // 2)), new((n, h))
         lib, p = _lib.kernels(), _lib.ptr
         _lib.check(lib.b200_gemm_grouped_swiglu(p(x_perm), p(w_gu), p(counts), p(gu), p(act), n, two_f // 2, h, E,
                                                 _lib.stream()), "b200_gemm_grouped_swiglu")
@@ -168,7 +168,7 @@ def moe_mlp(n2: torch.Tensor, w_router: torch.Tensor, w_gu: torch.Tensor, w_d: t
     T, h = n2.shape
     _, top_e, top_w = route(n2, w_router, k, renorm)
     _, inverse, tok, counts = sorted_pairs(top_e, w_gu.shape[0])
-    _, _, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d)
+    _, _, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d, keep_gu=False)
     if shared is None:
         out = combine(y, inverse, top_w, None)
         if out is not None:
@@ -309,7 +309,8 @@ class MoEBlockFn(torch.autograd.Function):
         order, inverse, tok, counts = sorted_pairs(top_e, w_gu.shape[0])
         ctx.device_counts = counts
         ctx.counts = counts.tolist() if any(ctx.needs_input_grad) else None      # only the backward pass reads them
-        gu, act, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d, ctx.counts)
+        gu, act, y = experts_forward(n2.index_select(0, tok), counts, w_gu, w_d, ctx.counts,
+                                     any(ctx.needs_input_grad) and not recompute)
         shared_saved = ()
         h2 = combine(y, inverse, top_w, h1, rmul) if w_sgu is None else None
         if h2 is None:

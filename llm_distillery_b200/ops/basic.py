@@ -420,20 +420,23 @@ def swiglu_fusable(x: torch.Tensor, w_gu: torch.Tensor) -> bool:
 
 
 def linear_swiglu_fwd(x: torch.Tensor, w_gu: torch.Tensor, out_gu: torch.Tensor | None = None,
-                      out_act: torch.Tensor | None = None, split_k: bool = False) -> tuple[torch.Tensor, torch.Tensor]:
+                      out_act: torch.Tensor | None = None, split_k: bool = False,
+                      keep_gu: bool = True) -> tuple[torch.Tensor | None, torch.Tensor]:
     """(gu, act) with gu[T, 2f] = x w_gu^T (gate rows first, then up rows) and act[T, f] = silu(gate) * up. On the GPU
     one launch does both when the shape allows (bf16, f a multiple of 128): the SwiGLU sits in the
     epilogue of the gate / up GEMM. Same values as ``linear_fwd`` followed by ``swiglu_fwd``.
-    ``out_gu`` / ``out_act`` (row slices of larger buffers are fine) receive the results when given."""
+    ``out_gu`` / ``out_act`` (row slices of larger buffers are fine) receive the results when given. Without ``keep_gu``
+    the one launch does not write gu (None instead)."""
     T = x.shape[0]
     f = w_gu.shape[0] // 2
     _same_reduction("linear_swiglu_fwd", x.shape[1], w_gu.shape[1])
     if swiglu_fusable(x, w_gu):
-        gu, act = _target(out_gu, T, 2 * f, x.device), _target(out_act, T, f, x.device)
+        gu = _target(out_gu, T, 2 * f, x.device) if keep_gu else None
+        act = _target(out_act, T, f, x.device)
         _lib.check(_lib.kernels().b200_gemm_swiglu(_lib.ptr(x), _lib.ptr(w_gu), _lib.ptr(gu), _lib.ptr(act), T, f,
-                                                   x.shape[1], x.stride(0), w_gu.stride(0), gu.stride(0), act.stride(0),
-                                                   int(split_k), _lib.stream()), "b200_gemm_swiglu")
-        return _deliver(gu, out_gu), _deliver(act, out_act)
+                                                   x.shape[1], x.stride(0), w_gu.stride(0), gu.stride(0) if keep_gu else 0,
+                                                   act.stride(0), int(split_k), _lib.stream()), "b200_gemm_swiglu")
+        return _deliver(gu, out_gu) if keep_gu else None, _deliver(act, out_act)
     gu = gemm(x, w_gu, out=out_gu, split_k=split_k)
     return gu, _deliver(swiglu_fwd(gu), out_act)
 

@@ -335,3 +335,16 @@ def test_fused_epilogues_copy_to_outputs_they_cannot_store_to(T, form):
     dgu = basic.linear_dgrad_swiglu_bwd(x, wd, gu)
     assert basic.linear_dgrad_swiglu_bwd(x, wd, gu, out=od) is od and torch.equal(od, dgu.to(od.dtype))
     assert _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("T,f,K,split", [(93, 1408, 512, True), (93, 1408, 512, False), (777, 384, 896, False),
+                                         (5003, 1408, 520, False), (4737, 1152, 264, True)])
+def test_swiglu_epilogue_without_the_gate_and_up_values(T, f, K, split):
+    """Few-tile and pair kernels: the same activation, nothing written behind it."""
+    g = torch.Generator("cuda").manual_seed(T)
+    x, w = torch.randn(T, K, device=DEV, generator=g).bfloat16(), (torch.randn(2 * f, K, device=DEV, generator=g) * 0.05).bfloat16()
+    gu, act = basic.linear_swiglu_fwd(x, w, split_k=split)
+    buf = torch.full((T + 1, f), 7.0, device=DEV, dtype=torch.bfloat16)
+    none, alone = basic.linear_swiglu_fwd(x, w, out_act=buf[:T], split_k=split, keep_gu=False)
+    assert none is None and gu.shape == (T, 2 * f) and torch.equal(act, alone) and alone.data_ptr() == buf.data_ptr()
+    assert (buf[T] == 7).all() and _lib.take_device_error() == 0
