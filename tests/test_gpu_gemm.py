@@ -348,3 +348,19 @@ def test_swiglu_epilogue_without_the_gate_and_up_values(T, f, K, split):
     none, alone = basic.linear_swiglu_fwd(x, w, out_act=buf[:T], split_k=split, keep_gu=False)
     assert none is None and gu.shape == (T, 2 * f) and torch.equal(act, alone) and alone.data_ptr() == buf.data_ptr()
     assert (buf[T] == 7).all() and _lib.take_device_error() == 0
+
+
+@pytest.mark.parametrize("T", [450, 777])
+def test_few_tile_kernel_beyond_the_resident_grid(T):
+    """Several waves of small tiles where the large ones would just miss whole rounds: the bits of the large tiles, which a call
+    with more rows of output takes."""
+    g = torch.Generator("cuda").manual_seed(T)
+    x, w = torch.randn(8192, 896, device=DEV, generator=g).bfloat16(), (torch.randn(2 * 4864, 896, device=DEV, generator=g) * 0.1).bfloat16()
+    for few, many in zip(basic.linear_swiglu_fwd(x[:T], w), basic.linear_swiglu_fwd(x, w)):
+        assert torch.equal(few, many[:T])
+    dy = torch.randn(T, 4 * 9728, device=DEV, generator=g).bfloat16()
+    few, many = (basic.gemm(d, x[:T], a_mn=True, b_mn=True, out_dtype=torch.float32) for d in (dy[:, :9728].contiguous(), dy))
+    assert torch.equal(few, many[:9728])
+    both = basic.gemm(dy[:, :9728].contiguous(), x[:T], a_mn=True, b_mn=True, out=few.clone(), accumulate=True)
+    assert torch.equal(both, basic.gemm(dy, x[:T], a_mn=True, b_mn=True, out=many.clone(), accumulate=True)[:9728])
+    assert _lib.take_device_error() == 0
